@@ -71,6 +71,7 @@ struct DevIndex {
     const uint64_t* valSig[2];
     const uint64_t* sufSig[2];
     int32_t nHub;
+    int32_t hubMinLen;   // edges of the shortest hub row (INT_MAX without any)
     uint32_t hashMask;
     int32_t nPred;
     int32_t nEnt;

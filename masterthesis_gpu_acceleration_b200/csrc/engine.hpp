@@ -390,6 +390,10 @@ struct Context {
         dix.sufSig[0] = reinterpret_cast<const uint64_t*>(base + off[k++]);
         dix.sufSig[1] = reinterpret_cast<const uint64_t*>(base + off[k++]);
         dix.nHub = (int32_t)h.hubOff.size();
+        dix.hubMinLen = INT_MAX;
+        for (int d = 0; d < 2; ++d)
+            for (size_t r = 0; r < h.hubOf[d].size(); ++r)
+                if (h.hubOf[d][r] >= 0) dix.hubMinLen = std::min(dix.hubMinLen, h.rowBeg[d][r + 1] - h.rowBeg[d][r]);
         dix.hashMask = h.hashMask;
         dix.nPred = h.nPred;
         dix.nEnt = h.nEnt;
