@@ -63,12 +63,12 @@ struct BlockState {
     int stop;                       // the block's deadline passed: abandon the task
     unsigned long long deadline;    // global-timer ns (0: none)
     int curItem[kMaxBody + 1];      // a level's position, saved when the search descends below it
-    long long curOff[kMaxBody + 1];
+    int curOff[kMaxBody + 1];
     int count[kMaxBody + 1];
     int firstFail;                  // first candidate of a wide round that found the next level full
     unsigned safeLevels;            // bit l: level l takes capacity-sized rounds until exhausted
     int levelOff[kMaxBody + 1];
-    long long warpSum[kWarps];
+    int warpSum[kWarps];
     unsigned long long red[kWarps];
     int exRank[kWarps][kMaxVars];   // per warp: hO-domain ranks of the bound values of a hub item
 };
@@ -78,8 +78,8 @@ struct Smem {
     DevPlan plan;
     BlockState<B> st;
     int wBeg[B];
-    long long wLen[B];
-    long long wLoc[B];   // inclusive prefix of wLen within the item's warp
+    int wLen[B];
+    int wLoc[B];   // inclusive prefix of wLen within the item's warp
     int pool[Geom::pool_for(B)];   // frontier levels, then the dedup bitmap at plan.bitmapOff
 };
 
@@ -158,11 +158,11 @@ struct Smem;
 // totals of the warps before i's warp plus wLoc[i] (WinCursor reads it
 // that way).  The barrier also ORs `flag` over the block.
 template <int B>
-__device__ __forceinline__ bool publish_window(long long x, bool flag, Smem<B>& sm) {
+__device__ __forceinline__ bool publish_window(int x, bool flag, Smem<B>& sm) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
-        const long long y = __shfl_up_sync(0xffffffffu, x, d);
+        const int y = __shfl_up_sync(0xffffffffu, x, d);
         if (lane >= d) x += y;
     }
     sm.wLoc[threadIdx.x] = x;
@@ -174,15 +174,15 @@ __device__ __forceinline__ bool publish_window(long long x, bool flag, Smem<B>& 
 // (Up to 256 threads the eight totals are added directly; the two forms
 // differ only in the registers the kernel needs around them.)
 template <int B>
-__device__ __forceinline__ long long window_total(const Smem<B>& sm) {
+__device__ __forceinline__ int window_total(const Smem<B>& sm) {
     if constexpr (B <= 256) {
-        long long v = 0;
+        int v = 0;
 #pragma unroll
         for (int w = 0; w < B / 32; ++w) v += sm.st.warpSum[w];
         return v;
     } else {
         const int lane = threadIdx.x & 31;
-        long long v = lane < B / 32 ? sm.st.warpSum[lane] : 0;
+        int v = lane < B / 32 ? sm.st.warpSum[lane] : 0;
 #pragma unroll
         for (int d = 16; d; d >>= 1) v += __shfl_xor_sync(0xffffffffu, v, d);
         return v;
@@ -196,10 +196,10 @@ __device__ __forceinline__ long long window_total(const Smem<B>& sm) {
 template <int B>
 struct WinCursor {
     int item = 0, warp = 0;
-    long long base = 0;   // candidates of the warps before `warp`
-    __device__ __forceinline__ void seek(const Smem<B>& sm, int nw, long long j) {
+    int base = 0;   // candidates of the warps before `warp`
+    __device__ __forceinline__ void seek(const Smem<B>& sm, int nw, int j) {
         if (base + sm.wLoc[item] > j) return;
-        long long end = base + sm.st.warpSum[warp];
+        int end = base + sm.st.warpSum[warp];
         while (end <= j) {
             base = end;
             ++warp;
@@ -213,7 +213,7 @@ struct WinCursor {
         item = lo;
     }
     // index of the item's first candidate
-    __device__ __forceinline__ long long first(const Smem<B>& sm) const { return base + sm.wLoc[item] - sm.wLen[item]; }
+    __device__ __forceinline__ int first(const Smem<B>& sm) const { return base + sm.wLoc[item] - sm.wLen[item]; }
 };
 
 template <int B>
@@ -624,6 +624,11 @@ __device__ __forceinline__ void run_task(Smem<B>& sm, const DevIndex& ix, const 
     // (most candidates die on it): more than the next level's capacity, so
     // a round may find that level full (see `wide` below)
     constexpr int kWideChunk = 8 * B;
+    // A window takes at most this many candidates of one item, so that its
+    // prefix sums fit 32 bits; no round consumes as many, so a longer item
+    // always has candidates left for the next window.
+    constexpr int kMaxSeg = 1 << 21;
+    static_assert(kLeafChunk < kMaxSeg && (long long)B * kMaxSeg <= 1 << 30, "window sums fit an int");
     // candidates per thread per group (1, 2 and 4 measured on c3: 44.96,
     // 45.22 and 46.92 ms per launch; 8 makes compilation impractical)
     constexpr int kU = 1;
@@ -763,8 +768,7 @@ __device__ __forceinline__ void run_task(Smem<B>& sm, const DevIndex& ix, const 
         // publishes the window's prefix sums, one closes the round.  Reads
         // of the shared counters that a later step may reset can only see
         // the reset when the decision they feed is the same either way.
-        int k = 0, w0 = 0;
-        long long off = 0;
+        int k = 0, w0 = 0, off = 0;
         for (;;) {
             const int cnt = min(S.count[k], P.cap);
             if (w0 >= cnt) {
@@ -802,7 +806,7 @@ __device__ __forceinline__ void run_task(Smem<B>& sm, const DevIndex& ix, const 
 
             // window: the stored neighbour segment of each item
             int myBeg = 0;
-            long long myLen = 0;
+            int myLen = 0;
             if (tid < nw) {
                 int* it = items + S.levelOff[k] + (w0 + tid) * strideK;
                 bool pruned = false;
@@ -829,7 +833,7 @@ __device__ __forceinline__ void run_task(Smem<B>& sm, const DevIndex& ix, const 
                         if (code == kItemNew && myLen > 0) {
                             code = kItemEnum;
                             if (myLen >= ix.hubMinLen && !(tid == 0 && off != 0)) {
-                                const int c = classify_item(P, ix, stp, it, lenK, pathKind, myBeg, (int)myLen, fb,
+                                const int c = classify_item(P, ix, stp, it, lenK, pathKind, myBeg, myLen, fb,
                                                             heavy, mt);
                                 if (c == -4) myNew += 1;   // a new found bit of a split root
                                 if (c != -1) code = c >= 0 ? kItemHub + c : kItemDone;
@@ -845,16 +849,17 @@ __device__ __forceinline__ void run_task(Smem<B>& sm, const DevIndex& ix, const 
                         }
                     }
                     if (tid == 0 && !isHub) {
-                        myBeg += (int)off;
+                        myBeg += off;
                         myLen = myLen > off ? myLen - off : 0;
                     }
+                    myLen = min(myLen, kMaxSeg);
                 }
             }
             sm.wBeg[tid] = myBeg;
             sm.wLen[tid] = myLen;
             if (tid == 0 && !leaf) S.count[k + 1] = 0;
             const bool anyHub = publish_window<B>(myLen, isHub, sm) && (hubPath || memoPath);
-            const long long total = window_total<B>(sm);
+            const int total = window_total<B>(sm);
             // When the next step expands from the value this step binds,
             // that value's row signature (stored beside it) drops most
             // candidates whose next row is absent before any lookup.
@@ -871,7 +876,7 @@ __device__ __forceinline__ void run_task(Smem<B>& sm, const DevIndex& ix, const 
             // capacity-sized rounds: its key count must not depend on how
             // the threads raced (a launch is staged again with that count).
             const bool wide = sigTest && !sortMode && !((S.safeLevels >> k) & 1u);
-            const long long take = min(total, (long long)(leaf ? kLeafChunk : (wide ? kWideChunk : P.cap)));
+            const int take = min(total, leaf ? kLeafChunk : (wide ? kWideChunk : P.cap));
             const int lenN = leaf ? 0 : P.tupleLen[k + 1];
             const int strideN = lenN + 2;
             int* baseN = leaf ? nullptr : items + S.levelOff[k + 1];
@@ -959,18 +964,18 @@ __device__ __forceinline__ void run_task(Smem<B>& sm, const DevIndex& ix, const 
             const int sigBit = sig_bit(P.steps[k + 1 < P.m ? k + 1 : k].pred, P.steps[k + 1 < P.m ? k + 1 : k].dir);
             const uint32_t* sigWords = reinterpret_cast<const uint32_t*>(ix.valSig[stp.dir]) + (sigBit >> 5);
             WinCursor<B> cur;
-            for (long long jb = tid; jb < take; jb += (long long)B * kU) {
+            for (int jb = tid; jb < take; jb += B * kU) {
                 int lo_[kU], e_[kU], n0_[kU], n1_[kU], rk_[kU];
                 uint32_t sw_[kU];
 #pragma unroll
                 for (int u = 0; u < kU; ++u) {
-                    const long long j = jb + (long long)u * B;
+                    const int j = jb + u * B;
                     lo_[u] = -1;
                     e_[u] = 0;
                     if (j < take) {
                         cur.seek(sm, nw, j);
                         lo_[u] = cur.item;
-                        e_[u] = sm.wBeg[cur.item] + (int)(j - cur.first(sm));
+                        e_[u] = sm.wBeg[cur.item] + (j - cur.first(sm));
                     }
                 }
 #pragma unroll
@@ -986,14 +991,14 @@ __device__ __forceinline__ void run_task(Smem<B>& sm, const DevIndex& ix, const 
 #pragma unroll
                 for (int u = 0; u < kU; ++u)
                     if (lo_[u] >= 0 && ((sw_[u] >> (sigBit & 31)) & 1u))
-                        eval(lo_[u], e_[u], n0_[u], n1_[u], rk_[u], (int)(jb + (long long)u * B));
+                        eval(lo_[u], e_[u], n0_[u], n1_[u], rk_[u], jb + u * B);
             }
             // where the next round at this level starts: the item holding
             // candidate `take` (items before it are consumed), and how much
             // of it is (computed here, not before the candidates, so that it
             // holds no registers across them)
             int cut = nw;
-            long long cutOff = 0;
+            int cutOff = 0;
             {
                 if (take < window_total<B>(sm)) {
                     WinCursor<B> c;
