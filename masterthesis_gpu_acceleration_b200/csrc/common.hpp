@@ -149,12 +149,14 @@ struct DevPlan {
                                   // kExist plans ending in x -> y and the check (h, y) (memo_exists)
     int32_t memoP2, memoD2;       // the memo's second relation: y -> h through (memoP2, memoD2) rows
     TermRef memoH;                // kExist: tuple ref of h
-    int8_t memoSteps;             // kPairs: 3 for a three-step suffix memo x -> v2 -> v3 -> hO (memo3_item),
-                                  // otherwise the two-step one
+    int8_t memoSteps;             // kPairs: 3 when items of level 1 may also use a three-step suffix memo
+                                  // x -> v2 -> v3 -> hO (memo3Tab), else 0
     int8_t pad2;
     int32_t memoWords;            // words per memo bitmap (the rows of (memoP2, 1 - memoD2))
     const int32_t* memoTab;       // per hub row: memo slot or -1 (null: no memo)
     const uint32_t* memoBits;     // per slot: S1 then S2, memoWords words each
+    const int32_t* memo3Tab;      // the same for the three-step memo: per slot S1, then one path count per rank
+    const uint32_t* memo3Bits;
     // kPairs deduplication outside the shared pool (per launch; see DedupMode):
     int64_t gBlockWords;          // > 0: block rows, each block owns gBitmap + blockIdx.x * gBlockWords
                                   // words for its current task's rows (cleared at task start)
@@ -168,28 +170,35 @@ struct DevPlan {
     // for j < supN, results[supSlot[j]] gains the number of head triples
     // (hS, supPred[j], b), b != hS, whose pair (hS, b) the plan's rows hold;
     // b's rank is that of its row in (supDomPred, supDomDir), hO's domain.
-    int32_t supN;
+    // supDir 1: the plan's roots are the head's objects (the pairs counted
+    // from hO's end), so the head triples are looked up by object.
+    int32_t supN, supDir;
     int32_t supDomPred, supDomDir;
     int32_t supPred[kMaxSupFused];
     int32_t supSlot[kMaxSupFused];
-    int32_t pad4;
-    // Hub items of the leaf (see kHubSeen): per resident block kHubSeen
-    // claim entries at hubSeen + blockIdx.x * kHubSeen (null: every hub item
-    // is OR-ed).  Set for plans whose leaf items are (hS, u, w) expanding
-    // from u or w with nothing to test but injectivity.
+    // Hub items of the leaf or memo items of the level above it (see
+    // kHubSeen): per resident block kHubSeen claim entries at hubSeen +
+    // blockIdx.x * kHubSeen (null: no item is skipped).  Set for plans whose
+    // items of level claimLevel are (hS, u, w) expanding from u or w with
+    // nothing to test but injectivity from there on.
+    int32_t claimLevel, pad4;
     unsigned long long* hubSeen;
 };
 
-// Leaf hub items of one root and one hub row differ only in the one bound
-// value that is neither the root nor the row key (the middle value), and
-// each excludes only its own bound values from the row: two items with
-// different middle values already cover every value any further one would
-// add.  A task claims its (root, hub) pairs in a direct-mapped table of
-// kHubSeen 64-bit entries [root 10 bits | hub 20 | state 2 | first middle
-// value 32] (state 1: one middle value seen, 2: two) and skips the items
-// that come after two different middle values.  The same item may come
-// twice (a wide round makes some items again); it never counts as a second
-// value, and a displaced entry only costs repeats.
+// Hub items of the leaf and memo items of the level above it, of one root
+// and one hub row, differ only in the one bound value that is neither the
+// root nor the row key (the middle value).  Each keeps its bound values out
+// of the q values still to be bound (q = 1 for the leaf, 2 for a memo item).
+// A choice of those q that some middle value allows meets at most q of q + 1
+// different middle values, so q + 1 items cover every pair that any further
+// one would add.  A task claims its (root, hub or memo slot) pairs in a
+// direct-mapped table of kHubSeen 64-bit entries [root 10 bits | hub 20 |
+// state 2 | 16-bit hashes of the second and first middle value] (state: the
+// different middle values seen) and skips the items after q + 1 of them.
+// The same item may come twice (a wide round makes some items again), and
+// values with one hash look alike: neither counts as another value, and
+// neither is skipped before q + 1 are seen.  A displaced entry only costs
+// repeats.
 constexpr int kHubSeenBits = 8;
 constexpr int kHubSeen = 1 << kHubSeenBits;
 

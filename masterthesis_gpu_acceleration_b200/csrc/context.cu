@@ -44,14 +44,21 @@ double host_ms() {
     return std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now().time_since_epoch()).count();
 }
 
-// Plans whose leaf hub items may skip repeats (see kHubSeen): the leaf
-// tuple holds hS and two more values, the leaf step expands from one of
-// those two, binds hO and tests nothing but injectivity.
-bool hub_leaf_claims(const DevPlan& P) {
-    if (P.mode != kPairs || P.m < 1) return false;
-    const DevStep& st = P.steps[P.m - 1];
-    return P.tupleLen[P.m - 1] == kTupleHead + 3 && st.kind == kExpand && st.nNew == 1 && st.hoWhich != 0 &&
-           (st.keyRef == kTupleHead + 1 || st.keyRef == kTupleHead + 2) && P.chkN[P.m] == 0 && P.usedN[P.m] == 0;
+// The level whose hub or memo items may skip repeats (see kHubSeen), or -1:
+// its tuple holds hS and two more values, its step expands from one of those
+// two, and it is the leaf (binding hO, testing nothing but injectivity) or
+// the level of the two-step memo.
+int claim_level(const DevPlan& P) {
+    if (P.mode != kPairs) return -1;
+    auto shaped = [&](int k) {
+        const DevStep& st = P.steps[k];
+        return P.tupleLen[k] == kTupleHead + 3 && st.kind == kExpand && st.nNew == 1 &&
+               (st.keyRef == kTupleHead + 1 || st.keyRef == kTupleHead + 2);
+    };
+    const int k = P.m - 1;
+    if (k >= 0 && shaped(k) && P.steps[k].hoWhich != 0 && P.chkN[P.m] == 0 && P.usedN[P.m] == 0) return k;
+    if (P.memoLevel > 0 && shaped(P.memoLevel - 1)) return P.memoLevel - 1;
+    return -1;
 }
 
 // Bits that hold the values 0 .. n - 1 (at least one).
@@ -192,18 +199,26 @@ void Staged::stage(Context& c, std::vector<DevPlan>& plans, const std::vector<co
     std::vector<std::array<int, 6>> memoKeys;
     auto memo_key_of = [](const DevPlan& P) -> std::array<int, 6> {
         const DevStep& a = P.steps[P.memoLevel - 1];
-        if (P.memoSteps == 3) {
-            const DevStep& c3 = P.steps[P.memoLevel + 1];
-            return {a.pred, a.dir, P.memoP2, P.memoD2, c3.pred, c3.dir};
-        }
         return {a.pred, a.dir, P.memoP2, P.memoD2, -1, 0};
     };
+    auto memo3_key_of = [](const DevPlan& P) -> std::array<int, 6> {
+        return {P.steps[1].pred, P.steps[1].dir, P.steps[2].pred, P.steps[2].dir, P.steps[3].pred, P.steps[3].dir};
+    };
     for (int i = 0; i < nPlans; ++i) {
-        if (plans[i].memoSteps == 3 && !c.memo3) {   // three-step memos switched off: enumerate
-            plans[i].memoLevel = 0;
-            plans[i].memoSteps = 0;
+        if (!c.memo3) plans[i].memoSteps = 0;   // three-step memos switched off
+        if (plans[i].memoLevel > 0) {
+            // the memo leaves x out of x's own neighbours, as injectivity
+            // does for a variable; a constant that is its own neighbour stays
+            // one, so such a plan enumerates
+            const DevStep& a = plans[i].steps[plans[i].memoLevel - 1];
+            if (a.keyRef < 0) {
+                const int32_t e = plans[i].consts[-1 - a.keyRef];
+                if (e >= 0 && c.hix.has_triple(a.pred, e, e)) plans[i].memoLevel = 0;
+            }
         }
-        if (plans[i].memoLevel > 0 && dedup[i] != kDedupSort) memoKeys.push_back(memo_key_of(plans[i]));
+        if (dedup[i] == kDedupSort) continue;
+        if (plans[i].memoLevel > 0) memoKeys.push_back(memo_key_of(plans[i]));
+        if (plans[i].memoSteps == 3) memoKeys.push_back(memo3_key_of(plans[i]));
     }
     if (!memoKeys.empty()) c.ensure_memos(memoKeys, s);
     hostSect[1] += host_ms() - tSect;
@@ -235,19 +250,26 @@ void Staged::stage(Context& c, std::vector<DevPlan>& plans, const std::vector<co
     std::vector<DevTask> tasks;
     std::vector<double> cost;
     bool anyClaims = false;
-    for (int i = 0; i < nPlans; ++i) anyClaims |= c.hubClaims && dedup[i] != kDedupSort && hub_leaf_claims(plans[i]);
+    for (int i = 0; i < nPlans; ++i) anyClaims |= c.hubClaims && dedup[i] != kDedupSort && claim_level(plans[i]) >= 0;
     if (anyClaims) dHubSeen.ensure((size_t)std::max(c.grid, 1) * kHubSeen * 8, as);
     for (int i = 0; i < nPlans; ++i) {
-        plans[i].memoTab = nullptr;
-        plans[i].memoBits = nullptr;
+        plans[i].memoTab = plans[i].memo3Tab = nullptr;
+        plans[i].memoBits = plans[i].memo3Bits = nullptr;
         if (plans[i].memoLevel > 0) {
             const std::array<int, 6> k = memo_key_of(plans[i]);
             const SuffixMemo* m = c.memo_for(k[0], k[1], k[2], k[3], k[4], k[5]);
-            if (m && (plans[i].mode != kPairs || m->words == plans[i].rowWords) &&
-                (plans[i].memoSteps != 3 || m->wo == plans[i].wo)) {
+            if (m && (plans[i].mode != kPairs || m->words == plans[i].rowWords)) {
                 plans[i].memoTab = m->tab;
                 plans[i].memoBits = m->bits;
                 plans[i].memoWords = m->words;
+            }
+        }
+        if (plans[i].memoSteps == 3) {
+            const std::array<int, 6> k = memo3_key_of(plans[i]);
+            const SuffixMemo* m = c.memo_for(k[0], k[1], k[2], k[3], k[4], k[5]);
+            if (m && m->words == plans[i].rowWords && m->wo == plans[i].wo) {
+                plans[i].memo3Tab = m->tab;
+                plans[i].memo3Bits = m->bits;
             }
         }
         plans[i].resultSlot = i;
@@ -257,7 +279,8 @@ void Staged::stage(Context& c, std::vector<DevPlan>& plans, const std::vector<co
         plans[i].gRowBase = (dm == kDedupRows || dm == kDedupSort) ? phases[i]->rootBeg : 0;
         plans[i].gBlockWords = dm == kDedupBlockRows ? (int64_t)blockWords : 0;
         plans[i].gHeavy = (pts[i].heavyRows && dm != kDedupSort) ? static_cast<uint32_t*>(dHeavy.p) + hOff[i] : nullptr;
-        plans[i].hubSeen = (anyClaims && dm != kDedupSort && hub_leaf_claims(plans[i]))
+        plans[i].claimLevel = claim_level(plans[i]);
+        plans[i].hubSeen = (anyClaims && dm != kDedupSort && plans[i].claimLevel >= 0)
                                ? static_cast<unsigned long long*>(dHubSeen.p) : nullptr;
         plans[i].pairKeys = nullptr;
         plans[i].keyCursor = nullptr;
@@ -272,8 +295,8 @@ void Staged::stage(Context& c, std::vector<DevPlan>& plans, const std::vector<co
             plans[i].keyCap = keyCap;
             plans[i].keyBase = (unsigned long long)k << sortSlotShift;
             plans[i].rankBits = rankBits;
-            plans[i].memoTab = nullptr;   // memos set bitmap words; keys carry every pair
-            plans[i].memoBits = nullptr;
+            plans[i].memoTab = plans[i].memo3Tab = nullptr;   // memos set bitmap words; keys carry every pair
+            plans[i].memoBits = plans[i].memo3Bits = nullptr;
         }
         tasks.insert(tasks.end(), pts[i].tasks.begin(), pts[i].tasks.end());
         cost.insert(cost.end(), pts[i].cost.begin(), pts[i].cost.end());
@@ -468,12 +491,8 @@ void Context::ensure_memos(const std::vector<std::array<int, 6>>& keys, cudaStre
         for (size_t j = 0; j < rows.size(); ++j) {
             tab[h.hubOf[d1][rows[j]]] = (int32_t)j;
             m->rowHasMemo[(size_t)(rows[j] - h.predRow[d1][p1])] = 1;
-            if (p3 < 0) {
-                all.push_back(MemoJob{p1, d1, p2, d2, rows[j], words, p3, d3, wo, 0, -1, 0, bits + j * stride});
-                continue;
-            }
-            // three steps: one block per slice of the row's values, so that
-            // the paths of a long row spread over the SMs
+            // one block per slice of the row's values, so that the paths of a
+            // long row spread over the SMs
             constexpr int32_t kSlice = 64;
             const int32_t len = h.rowBeg[d1][rows[j] + 1] - h.rowBeg[d1][rows[j]];
             for (int32_t b0 = 0; b0 < len; b0 += kSlice)
@@ -662,7 +681,7 @@ bool fusing(const Context& c) { return c.fuseSupport && (c.batchPhases & 3) == 3
 // issued back to back with one host synchronisation; a fused support takes
 // no launch of its own.
 int evaluate_parsed(Context& c, const Rule& rule, GpuRuleResult* out) {
-    RulePlan rp = plan_rule(rule, c.hix, c.geom);
+    RulePlan rp = plan_rule(rule, c.hix, c.geom, c.fans.get());
     int64_t sup = rp.support.value, body = rp.body.value;
     float supMs = 0.f, confMs = 0.f;
     const bool runS = rp.status == kRuleOk && rp.support.how == kDevice;
@@ -712,7 +731,7 @@ int evaluate_parsed(Context& c, const Rule& rule, GpuRuleResult* out) {
 // (hS, hO) pairs of different hS never collide.  Static parts count in
 // slice 0 only.
 void evaluate_shard(Context& c, const Rule& rule, int shard, int nShards, long long* counts) {
-    RulePlan rp = plan_rule(rule, c.hix, c.geom);
+    RulePlan rp = plan_rule(rule, c.hix, c.geom, c.fans.get());
     int64_t part[2] = {shard == 0 ? rp.support.value : 0, shard == 0 ? rp.body.value : 0};
     PhasePlan* phs[2] = {&rp.support, &rp.body};
     for (int k = 0; k < 2 && rp.status == kRuleOk; ++k) {
@@ -756,7 +775,7 @@ void prepare(Batch& b, Context& c, const char* const* rules, int n, int isJson, 
         if (!rules[i]) { b.parseStatus[i] = -1; return; }
         try {
             Rule r = isJson ? c.parser->parse_json(rules[i]) : c.parser->parse_text(rules[i]);
-            b.rps[i] = plan_rule(r, c.hix, c.geom);
+            b.rps[i] = plan_rule(r, c.hix, c.geom, c.fans.get());
             if (b.rps[i].status == kRuleOk) {
                 if (b.rps[i].support.how == kDevice) hash[2 * i] = phase_hash(b.rps[i].support);
                 if (b.rps[i].body.how == kDevice) hash[2 * i + 1] = phase_hash(b.rps[i].body);
@@ -939,6 +958,9 @@ void finish_load(Context* c) {
     // GPU_RULES_HOST_PROFILE=1: one stderr line of host-side times per one-shot batch
     if (const char* h = std::getenv("GPU_RULES_HOST_PROFILE")) c->hostProfile = std::atoi(h) != 0;
     c->tasks.reset(new TaskBuilder(c->hix));
+    // GPU_RULES_PLAN_BOTH_ENDS=0: body sizes always from the head subject's end
+    const char* ends = std::getenv("GPU_RULES_PLAN_BOTH_ENDS");
+    if (!ends || std::atoi(ends) != 0) c->fans.reset(new FanSamples(c->hix));
     c->tasks->memoRows = [c](int p1, int d1, int p2, int d2, int p3, int d3,
                              double* cost) -> const std::vector<uint8_t>* {
         auto it = c->memos.find(memo_key(p1, d1, p2, d2, p3, d3));
@@ -1480,7 +1502,7 @@ extern "C" int gpu_evaluate_rule_noalloc(void* ctx, const char* ruleText, GpuRul
         ck(cudaSetDevice(c.device), "cudaSetDevice");
         char* scratch = static_cast<char*>(noalloc_scratch(c.device));
         Rule r = c.parser->parse_text(ruleText);
-        RulePlan rp = plan_rule(r, c.hix, c.geom);
+        RulePlan rp = plan_rule(r, c.hix, c.geom, c.fans.get());
         int64_t sup = rp.support.value, body = rp.body.value;
         float supMs = 0.f, confMs = 0.f;
         if (rp.status == kRuleOk && rp.support.how == kDevice) sup = run_phase_noalloc(c, rp.support, scratch, &supMs);

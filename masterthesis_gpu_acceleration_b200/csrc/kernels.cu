@@ -342,17 +342,23 @@ __device__ __forceinline__ int memo3_exceptions(const DevPlan& P, const DevIndex
     n = __shfl_sync(0xffffffffu, n, 0);
     __syncwarp();
     if (lane < n) {
-        const uint32_t* C = P.memoBits + (long long)slot * ((long long)words + ((P.wo + 3) >> 2)) + words;
+        const uint32_t* C = P.memo3Bits + (long long)slot * ((long long)words + ((P.wo + 3) >> 2)) + words;
         if (memo3_keep(P, ix, par, lenK, ex[lane], kv, C, mt)) ex[lane] = -1;   // still reached: keep its bit
     }
     __syncwarp();
     return n + 1;
 }
 
+// The variable whose row a memo item expands (-1: a constant's row; plans
+// whose constant is its own neighbour get no memo).
+__device__ __forceinline__ int memo_row_value(const DevStep& stA, const int* it) {
+    return stA.keyRef >= kTupleHead ? it[stA.keyRef] : -1;
+}
+
 // One level-k item whose first suffix step expands a hub row x with a memo:
 // for the plan suffix x -[stA]-> y -[stB]-> hO, the memo holds, over hO's
-// rank domain, S1 = {h : at least one y in N1(x) with h in N2(y), h != y}
-// and S2 = {h : at least two such y}.  The item's valid hO are S1 minus the
+// rank domain, S1 = {h : at least one y in N1(x), y != x, with h in N2(y),
+// h != y} and S2 = {h : at least two such y}.  The item's valid hO are S1 minus the
 // ranks of its bound values (injectivity on hO) minus, when one bound value
 // y0 lies in N1(x) (injectivity on y), the h in N2(y0) that have no witness
 // but y0 (those outside S2).  Ranks within a row ascend with the values, so
@@ -367,7 +373,8 @@ __device__ __noinline__ unsigned long long memo_item(const DevPlan& P, const Dev
                                                      bool sharedDst, int nEx3) {
     unsigned long long myNew = 0;
     const bool three = nEx3 > 0;
-    const uint32_t* S1 = P.memoBits + (long long)slot * (three ? (long long)words + ((P.wo + 3) >> 2) : 2LL * words);
+    const uint32_t* S1 = three ? P.memo3Bits + (long long)slot * ((long long)words + ((P.wo + 3) >> 2))
+                               : P.memoBits + (long long)slot * (2LL * words);
     int nEx = lenK - kTupleHead;
     unsigned wmask = 0;
     if (three) {
@@ -380,7 +387,7 @@ __device__ __noinline__ unsigned long long memo_item(const DevPlan& P, const Dev
             const int u = par[kTupleHead + lane];
             const int2 r = row_lookup(ix, stB.pred, exDir, u, mt);
             ex[lane] = r.y > r.x ? __ldg(ix.srcRank[exDir] + r.x) : -1;
-            isW = seg_has(ix.val[stA.dir], segBeg, segLen, u, mt);
+            isW = u != memo_row_value(stA, par) && seg_has(ix.val[stA.dir], segBeg, segLen, u, mt);
         }
         wmask = __ballot_sync(0xffffffffu, isW);
         __syncwarp();
@@ -448,10 +455,11 @@ __device__ __noinline__ int memo_exists(const DevPlan& P, const DevIndex& ix, co
     const int2 hr = row_lookup(ix, P.memoP2, dDom, h, mt);
     if (hr.y <= hr.x) return 0;   // no y reaches h at all
     const int rank = __ldg(ix.srcRank[dDom] + hr.x);
+    const int x = memo_row_value(stA, it);
     int nRem = 0;
     for (int q = kTupleHead; q < lenK; ++q) {
         const int u = it[q];
-        if (u == h || !seg_has(ix.val[stA.dir], segBeg, segLen, u, mt)) continue;
+        if (u == h || u == x || !seg_has(ix.val[stA.dir], segBeg, segLen, u, mt)) continue;
         if (!has_edge(ix, P.memoP2, P.memoD2, u, h, mt)) continue;
         if (++nRem >= 2) return -1;
     }
@@ -485,7 +493,8 @@ __device__ __forceinline__ bool memo3_fits(const DevPlan& P, const DevIndex& ix,
 // segment is a memoised hub row with at most one bound value among its
 // neighbours (returns the memo slot); 3: a kExist leaf item decided by the
 // existence memo (returns -3, its found bit set; -4 when the bit is new and
-// the task counts on insertion).  -1: enumerate as usual.
+// the task counts on insertion); 4: as 2 for the three-step memo of level 1.
+// -1: enumerate as usual.
 template <bool kC>
 __device__ __noinline__ int classify_item(const DevPlan& P, const DevIndex& ix, const DevStep stp, const int* it,
                                           int lenK, int kind, int segBeg, int segLen, uint32_t* fb, bool heavy,
@@ -496,15 +505,17 @@ __device__ __noinline__ int classify_item(const DevPlan& P, const DevIndex& ix, 
     if (h < 0 || __ldg(ix.rowBeg[stp.dir] + row) != segBeg || __ldg(ix.rowBeg[stp.dir] + row + 1) - segBeg != segLen)
         return -1;
     if (kind == 1) return h;
-    const int slot = __ldg(P.memoTab + h);
+    const int slot = __ldg((kind == 4 ? P.memo3Tab : P.memoTab) + h);
     if (slot < 0) return -1;
+    if (kind == 4) return memo3_fits(P, ix, it[kTupleHead], mt) ? slot : -1;
     if (kind == 2) {
-        if (P.memoSteps == 3) return memo3_fits(P, ix, it[kTupleHead], mt) ? slot : -1;
         // bound values that are also first-step neighbours are witnesses the
-        // memo must not count; one is corrected exactly, more enumerate
+        // memo must not count (x itself never is one); one is corrected
+        // exactly, more enumerate
+        const int x = memo_row_value(stp, it);
         int nR = 0;
         for (int q = kTupleHead; q < lenK && nR < 2; ++q)
-            nR += seg_has(ix.val[stp.dir], segBeg, segLen, it[q], mt) ? 1 : 0;
+            nR += it[q] != x && seg_has(ix.val[stp.dir], segBeg, segLen, it[q], mt) ? 1 : 0;
         return nR <= 1 ? slot : -1;
     }
     const int res = memo_exists(P, ix, stp, it, lenK, segBeg, segLen, slot, mt);
@@ -541,23 +552,25 @@ __device__ __forceinline__ void emit_pair(const DevPlan& P, long long row, int r
     if (slot < P.keyCap) P.pairKeys[slot] = key;
 }
 
-// Claims a leaf hub item of (root, hub) with middle value `mid` in the
-// task's table (see kHubSeen); false when two other middle values are
-// claimed already.
-__device__ __forceinline__ bool hub_claim(unsigned long long* seen, int root, int hub, int mid) {
+// Claims a hub item of (root, hub) with middle value `mid` in the task's
+// table (see kHubSeen); false when `need` other middle values are claimed
+// already.
+__device__ __forceinline__ bool hub_claim(unsigned long long* seen, int root, int hub, int mid, unsigned need) {
     const unsigned long long key = ((unsigned long long)root << 20) | (unsigned long long)hub;   // 30 bits
     unsigned long long* w = seen + (((uint32_t)key * 0x9E3779B1u) >> (32 - kHubSeenBits));
-    const unsigned long long m = (uint32_t)mid;
+    const unsigned h = ((uint32_t)mid * 0x85EBCA6Bu) >> 16;
     unsigned long long old = __ldcg(w);
     for (int t = 0; t < 8; ++t) {
         unsigned long long want;
         const unsigned state = (unsigned)(old >> 32) & 3u;
         if ((old >> 34) == key && state != 0u) {
-            if (state >= 2u) return false;
-            if ((old & 0xffffffffull) == m) return true;   // the first value again
-            want = (old & ~(3ull << 32)) | (2ull << 32);
+            if (state >= need) return false;
+            const unsigned h1 = (unsigned)old & 0xffffu, h2 = (unsigned)(old >> 16) & 0xffffu;
+            if (h == h1 || (state == 2u && h == h2)) return true;   // a claimed value again (or its hash)
+            want = (old & ~(3ull << 32)) | ((unsigned long long)(state + 1u) << 32);
+            if (state == 1u) want |= (unsigned long long)h << 16;
         } else {
-            want = (key << 34) | (1ull << 32) | m;   // displaces another pair: it may repeat items, never lose one
+            want = (key << 34) | (1ull << 32) | h;   // displaces another pair: it may repeat items, never lose one
         }
         const unsigned long long prev = atomicCAS(w, old, want);
         if (prev == old) return true;
@@ -566,23 +579,24 @@ __device__ __forceinline__ bool hub_claim(unsigned long long* seen, int root, in
     return true;
 }
 
-// The claims of a round's leaf hub items [0, cut) (items at `items`,
+// The claims of a round's hub or memo items [0, cut) (items at `items`,
 // `stride` ints apart): items that add nothing get wBeg -1.  Out of line,
 // so that the caller's loop keeps its registers.
 __device__ __noinline__ void hub_claims(unsigned long long* seen, const int* items, int stride, int cut, int midAt,
-                                        int* wBeg, int nThreads) {
+                                        int* wBeg, int nThreads, unsigned need) {
     for (int i = threadIdx.x; i < cut; i += nThreads) {
         const int wb = wBeg[i];
         if (wb <= -2) {
             const int* it = items + i * stride;
-            if (!hub_claim(seen, it[0], -2 - wb, it[midAt])) wBeg[i] = -1;
+            if (!hub_claim(seen, it[0], -2 - wb, it[midAt], need)) wBeg[i] = -1;
         }
     }
 }
 
 // Fused support (plans with supN > 0): the head triples (hS, supPred[j],
 // b), b != hS, of rule j whose pair (hS, b) is set in the plan's row of
-// root i (rows at bm + i * rowWords for the roots rootBeg + i, i < G).
+// root i (rows at bm + i * rowWords for the roots rootBeg + i, i < G); with
+// supDir 1 the roots are the objects of the head triples.
 // Warps take the roots, lanes a root's head triples; returns this lane's
 // count.  Out of line and small: it runs once per task, after the search.
 // `part` of `nParts` takes every nParts-th group of 32 head triples.
@@ -595,10 +609,10 @@ __device__ __noinline__ unsigned long long fused_support(const DevPlan& P, const
     for (int i = warp; i < G; i += nWarps) {
         const int a = __ldg(ix.rowKey[P.rootDir] + rootBeg + i);
         mt.add(4);
-        const int2 hr = row_lookup(ix, hp, 0, a, mt);
+        const int2 hr = row_lookup(ix, hp, P.supDir, a, mt);
         const uint32_t* row = bm + (long long)i * P.rowWords;
         for (int e = hr.x + 32 * part + lane; e < hr.y; e += 32 * nParts) {
-            const int b = __ldg(ix.val[0] + e);
+            const int b = __ldg(ix.val[P.supDir] + e);
             mt.add(4);
             if (b == a) continue;
             const int2 br = row_lookup(ix, dp, dd, b, mt);
@@ -672,7 +686,7 @@ __device__ __forceinline__ void run_task(Smem<B>& sm, const DevIndex& ix, const 
         for (long long i = tid; i < n4; i += B) b4[i] = make_uint4(0u, 0u, 0u, 0u);
         if (tid == 0) mt.add(16 * (unsigned long long)n4);
     }
-    // leaf hub items: the task's claim table (roots and hubs must fit its fields)
+    // hub and memo items: the task's claim table (roots and slots must fit its fields)
     const bool claims = P.hubSeen && G <= 1024 && ix.nHub <= (1 << 20);
     if (claims)
         for (int i = tid; i < kHubSeen; i += B) P.hubSeen[(long long)blockIdx.x * kHubSeen + i] = 0ull;
@@ -798,10 +812,12 @@ __device__ __forceinline__ void run_task(Smem<B>& sm, const DevIndex& ix, const 
             // nothing but injectivity to test; an item whose first segment
             // is a hub row with a suffix memo is counted from the memo's
             // "one witness y" / "two witnesses y" bitmaps (see below).
+            // A four-step plan may also have the three-step memo, at level 1.
+            const bool memo3Path = !leaf && pairs && !sortMode && P.memo3Tab != nullptr && k == 1;
             const bool memoPath = !leaf && pairs && !sortMode && P.memoTab != nullptr && k + 1 == P.memoLevel;
             const bool existMemo = leaf && !pairs && P.memoTab != nullptr && k + 1 == P.memoLevel &&
                                    !(heavy && k == 0);
-            const int pathKind = hubPath ? 1 : (memoPath ? 2 : (existMemo ? 3 : 0));
+            const int pathKind = hubPath ? 1 : (memoPath ? 2 : (existMemo ? 3 : (memo3Path ? 4 : 0)));
             bool isHub = false;   // item marked for the hub or memo pass
 
             // window: the stored neighbour segment of each item
@@ -858,7 +874,7 @@ __device__ __forceinline__ void run_task(Smem<B>& sm, const DevIndex& ix, const 
             sm.wBeg[tid] = myBeg;
             sm.wLen[tid] = myLen;
             if (tid == 0 && !leaf) S.count[k + 1] = 0;
-            const bool anyHub = publish_window<B>(myLen, isHub, sm) && (hubPath || memoPath);
+            const bool anyHub = publish_window<B>(myLen, isHub, sm) && (hubPath || memoPath || memo3Path);
             const int total = window_total<B>(sm);
             // When the next step expands from the value this step binds,
             // that value's row signature (stored beside it) drops most
@@ -1007,10 +1023,11 @@ __device__ __forceinline__ void run_task(Smem<B>& sm, const DevIndex& ix, const 
                     cutOff = take - c.first(sm) + (c.item == 0 ? off : 0);
                 }
             }
-            if (anyHub && leaf && claims) {
-                // leaf hub items of a (root, hub) after two middle values add nothing
+            if (anyHub && claims && k == P.claimLevel) {
+                // items of a (root, hub row) after enough middle values add nothing
                 hub_claims(P.hubSeen + (long long)blockIdx.x * kHubSeen, baseK + w0 * strideK, strideK, cut,
-                           stp.keyRef == kTupleHead + 1 ? kTupleHead + 2 : kTupleHead + 1, sm.wBeg, B);
+                           stp.keyRef == kTupleHead + 1 ? kTupleHead + 2 : kTupleHead + 1, sm.wBeg, B,
+                           leaf ? 2u : 3u);
                 __syncthreads();
             }
             if (anyHub) {
@@ -1036,7 +1053,7 @@ __device__ __forceinline__ void run_task(Smem<B>& sm, const DevIndex& ix, const 
                         const int* par = baseK + (w0 + item) * strideK;
                         if (!leaf) {
                             const int slot = -2 - sm.wBeg[item];
-                            const int nEx3 = P.memoSteps == 3
+                            const int nEx3 = memo3Path
                                 ? memo3_exceptions(P, ix, par, lenK, slot, words, S.exRank[warp], lane, mt) : 0;
                             myNew += memo_item(P, ix, stp, P.steps[k + 1], par, lenK, slot,
                                                bm + (rowBase + par[0]) * (long long)words, words, S.exRank[warp],
@@ -1341,8 +1358,10 @@ __global__ void memo_build_kernel(DevIndex ix, const MemoJob* jobs, int nJobs) {
         }
         return;
     }
+    const int x = ix.rowKey[job.d1][job.row];
     for (int i = b + warp; i < e; i += nWarps) {
         const int y = __ldg(ix.val[job.d1] + i);
+        if (y == x) continue;   // x is bound wherever the memo is used: never a witness
         const int2 r = row_lookup(ix, job.p2, job.d2, y, mt);
         for (int j = r.x + lane; j < r.y; j += 32) {
             if (__ldg(ix.val[job.d2] + j) == y) continue;

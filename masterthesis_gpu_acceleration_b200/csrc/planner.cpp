@@ -4,7 +4,8 @@
 //  * support (474-552): head triples that match the head pattern injectively
 //    (9-34) and admit a body grounding; the head triple counts as used.
 //  * body size (563-631): distinct (hS, hO) over body groundings, with the
-//    keys of the smallest body atom containing hS as hS candidates; hS == hO,
+//    keys of the smallest body atom containing hS as hS candidates (or the
+//    same pairs from hO's end, whichever costs less); hS == hO,
 //    or hO absent from the body, counts candidates with a grounding.
 //  * injective bindings: a newly bound variable differs from every bound
 //    variable (SupportCounting.hpp:43-48); constants take no part.
@@ -28,6 +29,7 @@
 #include <algorithm>
 #include <cstring>
 #include <limits>
+#include <mutex>
 
 namespace gr {
 namespace {
@@ -261,9 +263,139 @@ bool finish_capacity(DevPlan& P, const Geom& geom) {
     return local;
 }
 
+// The body-size phase with head variable hS as the root and hO as the other
+// end (pairs: distinct (hS, hO) are counted, else hS values).  Returns false
+// for plans beyond the engine's limits; `B` stays static (count 0) when hS is
+// in no body atom or two atoms always collide.
+bool build_body(const Rule& rule, const HostIndex& ix, const Geom& geom, int32_t hS, int32_t hO, bool pairs,
+                PhasePlan& B) {
+    int seedPred = -1, seedDir = 0;
+    int64_t bestSize = std::numeric_limits<int32_t>::max();
+    for (const auto& a : rule.body) {
+        int64_t sz = ix.pred_size(a.pred);
+        if (a.s.isVar && a.s.id == hS && sz < bestSize) { seedPred = a.pred; seedDir = 0; bestSize = sz; }
+        if (a.o.isVar && a.o.id == hS && sz < bestSize) { seedPred = a.pred; seedDir = 1; bestSize = sz; }
+    }
+    if (seedPred < 0) return true;
+    DevPlan& P = B.plan;
+    std::memset(&P, 0, sizeof(P));
+    Builder b(ix, P);
+    P.mode = pairs ? kPairs : kExist;
+    P.rootKind = kRootRows;
+    P.rootDir = seedDir;
+    P.rootPred = seedPred;
+    b.bind(hS);
+    if (!build_steps(b, rule.body, nullptr, hO, pairs)) return true;
+    if (!b.ok) return false;
+    if (pairs) {
+        for (int l = 0; l < P.m; ++l) {
+            const DevStep& st = P.steps[l];
+            if (!st.hoWhich) continue;
+            P.hoLevel = l + 1;
+            if (st.kind == kExpand) P.wo = (int32_t)ix.pred_rows(st.pred, 1 - st.dir);
+            else P.wo = (int32_t)ix.pred_rows(st.pred, st.hoWhich == 1 ? 0 : 1);
+        }
+    }
+    const bool local = finish_capacity(P, geom);
+    // suffix memo eligibility: the last two steps expand x -> y -> hO
+    // (y bound by the first, keying the second) with no test at
+    // either level but injectivity
+    if (pairs && P.m >= 2) {
+        const int k = P.m - 2;
+        const DevStep& a = P.steps[k];
+        const DevStep& c = P.steps[k + 1];
+        if (a.kind == kExpand && a.nNew == 1 && a.hoWhich == 0 && c.kind == kExpand && c.nNew == 1 &&
+            c.hoWhich != 0 && c.keyRef == P.tupleLen[k] && P.chkN[k + 1] == 0 && P.usedN[k + 1] == 0 &&
+            P.chkN[k + 2] == 0 && P.usedN[k + 2] == 0) {
+            P.memoLevel = k + 1;
+            P.memoP2 = c.pred;
+            P.memoD2 = c.dir;
+        }
+    }
+    // three-step suffix memo: hS -> x, then x -> v2 -> v3 -> hO,
+    // each step keyed by the value the one before bound, and no
+    // test after x but injectivity; items (hS, x) whose x is a
+    // memoised hub row are answered by it, the others reach
+    // level 2, whose hub rows have the two-step memo
+    if (pairs && P.m == 4 && P.tupleLen[0] == kTupleHead + 1) {
+        bool ok = true;
+        for (int l = 0; l < 4 && ok; ++l) {
+            const DevStep& st = P.steps[l];
+            ok = st.kind == kExpand && st.nNew == 1 && st.keyRef == P.tupleLen[l] - 1 &&
+                 (st.hoWhich != 0) == (l == 3);
+        }
+        for (int l = 2; l <= 4 && ok; ++l) ok = P.chkN[l] == 0 && P.usedN[l] == 0;
+        if (ok) P.memoSteps = 3;
+    }
+    B.how = kDevice;
+    B.rootBeg = ix.predRow[seedDir][seedPred];
+    B.rootEnd = ix.predRow[seedDir][seedPred + 1];
+    B.needsGlobalBitmap = pairs && !local;
+    B.estCost = (double)(ix.predEdge[seedDir][seedPred + 1] - ix.predEdge[seedDir][seedPred]);
+    return true;
+}
+
+// Candidates a body-size plan is expected to visit, level by level: the mean
+// next row length of the values each step leads to (sampled), long rows
+// counted as kHubMinDegree where a hub row costs no more (the leaf, and the
+// levels with a suffix memo), plus the clearing of the roots' bitmap rows.
+double plan_cost(const PhasePlan& ph, FanSamples& fans) {
+    const DevPlan& P = ph.plan;
+    double w = std::max(1, ph.rootEnd - ph.rootBeg);
+    double cost = w * (2.0 + P.rowWords / 64.0);
+    for (int s = 0; s < P.m; ++s) {
+        const DevStep& st = P.steps[s];
+        const bool cap = s == P.m - 1 || (P.memoLevel > 0 && s == P.memoLevel - 1) || (P.memoSteps == 3 && s == 1);
+        FanSamples::Fan f;
+        int by = -1;   // the step that bound the key (-1: the root, or a constant)
+        if (st.kind == kExpand)
+            for (int q = 0; q < s; ++q)
+                if (st.keyRef >= P.tupleLen[q] && st.keyRef < P.tupleLen[q + 1]) by = q;
+        if (st.kind == kScan) f.all = f.capped = (float)fans.index().pred_size(st.pred);
+        else if (by >= 0 && P.steps[by].kind == kExpand) f = fans.edges(P.steps[by].pred, P.steps[by].dir, st.pred, st.dir);
+        else if (by < 0 && st.keyRef == kTupleHead) f = fans.rows(P.rootPred, P.rootDir, st.pred, st.dir);
+        else f.all = f.capped = (float)fans.index().avg_degree(st.pred, st.dir);
+        w *= cap ? f.capped : f.all;
+        cost += w * (s == P.m - 1 ? 1.0 : 2.0);
+    }
+    return cost;
+}
+
 }  // namespace
 
-RulePlan plan_rule(const Rule& rule, const HostIndex& ix, const Geom& geom) {
+FanSamples::FanSamples(const HostIndex& ix) : ix_(ix), shards_(new Shard[kShards]) {}
+
+FanSamples::Fan FanSamples::get(int32_t p0, int d0, int32_t p1, int d1, bool perEdge) {
+    const uint64_t key = ((uint64_t)(uint32_t)p0 << 35) | ((uint64_t)(uint32_t)p1 << 3) | (uint64_t)(d0 << 2) |
+                         (uint64_t)(d1 << 1) | (perEdge ? 1u : 0u);
+    Shard& sh = shards_[(key * 0x9E3779B97F4A7C15ull) >> 58];
+    {
+        std::shared_lock<std::shared_mutex> lk(sh.mu);
+        auto it = sh.map.find(key);
+        if (it != sh.map.end()) return it->second;
+    }
+    const int32_t beg = perEdge ? ix_.predEdge[d0][p0] : ix_.predRow[d0][p0];
+    const int32_t n = (perEdge ? ix_.predEdge[d0][p0 + 1] : ix_.predRow[d0][p0 + 1]) - beg;
+    const int32_t k = std::min(n, kSamples);
+    double all = 0, capped = 0;
+    for (int32_t i = 0; i < k; ++i) {
+        const int32_t at = beg + (int32_t)(((int64_t)2 * i + 1) * n / (2 * k));   // evenly spaced
+        const auto r = ix_.row_range(p1, d1, perEdge ? ix_.val[d0][at] : ix_.rowKey[d0][at]);
+        const double len = r.second - r.first;
+        all += len;
+        capped += std::min(len, (double)kHubMinDegree);
+    }
+    Fan f;
+    if (k > 0) {
+        f.all = (float)(all / k);
+        f.capped = (float)(capped / k);
+    }
+    std::unique_lock<std::shared_mutex> lk(sh.mu);
+    sh.map.emplace(key, f);
+    return f;
+}
+
+RulePlan plan_rule(const Rule& rule, const HostIndex& ix, const Geom& geom, FanSamples* fans) {
     RulePlan rp;
     const Atom& h = rule.head;
     int nb = (int)rule.body.size();
@@ -354,79 +486,26 @@ RulePlan plan_rule(const Rule& rule, const HostIndex& ix, const Geom& geom) {
     B.how = kStatic;
     B.value = 0;
     if (nb > 0 && h.s.isVar && h.o.isVar && !bodyUnknown && !bodyDup) {
-        int32_t hS = h.s.id, hO = h.o.id;
-        int seedPred = -1, seedDir = 0;
-        int64_t bestSize = std::numeric_limits<int32_t>::max();
-        for (const auto& a : rule.body) {
-            int64_t sz = ix.pred_size(a.pred);
-            if (a.s.isVar && a.s.id == hS && sz < bestSize) { seedPred = a.pred; seedDir = 0; bestSize = sz; }
-            if (a.o.isVar && a.o.id == hS && sz < bestSize) { seedPred = a.pred; seedDir = 1; bestSize = sz; }
-        }
+        const int32_t hS = h.s.id, hO = h.o.id;
         bool hoInBody = false;
         for (const auto& a : rule.body)
             hoInBody |= (a.s.isVar && a.s.id == hO) || (a.o.isVar && a.o.id == hO);
-        if (seedPred >= 0) {
-            DevPlan& P = B.plan;
-            std::memset(&P, 0, sizeof(P));
-            Builder b(ix, P);
-            bool pairs = hS != hO && hoInBody;
-            P.mode = pairs ? kPairs : kExist;
-            P.rootKind = kRootRows;
-            P.rootDir = seedDir;
-            P.rootPred = seedPred;
-            b.bind(hS);
-            if (build_steps(b, rule.body, nullptr, hO, pairs) && b.ok) {
-                if (pairs) {
-                    for (int l = 0; l < P.m; ++l) {
-                        const DevStep& st = P.steps[l];
-                        if (!st.hoWhich) continue;
-                        P.hoLevel = l + 1;
-                        if (st.kind == kExpand) P.wo = (int32_t)ix.pred_rows(st.pred, 1 - st.dir);
-                        else P.wo = (int32_t)ix.pred_rows(st.pred, st.hoWhich == 1 ? 0 : 1);
-                    }
-                }
-                const bool local = finish_capacity(P, geom);
-                // suffix memo eligibility: the last two steps expand x -> y -> hO
-                // (y bound by the first, keying the second) with no test at
-                // either level but injectivity
-                if (pairs && P.m >= 2) {
-                    const int k = P.m - 2;
-                    const DevStep& a = P.steps[k];
-                    const DevStep& c = P.steps[k + 1];
-                    if (a.kind == kExpand && a.nNew == 1 && a.hoWhich == 0 && c.kind == kExpand && c.nNew == 1 &&
-                        c.hoWhich != 0 && c.keyRef == P.tupleLen[k] && P.chkN[k + 1] == 0 && P.usedN[k + 1] == 0 &&
-                        P.chkN[k + 2] == 0 && P.usedN[k + 2] == 0) {
-                        P.memoLevel = k + 1;
-                        P.memoP2 = c.pred;
-                        P.memoD2 = c.dir;
-                    }
-                }
-                // three-step suffix memo: hS -> x, then x -> v2 -> v3 -> hO,
-                // each step keyed by the value the one before bound, and no
-                // test after x but injectivity; items (hS, x) whose x is a
-                // memoised hub row are answered by memo3_item (kernels.cu)
-                if (pairs && P.m == 4 && P.tupleLen[0] == kTupleHead + 1) {
-                    bool ok = true;
-                    for (int l = 0; l < 4 && ok; ++l) {
-                        const DevStep& st = P.steps[l];
-                        ok = st.kind == kExpand && st.nNew == 1 && st.keyRef == P.tupleLen[l] - 1 &&
-                             (st.hoWhich != 0) == (l == 3);
-                    }
-                    for (int l = 2; l <= 4 && ok; ++l) ok = P.chkN[l] == 0 && P.usedN[l] == 0;
-                    if (ok) {
-                        P.memoLevel = 2;
-                        P.memoP2 = P.steps[2].pred;
-                        P.memoD2 = P.steps[2].dir;
-                        P.memoSteps = 3;
-                    }
-                }
-                B.how = kDevice;
-                B.rootBeg = ix.predRow[seedDir][seedPred];
-                B.rootEnd = ix.predRow[seedDir][seedPred + 1];
-                B.needsGlobalBitmap = pairs && !local;
-                B.estCost = (double)(ix.predEdge[seedDir][seedPred + 1] - ix.predEdge[seedDir][seedPred]);
-            } else if (!b.ok) {
-                rp.status = kRuleUnsupported;
+        const bool pairs = hS != hO && hoInBody;
+        if (!build_body(rule, ix, geom, hS, hO, pairs, B)) rp.status = kRuleUnsupported;
+        // Distinct (hS, hO) pairs can be counted from either end: rows of hS
+        // values with bits for hO, or the reverse.  What a grounding order
+        // costs is the bindings of its inner levels, and a hub costs least
+        // where its row is the last expanded (OR-ed 32 values a word) or
+        // memoised, so the end with the lower estimate is taken (half or
+        // less, as the estimates are sampled).
+        // Plans whose rows do not fit the shared pool keep hS's end: their
+        // memory (and what a scratch limit refuses) depends on it.
+        if (fans && pairs && rp.status == kRuleOk && B.how == kDevice && B.plan.m >= 2 && !B.needsGlobalBitmap) {
+            PhasePlan R;
+            if (build_body(rule, ix, geom, hO, hS, true, R) && R.how == kDevice &&
+                !R.needsGlobalBitmap && plan_cost(R, *fans) < 0.5 * plan_cost(B, *fans)) {
+                R.plan.supDir = 1;
+                B = R;
             }
         }
     }

@@ -1,6 +1,9 @@
 // planner.hpp — rule -> device plans (support phase and body-size phase).
 #pragma once
 #include <cstdint>
+#include <memory>
+#include <shared_mutex>
+#include <unordered_map>
 #include <utility>
 #include <vector>
 
@@ -46,9 +49,37 @@ struct RulePlan {
 // pair (the step binding hO looks its value up there).
 std::pair<int32_t, int32_t> ho_domain(const DevPlan& P);
 
+// Mean row lengths of predicate transitions, estimated from a few evenly
+// spaced edges (or rows) of the first predicate and cached: what the planner
+// compares grounding orders by.  Safe to call from several threads.
+class FanSamples {
+public:
+    struct Fan {
+        float all = 0.f, capped = 0.f;   // rows above kHubMinDegree edges count as kHubMinDegree in `capped`
+    };
+    explicit FanSamples(const HostIndex& ix);
+    const HostIndex& index() const { return ix_; }
+    // row length under (p1, d1) of the value an edge of (p0, d0) leads to
+    Fan edges(int32_t p0, int d0, int32_t p1, int d1) { return get(p0, d0, p1, d1, true); }
+    // row length under (p1, d1) of a row key of (p0, d0)
+    Fan rows(int32_t p0, int d0, int32_t p1, int d1) { return get(p0, d0, p1, d1, false); }
+
+private:
+    static constexpr int kShards = 64;
+    static constexpr int32_t kSamples = 64;
+    struct Shard {
+        std::shared_mutex mu;
+        std::unordered_map<uint64_t, Fan> map;
+    };
+    const HostIndex& ix_;
+    std::unique_ptr<Shard[]> shards_;
+    Fan get(int32_t p0, int d0, int32_t p1, int d1, bool perEdge);
+};
+
 // Plans both phases.  Semantics follow CPU_01_nonparallel/SupportCounting.cpp:
 // support (474-552) with the head triple counted as used, body size
-// (563-631) with the seed atom's keys as headS candidates.
-RulePlan plan_rule(const Rule& rule, const HostIndex& ix, const Geom& geom);
+// (563-631) with the seed atom's keys as headS candidates, or from hO's end
+// where `fans` (optional) says that costs less.
+RulePlan plan_rule(const Rule& rule, const HostIndex& ix, const Geom& geom, FanSamples* fans = nullptr);
 
 }  // namespace gr

@@ -185,7 +185,7 @@ struct Server {
             Planned& q = qs[i];
             q.req = std::move(got[i]);
             try {
-                q.rp = plan_rule(c->parser->parse_text(q.req.text), c->hix, c->geom);
+                q.rp = plan_rule(c->parser->parse_text(q.req.text), c->hix, c->geom, c->fans.get());
             } catch (const std::exception&) {
                 q.status = -1;
             }

@@ -31,6 +31,8 @@ DevPlan plan_identity(const PhasePlan& ph) {
     p.rowWords = 0;
     p.memoTab = nullptr;
     p.memoBits = nullptr;
+    p.memo3Tab = nullptr;
+    p.memo3Bits = nullptr;
     p.memoWords = 0;
     p.gBlockWords = 0;
     p.pairKeys = nullptr;
