@@ -154,7 +154,7 @@ struct DevPlan {
     int8_t pad2;
     int32_t memoWords;            // words per memo bitmap (the rows of (memoP2, 1 - memoD2))
     const int32_t* memoTab;       // per hub row: memo slot or -1 (null: no memo)
-    const uint32_t* memoBits;     // per slot: S1 then S2, memoWords words each
+    const uint32_t* memoBits;     // per slot: S1, S2 and S3, memoWords words each
     const int32_t* memo3Tab;      // the same for the three-step memo: per slot S1, then one path count per rank
     const uint32_t* memo3Bits;
     // kPairs deduplication outside the shared pool (per launch; see DedupMode):
@@ -238,13 +238,12 @@ struct Geom {
     int poolInts() const { return pool_for(block); }
 };
 
-// Profiling outputs of the instrumented kernel variant (null members are
-// skipped): requested global-memory bytes, and per task its start and end
-// time (globaltimer ns).
+constexpr int kMemoMaps = 3;   // S1, S2, S3 of a two-step memo: at least one, two, three witnesses
+
 // One suffix memo to build for hub row `row` of (p1, d1), or the part that
 // starts from the row's values [b0, b1) (b1 < 0: all of them; the parts of
 // one memo add into the same bits).  Two steps (p3 < 0): through (p2, d2),
-// bitmaps S1 then S2 of `words` words at `bits`.  Three steps: through
+// kMemoMaps bitmaps of `words` words at `bits`.  Three steps: through
 // (p2, d2) then (p3, d3), the bitmap S1 (`words` words) then one path count
 // per rank of the domain (`wo` ranks), a byte each (four to a word) that
 // saturates at 255.
@@ -257,6 +256,9 @@ struct MemoJob {
 // per rank) when the domain has at most this many ranks.
 constexpr int kMemoSmemRanks = 16384;
 
+// Profiling outputs of the instrumented kernel variant (null members are
+// skipped): requested global-memory bytes, and per task its start and end
+// time (globaltimer ns).
 struct EngineProfile {
     unsigned long long* bytes = nullptr;
     unsigned long long* taskNs = nullptr;

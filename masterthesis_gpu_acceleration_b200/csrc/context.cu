@@ -449,10 +449,10 @@ void Context::ensure_memos(const std::vector<std::array<int, 6>>& keys, cudaStre
             if (cand >= need) rowsOf[i].push_back(r);
         }
     }, 1);
-    // per memo slot: S1 and S2 (two steps), or S1 and one count per rank
+    // per memo slot: kMemoMaps bitmaps (two steps), or S1 and one count per rank
     auto slot_words = [&](const std::array<int, 6>& k) -> size_t {
         const size_t words = (size_t)((domain(k) + 31) / 32);
-        return k[4] >= 0 ? words + (size_t)(domain(k) + 3) / 4 : 2 * words;
+        return k[4] >= 0 ? words + (size_t)(domain(k) + 3) / 4 : kMemoMaps * words;
     };
     // within the memory budget, in key order: one device allocation holding
     // every new memo's hub table, then every new memo's bits

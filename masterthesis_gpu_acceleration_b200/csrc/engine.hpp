@@ -254,7 +254,7 @@ struct Staged {
 };
 
 // Suffix memo of one predicate transition (p1, d1) -> (p2, d2): per hub row
-// of (p1, d1) worth it, the S1/S2 bitmaps over (p2, 1 - d2)'s rows (see
+// of (p1, d1) worth it, the S1, S2 and S3 bitmaps over (p2, 1 - d2)'s rows (see
 // memo_item in kernels.cu).  Built once per context, never moved.
 constexpr size_t kMemoBudgetBytes = size_t(1) << 30;   // all suffix memos of a context
 

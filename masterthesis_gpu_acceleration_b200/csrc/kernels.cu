@@ -358,14 +358,15 @@ __device__ __forceinline__ int memo_row_value(const DevStep& stA, const int* it)
 // One level-k item whose first suffix step expands a hub row x with a memo:
 // for the plan suffix x -[stA]-> y -[stB]-> hO, the memo holds, over hO's
 // rank domain, S1 = {h : at least one y in N1(x), y != x, with h in N2(y),
-// h != y} and S2 = {h : at least two such y}.  The item's valid hO are S1 minus the
-// ranks of its bound values (injectivity on hO) minus, when one bound value
-// y0 lies in N1(x) (injectivity on y), the h in N2(y0) that have no witness
-// but y0 (those outside S2).  Ranks within a row ascend with the values, so
-// each lane merges its own run of words with N2(y0)'s sorted ranks.  The
-// whole warp calls this; new pair bits are counted on insertion and
-// returned (per lane).  Steps come by value and counts go back as the
-// result, so that the caller's loop state never needs an address.
+// h != y} and S2, S3 = {h : at least two, three such y}.  The item's valid hO are S1 minus the
+// ranks of its bound values (injectivity on hO) minus the h left without a
+// witness when bound values are witnesses themselves (u in N1(x), injectivity
+// on y): with one such u, the h in N2(u) outside S2; with two, also the h in
+// both N2(u)s outside S3.  Ranks within a row ascend with the values, so each
+// lane merges its own run of words with the N2(u)s' sorted ranks.  The whole
+// warp calls this; new pair bits are counted on insertion and returned (per
+// lane).  Steps come by value and counts go back as the result, so that the
+// caller's loop state never needs an address.
 template <bool kC>
 __device__ __noinline__ unsigned long long memo_item(const DevPlan& P, const DevIndex& ix, const DevStep stA,
                                                      const DevStep stB, const int* par, int lenK, int slot,
@@ -374,7 +375,7 @@ __device__ __noinline__ unsigned long long memo_item(const DevPlan& P, const Dev
     unsigned long long myNew = 0;
     const bool three = nEx3 > 0;
     const uint32_t* S1 = three ? P.memo3Bits + (long long)slot * ((long long)words + ((P.wo + 3) >> 2))
-                               : P.memoBits + (long long)slot * (2LL * words);
+                               : P.memoBits + (long long)slot * ((long long)kMemoMaps * words);
     int nEx = lenK - kTupleHead;
     unsigned wmask = 0;
     if (three) {
@@ -392,44 +393,50 @@ __device__ __noinline__ unsigned long long memo_item(const DevPlan& P, const Dev
         wmask = __ballot_sync(0xffffffffu, isW);
         __syncwarp();
     }
-    int e0 = 0, e1 = 0;
-    if (wmask) {
-        const int2 r = row_lookup(ix, stB.pred, stB.dir, par[kTupleHead + __ffs(wmask) - 1], mt);
-        e0 = r.x;
-        e1 = r.y;
-    }
-    const uint32_t* S2 = S1 + words;
+    // the witnesses' rows (the second is empty for most items)
+    int e[2] = {0, 0}, e1[2] = {0, 0};
     const int* rk = ix.valRank[stB.dir];
     const int per = (words + 31) >> 5;
     const int wb = min(words, lane * per), we = min(words, wb + per);
-    int e = e0;
-    if (e1 > e0 && wb < we) {
-        int lo = e0, hi = e1;
-        const int key = wb << 5;
-        while (lo < hi) {
-            const int mid = (lo + hi) >> 1;
-            mt.add(4);
-            if (__ldg(rk + mid) < key) lo = mid + 1; else hi = mid;
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        if (!wmask) break;
+        const int2 r = row_lookup(ix, stB.pred, stB.dir, par[kTupleHead + __ffs(wmask) - 1], mt);
+        wmask &= wmask - 1;
+        e[k] = r.x;
+        e1[k] = r.y;
+        if (r.y > r.x && wb < we) {
+            int lo = r.x, hi = r.y;
+            const int key = wb << 5;
+            while (lo < hi) {
+                const int mid = (lo + hi) >> 1;
+                mt.add(4);
+                if (__ldg(rk + mid) < key) lo = mid + 1; else hi = mid;
+            }
+            e[k] = lo;
         }
-        e = lo;
     }
+    const uint32_t* S2 = S1 + words;
     for (int w = wb; w < we; ++w) {
         uint32_t m = __ldg(S1 + w);
         mt.add(4);
         for (int q = 0; q < nEx; ++q)
             if (ex[q] >= 0 && (ex[q] >> 5) == w) m &= ~(1u << (ex[q] & 31));
-        if (e < e1) {
-            const int lim = (w + 1) << 5;
-            uint32_t s2 = 0u;
-            bool s2Loaded = false;
-            while (e < e1) {
-                const int r = __ldg(rk + e);
+        uint32_t hit[2] = {0u, 0u};
+        const int lim = (w + 1) << 5;
+#pragma unroll
+        for (int k = 0; k < 2; ++k)
+            while (e[k] < e1[k]) {
+                const int r = __ldg(rk + e[k]);
                 if (r >= lim) break;
-                if (!s2Loaded) { s2 = __ldg(S2 + w); s2Loaded = true; mt.add(4); }
-                if (!((s2 >> (r & 31)) & 1u)) m &= ~(1u << (r & 31));
-                ++e;
+                hit[k] |= 1u << (r & 31);
+                ++e[k];
                 mt.add(4);
             }
+        if (hit[0] | hit[1]) {
+            m &= ~((hit[0] | hit[1]) & ~__ldg(S2 + w));
+            mt.add(4);
+            if (hit[0] & hit[1]) { m &= ~(hit[0] & hit[1] & ~__ldg(S2 + words + w)); mt.add(4); }
         }
         if (m) {
             const uint32_t old = atomicOr(dst + w, m);
@@ -444,8 +451,9 @@ __device__ __noinline__ unsigned long long memo_item(const DevPlan& P, const Dev
 // kExist counterpart of memo_item: the item's last step expands a hub row x
 // with a memo and its only remaining test is the check (h, y) for a bound
 // variable h.  A valid y exists iff h has a witness y in N1(x) other than
-// the bound values: with no bound value among h's witnesses that is the S1
-// bit of h, with one the S2 bit; with more the item is left to enumeration.
+// the bound values: with n bound values among h's witnesses that is the bit
+// of h in the n-th map after S1; beyond the last map the item is left to
+// enumeration.
 // Returns 1 (a grounding exists), 0 (none) or -1 (undecided).
 template <bool kC>
 __device__ __noinline__ int memo_exists(const DevPlan& P, const DevIndex& ix, const DevStep stA, const int* it,
@@ -461,9 +469,9 @@ __device__ __noinline__ int memo_exists(const DevPlan& P, const DevIndex& ix, co
         const int u = it[q];
         if (u == h || u == x || !seg_has(ix.val[stA.dir], segBeg, segLen, u, mt)) continue;
         if (!has_edge(ix, P.memoP2, P.memoD2, u, h, mt)) continue;
-        if (++nRem >= 2) return -1;
+        if (++nRem >= kMemoMaps) return -1;
     }
-    const uint32_t* S = P.memoBits + ((long long)slot * 2 + nRem) * P.memoWords;
+    const uint32_t* S = P.memoBits + ((long long)slot * kMemoMaps + nRem) * P.memoWords;
     mt.add(4);
     return (int)((__ldg(S + (rank >> 5)) >> (rank & 31)) & 1u);
 }
@@ -490,7 +498,7 @@ __device__ __forceinline__ bool memo3_fits(const DevPlan& P, const DevIndex& ix,
 // Items of a round that may skip enumeration, kept out of line so that the
 // main loop's registers stay free.  kind 1: a leaf item whose segment is a
 // whole hub row (returns the hub index); 2: an item at the memo level whose
-// segment is a memoised hub row with at most one bound value among its
+// segment is a memoised hub row with at most two bound values among its
 // neighbours (returns the memo slot); 3: a kExist leaf item decided by the
 // existence memo (returns -3, its found bit set; -4 when the bit is new and
 // the task counts on insertion); 4: as 2 for the three-step memo of level 1.
@@ -510,13 +518,13 @@ __device__ __noinline__ int classify_item(const DevPlan& P, const DevIndex& ix, 
     if (kind == 4) return memo3_fits(P, ix, it[kTupleHead], mt) ? slot : -1;
     if (kind == 2) {
         // bound values that are also first-step neighbours are witnesses the
-        // memo must not count (x itself never is one); one is corrected
-        // exactly, more enumerate
+        // memo must not count (x itself never is one); up to two are
+        // corrected exactly, more enumerate
         const int x = memo_row_value(stp, it);
         int nR = 0;
-        for (int q = kTupleHead; q < lenK && nR < 2; ++q)
+        for (int q = kTupleHead; q < lenK && nR < 3; ++q)
             nR += it[q] != x && seg_has(ix.val[stp.dir], segBeg, segLen, it[q], mt) ? 1 : 0;
-        return nR <= 1 ? slot : -1;
+        return nR <= 2 ? slot : -1;
     }
     const int res = memo_exists(P, ix, stp, it, lenK, segBeg, segLen, slot, mt);
     if (res < 0) return -1;
@@ -1260,8 +1268,8 @@ static void launch_b(const DevIndex& ix, const DevPlan* plans, const DevTask* ta
 
 // Suffix memos (see memo_item): one block per job (a hub row x of one
 // transition); warps take the y in N1(x), lanes the h in N2(y).  The first
-// witness of h sets its S1 bit, any later one its S2 bit (atomicOr returns
-// the old word).
+// witness of h sets its S1 bit, the second its S2 bit, later ones its S3 bit
+// (atomicOr returns the old word).
 // Adds one path ending at `rank` to a three-step memo's counts: a 32-bit
 // shared counter, or the saturating byte in global memory.
 __device__ __forceinline__ void memo3_count_path(uint32_t* smemCnt, uint32_t* cnt, uint32_t* S1, int rank) {
@@ -1369,7 +1377,7 @@ __global__ void memo_build_kernel(DevIndex ix, const MemoJob* jobs, int nJobs) {
             if (rank < 0 || rank >= (job.words << 5)) continue;
             const uint32_t bit = 1u << (rank & 31);
             const uint32_t old = atomicOr(S1 + (rank >> 5), bit);
-            if (old & bit) atomicOr(S2 + (rank >> 5), bit);
+            if ((old & bit) && (atomicOr(S2 + (rank >> 5), bit) & bit)) atomicOr(S2 + job.words + (rank >> 5), bit);
         }
     }
 }
