@@ -18,6 +18,7 @@ constexpr int kTupleHead = 2;                  // [root index, hO rank]
 constexpr int kMaxTuple = kTupleHead + kMaxVars;
 constexpr int kMaxChecks = 16;
 constexpr int kMaxUsed = 40;
+constexpr int kAnyValue = -1;     // bound value of a free variable with values to spare
 constexpr int kMaxSupFused = 4;   // rules whose support one body-size plan counts
 
 // One slot of the (predicate, direction, key) -> edge range table.
@@ -93,17 +94,18 @@ struct DevUsed {         // used-triple rule: reject when the two triples are eq
     TermRef sA, oA, sB, oB;
 };
 
-enum StepKind : int8_t { kExpand = 0, kScan = 1 };
+enum StepKind : int8_t { kExpand = 0, kScan = 1, kRowScan = 2 };
 
 struct DevStep {
     int32_t pred;
-    int8_t dir;          // EXPAND: direction of the lookup; SCAN: always 0
-    int8_t kind;
+    int8_t dir;          // EXPAND: direction of the lookup; SCAN: always 0; ROWSCAN: direction of the rows
+    int8_t kind;         // ROWSCAN binds the keys of the predicate's rows (no atom is grounded by it)
     int8_t sameVar;      // SCAN with one variable in both positions
     int8_t nNew;         // values appended to the tuple (1 or 2)
     TermRef keyRef;      // EXPAND: the bound key
     int8_t hoWhich;      // 0: hO not bound here; 1/2: hO is the first/second new value
-    int8_t pad;
+    int8_t free;         // EXPAND: the new value occurs nowhere else in the rule (see freeMin);
+                         // ROWSCAN: the plan's scan level
 };
 
 enum PlanMode : int32_t { kExist = 0, kPairs = 1 };
@@ -139,7 +141,12 @@ struct DevPlan {
     DevStep steps[kMaxBody];
     DevCheck checks[kMaxChecks];
     DevUsed used[kMaxUsed];
-    int32_t pad1;                 // explicit: plans are compared and hashed byte by byte
+    // A step with `free` set binds a variable that only has to differ from
+    // the rule's other variables.  A row of at least freeMin values (the
+    // rule's variables) always holds one that does, whatever the others are
+    // bound to: such a row counts as the one value kAnyValue, shorter rows
+    // are enumerated.
+    int32_t freeMin;
     uint32_t* gBitmap;            // kPairs with a global bitmap (null: shared memory)
     int64_t gRowBase;             // first root of the plan, for global bitmap rows
     uint32_t* gHeavy;             // global dedup rows of split heavy roots
@@ -157,6 +164,12 @@ struct DevPlan {
     const uint32_t* memoBits;     // per slot: S1, S2 and S3, memoWords words each
     const int32_t* memo3Tab;      // the same for the three-step memo: per slot S1, then one path count per rank
     const uint32_t* memo3Bits;
+    // kPairs plans ending in a ROWSCAN that binds hO and a free step keyed on
+    // it (scanLevel: the ROWSCAN's level + 1, 0: none): three maps as those
+    // of a memo slot, with the row's values in the place of the witnesses.
+    const uint32_t* scanBits;
+    int32_t scanLevel;
+    int32_t pad1;                 // explicit: plans are compared and hashed byte by byte
     // kPairs deduplication outside the shared pool (per launch; see DedupMode):
     int64_t gBlockWords;          // > 0: block rows, each block owns gBitmap + blockIdx.x * gBlockWords
                                   // words for its current task's rows (cleared at task start)
@@ -243,7 +256,8 @@ constexpr int kMemoMaps = 3;   // S1, S2, S3 of a two-step memo: at least one, t
 // One suffix memo to build for hub row `row` of (p1, d1), or the part that
 // starts from the row's values [b0, b1) (b1 < 0: all of them; the parts of
 // one memo add into the same bits).  Two steps (p3 < 0): through (p2, d2),
-// kMemoMaps bitmaps of `words` words at `bits`.  Three steps: through
+// kMemoMaps bitmaps of `words` words at `bits` (row < 0: the scan memo of
+// (p1, d1) instead, from the predicate's rows [b0, b1)).  Three steps: through
 // (p2, d2) then (p3, d3), the bitmap S1 (`words` words) then one path count
 // per rank of the domain (`wo` ranks), a byte each (four to a word) that
 // saturates at 255.

@@ -201,6 +201,11 @@ void Staged::stage(Context& c, std::vector<DevPlan>& plans, const std::vector<co
         const DevStep& a = P.steps[P.memoLevel - 1];
         return {a.pred, a.dir, P.memoP2, P.memoD2, -1, 0};
     };
+    // scan memos have no first step (p1 = -1)
+    auto scan_key_of = [](const DevPlan& P) -> std::array<int, 6> {
+        const DevStep& a = P.steps[P.scanLevel - 1];
+        return {-1, 0, a.pred, a.dir, -1, 0};
+    };
     auto memo3_key_of = [](const DevPlan& P) -> std::array<int, 6> {
         return {P.steps[1].pred, P.steps[1].dir, P.steps[2].pred, P.steps[2].dir, P.steps[3].pred, P.steps[3].dir};
     };
@@ -217,6 +222,7 @@ void Staged::stage(Context& c, std::vector<DevPlan>& plans, const std::vector<co
             }
         }
         if (dedup[i] == kDedupSort) continue;
+        if (plans[i].scanLevel > 0) memoKeys.push_back(scan_key_of(plans[i]));
         if (plans[i].memoLevel > 0) memoKeys.push_back(memo_key_of(plans[i]));
         if (plans[i].memoSteps == 3) memoKeys.push_back(memo3_key_of(plans[i]));
     }
@@ -254,7 +260,12 @@ void Staged::stage(Context& c, std::vector<DevPlan>& plans, const std::vector<co
     if (anyClaims) dHubSeen.ensure((size_t)std::max(c.grid, 1) * kHubSeen * 8, as);
     for (int i = 0; i < nPlans; ++i) {
         plans[i].memoTab = plans[i].memo3Tab = nullptr;
-        plans[i].memoBits = plans[i].memo3Bits = nullptr;
+        plans[i].memoBits = plans[i].memo3Bits = plans[i].scanBits = nullptr;
+        if (plans[i].scanLevel > 0) {
+            const std::array<int, 6> k = scan_key_of(plans[i]);
+            const SuffixMemo* m = c.memo_for(k[0], k[1], k[2], k[3], k[4], k[5]);
+            if (m && m->words == plans[i].rowWords) plans[i].scanBits = m->bits;
+        }
         if (plans[i].memoLevel > 0) {
             const std::array<int, 6> k = memo_key_of(plans[i]);
             const SuffixMemo* m = c.memo_for(k[0], k[1], k[2], k[3], k[4], k[5]);
@@ -296,7 +307,7 @@ void Staged::stage(Context& c, std::vector<DevPlan>& plans, const std::vector<co
             plans[i].keyBase = (unsigned long long)k << sortSlotShift;
             plans[i].rankBits = rankBits;
             plans[i].memoTab = plans[i].memo3Tab = nullptr;   // memos set bitmap words; keys carry every pair
-            plans[i].memoBits = plans[i].memo3Bits = nullptr;
+            plans[i].memoBits = plans[i].memo3Bits = plans[i].scanBits = nullptr;
         }
         tasks.insert(tasks.end(), pts[i].tasks.begin(), pts[i].tasks.end());
         cost.insert(cost.end(), pts[i].cost.begin(), pts[i].cost.end());
@@ -410,14 +421,16 @@ void Context::ensure_memos(const std::vector<std::array<int, 6>>& keys, cudaStre
         const uint64_t key = memo_key(k[0], k[1], k[2], k[3], k[4], k[5]);
         if (memos.count(key)) continue;
         memos[key] = nullptr;
-        if (memoGain < 0 || nHub == 0 || p1 < 0 || p2 < 0 || p1 >= h.nPred || p2 >= h.nPred || p3 >= h.nPred) continue;
+        const bool scan = p1 < 0;
+        if (memoGain < 0 || (nHub == 0 && !scan) || p2 < 0 || p1 >= h.nPred || p2 >= h.nPred || p3 >= h.nPred) continue;
         if (p3 >= 0 && h.nPred >= (1 << 20)) continue;
         fresh.push_back(k);
     }
     if (fresh.empty()) return;
     // the rank domain of a memo: the rows of its last step's predicate in
-    // the other direction
+    // the other direction (a scan memo's: the rows it scans)
     auto domain = [&](const std::array<int, 6>& k) -> int64_t {
+        if (k[0] < 0) return h.pred_rows(k[2], k[3]);
         return k[4] >= 0 ? h.pred_rows(k[4], 1 - k[5]) : h.pred_rows(k[2], 1 - k[3]);
     };
     // the hub rows of (p1, d1) worth a memo, per new key, on host threads:
@@ -428,6 +441,10 @@ void Context::ensure_memos(const std::vector<std::array<int, 6>>& keys, cudaStre
     parallel_for(fresh.size(), [&](size_t i) {
         const int p1 = fresh[i][0], d1 = fresh[i][1], p2 = fresh[i][2], d2 = fresh[i][3];
         const int p3 = fresh[i][4], d3 = fresh[i][5];
+        if (p1 < 0) {   // scan memos: one slot
+            rowsOf[i].push_back(-1);
+            return;
+        }
         const int words = (int)((domain(fresh[i]) + 31) / 32);
         const double need = memoGain * words;
         // the count only grows: a row stops being summed once it qualifies
@@ -489,6 +506,12 @@ void Context::ensure_memos(const std::vector<std::array<int, 6>>& keys, cudaStre
         m->rowHasMemo.assign((size_t)h.pred_rows(p1, d1), 0);
         const std::vector<int32_t>& rows = rowsOf[i];
         for (size_t j = 0; j < rows.size(); ++j) {
+            if (p1 < 0) {
+                constexpr int32_t kRows = 2048;   // rows a block
+                for (int32_t b0 = 0; b0 < wo; b0 += kRows)
+                    all.push_back(MemoJob{p2, d2, p2, d2, -1, words, -1, 0, wo, b0, std::min(wo, b0 + kRows), 0, bits});
+                continue;
+            }
             tab[h.hubOf[d1][rows[j]]] = (int32_t)j;
             m->rowHasMemo[(size_t)(rows[j] - h.predRow[d1][p1])] = 1;
             // one block per slice of the row's values, so that the paths of a

@@ -335,7 +335,12 @@ struct Context {
         const HostIndex& h = hix;
         std::vector<std::pair<const void*, size_t>> parts;
         auto add = [&](const void* p, size_t n) { parts.push_back({p, n}); };
+        // per-edge arrays have one element more on the device: the edge that
+        // stands for a free variable's long row (its value is kAnyValue, the
+        // rest zero)
+        std::vector<size_t> valParts;
         for (int d = 0; d < 2; ++d) {
+            valParts.push_back(parts.size());
             add(h.val[d].data(), h.val[d].size() * 4);
             add(h.valRank[d].data(), h.valRank[d].size() * 4);
             add(h.src[d].data(), h.src[d].size() * 4);
@@ -358,7 +363,7 @@ struct Context {
         std::vector<size_t> off;
         for (auto& pp : parts) {
             off.push_back(total);
-            total += (pp.second + 255) & ~size_t(255);
+            total += (pp.second + 8 + 255) & ~size_t(255);
         }
         size_t freeB = 0, totB = 0;
         ck(cudaMemGetInfo(&freeB, &totB), "cudaMemGetInfo");
@@ -370,6 +375,10 @@ struct Context {
         for (size_t i = 0; i < parts.size(); ++i)
             if (parts[i].second)
                 ck(cudaMemcpy(base + off[i], parts[i].first, parts[i].second, cudaMemcpyHostToDevice), "cudaMemcpy(index)");
+        for (size_t i = 0; i < parts.size(); ++i)
+            ck(cudaMemset(base + off[i] + parts[i].second, 0, 8), "cudaMemset(index)");
+        static_assert(kAnyValue == -1, "set by bytes");
+        for (size_t i : valParts) ck(cudaMemset(base + off[i] + parts[i].second, 0xff, 4), "cudaMemset(index)");
         size_t k = 0;
         for (int d = 0; d < 2; ++d) {
             dix.val[d] = reinterpret_cast<const int32_t*>(base + off[k++]);

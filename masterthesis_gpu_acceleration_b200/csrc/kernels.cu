@@ -144,8 +144,14 @@ __device__ __forceinline__ bool pass_filters(const DevPlan& P, const DevIndex& i
 template <bool kC, class Val>
 __device__ __forceinline__ int2 step_segment(const DevPlan& P, const DevIndex& ix, int s, Meter<kC>& mt, Val val) {
     const DevStep& st = P.steps[s];
-    if (st.kind == kExpand) return row_lookup(ix, st.pred, st.dir, val(st.keyRef), mt);
+    if (st.kind == kExpand) {
+        const int2 r = row_lookup(ix, st.pred, st.dir, val(st.keyRef), mt);
+        // a free variable's long row: the one edge past the last, whose value is kAnyValue
+        if (st.free && r.y - r.x >= P.freeMin) return make_int2((int)ix.nTriples, (int)ix.nTriples + 1);
+        return r;
+    }
     mt.add(8);
+    if (st.kind == kRowScan) return make_int2(__ldg(ix.predRow[st.dir] + st.pred), __ldg(ix.predRow[st.dir] + st.pred + 1));
     return make_int2(__ldg(ix.predEdge[0] + st.pred), __ldg(ix.predEdge[0] + st.pred + 1));
 }
 
@@ -367,15 +373,20 @@ __device__ __forceinline__ int memo_row_value(const DevStep& stA, const int* it)
 // warp calls this; new pair bits are counted on insertion and returned (per
 // lane).  Steps come by value and counts go back as the result, so that the
 // caller's loop state never needs an address.
+// Scan items (plans with a scanLevel: hO from the rows of (p, d), then only a
+// free value behind it) are the same with every value in the place of N1(x):
+// h = hO, its row's values as witnesses, and stB the step (p, 1 - d) from a
+// witness to its h.
 template <bool kC>
 __device__ __noinline__ unsigned long long memo_item(const DevPlan& P, const DevIndex& ix, const DevStep stA,
                                                      const DevStep stB, const int* par, int lenK, int slot,
                                                      uint32_t* dst, int words, int* ex, int lane, Meter<kC>& mt,
-                                                     bool sharedDst, int nEx3) {
+                                                     bool sharedDst, int nEx3, bool scan) {
     unsigned long long myNew = 0;
     const bool three = nEx3 > 0;
-    const uint32_t* S1 = three ? P.memo3Bits + (long long)slot * ((long long)words + ((P.wo + 3) >> 2))
-                               : P.memoBits + (long long)slot * ((long long)kMemoMaps * words);
+    const uint32_t* S1 = scan ? P.scanBits
+                              : (three ? P.memo3Bits + (long long)slot * ((long long)words + ((P.wo + 3) >> 2))
+                                       : P.memoBits + (long long)slot * ((long long)kMemoMaps * words));
     int nEx = lenK - kTupleHead;
     unsigned wmask = 0;
     if (three) {
@@ -388,7 +399,12 @@ __device__ __noinline__ unsigned long long memo_item(const DevPlan& P, const Dev
             const int u = par[kTupleHead + lane];
             const int2 r = row_lookup(ix, stB.pred, exDir, u, mt);
             ex[lane] = r.y > r.x ? __ldg(ix.srcRank[exDir] + r.x) : -1;
-            isW = u != memo_row_value(stA, par) && seg_has(ix.val[stA.dir], segBeg, segLen, u, mt);
+            if (scan) {   // every bound value may be the free value of some row
+                const int2 w = row_lookup(ix, stB.pred, stB.dir, u, mt);
+                isW = w.y > w.x;
+            } else {
+                isW = u != memo_row_value(stA, par) && seg_has(ix.val[stA.dir], segBeg, segLen, u, mt);
+            }
         }
         wmask = __ballot_sync(0xffffffffu, isW);
         __syncwarp();
@@ -501,12 +517,21 @@ __device__ __forceinline__ bool memo3_fits(const DevPlan& P, const DevIndex& ix,
 // segment is a memoised hub row with at most two bound values among its
 // neighbours (returns the memo slot); 3: a kExist leaf item decided by the
 // existence memo (returns -3, its found bit set; -4 when the bit is new and
-// the task counts on insertion); 4: as 2 for the three-step memo of level 1.
+// the task counts on insertion); 4: as 2 for the three-step memo of level 1;
+// 5: an item of the scan level, for the scan memo (returns 0).
 // -1: enumerate as usual.
 template <bool kC>
 __device__ __noinline__ int classify_item(const DevPlan& P, const DevIndex& ix, const DevStep stp, const int* it,
                                           int lenK, int kind, int segBeg, int segLen, uint32_t* fb, bool heavy,
                                           Meter<kC>& mt) {
+    if (kind == 5) {
+        int nR = 0;   // bound values that are some row's free value
+        for (int q = kTupleHead; q < lenK; ++q) {
+            const int2 r = row_lookup(ix, stp.pred, 1 - stp.dir, it[q], mt);
+            nR += r.y > r.x ? 1 : 0;
+        }
+        return nR <= 2 ? 0 : -1;
+    }
     const int row = __ldg(ix.predRow[stp.dir] + stp.pred) + __ldg(ix.srcRank[stp.dir] + segBeg);
     const int h = __ldg(ix.hubOf[stp.dir] + row);
     mt.add(12);
@@ -825,7 +850,11 @@ __device__ __forceinline__ void run_task(Smem<B>& sm, const DevIndex& ix, const 
             const bool memoPath = !leaf && pairs && !sortMode && P.memoTab != nullptr && k + 1 == P.memoLevel;
             const bool existMemo = leaf && !pairs && P.memoTab != nullptr && k + 1 == P.memoLevel &&
                                    !(heavy && k == 0);
-            const int pathKind = hubPath ? 1 : (memoPath ? 2 : (existMemo ? 3 : (memo3Path ? 4 : 0)));
+            // Scan path: the plan ends in a row scan binding hO and the free
+            // value behind it; the rows are counted from their scan memo.
+            const bool scanPath = !leaf && pairs && !sortMode && P.scanBits != nullptr && k + 1 == P.scanLevel &&
+                                  !(heavy && k == 0);
+            const int pathKind = hubPath ? 1 : (memoPath ? 2 : (existMemo ? 3 : (memo3Path ? 4 : (scanPath ? 5 : 0))));
             bool isHub = false;   // item marked for the hub or memo pass
 
             // window: the stored neighbour segment of each item
@@ -856,7 +885,7 @@ __device__ __forceinline__ void run_task(Smem<B>& sm, const DevIndex& ix, const 
                         int code = it[1];
                         if (code == kItemNew && myLen > 0) {
                             code = kItemEnum;
-                            if (myLen >= ix.hubMinLen && !(tid == 0 && off != 0)) {
+                            if ((myLen >= ix.hubMinLen || scanPath) && !(tid == 0 && off != 0)) {
                                 const int c = classify_item(P, ix, stp, it, lenK, pathKind, myBeg, myLen, fb,
                                                             heavy, mt);
                                 if (c == -4) myNew += 1;   // a new found bit of a split root
@@ -882,7 +911,7 @@ __device__ __forceinline__ void run_task(Smem<B>& sm, const DevIndex& ix, const 
             sm.wBeg[tid] = myBeg;
             sm.wLen[tid] = myLen;
             if (tid == 0 && !leaf) S.count[k + 1] = 0;
-            const bool anyHub = publish_window<B>(myLen, isHub, sm) && (hubPath || memoPath || memo3Path);
+            const bool anyHub = publish_window<B>(myLen, isHub, sm) && (hubPath || memoPath || memo3Path || scanPath);
             const int total = window_total<B>(sm);
             // When the next step expands from the value this step binds,
             // that value's row signature (stored beside it) drops most
@@ -920,10 +949,11 @@ __device__ __forceinline__ void run_task(Smem<B>& sm, const DevIndex& ix, const 
                 const int root = par[0];
                 if (!pairs && ((fb[root >> 5] >> (root & 31)) & 1u)) return;
                 if (stp.kind == kScan && (stp.sameVar ? (n0 != n1) : (n0 == n1))) return;
-                for (int q = kTupleHead; q < lenK; ++q) {
-                    const int x = par[q];
-                    if (x == n0 || (stp.nNew == 2 && x == n1)) return;
-                }
+                if (n0 != kAnyValue)
+                    for (int q = kTupleHead; q < lenK; ++q) {
+                        const int x = par[q];
+                        if (x == n0 || (stp.nNew == 2 && x == n1)) return;
+                    }
                 auto valN = [&](TermRef ref) -> int {
                     if (ref < 0) return P.consts[-1 - ref];
                     if (ref < lenK) return par[ref];
@@ -981,7 +1011,8 @@ __device__ __forceinline__ void run_task(Smem<B>& sm, const DevIndex& ix, const 
             // Candidates j = tid, tid + B, ... in groups of kU per thread: all
             // group members are located first, then their loads are issued
             // together, then they are evaluated.
-            const int* vbase = stp.kind == kExpand ? ix.val[stp.dir] : ix.src[0];
+            const int* vbase = stp.kind == kExpand ? ix.val[stp.dir]
+                                                   : (stp.kind == kRowScan ? ix.rowKey[stp.dir] : ix.src[0]);
             const int* rbase = stp.kind == kExpand ? ix.valRank[stp.dir]
                                                    : (stp.hoWhich == 1 ? ix.srcRank[0] : ix.valRank[0]);
             const bool wantRank = pairs && stp.hoWhich;
@@ -1010,7 +1041,11 @@ __device__ __forceinline__ void run_task(Smem<B>& sm, const DevIndex& ix, const 
                     if (sigTest) { sw_[u] = __ldg(sigWords + 2 * (long long)e_[u]); mt.add(4); }
                     n0_[u] = __ldg(vbase + e_[u]);
                     if (stp.kind == kScan) { n1_[u] = __ldg(ix.val[0] + e_[u]); mt.add(8); } else mt.add(4);
-                    if (wantRank) { rk_[u] = __ldg(rbase + e_[u]); mt.add(4); }
+                    if (wantRank) {   // a row scan's rank is the row's place among the predicate's
+                        rk_[u] = stp.kind == kRowScan ? e_[u] - __ldg(ix.predRow[stp.dir] + stp.pred)
+                                                      : __ldg(rbase + e_[u]);
+                        mt.add(4);
+                    }
                 }
 #pragma unroll
                 for (int u = 0; u < kU; ++u)
@@ -1063,9 +1098,11 @@ __device__ __forceinline__ void run_task(Smem<B>& sm, const DevIndex& ix, const 
                             const int slot = -2 - sm.wBeg[item];
                             const int nEx3 = memo3Path
                                 ? memo3_exceptions(P, ix, par, lenK, slot, words, S.exRank[warp], lane, mt) : 0;
-                            myNew += memo_item(P, ix, stp, P.steps[k + 1], par, lenK, slot,
+                            DevStep stB = P.steps[k + 1];
+                            if (scanPath) stB.dir = (int8_t)(1 - stB.dir);
+                            myNew += memo_item(P, ix, stp, stB, par, lenK, slot,
                                                bm + (rowBase + par[0]) * (long long)words, words, S.exRank[warp],
-                                               lane, mt, shared, nEx3);
+                                               lane, mt, shared, nEx3, scanPath);
                             continue;
                         }
                         // hO must differ from every bound value: their ranks in hO's domain
@@ -1295,6 +1332,19 @@ __global__ void memo_build_kernel(DevIndex ix, const MemoJob* jobs, int nJobs) {
     uint32_t* S1 = job.bits;
     uint32_t* S2 = S1 + job.words;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nWarps = blockDim.x >> 5;
+    if (job.row < 0) {
+        // scan memo of (p1, d1): its rows [b0, b1), by their number of values
+        // other than the key
+        const int base = ix.predRow[job.d1][job.p1];
+        for (int r = job.b0 + (int)threadIdx.x; r < job.b1; r += blockDim.x) {
+            const int key = ix.rowKey[job.d1][base + r];
+            const int e0 = ix.rowBeg[job.d1][base + r], e1 = ix.rowBeg[job.d1][base + r + 1];
+            int n = 0;
+            for (int e = e0; e < e1 && n < kMemoMaps; ++e) n += __ldg(ix.val[job.d1] + e) != key ? 1 : 0;
+            for (int q = 0; q < n; ++q) atomicOr(S1 + q * job.words + (r >> 5), 1u << (r & 31));
+        }
+        return;
+    }
     const int rb = ix.rowBeg[job.d1][job.row], re = ix.rowBeg[job.d1][job.row + 1];
     const int b = rb + job.b0, e = job.b1 < 0 ? re : rb + job.b1;
     Meter<false> mt;

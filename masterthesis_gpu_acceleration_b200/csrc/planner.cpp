@@ -20,7 +20,8 @@
 // in binding order.  Atoms are grounded greedily: every atom whose terms are
 // all bound becomes a membership check as soon as possible; otherwise the
 // atom with one bound term and the smallest average fan-out is expanded from
-// that term; otherwise the smallest predicate is scanned.  The order only
+// that term; otherwise the smallest predicate is scanned (by rows where a
+// free variable allows it, see build_steps).  The order only
 // affects speed: every complete grounding satisfies the same constraints
 // whichever order finds it (the reference's greedy choice in
 // SupportCounting.cpp:38-79 is likewise a speed heuristic).
@@ -77,7 +78,16 @@ int check_dir(const HostIndex& ix, int32_t p) {
 // Grounding order for `body` given the variables already bound in `b`.
 // `head` (support phase) is the used head triple, or null.  Returns false
 // when two atoms always ground to the same triple.
-bool build_steps(Builder& b, const std::vector<Atom>& body, const Atom* head, int32_t hO, bool pairs) {
+//
+// Free variables: one that occurs once in the body and not in the head, in
+// an atom that can never ground to another atom's triple (or the head's),
+// only has to exist.  Its atom is grounded by a free step (see
+// DevPlan::freeMin) as soon as its other term is bound; where a part of the
+// body that nothing bound reaches would be scanned edge by edge, the rows of
+// such an atom are scanned instead, and its free variable is looked for
+// behind each.
+bool build_steps(Builder& b, const Rule& rule, const Atom* head, int32_t hO, bool pairs) {
+    const std::vector<Atom>& body = rule.body;
     DevPlan& P = b.P;
     const HostIndex& ix = b.ix;
     const int nb = (int)body.size();   // at most kMaxBody (plan_rule checks)
@@ -101,6 +111,28 @@ bool build_steps(Builder& b, const std::vector<Atom>& body, const Atom* head, in
             found[nFound++] = LevelCheck{lvl, c};
         }
     };
+    // per atom: 0 no free variable, 1 the subject is free, 2 the object
+    int freeSide[kMaxBody];
+    for (int i = 0; i < nb; ++i) {
+        freeSide[i] = 0;
+        auto occurs = [&](const Term& t) {
+            int n = 0;
+            for (const Atom& a : body) n += (a.s.isVar && a.s.id == t.id) + (a.o.isVar && a.o.id == t.id);
+            for (const Term& u : {rule.head.s, rule.head.o}) n += u.isVar && u.id == t.id;
+            return n;
+        };
+        const Atom& a = body[i];
+        auto collides = [&](const Atom& c) {
+            return c.pred == a.pred && rel(a.s, c.s) != kNe && rel(a.o, c.o) != kNe;
+        };
+        bool alone = !collides(rule.head);
+        for (int j = 0; j < nb; ++j) alone &= j == i || !collides(body[j]);
+        if (!alone) continue;
+        if (a.o.isVar && occurs(a.o) == 1) freeSide[i] = 2;
+        else if (a.s.isVar && occurs(a.s) == 1) freeSide[i] = 1;
+    }
+    P.freeMin = std::max(rule.nVars, 1);
+    int steps = nb;   // upper bound of the plan's steps: the atoms and the row scans
     P.tupleLen[0] = b.tupleLen;
     add_checks(0);
     int lvl = 0;
@@ -113,6 +145,8 @@ bool build_steps(Builder& b, const std::vector<Atom>& body, const Atom* head, in
             if (sB == oB) continue;
             int d = sB ? 0 : 1;
             double fan = ix.avg_degree(body[i].pred, d);
+            // (the atom's unbound term is the free one: the other is bound)
+            if (freeSide[i]) fan = std::min(fan, 1.0);
             if (fan < bestFan) { bestFan = fan; best = i; bestDir = d; }
         }
         ++lvl;
@@ -128,14 +162,29 @@ bool build_steps(Builder& b, const std::vector<Atom>& body, const Atom* head, in
             b.bind(nv.id);
             st.nNew = 1;
             st.hoWhich = (pairs && nv.id == hO) ? 1 : 0;
+            st.free = freeSide[best] == (bestDir == 0 ? 2 : 1) ? 1 : 0;
         } else {
             int64_t bestSize = std::numeric_limits<int64_t>::max();
             for (int i = 0; i < nb; ++i) {
                 if (level[i] >= 0) continue;
-                int64_t sz = ix.pred_size(body[i].pred);
+                const bool rows = freeSide[i] && steps < kMaxBody;
+                int64_t sz = rows ? ix.pred_rows(body[i].pred, freeSide[i] == 2 ? 0 : 1) : ix.pred_size(body[i].pred);
                 if (sz < bestSize) { bestSize = sz; best = i; }
             }
             const Atom& a = body[best];
+            if (freeSide[best] && steps < kMaxBody) {
+                ++steps;
+                const Term& key = freeSide[best] == 2 ? a.s : a.o;
+                st.kind = kRowScan;
+                st.pred = a.pred;
+                st.dir = (int8_t)(freeSide[best] == 2 ? 0 : 1);
+                st.nNew = 1;
+                b.bind(key.id);
+                st.hoWhich = (pairs && key.id == hO) ? 1 : 0;
+                P.tupleLen[lvl] = b.tupleLen;
+                add_checks(lvl);
+                continue;
+            }
             st.kind = kScan;
             st.pred = a.pred;
             st.dir = 0;
@@ -285,7 +334,7 @@ bool build_body(const Rule& rule, const HostIndex& ix, const Geom& geom, int32_t
     P.rootDir = seedDir;
     P.rootPred = seedPred;
     b.bind(hS);
-    if (!build_steps(b, rule.body, nullptr, hO, pairs)) return true;
+    if (!build_steps(b, rule, nullptr, hO, pairs)) return true;
     if (!b.ok) return false;
     if (pairs) {
         for (int l = 0; l < P.m; ++l) {
@@ -293,6 +342,7 @@ bool build_body(const Rule& rule, const HostIndex& ix, const Geom& geom, int32_t
             if (!st.hoWhich) continue;
             P.hoLevel = l + 1;
             if (st.kind == kExpand) P.wo = (int32_t)ix.pred_rows(st.pred, 1 - st.dir);
+            else if (st.kind == kRowScan) P.wo = (int32_t)ix.pred_rows(st.pred, st.dir);
             else P.wo = (int32_t)ix.pred_rows(st.pred, st.hoWhich == 1 ? 0 : 1);
         }
     }
@@ -310,6 +360,19 @@ bool build_body(const Rule& rule, const HostIndex& ix, const Geom& geom, int32_t
             P.memoLevel = k + 1;
             P.memoP2 = c.pred;
             P.memoD2 = c.dir;
+        }
+    }
+    // scan memo: a row scan that binds hO, then only the free value behind it
+    if (pairs && P.m >= 2) {
+        const int k = P.m - 2;
+        const DevStep& a = P.steps[k];
+        const DevStep& c = P.steps[k + 1];
+        if (a.kind == kRowScan && a.hoWhich == 1 && c.kind == kExpand && c.free && c.pred == a.pred &&
+            c.dir == a.dir && c.keyRef == P.tupleLen[k] && P.chkN[k + 1] == 0 && P.usedN[k + 1] == 0 &&
+            P.chkN[k + 2] == 0 && P.usedN[k + 2] == 0)
+        {
+            P.scanLevel = k + 1;
+            P.steps[k].free = 1;   // for the estimates: its rows cost a word for 32
         }
     }
     // three-step suffix memo: hS -> x, then x -> v2 -> v3 -> hO,
@@ -352,11 +415,23 @@ double plan_cost(const PhasePlan& ph, FanSamples& fans) {
             for (int q = 0; q < s; ++q)
                 if (st.keyRef >= P.tupleLen[q] && st.keyRef < P.tupleLen[q + 1]) by = q;
         if (st.kind == kScan) f.all = f.capped = (float)fans.index().pred_size(st.pred);
+        else if (st.kind == kRowScan) {
+            f.all = f.capped = (float)fans.index().pred_rows(st.pred, st.dir);
+            if (P.scanLevel == s + 1) f.all = f.capped = 1.f + f.all / 32.f;   // the scan memo's words
+        }
         else if (by >= 0 && P.steps[by].kind == kExpand) f = fans.edges(P.steps[by].pred, P.steps[by].dir, st.pred, st.dir);
         else if (by < 0 && st.keyRef == kTupleHead) f = fans.rows(P.rootPred, P.rootDir, st.pred, st.dir);
         else f.all = f.capped = (float)fans.index().avg_degree(st.pred, st.dir);
+        if (st.free) f.all = f.capped = std::min(f.all, 2.f);
         w *= cap ? f.capped : f.all;
         cost += w * (s == P.m - 1 ? 1.0 : 2.0);
+        // a check passes as often as a random pair of its predicate's
+        // subjects and objects is a triple
+        for (int k = 0; k < P.chkN[s + 1]; ++k) {
+            const int32_t p = P.checks[P.chkBeg[s + 1] + k].pred;
+            const double cells = (double)fans.index().pred_rows(p, 0) * (double)fans.index().pred_rows(p, 1);
+            w *= cells > 0 ? (double)fans.index().pred_size(p) / cells : 0.0;
+        }
     }
     return cost;
 }
@@ -468,7 +543,7 @@ RulePlan plan_rule(const Rule& rule, const HostIndex& ix, const Geom& geom, FanS
                 range = ix.row_range(h.pred, 0, h.s.id);
                 P.rootValConst = b.ref(h.o);
             }
-            if (build_steps(b, rule.body, &h, -1, false) && b.ok) {
+            if (build_steps(b, rule, &h, -1, false) && b.ok) {
                 finish_capacity(P, geom);
                 exist_memo_eligibility(P);
                 S.how = kDevice;
@@ -529,6 +604,7 @@ RulePlan plan_rule(const Rule& rule, const HostIndex& ix, const Geom& geom, FanS
 std::pair<int32_t, int32_t> ho_domain(const DevPlan& P) {
     const DevStep& st = P.steps[P.hoLevel - 1];
     if (st.kind == kExpand) return {st.pred, 1 - st.dir};
+    if (st.kind == kRowScan) return {st.pred, st.dir};
     return {st.pred, st.hoWhich == 1 ? 0 : 1};
 }
 

@@ -33,6 +33,7 @@ DevPlan plan_identity(const PhasePlan& ph) {
     p.memoBits = nullptr;
     p.memo3Tab = nullptr;
     p.memo3Bits = nullptr;
+    p.scanBits = nullptr;
     p.memoWords = 0;
     p.gBlockWords = 0;
     p.pairKeys = nullptr;
@@ -41,7 +42,6 @@ DevPlan plan_identity(const PhasePlan& ph) {
     p.keyBase = 0;
     p.rankBits = 0;
     p.pad0 = 0;
-    p.pad1 = 0;
     p.pad2 = 0;
     p.pad3 = 0;
     return p;
@@ -117,7 +117,12 @@ double TaskBuilder::sb_fan(int32_t pred, int dir) { return sbFan_[(size_t)pred *
 
 double TaskBuilder::avg_fan(const DevStep& st) const {
     if (st.kind == kScan) return (double)ix_.pred_size(st.pred);
-    return std::max(1.0, ix_.avg_degree(st.pred, st.dir));
+    if (st.kind == kRowScan) {   // free: counted from the scan memo, 32 rows a word
+        const double rows = (double)ix_.pred_rows(st.pred, st.dir);
+        return st.free ? 1.0 + rows / 32.0 : rows;
+    }
+    const double f = std::max(1.0, ix_.avg_degree(st.pred, st.dir));
+    return st.free ? std::min(f, 2.0) : f;   // a long row of a free step is one candidate
 }
 
 double TaskBuilder::estimate(const PhasePlan& ph, bool hubAware) {
@@ -126,7 +131,7 @@ double TaskBuilder::estimate(const PhasePlan& ph, bool hubAware) {
     for (int s = 0; s < P.m; ++s) {
         const DevStep& st = P.steps[s];
         double f = avg_fan(st);
-        if (hubAware && st.kind == kExpand) f = std::max(f, sb_fan(st.pred, st.dir));
+        if (hubAware && st.kind == kExpand && !st.free) f = std::max(f, sb_fan(st.pred, st.dir));
         w *= std::max(1.0, f);
         if (w > 1e18) return 1e18;
     }
@@ -190,7 +195,7 @@ double TaskBuilder::chain_tail(const DevPlan& P) {
         const DevStep& st = P.steps[s];
         const DevStep& pv = P.steps[s - 1];
         double f;
-        if (st.kind == kExpand && pv.kind == kExpand && pv.nNew == 1 && st.keyRef == P.tupleLen[s - 1]) {
+        if (st.kind == kExpand && !st.free && pv.kind == kExpand && pv.nNew == 1 && st.keyRef == P.tupleLen[s - 1]) {
             const bool capped = s == P.m - 1 && P.mode == kPairs && P.hoLevel == P.m && !ix_.hubOff.empty();
             f = transition(pv.pred, pv.dir, st.pred, st.dir, capped);
         } else
@@ -201,7 +206,7 @@ double TaskBuilder::chain_tail(const DevPlan& P) {
 }
 
 bool TaskBuilder::chain_shaped(const DevPlan& P) const {
-    return P.m >= 2 && P.steps[0].kind == kExpand && P.steps[1].kind == kExpand &&
+    return P.m >= 2 && P.steps[0].kind == kExpand && P.steps[1].kind == kExpand && !P.steps[1].free &&
            P.steps[1].keyRef == P.tupleLen[0] && (P.steps[0].keyRef < 0 || P.steps[0].keyRef < P.tupleLen[0]);
 }
 
@@ -250,6 +255,9 @@ static int32_t resolve(const DevPlan& P, TermRef ref, const int32_t* vals, int32
 std::pair<int32_t, int32_t> TaskBuilder::first_segment(const DevPlan& P, int32_t r, const int32_t* vals) const {
     const DevStep& st = P.steps[0];
     if (st.kind == kScan) return {ix_.predEdge[0][st.pred], ix_.predEdge[0][st.pred + 1]};
+    if (st.kind == kRowScan) return {ix_.predRow[st.dir][st.pred], ix_.predRow[st.dir][st.pred + 1]};
+    // a free first step's row is split by its values as any other, although
+    // a long one counts as one (the first slice takes it, the others are empty)
     // the first step expands the root's own row: no lookup
     if (P.rootKind == kRootRows && P.rootDir == st.dir && P.rootPred == st.pred && st.keyRef == kTupleHead)
         return {ix_.rowBeg[st.dir][r], ix_.rowBeg[st.dir][r + 1]};
@@ -262,10 +270,11 @@ double TaskBuilder::child_work(const DevPlan& P, const int32_t* vals, int32_t e,
     const DevStep& s0 = P.steps[0];
     int32_t n0, n1 = -1;
     if (s0.kind == kExpand) n0 = ix_.val[s0.dir][e];
+    else if (s0.kind == kRowScan) n0 = ix_.rowKey[s0.dir][e];
     else { n0 = ix_.src[0][e]; n1 = ix_.val[0][e]; }
     const DevStep& s1 = P.steps[1];
     double d2;
-    if (s1.kind == kScan) d2 = (double)ix_.pred_size(s1.pred);
+    if (s1.kind != kExpand || s1.free) d2 = avg_fan(s1);
     else {
         int32_t k = resolve(P, s1.keyRef, vals, n0, n1);
         d2 = (k >= 0 && k < ix_.nEnt) ? deg2[k] : 0.0;
@@ -304,7 +313,7 @@ TaskBuilder::Walk TaskBuilder::compute_walk(const PhasePlan& ph) {
     }
     // a second step that scans, or expands from a root value or a constant,
     // costs the same after every edge of the first step
-    const bool uniformChild = P.m >= 2 && (s1.kind == kScan || s1.keyRef < P.tupleLen[0]);
+    const bool uniformChild = P.m >= 2 && (s1.kind != kExpand || s1.keyRef < P.tupleLen[0]);
     std::vector<float> w((size_t)(ph.rootEnd - ph.rootBeg));
     int32_t vals[2];
     for (int32_t r = ph.rootBeg; r < ph.rootEnd; ++r) {
@@ -400,7 +409,7 @@ void TaskBuilder::build(const std::vector<const PhasePlan*>& phases, int blocks,
             // otherwise every first-segment edge
             double edges = chain_shaped(ph.plan) ? (double)(ph.rootEnd - ph.rootBeg)
                          : (double)(ph.rootEnd - ph.rootBeg) *
-                           (s0.kind == kExpand ? std::max(1.0, ix_.avg_degree(s0.pred, s0.dir)) : (double)ix_.pred_size(s0.pred));
+                           (s0.kind == kExpand ? std::max(1.0, ix_.avg_degree(s0.pred, s0.dir)) : avg_fan(s0));
             if (!forced[i] && !cached[i] && used + edges > walkBudget) continue;
             // a walk whose own cost exceeds the phase's expected device time
             // cannot pay for itself (a single rule on the whole GPU)
