@@ -241,6 +241,50 @@ struct DevTask {
     int32_t gRow;            // heavy root: global dedup row, else -1
 };
 
+// The work a block gives away when it still runs a long task while the queue
+// is empty and other blocks are idle: the frontier items it has not expanded,
+// as records (tuple, segment) that a follow-up launch spreads over the GPU.
+// A spill task is a run of records of one task and level; its dedup rows (the
+// task's own, copied from shared memory, or its global ones) are shared by
+// all of them.
+struct SpillTask {
+    int32_t plan, level;
+    int32_t recBeg, recN;
+    int32_t beg, G;            // the task's roots [beg, beg + G)
+    uint32_t* rows;            // row of the first root (kExist: the found bits)
+};
+constexpr int kSpillRecInts = kMaxTuple + 2;   // tuple, first edge, edges
+constexpr int kSpillTasks = 8192;              // capacities of one list
+constexpr int kSpillRecs = 65536;
+constexpr int kSpillSups = 2048;
+constexpr long long kSpillRowWords = 1 << 21;  // rows copied out of shared memory (8 MiB a launch)
+
+// Spilled tasks of plans with fused support: counted after the last launch.
+struct SpillSup {
+    int32_t plan, beg, G, pad;
+    const uint32_t* rows;
+};
+
+// Counters of one launch's spilling (all zero before it).
+struct SpillCtl {
+    unsigned long long used[2];   // per list: tasks << 32 | records
+    unsigned long long rowWords;
+    int32_t next[2];              // task counters of the follow-up launches
+    int32_t sups;
+    int32_t pad;
+};
+
+struct SpillArgs {
+    SpillCtl* ctl = nullptr;      // null: no spilling
+    SpillTask* tasks[2] = {nullptr, nullptr};
+    int32_t* recs[2] = {nullptr, nullptr};
+    uint32_t* rows = nullptr;
+    SpillSup* sups = nullptr;
+    int32_t in = -1;              // list a follow-up launch runs (-1: the launch's own tasks)
+    int32_t out = -1;             // list it may spill into (-1: none)
+    int32_t always = 0;           // 1: every task spills after its first round (tests)
+};
+
 // Engine launch geometry: block size B (128, 256 or 512 threads) with a
 // shared-memory pool of 48 ints per thread that each plan splits between
 // its frontier levels and its dedup bitmap, so 1024 / B blocks stay

@@ -70,6 +70,19 @@ int bits_for(uint64_t n) {
 constexpr unsigned long long kMaxSortKeys = 0xffffffffull;   // the sort's 32-bit positions
 }  // namespace
 
+namespace {
+// Layout of Staged::dSpill: two lists of tasks and records, support jobs, rows.
+size_t spill_part(int part) {
+    const size_t sizes[] = {kSpillTasks * sizeof(SpillTask), kSpillTasks * sizeof(SpillTask),
+                            (size_t)kSpillRecs * kSpillRecInts * 4, (size_t)kSpillRecs * kSpillRecInts * 4,
+                            kSpillSups * sizeof(SpillSup), (size_t)kSpillRowWords * 4};
+    size_t at = 0;
+    for (int i = 0; i < part; ++i) at += (sizes[i] + 255) & ~size_t(255);
+    return at;
+}
+size_t spill_bytes() { return spill_part(6); }
+}  // namespace
+
 void Staged::stage(Context& c, std::vector<DevPlan>& plans, const std::vector<const PhasePlan*>& phases,
                    bool sortTasks, cudaStream_t s, double walkBudget, bool costAware, bool allowSort) {
     nPlans = (int)plans.size();
@@ -381,7 +394,16 @@ void Staged::stage(Context& c, std::vector<DevPlan>& plans, const std::vector<co
     dBlob.ensure(blob, as);
     nResults = nPlans + extraResults;
     dResults.ensure((size_t)nResults * sizeof(unsigned long long), as);
-    dCtl.ensure(64, as);
+    dCtl.ensure(kCtlBytes, as);
+    // Spilling pays where a task can outlast the others: not for launches
+    // whose estimated work is below about 60 us of the whole GPU (their
+    // follow-up launches, a few us, would cost more than a tail saves), and
+    // not for sort mode, whose key count must not depend on it.
+    double workNs = 0;
+    for (int i = 0; i < nPlans; ++i) workNs += pts[i].work * pts[i].scale;
+    spillAlways = c.spill == 2;
+    spillable = c.spill && nSort == 0 && (spillAlways || workNs > 60e3 * std::max(c.grid, 1));
+    if (spillable) dSpill.ensure(spill_bytes(), as);
     hResults.ensure((size_t)nResults * sizeof(unsigned long long));
     hCtl.ensure(64);
     ck(cudaMemcpyAsync(dBlob.p, hBlob.p, blob, cudaMemcpyHostToDevice, s), "H2D plans");
@@ -541,6 +563,37 @@ void Context::ensure_memos(const std::vector<std::array<int, 6>>& keys, cudaStre
     ck(cudaStreamSynchronize(s), "memo build");   // memos are shared by every stream afterwards
 }
 
+SpillArgs Staged::spill_args() const {
+    SpillArgs a;
+    if (!spillable) return a;
+    char* p = static_cast<char*>(dSpill.p);
+    a.ctl = reinterpret_cast<SpillCtl*>(static_cast<char*>(dCtl.p) + kSpillCtlAt);
+    for (int k = 0; k < 2; ++k) {
+        a.tasks[k] = reinterpret_cast<SpillTask*>(p + spill_part(k));
+        a.recs[k] = reinterpret_cast<int32_t*>(p + spill_part(2 + k));
+    }
+    a.sups = reinterpret_cast<SpillSup*>(p + spill_part(4));
+    a.rows = reinterpret_cast<uint32_t*>(p + spill_part(5));
+    a.out = 0;
+    a.always = spillAlways ? 1 : 0;
+    return a;
+}
+
+// The launches that run what the one before spilled; the last may not spill.
+void Staged::enqueue_follow_ups(Context& c, cudaStream_t s, unsigned long long* results, int* status,
+                                unsigned long long* span) {
+    if (!spillable) return;
+    EngineProfile prof;
+    prof.span = span;
+    for (int k = 0; k < kFollowUps; ++k) {
+        SpillArgs a = spill_args();
+        a.in = k;
+        a.out = k + 1 < kFollowUps ? k + 1 : -1;
+        ck(engine_launch(c.dix, dPlans, dTasks, 0, nullptr, results, status, c.grid, c.geom.block, s, &prof, a),
+           "engine follow-up launch");
+    }
+}
+
 void Staged::enqueue_sort(Context& c, cudaStream_t s, unsigned long long* results, int* status) {
     if (!nSort) return;
     char* base = static_cast<char*>(dSort.p);
@@ -576,7 +629,7 @@ void Staged::enqueue(Context& c, cudaStream_t s, int instr, int gridCap, unsigne
     if (!nPlans) return;
     check_geometry(c);
     ck(cudaMemsetAsync(dResults.p, 0, (size_t)nResults * sizeof(unsigned long long), s), "memset results");
-    ck(cudaMemsetAsync(dCtl.p, 0, 8, s), "memset ctl");
+    ck(cudaMemsetAsync(dCtl.p, 0, kCtlBytes, s), "memset ctl");
     if (bitmapWords) ck(cudaMemsetAsync(dBitmap.p, 0, bitmapWords * 4, s), "memset bitmap");
     if (heavyWords) ck(cudaMemsetAsync(dHeavy.p, 0, heavyWords * 4, s), "memset heavy rows");
     if (nSort) ck(cudaMemsetAsync(dSort.p, 0, 8, s), "memset key cursor");
@@ -602,10 +655,13 @@ void Staged::enqueue(Context& c, cudaStream_t s, int instr, int gridCap, unsigne
     if (blockWords && (size_t)grid > blockRegions) throw CudaError("launch grid exceeds the block-row regions");
     ck(engine_launch(c.dix, dPlans, dTasks, nTasks, static_cast<int*>(dCtl.p),
                      static_cast<unsigned long long*>(dResults.p), static_cast<int*>(dCtl.p) + 1, grid,
-                     c.geom.block, s, instr ? &prof : nullptr),
+                     c.geom.block, s, instr ? &prof : nullptr, instr ? SpillArgs{} : spill_args()),
        "engine launch");
-    ck(support_rows(c.dix, dPlans, dSupJobs, nSupJobs, static_cast<unsigned long long*>(dResults.p), s),
-       "fused support of split roots");
+    if (!instr)
+        enqueue_follow_ups(c, s, static_cast<unsigned long long*>(dResults.p), static_cast<int*>(dCtl.p) + 1, nullptr);
+    ck(support_rows(c.dix, dPlans, dSupJobs, nSupJobs, static_cast<unsigned long long*>(dResults.p), s,
+                    !instr && extraResults > 0 ? spill_args() : SpillArgs{}, c.sms),
+       "fused support of split roots and spilled tasks");
     enqueue_sort(c, s, static_cast<unsigned long long*>(dResults.p), static_cast<int*>(dCtl.p) + 1);
 }
 
@@ -616,7 +672,7 @@ void Staged::enqueue_per_plan(Context& c, cudaStream_t s) {
     // control words: [0..1] task counters, [2] status (int), per plan two
     // u64 span words at byte 16 + 16 * i and its u64 result at
     // kPerPlanResults + 8 * i; all start at zero
-    ck(cudaMemsetAsync(dCtl.p, 0, 64, s), "memset ctl");
+    ck(cudaMemsetAsync(dCtl.p, 0, kCtlBytes, s), "memset ctl");
     if (bitmapWords) ck(cudaMemsetAsync(dBitmap.p, 0, bitmapWords * 4, s), "memset bitmap");
     if (heavyWords) ck(cudaMemsetAsync(dHeavy.p, 0, heavyWords * 4, s), "memset heavy rows");
     if (nSort) ck(cudaMemsetAsync(dSort.p, 0, 8, s), "memset key cursor");
@@ -629,12 +685,19 @@ void Staged::enqueue_per_plan(Context& c, cudaStream_t s) {
         if (blockWords && (size_t)grid > blockRegions) throw CudaError("launch grid exceeds the block-row regions");
         ck(engine_launch(c.dix, dPlans, dTasks + b, e - b, ctl + i,
                          reinterpret_cast<unsigned long long*>(static_cast<char*>(dCtl.p) + kPerPlanResults), ctl + 2,
-                         grid, c.geom.block, s, &prof),
+                         grid, c.geom.block, s, &prof, spill_args()),
            "engine launch");
     }
+    // (timed with the last plan's phase, the body size where there is one)
+    enqueue_follow_ups(c, s, reinterpret_cast<unsigned long long*>(static_cast<char*>(dCtl.p) + kPerPlanResults), ctl + 2,
+                       reinterpret_cast<unsigned long long*>(static_cast<char*>(dCtl.p) + 16 + 16 * (nPlans - 1)));
+    bool fusedHere = false;
+    for (const DevPlan* P = static_cast<const DevPlan*>(hBlob.p); P != static_cast<const DevPlan*>(hBlob.p) + nPlans; ++P)
+        fusedHere |= P->supN > 0;
     ck(support_rows(c.dix, dPlans, dSupJobs, nSupJobs,
-                    reinterpret_cast<unsigned long long*>(static_cast<char*>(dCtl.p) + kPerPlanResults), s),
-       "fused support of split roots");
+                    reinterpret_cast<unsigned long long*>(static_cast<char*>(dCtl.p) + kPerPlanResults), s,
+                    fusedHere ? spill_args() : SpillArgs{}, c.sms),
+       "fused support of split roots and spilled tasks");
     enqueue_sort(c, s, reinterpret_cast<unsigned long long*>(static_cast<char*>(dCtl.p) + kPerPlanResults), ctl + 2);
 }
 
@@ -978,6 +1041,9 @@ void finish_load(Context* c) {
     if (const char* m = std::getenv("GPU_RULES_MEMO3")) c->memo3 = std::atoi(m) != 0;
     if (const char* f = std::getenv("GPU_RULES_FUSE_SUPPORT")) c->fuseSupport = std::atoi(f) != 0;
     if (const char* h = std::getenv("GPU_RULES_HUB_CLAIMS")) c->hubClaims = std::atoi(h) != 0;
+    // GPU_RULES_SPILL=0: long tasks run to their end on one block; 2: every
+    // task spills after its first round
+    if (const char* h = std::getenv("GPU_RULES_SPILL")) c->spill = std::max(0, std::min(2, std::atoi(h)));
     // GPU_RULES_HOST_PROFILE=1: one stderr line of host-side times per one-shot batch
     if (const char* h = std::getenv("GPU_RULES_HOST_PROFILE")) c->hostProfile = std::atoi(h) != 0;
     c->tasks.reset(new TaskBuilder(c->hix));

@@ -31,11 +31,13 @@ cudaError_t engine_configure();
 cudaError_t memo_build(const DevIndex& ix, const MemoJob* jobs, int nJobs, int maxWo, cudaStream_t stream);
 // Fused support of split heavy roots, after the engine launch that filled
 // their rows (see DevPlan::supN).
+// spillBlocks: blocks for the tasks that a launch with spilling gave away.
 cudaError_t support_rows(const DevIndex& ix, const DevPlan* plans, const SupJob* jobs, int nJobs,
-                         unsigned long long* results, cudaStream_t stream);
+                         unsigned long long* results, cudaStream_t stream, const SpillArgs& sp = SpillArgs{},
+                         int spillBlocks = 0);
 cudaError_t engine_launch(const DevIndex& ix, const DevPlan* plans, const DevTask* tasks, int nTasks,
                           int* taskCounter, unsigned long long* results, int* status, int grid, int block,
-                          cudaStream_t stream, const EngineProfile* prof);
+                          cudaStream_t stream, const EngineProfile* prof, const SpillArgs& sp = SpillArgs{});
 // Sort mode (sort.cu): radix sort of the appended pair keys and the count of
 // each plan's distinct keys into its result slot.
 size_t pairs_sort_hist_words(unsigned long long cap);
@@ -148,7 +150,19 @@ struct Staged {
     int nResults = 0;
     int nSupJobs = 0;
     const SupJob* dSupJobs = nullptr;      // in dBlob
-    DevBuf dHubSeen;                       // leaf hub claims: kHubSeen words per resident block
+    DevBuf dHubSeen;                       // hub and memo claims: kHubSeen words per resident block
+    DevBuf dSpill;                         // spill lists, rows and support jobs (see spill_args)
+    // Where the control words of one launch lie in dCtl (kCtlBytes, cleared
+    // before it): counters, status and per-plan words first, then spilling's.
+    static constexpr size_t kSpillCtlAt = 64, kCtlBytes = 128;
+    static_assert(kSpillCtlAt + sizeof(SpillCtl) <= kCtlBytes, "control words");
+    bool spillable = false;                // launches of this staging may spill
+    bool spillAlways = false;
+    // Follow-up launches after a launch that may spill (a list each).
+    static constexpr int kFollowUps = 2;
+    SpillArgs spill_args() const;
+    void enqueue_follow_ups(Context& c, cudaStream_t s, unsigned long long* results, int* status,
+                            unsigned long long* span);
     // host ms of the staging sections (dedup and fusion, memos, task build,
     // plan fields, task order, upload), summed until read
     double hostSect[6] = {0, 0, 0, 0, 0, 0};
@@ -176,12 +190,13 @@ struct Staged {
         return nSort > 0 && *static_cast<const unsigned long long*>(hSort.p) > keyCap;
     }
     void restage(Context& c, cudaStream_t s);
-    // Kernels one enqueue() launches: the engine, the fused support of split
-    // roots when there are any, and the pair sort (three kernels per 8-bit
+    // Kernels one enqueue() launches: the engine and its follow-ups, the fused
+    // support of split roots and spilled tasks, and the pair sort (three kernels per 8-bit
     // pass and the count) when sort mode is staged.
     int kernels_per_enqueue() const {
         if (!nPlans) return 0;
-        return (nTasks > 0 ? 1 : 0) + (nSupJobs > 0 ? 1 : 0) + (nSort ? 3 * ((sortBits + 7) / 8) + 1 : 0);
+        return (nTasks > 0 ? 1 : 0) + (nTasks > 0 && spillable ? kFollowUps : 0) +
+               (nSupJobs > 0 || (spillable && extraResults > 0) ? 1 : 0) + (nSort ? 3 * ((sortBits + 7) / 8) + 1 : 0);
     }
     // instr: 0 plain, 1 task times into dTaskNs, 2 also algorithmic bytes
     // into dBytes.  gridCap > 0 limits the launch to that many blocks (a
@@ -223,7 +238,7 @@ struct Staged {
         hBlob.ensure(blob);
         dResults.ensure(plans * sizeof(unsigned long long), s);
         hResults.ensure(plans * sizeof(unsigned long long));
-        dCtl.ensure(64, s);
+        dCtl.ensure(kCtlBytes, s);
         hCtl.ensure(64);
         dHeavy.ensure(1 << 20, s);
         dBitmap.ensure(1 << 20, s);
@@ -289,6 +304,7 @@ struct Context {
     double memoGain = 0.25;
     bool memo3 = true;         // three-step suffix memos (memo3_item) for the plans that admit one
     bool fuseSupport = true;   // batches count a rule's support in its body-size plan where it can
+    int spill = 1;             // 1: long tasks spill into follow-up launches (see SpillTask); 2: every task (tests)
     bool hubClaims = true;     // repeated leaf hub items of a root are skipped (see kHubSeen)
     bool hostProfile = false;  // one-shot batches print their host-side times
     std::unordered_map<uint64_t, std::unique_ptr<SuffixMemo>> memos;

@@ -71,6 +71,16 @@ struct BlockState {
     int warpSum[kWarps];
     unsigned long long red[kWarps];
     int exRank[kWarps][kMaxVars];   // per warp: hO-domain ranks of the bound values of a hub item
+    int spill;                      // 1: the block gives its open items away
+    long long lookAt;               // thread 0: the clock at its last look at the queue,
+    int looks;                      // and the looks in a row that found idle blocks
+    int base;                       // the level the task's search starts at
+    int nTasks;                     // of the launch, and its counter
+    const int* queue;
+    int spillN[kMaxBody + 1];       // records per level, then their write positions
+    int spillAt;                    // first task slot, first record slot
+    int spillRec;
+    uint32_t* spillRows;
 };
 
 template <int B>
@@ -663,9 +673,158 @@ __device__ __noinline__ unsigned long long fused_support(const DevPlan& P, const
 // items) or memo slot of an item that the hub or memo pass takes.
 constexpr int kItemNew = 0, kItemEnum = 1, kItemDone = 2, kItemHub = 3;
 
-template <int B, bool kC, bool kD>
+// Clock cycles (about 8 us) between a block's looks at the task queue, and how
+// many looks in a row must find idle blocks before it spills (a follow-up
+// launch costs a few us; a round of memo items can take hundreds).
+constexpr long long kSpillEvery = 16000;
+constexpr int kSpillLooks = 2;
+// Records of a spill task, and candidates of a record, at inner levels and at
+// the leaf: about a round's work each.
+constexpr int kSpillChunk = 8, kSpillChunkLeaf = 32;
+constexpr int kSpillSeg = 256, kSpillSegLeaf = 8192;
+
+// Gives the open items of levels kBase..k away (see SpillTask); false when a
+// list is full (the block then carries on).  The task's dedup rows start at
+// `rows`; `shared`: they are nWords words in shared memory and move to global
+// ones.  The whole block calls this between two rounds;
+// level k continues at item w0, `off` candidates of it consumed.  Out of line:
+// it runs at most once per task.
+template <int B>
+__device__ __noinline__ bool spill_items(Smem<B>& sm, const DevTask& task, const SpillArgs& sp, uint32_t* rows,
+                                         int nWords, bool shared, bool sup, int kBase, int k,
+                                         int w0, int off) {
+    const DevPlan& P = sm.plan;
+    BlockState<B>& S = sm.st;
+    const int tid = threadIdx.x;
+    // a level's first open item and the candidates of it already consumed
+    auto level_pos = [&](int l, int& at, int& skip) {
+        at = l == k ? w0 : S.curItem[l];
+        skip = l == k ? off : S.curOff[l];
+    };
+    // records an item takes: none when nothing is left of it, one when a memo
+    // or hub row answers it, else its segment in pieces
+    auto pieces = [&](int l, const int* it, int skip) {
+        const int lenL = P.tupleLen[l];
+        const bool hasRank = P.mode == kPairs && P.hoLevel >= 1 && l >= P.hoLevel;
+        const int left = it[lenL + 1] - skip;
+        if (left <= 0 || (!hasRank && it[1] == kItemDone)) return 0;
+        if (!hasRank && it[1] >= kItemHub) return 1;
+        // (not classified yet at a level that may: whole, or its row would not be known as a hub's)
+        if (!hasRank && it[1] == kItemNew &&
+            (l + 1 == P.m || l + 1 == P.memoLevel || l + 1 == P.scanLevel || (l == 1 && P.memo3Tab)))
+            return 1;
+        const int seg = l + 1 == P.m ? kSpillSegLeaf : kSpillSeg;
+        return (left + seg - 1) / seg;
+    };
+    for (int l = tid; l <= kMaxBody; l += B) S.spillN[l] = 0;
+    __syncthreads();
+    for (int l = kBase; l <= k; ++l) {
+        int at, skip;
+        level_pos(l, at, skip);
+        const int cnt = min(S.count[l], P.cap), stride = P.tupleLen[l] + 2;
+        int n = 0;
+        for (int i = at + tid; i < cnt; i += B)
+            n += pieces(l, sm.pool + S.levelOff[l] + i * stride, i == at ? skip : 0);
+        n = __reduce_add_sync(0xffffffffu, n);
+        if ((tid & 31) == 0 && n) atomicAdd(&S.spillN[l], n);
+    }
+    __syncthreads();
+    if (tid == 0) {
+        unsigned nRec = 0, nTask = 0;
+        for (int l = kBase; l <= k; ++l) {
+            const int c = l + 1 == P.m ? kSpillChunkLeaf : kSpillChunk;
+            nRec += S.spillN[l];
+            nTask += (S.spillN[l] + c - 1) / c;
+        }
+        bool ok = nTask > 1 && nRec <= (unsigned)kSpillRecs;   // one task would gain nothing
+        uint32_t* dst = rows;
+        int supAt = -1;
+        if (ok && shared) {
+            const unsigned long long need = (unsigned long long)((nWords + 3) & ~3);
+            const unsigned long long at = atomicAdd(&sp.ctl->rowWords, need);
+            ok = at + need <= (unsigned long long)kSpillRowWords;
+            dst = sp.rows + at;
+            if (ok && sup) {
+                supAt = atomicAdd(&sp.ctl->sups, 1);
+                ok = supAt < kSpillSups;
+            }
+        }
+        unsigned long long old = 0;
+        if (ok) {
+            unsigned long long* used = &sp.ctl->used[sp.out];
+            old = *reinterpret_cast<volatile unsigned long long*>(used);
+            for (;;) {
+                const unsigned t0 = (unsigned)(old >> 32), r0 = (unsigned)old;
+                ok = t0 + nTask <= (unsigned)kSpillTasks && r0 + nRec <= (unsigned)kSpillRecs;
+                if (!ok) break;
+                const unsigned long long seen =
+                    atomicCAS(used, old, (unsigned long long)(t0 + nTask) << 32 | (r0 + nRec));
+                if (seen == old) break;
+                old = seen;
+            }
+        }
+        // (rows or a support slot taken before a list turned out full are lost to this launch)
+        if (supAt >= 0 && supAt < kSpillSups)
+            sp.sups[supAt] = SpillSup{ok ? task.plan : -1, task.beg, task.end - task.beg, 0, dst};
+        S.spill = ok ? 1 : 0;
+        S.spillAt = (int)(old >> 32);
+        S.spillRec = (int)(unsigned)old;
+        S.spillRows = dst;
+    }
+    __syncthreads();
+    if (!S.spill) return false;
+    uint32_t* const dst = S.spillRows;
+    if (shared)
+        for (int i = tid; i < nWords; i += B) dst[i] = rows[i];
+    // tasks, level by level; records of a level in the order of their claims
+    int t = S.spillAt, r = S.spillRec;
+    for (int l = kBase; l <= k; ++l) {
+        const int n = S.spillN[l], c = l + 1 == P.m ? kSpillChunkLeaf : kSpillChunk;
+        for (int j = tid; j * c < n; j += B)
+            sp.tasks[sp.out][t + j] = SpillTask{task.plan, l, r + j * c, min(c, n - j * c), task.beg,
+                                                task.end - task.beg, dst};
+        t += (n + c - 1) / c;
+        r += n;
+    }
+    __syncthreads();
+    if (tid == 0) {
+        int at = S.spillRec;
+        for (int l = kBase; l <= k; ++l) {
+            const int n = S.spillN[l];
+            S.spillN[l] = at;
+            at += n;
+        }
+    }
+    __syncthreads();
+    for (int l = kBase; l <= k; ++l) {
+        int at, skip0;
+        level_pos(l, at, skip0);
+        const int lenL = P.tupleLen[l], cnt = min(S.count[l], P.cap), stride = lenL + 2;
+        const int seg = l + 1 == P.m ? kSpillSegLeaf : kSpillSeg;
+        for (int i = at + tid; i < cnt; i += B) {
+            const int* it = sm.pool + S.levelOff[l] + i * stride;
+            const int skip = i == at ? skip0 : 0;
+            const int n = pieces(l, it, skip);
+            if (!n) continue;
+            const int slot = atomicAdd(&S.spillN[l], n);
+            for (int q = 0; q < n; ++q) {
+                int* rec = sp.recs[sp.out] + (long long)(slot + q) * kSpillRecInts;
+                for (int j = 0; j < lenL; ++j) rec[j] = it[j];
+                const int b = skip + q * seg;
+                rec[lenL] = it[lenL] + b;
+                rec[lenL + 1] = n == 1 ? it[lenL + 1] - b : min(seg, it[lenL + 1] - b);
+            }
+        }
+    }
+    return true;
+}
+
+// kS: the task may be spilled; st: the spill task to resume (`task` its
+// roots), or null.
+template <int B, bool kC, bool kD, bool kS>
 __device__ __forceinline__ void run_task(Smem<B>& sm, const DevIndex& ix, const DevTask& task,
-                                         unsigned long long* results, int* status, Meter<kC>& mt) {
+                                         unsigned long long* results, int* status, Meter<kC>& mt, const SpillArgs& sp,
+                                         const SpillTask* st) {
     constexpr int kLeafChunk = 16 * B;
     // candidates of a non-leaf round whose next step has a signature test
     // (most candidates die on it): more than the next level's capacity, so
@@ -686,8 +845,11 @@ __device__ __forceinline__ void run_task(Smem<B>& sm, const DevIndex& ix, const 
     const bool pairs = P.mode == kPairs;
     // Dedup targets.  A split heavy root (one root, G == 1) uses its global
     // row for both the pair bits and the found bit; counting happens on
-    // insertion so that the slices of one root count each result once.
-    const bool heavy = task.gRow >= 0;
+    // insertion so that the slices of one root count each result once.  A
+    // resumed spill task does the same with the rows of all its roots.
+    const bool resumed = kS && st != nullptr;
+    const bool sliced = task.gRow >= 0;   // level 0 holds a slice of the root's segment
+    const bool heavy = resumed || sliced;
     // Sort mode appends pair keys instead of setting bits (no bitmap at
     // all); block rows keep the task's rows in the block's own region of a
     // global buffer instead of one row per root of the phase.
@@ -696,15 +858,17 @@ __device__ __forceinline__ void run_task(Smem<B>& sm, const DevIndex& ix, const 
     const bool shared = !heavy && !(pairs && (P.gBitmap || sortMode));
     uint32_t* sbits = reinterpret_cast<uint32_t*>(sm.pool + P.bitmapOff);
     int* const items = sm.pool;
-    uint32_t* bm = heavy ? (P.gHeavy ? P.gHeavy + (long long)task.gRow * P.rowWords : nullptr)
+    uint32_t* bm = resumed ? st->rows
+                   : heavy ? (P.gHeavy ? P.gHeavy + (long long)task.gRow * P.rowWords : nullptr)
                          : (shared ? sbits : (blockRows ? P.gBitmap + (long long)blockIdx.x * P.gBlockWords : P.gBitmap));
     uint32_t* fb = heavy ? bm : sbits;   // kExist found bits
-    const long long rowBase = (heavy || shared || blockRows) ? 0 : (long long)task.beg - P.gRowBase;
+    // per-phase global rows start at the phase's first root: bm is the row of
+    // the task's first one
+    if (pairs && !heavy && !shared && !blockRows && !sortMode) bm += ((long long)task.beg - P.gRowBase) * P.rowWords;
     const long long keyRow0 = (long long)task.beg - P.gRowBase;   // sort mode: key row of the task's root 0
 
     // clear the task's shared dedup bits
     // pair rows are word-aligned: row r occupies words [r * rowWords, (r + 1) * rowWords)
-    const long long rowBits = (long long)P.rowWords << 5;
     const int nWords = heavy ? 0 : (shared ? (int)(pairs ? (long long)G * P.rowWords : ((G + 31) >> 5))
                                            : (pairs ? 0 : ((G + 31) >> 5)));
     for (int i = tid; i < nWords; i += B) sbits[i] = 0u;
@@ -726,6 +890,9 @@ __device__ __forceinline__ void run_task(Smem<B>& sm, const DevIndex& ix, const 
     if (tid == 0) {
         S.firstFail = INT_MAX;
         S.safeLevels = 0;
+        S.spill = S.looks = 0;
+        S.lookAt = clock64();
+        S.base = resumed ? st->level : 0;
         int off = 0;
         for (int l = 0; l <= kMaxBody; ++l) {
             S.curItem[l] = 0;
@@ -738,8 +905,17 @@ __device__ __forceinline__ void run_task(Smem<B>& sm, const DevIndex& ix, const 
     }
     __syncthreads();
 
+    const int kBase = resumed ? st->level : 0;   // the search ends when this level is exhausted
+    if (resumed) {
+        const int lenL = P.tupleLen[kBase], ints = lenL + 2;
+        const int n = min(st->recN, P.cap);
+        for (int i = tid; i < n * ints; i += B) {
+            const int r = i / ints, q = i - r * ints;
+            items[S.levelOff[kBase] + i] = sp.recs[sp.in][(long long)(st->recBeg + r) * kSpillRecInts + q];
+        }
+        if (tid == 0) S.count[kBase] = n;
+    } else {
     // ---- level 0: roots (tuple, then the segment of step 1) ----
-    {
         const int len0 = P.tupleLen[0];
         const int stride0 = P.m > 0 ? len0 + 2 : len0;
         // as for deeper items: a root whose segment has no value able to
@@ -815,11 +991,19 @@ __device__ __forceinline__ void run_task(Smem<B>& sm, const DevIndex& ix, const 
         // publishes the window's prefix sums, one closes the round.  Reads
         // of the shared counters that a later step may reset can only see
         // the reset when the decision they feed is the same either way.
-        int k = 0, w0 = 0, off = 0;
+        int k = kBase, w0 = 0, off = 0;
         for (;;) {
+            if constexpr (kS) {
+                if (S.spill) {   // set before the last round's barrier: all threads are here
+                    if (spill_items<B>(sm, task, sp, pairs ? bm : fb,
+                                       pairs ? G * P.rowWords : (G + 31) >> 5, !heavy && (shared || !pairs),
+                                       P.supN > 0 && !heavy, S.base, k, w0, off))
+                        break;
+                }
+            }
             const int cnt = min(S.count[k], P.cap);
             if (w0 >= cnt) {
-                if (k == 0) break;
+                if (k == S.base) break;
                 // nobody reads level k's bit again before it is re-entered
                 if (tid == 0) S.safeLevels &= ~(1u << k);
                 --k;
@@ -840,7 +1024,7 @@ __device__ __forceinline__ void run_task(Smem<B>& sm, const DevIndex& ix, const 
             // counted by OR-ing the row's rank bitmap into its pair row (32
             // candidates per word) instead of candidate by candidate.
             const bool hubPath = leaf && pairs && !sortMode && stp.hoWhich != 0 && stp.kind == kExpand &&
-                                 stp.nNew == 1 && !hasFilters && ix.nHub > 0 && !(heavy && k == 0);
+                                 stp.nNew == 1 && !hasFilters && ix.nHub > 0 && !(sliced && k == 0);
             // Memo path: the plan ends in two expand steps x -> y -> hO with
             // nothing but injectivity to test; an item whose first segment
             // is a hub row with a suffix memo is counted from the memo's
@@ -849,11 +1033,11 @@ __device__ __forceinline__ void run_task(Smem<B>& sm, const DevIndex& ix, const 
             const bool memo3Path = !leaf && pairs && !sortMode && P.memo3Tab != nullptr && k == 1;
             const bool memoPath = !leaf && pairs && !sortMode && P.memoTab != nullptr && k + 1 == P.memoLevel;
             const bool existMemo = leaf && !pairs && P.memoTab != nullptr && k + 1 == P.memoLevel &&
-                                   !(heavy && k == 0);
+                                   !(sliced && k == 0);
             // Scan path: the plan ends in a row scan binding hO and the free
             // value behind it; the rows are counted from their scan memo.
             const bool scanPath = !leaf && pairs && !sortMode && P.scanBits != nullptr && k + 1 == P.scanLevel &&
-                                  !(heavy && k == 0);
+                                  !(sliced && k == 0);
             const int pathKind = hubPath ? 1 : (memoPath ? 2 : (existMemo ? 3 : (memo3Path ? 4 : (scanPath ? 5 : 0))));
             bool isHub = false;   // item marked for the hub or memo pass
 
@@ -867,8 +1051,7 @@ __device__ __forceinline__ void run_task(Smem<B>& sm, const DevIndex& ix, const 
                     pruned = (fb[it[0] >> 5] >> (it[0] & 31)) & 1u;
                     if (heavy) mt.add(4);
                 } else if (itemHasRank && !sortMode) {
-                    const long long bit = (rowBase + it[0]) * rowBits + it[1];
-                    pruned = (bm[bit >> 5] >> (bit & 31)) & 1u;
+                    pruned = (bm[(long long)it[0] * P.rowWords + (it[1] >> 5)] >> (it[1] & 31)) & 1u;
                     if (!shared) mt.add(4);
                 }
                 if (!pruned) {
@@ -964,9 +1147,8 @@ __device__ __forceinline__ void run_task(Smem<B>& sm, const DevIndex& ix, const 
                 if (pairs && stp.hoWhich) {
                     rank = rankLoaded;
                     if (!leaf && !sortMode) {
-                        const long long bit = (rowBase + root) * rowBits + rank;
                         if (!shared) mt.add(4);
-                        if ((bm[bit >> 5] >> (bit & 31)) & 1u) return;
+                        if ((bm[(long long)root * P.rowWords + (rank >> 5)] >> (rank & 31)) & 1u) return;
                     }
                 }
                 if (leaf) {
@@ -978,9 +1160,8 @@ __device__ __forceinline__ void run_task(Smem<B>& sm, const DevIndex& ix, const 
                         emit_pair(P, keyRow0 + root, rank);
                         mt.add(8);
                     } else {
-                        const long long bit = (rowBase + root) * rowBits + rank;
-                        const uint32_t mask = 1u << (bit & 31);
-                        const uint32_t old = atomicOr(&bm[bit >> 5], mask);
+                        const uint32_t mask = 1u << (rank & 31);
+                        const uint32_t old = atomicOr(bm + (long long)root * P.rowWords + (rank >> 5), mask);
                         if (!shared) mt.add(8);
                         myNew += (old & mask) ? 0ull : 1ull;
                     }
@@ -1101,7 +1282,7 @@ __device__ __forceinline__ void run_task(Smem<B>& sm, const DevIndex& ix, const 
                             DevStep stB = P.steps[k + 1];
                             if (scanPath) stB.dir = (int8_t)(1 - stB.dir);
                             myNew += memo_item(P, ix, stp, stB, par, lenK, slot,
-                                               bm + (rowBase + par[0]) * (long long)words, words, S.exRank[warp],
+                                               bm + (long long)par[0] * words, words, S.exRank[warp],
                                                lane, mt, shared, nEx3, scanPath);
                             continue;
                         }
@@ -1114,7 +1295,7 @@ __device__ __forceinline__ void run_task(Smem<B>& sm, const DevIndex& ix, const 
                         __syncwarp();
                         const int h = -2 - sm.wBeg[item];
                         const uint32_t* hb = ix.hubBits + __ldg(ix.hubOff + h);
-                        uint32_t* dst = bm + (rowBase + par[0]) * (long long)words;
+                        uint32_t* dst = bm + (long long)par[0] * words;
                         const int w0b = perWarp ? lane : tid;
                         const int step = perWarp ? 32 : B;
                         for (int w = w0b; w < words; w += step) {
@@ -1134,6 +1315,17 @@ __device__ __forceinline__ void run_task(Smem<B>& sm, const DevIndex& ix, const 
             }
             if constexpr (kD) {
                 if (tid == 0 && global_ns() > S.deadline) S.stop = 1;
+            }
+            if constexpr (kS) {
+                // blocks past the end of the queue are idle; when a quarter
+                // of the launch has been for a while, the items left here are
+                // worth a follow-up launch
+                if (tid == 0 && sp.out >= 0 && (clock64() - S.lookAt > kSpillEvery || sp.always)) {
+                    S.lookAt = clock64();
+                    const int idle = *reinterpret_cast<const volatile int*>(S.queue) - S.nTasks;
+                    S.looks = sp.always ? kSpillLooks : (idle * 4 >= (int)gridDim.x ? S.looks + 1 : 0);
+                    if (S.looks >= kSpillLooks && !sortMode && !blockRows) S.spill = 1;
+                }
             }
             __syncthreads();
             if constexpr (kD) {
@@ -1172,7 +1364,7 @@ __device__ __forceinline__ void run_task(Smem<B>& sm, const DevIndex& ix, const 
 
     // ---- fused support: every pair row of the task is complete here (a
     // split heavy root's row only after the launch: support_rows_kernel) ----
-    if (P.supN > 0 && !heavy) {
+    if (P.supN > 0 && !heavy && !(kS && S.spill)) {
         const int lane = tid & 31;
         for (int j = 0; j < P.supN; ++j) {
             unsigned long long n = fused_support(P, ix, j, task.beg, G, bm, tid >> 5, B / 32, lane, 0, 1, mt);
@@ -1202,15 +1394,27 @@ __device__ __forceinline__ void run_task(Smem<B>& sm, const DevIndex& ix, const 
 template <int B, int kI>
 __global__ void __launch_bounds__(B, 1024 / B)
 engine_kernel(const __grid_constant__ DevIndex ix, const DevPlan* __restrict__ plans, const DevTask* __restrict__ tasks,
-              int nTasks, int* taskCounter, unsigned long long* results, int* status, EngineProfile prof) {
+              int nTasks, int* taskCounter, unsigned long long* results, int* status, EngineProfile prof,
+              const __grid_constant__ SpillArgs sp) {
     constexpr bool kC = kI == 2;
     constexpr bool kD = kI == 3;
+    constexpr bool kS = kI == 0;   // only the plain variant spills: the others time whole tasks
     extern __shared__ __align__(16) unsigned char smem_raw[];
     Smem<B>& sm = *reinterpret_cast<Smem<B>*>(smem_raw);
     Meter<kC> mt;
     if (prof.span && threadIdx.x == 0) atomicMax(prof.span, ~global_ns());
     if constexpr (kD) {
         if (threadIdx.x == 0) sm.st.deadline = global_ns() + prof.budgetNs;
+    }
+    const bool follow = kS && sp.in >= 0;   // a follow-up launch: its tasks are a spill list
+    if (follow) {
+        nTasks = (int)(sp.ctl->used[sp.in] >> 32);
+        taskCounter = &sp.ctl->next[sp.in];
+        if (nTasks == 0) return;
+    }
+    if (threadIdx.x == 0) {
+        sm.st.nTasks = nTasks;
+        sm.st.queue = taskCounter;
     }
     for (;;) {
         if (threadIdx.x == 0) {
@@ -1220,7 +1424,14 @@ engine_kernel(const __grid_constant__ DevIndex ix, const DevPlan* __restrict__ p
         __syncthreads();
         const int t = sm.st.task;
         if (t >= nTasks) break;
-        const DevTask task = tasks[t];
+        const SpillTask* st = nullptr;
+        DevTask task;
+        if (follow) {
+            st = sp.tasks[sp.in] + t;
+            task = DevTask{st->plan, st->beg, st->beg + st->G, 0, 0, -1};
+        } else {
+            task = tasks[t];
+        }
         if constexpr (kD) {
             if (sm.st.stop) {   // past the deadline: the task is skipped and its plan marked
                 if (threadIdx.x == 0) atomicOr(prof.incomplete + task.plan, 1);
@@ -1239,7 +1450,7 @@ engine_kernel(const __grid_constant__ DevIndex ix, const DevPlan* __restrict__ p
         int* dst = reinterpret_cast<int*>(&sm.plan);
         for (int i = threadIdx.x; i < (int)(sizeof(DevPlan) / 4); i += B) dst[i] = src[i];
         __syncthreads();
-        run_task<B, kC, kD>(sm, ix, task, results, status, mt);
+        run_task<B, kC, kD, kS>(sm, ix, task, results, status, mt, sp, st);
         __syncthreads();
         if constexpr (kD) {
             if (threadIdx.x == 0 && sm.st.stop) atomicOr(prof.incomplete + task.plan, 1);
@@ -1290,17 +1501,17 @@ cudaError_t engine_configure() {
 template <int B>
 static void launch_b(const DevIndex& ix, const DevPlan* plans, const DevTask* tasks, int nTasks, int* taskCounter,
                      unsigned long long* results, int* status, int grid, cudaStream_t stream,
-                     const EngineProfile* prof) {
+                     const EngineProfile* prof, const SpillArgs& sp) {
     const size_t smem = sizeof(Smem<B>);
     const EngineProfile p = prof ? *prof : EngineProfile{};
     if (p.bytes)
-        engine_kernel<B, 2><<<grid, B, smem, stream>>>(ix, plans, tasks, nTasks, taskCounter, results, status, p);
+        engine_kernel<B, 2><<<grid, B, smem, stream>>>(ix, plans, tasks, nTasks, taskCounter, results, status, p, sp);
     else if (p.budgetNs && p.incomplete && p.taskNs)
-        engine_kernel<B, 3><<<grid, B, smem, stream>>>(ix, plans, tasks, nTasks, taskCounter, results, status, p);
+        engine_kernel<B, 3><<<grid, B, smem, stream>>>(ix, plans, tasks, nTasks, taskCounter, results, status, p, sp);
     else if (p.taskNs)
-        engine_kernel<B, 1><<<grid, B, smem, stream>>>(ix, plans, tasks, nTasks, taskCounter, results, status, p);
+        engine_kernel<B, 1><<<grid, B, smem, stream>>>(ix, plans, tasks, nTasks, taskCounter, results, status, p, sp);
     else
-        engine_kernel<B, 0><<<grid, B, smem, stream>>>(ix, plans, tasks, nTasks, taskCounter, results, status, p);
+        engine_kernel<B, 0><<<grid, B, smem, stream>>>(ix, plans, tasks, nTasks, taskCounter, results, status, p, sp);
 }
 
 // Suffix memos (see memo_item): one block per job (a hub row x of one
@@ -1432,28 +1643,42 @@ __global__ void memo_build_kernel(DevIndex ix, const MemoJob* jobs, int nJobs) {
     }
 }
 
-// Fused support of split heavy roots: one block per job, its warps share the
-// head triples of the job's root, counted against its completed global row.
+// Fused support of split heavy roots and of spilled tasks, whose rows are
+// complete after the launch.  The first nJobs blocks take one heavy root
+// each, their warps sharing its head triples; the others share the spilled
+// tasks, a warp per root.
 __global__ void support_rows_kernel(const __grid_constant__ DevIndex ix, const DevPlan* plans, const SupJob* jobs,
-                                    int nJobs, unsigned long long* results) {
+                                    int nJobs, unsigned long long* results, const __grid_constant__ SpillArgs sp) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nWarps = blockDim.x >> 5;
-    if ((int)blockIdx.x >= nJobs) return;
-    const SupJob jb = jobs[blockIdx.x];
-    const DevPlan& P = plans[jb.plan];
-    if (!P.gHeavy) return;
-    const uint32_t* row = P.gHeavy + (long long)jb.gRow * P.rowWords;
     Meter<false> mt;
-    for (int j = 0; j < P.supN; ++j) {
-        unsigned long long n = fused_support(P, ix, j, jb.root, 1, row, 0, 1, lane, warp, nWarps, mt);
+    auto add = [&](const DevPlan& P, int j, unsigned long long n) {
         for (int d = 16; d; d >>= 1) n += __shfl_down_sync(0xffffffffu, n, d);
         if (lane == 0 && n) atomicAdd(results + P.supSlot[j], n);
+    };
+    if ((int)blockIdx.x < nJobs) {
+        const SupJob jb = jobs[blockIdx.x];
+        const DevPlan& P = plans[jb.plan];
+        if (!P.gHeavy) return;
+        const uint32_t* row = P.gHeavy + (long long)jb.gRow * P.rowWords;
+        for (int j = 0; j < P.supN; ++j)
+            add(P, j, fused_support(P, ix, j, jb.root, 1, row, 0, 1, lane, warp, nWarps, mt));
+        return;
+    }
+    const int n = min(sp.ctl->sups, kSpillSups);
+    for (int i = (int)blockIdx.x - nJobs; i < n; i += (int)gridDim.x - nJobs) {
+        const SpillSup u = sp.sups[i];
+        if (u.plan < 0) continue;
+        const DevPlan& P = plans[u.plan];
+        for (int j = 0; j < P.supN; ++j)
+            add(P, j, fused_support(P, ix, j, u.beg, u.G, u.rows, warp, nWarps, lane, 0, 1, mt));
     }
 }
 
 cudaError_t support_rows(const DevIndex& ix, const DevPlan* plans, const SupJob* jobs, int nJobs,
-                         unsigned long long* results, cudaStream_t stream) {
-    if (nJobs <= 0) return cudaSuccess;
-    support_rows_kernel<<<nJobs, 256, 0, stream>>>(ix, plans, jobs, nJobs, results);
+                         unsigned long long* results, cudaStream_t stream, const SpillArgs& sp, int spillBlocks) {
+    const int grid = nJobs + (sp.ctl ? spillBlocks : 0);
+    if (grid <= 0) return cudaSuccess;
+    support_rows_kernel<<<grid, 256, 0, stream>>>(ix, plans, jobs, nJobs, results, sp);
     return cudaGetLastError();
 }
 
@@ -1474,12 +1699,12 @@ cudaError_t memo_build(const DevIndex& ix, const MemoJob* jobs, int nJobs, int m
 // prof->span is set (any variant).
 cudaError_t engine_launch(const DevIndex& ix, const DevPlan* plans, const DevTask* tasks, int nTasks,
                           int* taskCounter, unsigned long long* results, int* status, int grid, int block,
-                          cudaStream_t stream, const EngineProfile* prof) {
-    if (nTasks <= 0) return cudaSuccess;
+                          cudaStream_t stream, const EngineProfile* prof, const SpillArgs& sp) {
+    if (nTasks <= 0 && sp.in < 0) return cudaSuccess;
     switch (block) {
-        case 128: launch_b<128>(ix, plans, tasks, nTasks, taskCounter, results, status, grid, stream, prof); break;
-        case 256: launch_b<256>(ix, plans, tasks, nTasks, taskCounter, results, status, grid, stream, prof); break;
-        case 512: launch_b<512>(ix, plans, tasks, nTasks, taskCounter, results, status, grid, stream, prof); break;
+        case 128: launch_b<128>(ix, plans, tasks, nTasks, taskCounter, results, status, grid, stream, prof, sp); break;
+        case 256: launch_b<256>(ix, plans, tasks, nTasks, taskCounter, results, status, grid, stream, prof, sp); break;
+        case 512: launch_b<512>(ix, plans, tasks, nTasks, taskCounter, results, status, grid, stream, prof, sp); break;
         default: return cudaErrorInvalidValue;
     }
     return cudaGetLastError();
