@@ -28,6 +28,23 @@ struct alignas(16) HashSlot {
 };
 constexpr uint32_t kEmptyTag = 0xffffffffu;
 
+// A slot of that table on the device: with the edge range come the union of
+// the row's value signatures (sufSig of its first edge), the row's rank and
+// its hub index, all in the one 32-byte sector that a probe reads, so that
+// storing a new frontier item takes one dependent load instead of two, and
+// classifying it none.
+struct alignas(32) DevSlot {
+    uint32_t tag, key, beg, end;
+    uint32_t sig[2];
+    int32_t rank, hub;   // hub: -1 when the row is none
+};
+// The same by row index, for roots that start from their own row.
+struct alignas(32) DevRow {
+    int32_t key, beg, end, hub;
+    uint32_t sig[2];
+    int32_t pad[2];
+};
+
 __host__ __device__ inline uint32_t slot_hash(uint32_t tag, uint32_t key) {
     uint64_t x = ((uint64_t)tag << 32) | key;
     x ^= x >> 33; x *= 0xff51afd7ed558ccdull;
@@ -61,8 +78,9 @@ struct DevIndex {
     // per direction, per predicate
     const int32_t* predRow[2];   // P + 1 entries
     const int32_t* predEdge[2];  // P + 1 entries
-    // (predicate, direction, key) -> edge range, open addressing
-    const struct HashSlot* hash;
+    // (predicate, direction, key) -> row, open addressing; and the rows
+    const struct DevSlot* hash;
+    const struct DevRow* rows[2];
     // hub rows (rows whose values also exist as a rank bitmap)
     const int32_t* hubOf[2];     // per row: hub index or -1
     const int64_t* hubOff;       // per hub: first word in hubBits
@@ -72,7 +90,6 @@ struct DevIndex {
     const uint64_t* valSig[2];
     const uint64_t* sufSig[2];
     int32_t nHub;
-    int32_t hubMinLen;   // edges of the shortest hub row (INT_MAX without any)
     uint32_t hashMask;
     int32_t nPred;
     int32_t nEnt;

@@ -26,6 +26,10 @@ namespace gr {
 
 size_t engine_smem_bytes(int block);
 cudaError_t engine_configure();
+// Fills the device's lookup table from the host's (n slots) and the row
+// records, once every other array of the index is in place.
+cudaError_t build_lookup(const DevIndex& ix, const HashSlot* hash16, long long n, DevSlot* slots, DevRow* const* rows,
+                         const int* nRows);
 // maxWo: the largest three-step domain among the jobs (0: none), which
 // sizes the shared path counters.
 cudaError_t memo_build(const DevIndex& ix, const MemoJob* jobs, int nJobs, int maxWo, cudaStream_t stream);
@@ -366,7 +370,8 @@ struct Context {
             add(h.predRow[d].data(), h.predRow[d].size() * 4);
             add(h.predEdge[d].data(), h.predEdge[d].size() * 4);
         }
-        add(h.hash.data(), h.hash.size() * sizeof(HashSlot));
+        add(nullptr, h.hash.size() * sizeof(DevSlot));   // filled on the device, as the rows
+        for (int d = 0; d < 2; ++d) add(nullptr, h.rowKey[d].size() * sizeof(DevRow));
         add(h.hubOf[0].data(), h.hubOf[0].size() * 4);
         add(h.hubOf[1].data(), h.hubOf[1].size() * 4);
         add(h.hubOff.data(), h.hubOff.size() * 8);
@@ -389,7 +394,7 @@ struct Context {
         indexMem.ensure(std::max<size_t>(total, 256));
         char* base = static_cast<char*>(indexMem.p);
         for (size_t i = 0; i < parts.size(); ++i)
-            if (parts[i].second)
+            if (parts[i].first && parts[i].second)
                 ck(cudaMemcpy(base + off[i], parts[i].first, parts[i].second, cudaMemcpyHostToDevice), "cudaMemcpy(index)");
         for (size_t i = 0; i < parts.size(); ++i)
             ck(cudaMemset(base + off[i] + parts[i].second, 0, 8), "cudaMemset(index)");
@@ -406,7 +411,11 @@ struct Context {
             dix.predRow[d] = reinterpret_cast<const int32_t*>(base + off[k++]);
             dix.predEdge[d] = reinterpret_cast<const int32_t*>(base + off[k++]);
         }
-        dix.hash = reinterpret_cast<const HashSlot*>(base + off[k++]);
+        DevSlot* slots = reinterpret_cast<DevSlot*>(base + off[k++]);
+        DevRow* rows[2];
+        for (int d = 0; d < 2; ++d) rows[d] = reinterpret_cast<DevRow*>(base + off[k++]);
+        dix.hash = slots;
+        for (int d = 0; d < 2; ++d) dix.rows[d] = rows[d];
         dix.hubOf[0] = reinterpret_cast<const int32_t*>(base + off[k++]);
         dix.hubOf[1] = reinterpret_cast<const int32_t*>(base + off[k++]);
         dix.hubOff = reinterpret_cast<const int64_t*>(base + off[k++]);
@@ -416,14 +425,19 @@ struct Context {
         dix.sufSig[0] = reinterpret_cast<const uint64_t*>(base + off[k++]);
         dix.sufSig[1] = reinterpret_cast<const uint64_t*>(base + off[k++]);
         dix.nHub = (int32_t)h.hubOff.size();
-        dix.hubMinLen = INT_MAX;
-        for (int d = 0; d < 2; ++d)
-            for (size_t r = 0; r < h.hubOf[d].size(); ++r)
-                if (h.hubOf[d][r] >= 0) dix.hubMinLen = std::min(dix.hubMinLen, h.rowBeg[d][r + 1] - h.rowBeg[d][r]);
         dix.hashMask = h.hashMask;
         dix.nPred = h.nPred;
         dix.nEnt = h.nEnt;
         dix.nTriples = h.nTriples;
+        DevBuf hash16;   // the host's table, for the kernel that widens it
+        hash16.ensure(std::max<size_t>(h.hash.size() * sizeof(HashSlot), 16));
+        if (!h.hash.empty())
+            ck(cudaMemcpy(hash16.p, h.hash.data(), h.hash.size() * sizeof(HashSlot), cudaMemcpyHostToDevice),
+               "cudaMemcpy(lookup table)");
+        const int nRows[2] = {(int)h.rowKey[0].size(), (int)h.rowKey[1].size()};
+        ck(build_lookup(dix, static_cast<const HashSlot*>(hash16.p), (long long)h.hash.size(), slots, rows, nRows),
+           "lookup table");
+        ck(cudaDeviceSynchronize(), "lookup table");
     }
 
     bool set_block(int b) {

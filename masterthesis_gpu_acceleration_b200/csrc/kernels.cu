@@ -99,13 +99,43 @@ __device__ __forceinline__ int2 row_lookup(const DevIndex& ix, int pred, int dir
     const uint32_t tag = (uint32_t)pred * 2u + (uint32_t)dir;
     uint32_t i = slot_hash(tag, (uint32_t)key) & ix.hashMask;
     for (uint32_t probe = 0; probe <= ix.hashMask; ++probe) {
-        const uint4 s = __ldg(reinterpret_cast<const uint4*>(ix.hash) + i);
+        const uint4 s = __ldg(reinterpret_cast<const uint4*>(ix.hash + i));
         mt.add(16);
         if (s.x == kEmptyTag) break;
         if (s.x == tag && s.y == (uint32_t)key) return make_int2((int)s.z, (int)s.w);
         i = (i + 1) & ix.hashMask;
     }
     return make_int2(0, 0);
+}
+
+// A row and what its slot says of it.
+struct RowHit {
+    int2 seg;
+    uint2 sig;   // union of the values' signatures
+    int rank, hub;
+};
+
+template <bool kC>
+__device__ __forceinline__ RowHit row_find(const DevIndex& ix, int pred, int dir, int key, Meter<kC>& mt) {
+    RowHit h{make_int2(0, 0), make_uint2(0u, 0u), -1, -1};
+    if (key < 0) return h;
+    const uint32_t tag = (uint32_t)pred * 2u + (uint32_t)dir;
+    uint32_t i = slot_hash(tag, (uint32_t)key) & ix.hashMask;
+    for (uint32_t probe = 0; probe <= ix.hashMask; ++probe) {
+        const uint4* p = reinterpret_cast<const uint4*>(ix.hash + i);
+        const uint4 s = __ldg(p), t = __ldg(p + 1);   // one sector
+        mt.add(32);
+        if (s.x == kEmptyTag) break;
+        if (s.x == tag && s.y == (uint32_t)key) {
+            h.seg = make_int2((int)s.z, (int)s.w);
+            h.sig = make_uint2(t.x, t.y);
+            h.rank = (int)t.z;
+            h.hub = (int)t.w;
+            break;
+        }
+        i = (i + 1) & ix.hashMask;
+    }
+    return h;
 }
 
 template <bool kC>
@@ -150,19 +180,22 @@ __device__ __forceinline__ bool pass_filters(const DevPlan& P, const DevIndex& i
     return true;
 }
 
-// Edge range of step `s` (0-based) for a binding resolved by `val`.
+// The range step `s` (0-based) enumerates for a binding resolved by `val`.
 template <bool kC, class Val>
-__device__ __forceinline__ int2 step_segment(const DevPlan& P, const DevIndex& ix, int s, Meter<kC>& mt, Val val) {
+__device__ __forceinline__ RowHit step_row(const DevPlan& P, const DevIndex& ix, int s, Meter<kC>& mt, Val val) {
     const DevStep& st = P.steps[s];
     if (st.kind == kExpand) {
-        const int2 r = row_lookup(ix, st.pred, st.dir, val(st.keyRef), mt);
+        RowHit h = row_find(ix, st.pred, st.dir, val(st.keyRef), mt);
         // a free variable's long row: the one edge past the last, whose value is kAnyValue
-        if (st.free && r.y - r.x >= P.freeMin) return make_int2((int)ix.nTriples, (int)ix.nTriples + 1);
-        return r;
+        if (st.free && h.seg.y - h.seg.x >= P.freeMin) {
+            h.seg = make_int2((int)ix.nTriples, (int)ix.nTriples + 1);
+            h.hub = -1;
+        }
+        return h;
     }
     mt.add(8);
-    if (st.kind == kRowScan) return make_int2(__ldg(ix.predRow[st.dir] + st.pred), __ldg(ix.predRow[st.dir] + st.pred + 1));
-    return make_int2(__ldg(ix.predEdge[0] + st.pred), __ldg(ix.predEdge[0] + st.pred + 1));
+    const int* at = (st.kind == kRowScan ? ix.predRow[st.dir] : ix.predEdge[0]) + st.pred;
+    return RowHit{make_int2(__ldg(at), __ldg(at + 1)), make_uint2(~0u, ~0u), -1, -1};
 }
 
 template <int B>
@@ -313,8 +346,7 @@ __device__ __noinline__ int memo3_list(const DevPlan& P, const DevIndex& ix, con
         const int h = __ldg(ix.val[d3] + e3);
         if (h != x && h != a) ex[n++] = __ldg(ix.valRank[d3] + e3);
     }
-    const int2 ra = row_lookup(ix, p3, 1 - d3, a, mt);
-    ex[n] = ra.y > ra.x ? __ldg(ix.srcRank[1 - d3] + ra.x) : -1;
+    ex[n] = row_find(ix, p3, 1 - d3, a, mt).rank;
     return n;
 }
 
@@ -407,8 +439,7 @@ __device__ __noinline__ unsigned long long memo_item(const DevPlan& P, const Dev
         bool isW = false;
         if (lane < nEx) {
             const int u = par[kTupleHead + lane];
-            const int2 r = row_lookup(ix, stB.pred, exDir, u, mt);
-            ex[lane] = r.y > r.x ? __ldg(ix.srcRank[exDir] + r.x) : -1;
+            ex[lane] = row_find(ix, stB.pred, exDir, u, mt).rank;
             if (scan) {   // every bound value may be the free value of some row
                 const int2 w = row_lookup(ix, stB.pred, stB.dir, u, mt);
                 isW = w.y > w.x;
@@ -486,9 +517,8 @@ __device__ __noinline__ int memo_exists(const DevPlan& P, const DevIndex& ix, co
                                         int lenK, int segBeg, int segLen, int slot, Meter<kC>& mt) {
     const int h = it[P.memoH];
     const int dDom = 1 - P.memoD2;
-    const int2 hr = row_lookup(ix, P.memoP2, dDom, h, mt);
-    if (hr.y <= hr.x) return 0;   // no y reaches h at all
-    const int rank = __ldg(ix.srcRank[dDom] + hr.x);
+    const int rank = row_find(ix, P.memoP2, dDom, h, mt).rank;
+    if (rank < 0) return 0;   // no y reaches h at all
     const int x = memo_row_value(stA, it);
     int nRem = 0;
     for (int q = kTupleHead; q < lenK; ++q) {
@@ -522,17 +552,16 @@ __device__ __forceinline__ bool memo3_fits(const DevPlan& P, const DevIndex& ix,
 }
 
 // Items of a round that may skip enumeration, kept out of line so that the
-// main loop's registers stay free.  kind 1: a leaf item whose segment is a
-// whole hub row (returns the hub index); 2: an item at the memo level whose
-// segment is a memoised hub row with at most two bound values among its
-// neighbours (returns the memo slot); 3: a kExist leaf item decided by the
-// existence memo (returns -3, its found bit set; -4 when the bit is new and
-// the task counts on insertion); 4: as 2 for the three-step memo of level 1;
-// 5: an item of the scan level, for the scan memo (returns 0).
-// -1: enumerate as usual.
+// main loop's registers stay free.  The item's segment is hub row `hub` (kind
+// 5: none).  kind 2: an item at the memo level whose row has a memo and at
+// most two bound values among its neighbours (returns the memo slot); 3: a
+// kExist leaf item decided by the existence memo (returns -3, its found bit
+// set; -4 when the bit is new and the task counts on insertion); 4: as 2 for
+// the three-step memo of level 1; 5: an item of the scan level, for the scan
+// memo (returns 0).  -1: enumerate as usual.
 template <bool kC>
 __device__ __noinline__ int classify_item(const DevPlan& P, const DevIndex& ix, const DevStep stp, const int* it,
-                                          int lenK, int kind, int segBeg, int segLen, uint32_t* fb, bool heavy,
+                                          int lenK, int kind, int segBeg, int segLen, uint32_t* fb, bool heavy, int hub,
                                           Meter<kC>& mt) {
     if (kind == 5) {
         int nR = 0;   // bound values that are some row's free value
@@ -542,13 +571,8 @@ __device__ __noinline__ int classify_item(const DevPlan& P, const DevIndex& ix, 
         }
         return nR <= 2 ? 0 : -1;
     }
-    const int row = __ldg(ix.predRow[stp.dir] + stp.pred) + __ldg(ix.srcRank[stp.dir] + segBeg);
-    const int h = __ldg(ix.hubOf[stp.dir] + row);
-    mt.add(12);
-    if (h < 0 || __ldg(ix.rowBeg[stp.dir] + row) != segBeg || __ldg(ix.rowBeg[stp.dir] + row + 1) - segBeg != segLen)
-        return -1;
-    if (kind == 1) return h;
-    const int slot = __ldg((kind == 4 ? P.memo3Tab : P.memoTab) + h);
+    const int slot = __ldg((kind == 4 ? P.memo3Tab : P.memoTab) + hub);
+    mt.add(4);
     if (slot < 0) return -1;
     if (kind == 4) return memo3_fits(P, ix, it[kTupleHead], mt) ? slot : -1;
     if (kind == 2) {
@@ -658,20 +682,23 @@ __device__ __noinline__ unsigned long long fused_support(const DevPlan& P, const
             const int b = __ldg(ix.val[P.supDir] + e);
             mt.add(4);
             if (b == a) continue;
-            const int2 br = row_lookup(ix, dp, dd, b, mt);
-            if (br.y <= br.x) continue;   // b never binds hO
-            const int rank = __ldg(ix.srcRank[dd] + br.x);
-            mt.add(8);
+            const int rank = row_find(ix, dp, dd, b, mt).rank;
+            if (rank < 0) continue;   // b never binds hO
+            mt.add(4);
             if ((row[rank >> 5] >> (rank & 31)) & 1u) ++n;
         }
     }
     return n;
 }
 
-// What an item's rank slot holds before hO is bound: not classified yet,
-// enumerated as usual, nothing left to do, or kItemHub + the hub index (leaf
-// items) or memo slot of an item that the hub or memo pass takes.
+// What an item's rank slot holds before hO is bound: not looked at yet, with
+// hub index h (-1 - h) or with a scanned range (kItemNew); enumerated as
+// usual; nothing left to do; or kItemHub + the hub index (leaf items) or memo
+// slot of an item that the hub or memo pass takes.
 constexpr int kItemNew = 0, kItemEnum = 1, kItemDone = 2, kItemHub = 3;
+__device__ __forceinline__ int item_state(const DevStep& next, int hub) {
+    return next.kind != kExpand ? kItemNew : (hub >= 0 ? -1 - hub : kItemEnum);
+}
 
 // Clock cycles (about 8 us) between a block's looks at the task queue, and how
 // many looks in a row must find idle blocks before it spills (a follow-up
@@ -710,7 +737,7 @@ __device__ __noinline__ bool spill_items(Smem<B>& sm, const DevTask& task, const
         if (left <= 0 || (!hasRank && it[1] == kItemDone)) return 0;
         if (!hasRank && it[1] >= kItemHub) return 1;
         // (not classified yet at a level that may: whole, or its row would not be known as a hub's)
-        if (!hasRank && it[1] == kItemNew &&
+        if (!hasRank && it[1] <= kItemNew &&
             (l + 1 == P.m || l + 1 == P.memoLevel || l + 1 == P.scanLevel || (l == 1 && P.memo3Tab)))
             return 1;
         const int seg = l + 1 == P.m ? kSpillSegLeaf : kSpillSeg;
@@ -923,8 +950,10 @@ __device__ __forceinline__ void run_task(Smem<B>& sm, const DevIndex& ix, const 
         const bool lookTest0 = P.m >= 2 && P.steps[0].kind == kExpand && P.steps[1].kind == kExpand &&
                                P.steps[1].keyRef == len0;
         const int lookBit0 = lookTest0 ? sig_bit(P.steps[1].pred, P.steps[1].dir) : 0;
-        const uint32_t* lookWords0 =
-            reinterpret_cast<const uint32_t*>(ix.sufSig[lookTest0 ? P.steps[0].dir : 0]) + (lookBit0 >> 5);
+        // the first step expands the root's own row: its record has all
+        const bool ownRow = P.rootKind == kRootRows && P.m > 0 && P.steps[0].kind == kExpand && !P.steps[0].free &&
+                            P.steps[0].pred == P.rootPred && P.steps[0].dir == P.rootDir &&
+                            P.steps[0].keyRef == kTupleHead;
         for (int i = tid; i < G; i += B) {
             const int r = task.beg + i;
             int tv[kTupleHead + 2];
@@ -932,7 +961,14 @@ __device__ __forceinline__ void run_task(Smem<B>& sm, const DevIndex& ix, const 
             tv[1] = kItemNew;
             int nv = kTupleHead;
             bool ok = true;
-            if (P.rootKind == kRootRows) {
+            RowHit seg{make_int2(0, 0), make_uint2(0u, 0u), -1, -1};
+            if (ownRow) {
+                const uint4* p = reinterpret_cast<const uint4*>(ix.rows[P.rootDir] + r);
+                const uint4 s = __ldg(p), t = __ldg(p + 1);
+                mt.add(32);
+                tv[nv++] = (int)s.x;
+                seg = RowHit{make_int2((int)s.y, (int)s.z), make_uint2(t.x, t.y), -1, (int)s.w};
+            } else if (P.rootKind == kRootRows) {
                 tv[nv++] = __ldg(ix.rowKey[P.rootDir] + r);
                 mt.add(4);
             } else {
@@ -948,26 +984,30 @@ __device__ __forceinline__ void run_task(Smem<B>& sm, const DevIndex& ix, const 
             if (ok && nv != len0) { ok = false; atomicOr(status, 2); }
             auto val0 = [&](TermRef ref) -> int { return ref < 0 ? P.consts[-1 - ref] : tv[ref < nv ? ref : 0]; };
             if (ok) ok = pass_filters(P, ix, 0, mt, val0);
-            int2 seg = make_int2(0, 0);
             if (ok && P.m > 0) {
-                seg = step_segment(P, ix, 0, mt, val0);
-                if (heavy) {
-                    const int b0 = seg.x;
-                    seg.x = min(seg.y, b0 + task.sub0);
-                    seg.y = min(seg.y, b0 + task.sub1);
+                if (!ownRow) seg = step_row(P, ix, 0, mt, val0);
+                tv[1] = item_state(P.steps[0], seg.hub);
+                if (sliced) {
+                    const int b0 = seg.seg.x;
+                    seg.seg.x = min(seg.seg.y, b0 + task.sub0);
+                    seg.seg.y = min(seg.seg.y, b0 + task.sub1);
+                    // (a slice's values are not the whole row's: no hub or memo, and its own signatures)
+                    tv[1] = kItemEnum;
+                    if (lookTest0 && seg.seg.y > seg.seg.x) {
+                        const uint2 w = __ldg(reinterpret_cast<const uint2*>(ix.sufSig[P.steps[0].dir]) + seg.seg.x);
+                        seg.sig = w;
+                        mt.add(8);
+                    }
                 }
-                ok = seg.y > seg.x;
-                if (ok && lookTest0) {
-                    mt.add(4);
-                    ok = (__ldg(lookWords0 + 2 * (long long)seg.x) >> (lookBit0 & 31)) & 1u;
-                }
+                ok = seg.seg.y > seg.seg.x;
+                if (ok && lookTest0) ok = ((lookBit0 & 32 ? seg.sig.y : seg.sig.x) >> (lookBit0 & 31)) & 1u;
             }
             if (ok) {
                 const int slot = atomicAdd(&S.count[0], 1);
                 if (slot < P.cap) {
                     int* dst = items + S.levelOff[0] + slot * stride0;
                     for (int q = 0; q < len0; ++q) dst[q] = tv[q];
-                    if (P.m > 0) { dst[len0] = seg.x; dst[len0 + 1] = seg.y - seg.x; }
+                    if (P.m > 0) { dst[len0] = seg.seg.x; dst[len0 + 1] = seg.seg.y - seg.seg.x; }
                 } else {
                     atomicOr(status, 4);
                 }
@@ -1061,18 +1101,21 @@ __device__ __forceinline__ void run_task(Smem<B>& sm, const DevIndex& ix, const 
                         // A round consumes candidates, not items: an item may
                         // wait through many windows.  It is classified in its
                         // first one and the verdict kept in its rank slot
-                        // (unused before hO is bound).  Rows shorter than the
-                        // shortest hub row need no look at the index.
-                        // Per-round classification was 25 % of the block time
-                        // of a 5-atom biomedical rule (13.2M for 0.33M items).
+                        // (unused before hO is bound).  Per-round
+                        // classification was 25 % of the block time of a
+                        // 5-atom biomedical rule (13.2M for 0.33M items).
                         int code = it[1];
-                        if (code == kItemNew && myLen > 0) {
-                            code = kItemEnum;
-                            if ((myLen >= ix.hubMinLen || scanPath) && !(tid == 0 && off != 0)) {
-                                const int c = classify_item(P, ix, stp, it, lenK, pathKind, myBeg, myLen, fb,
-                                                            heavy, mt);
+                        if (code <= kItemNew) {
+                            const int hub = -1 - code;
+                            if (hub >= 0 ? pathKind == 5 : pathKind != 5) {
+                                code = kItemEnum;
+                            } else if (pathKind == 1) {
+                                code = kItemHub + hub;   // the segment is a whole hub row
+                            } else {
+                                const int c = classify_item(P, ix, stp, it, lenK, pathKind, myBeg, myLen, fb, heavy,
+                                                            hub, mt);
                                 if (c == -4) myNew += 1;   // a new found bit of a split root
-                                if (c != -1) code = c >= 0 ? kItemHub + c : kItemDone;
+                                code = c == -1 ? kItemEnum : (c >= 0 ? kItemHub + c : kItemDone);
                             }
                             it[1] = code;
                         }
@@ -1122,8 +1165,6 @@ __device__ __forceinline__ void run_task(Smem<B>& sm, const DevIndex& ix, const 
             const bool lookTest = k + 2 < P.m && P.steps[k + 1].kind == kExpand && P.steps[k + 2].kind == kExpand &&
                                   P.steps[k + 2].keyRef == P.tupleLen[k + 1];
             const int lookBit = lookTest ? sig_bit(P.steps[k + 2].pred, P.steps[k + 2].dir) : 0;
-            const uint32_t* lookWords =
-                reinterpret_cast<const uint32_t*>(ix.sufSig[lookTest ? P.steps[k + 1].dir : 0]) + (lookBit >> 5);
 
             // One candidate: its parent item `lo`, edge `e`, new value(s)
             // n0/n1 and (when this step binds hO) the loaded rank.
@@ -1143,7 +1184,7 @@ __device__ __forceinline__ void run_task(Smem<B>& sm, const DevIndex& ix, const 
                     return ref == lenK ? n0 : n1;
                 };
                 if (hasFilters && !pass_filters(P, ix, k + 1, mt, valN)) return;
-                int rank = itemHasRank ? par[1] : kItemNew;
+                int rank = par[1];
                 if (pairs && stp.hoWhich) {
                     rank = rankLoaded;
                     if (!leaf && !sortMode) {
@@ -1166,12 +1207,10 @@ __device__ __forceinline__ void run_task(Smem<B>& sm, const DevIndex& ix, const 
                         myNew += (old & mask) ? 0ull : 1ull;
                     }
                 } else {
-                    const int2 seg = step_segment(P, ix, k + 1, mt, valN);
-                    if (seg.y <= seg.x) return;
-                    if (lookTest) {
-                        mt.add(4);
-                        if (!((__ldg(lookWords + 2 * (long long)seg.x) >> (lookBit & 31)) & 1u)) return;
-                    }
+                    const RowHit hit = step_row(P, ix, k + 1, mt, valN);
+                    if (hit.seg.y <= hit.seg.x) return;
+                    if (lookTest && !(((lookBit & 32 ? hit.sig.y : hit.sig.x) >> (lookBit & 31)) & 1u)) return;
+                    if (!itemHasRank && !(pairs && stp.hoWhich)) rank = item_state(P.steps[k + 1], hit.hub);
                     const int slot = atomicAdd(&S.count[k + 1], 1);
                     if (slot >= P.cap) {
                         if (wide) atomicMin(&S.firstFail, j);
@@ -1184,8 +1223,8 @@ __device__ __forceinline__ void run_task(Smem<B>& sm, const DevIndex& ix, const 
                     for (int q = kTupleHead; q < lenK; ++q) dst[q] = par[q];
                     dst[lenK] = n0;
                     if (stp.nNew == 2) dst[lenK + 1] = n1;
-                    dst[lenN] = seg.x;
-                    dst[lenN + 1] = seg.y - seg.x;
+                    dst[lenN] = hit.seg.x;
+                    dst[lenN + 1] = hit.seg.y - hit.seg.x;
                 }
             };
 
@@ -1289,8 +1328,7 @@ __device__ __forceinline__ void run_task(Smem<B>& sm, const DevIndex& ix, const 
                         // hO must differ from every bound value: their ranks in hO's domain
                         int* ex = S.exRank[warp];
                         if (lane < nEx) {
-                            const int2 r = row_lookup(ix, stp.pred, exDir, par[kTupleHead + lane], mt);
-                            ex[lane] = r.y > r.x ? __ldg(ix.srcRank[exDir] + r.x) : -1;
+                            ex[lane] = row_find(ix, stp.pred, exDir, par[kTupleHead + lane], mt).rank;
                         }
                         __syncwarp();
                         const int h = -2 - sm.wBeg[item];
@@ -1406,6 +1444,7 @@ engine_kernel(const __grid_constant__ DevIndex ix, const DevPlan* __restrict__ p
     if constexpr (kD) {
         if (threadIdx.x == 0) sm.st.deadline = global_ns() + prof.budgetNs;
     }
+    int loaded = -1;   // the plan in shared memory
     const bool follow = kS && sp.in >= 0;   // a follow-up launch: its tasks are a spill list
     if (follow) {
         nTasks = (int)(sp.ctl->used[sp.in] >> 32);
@@ -1446,10 +1485,13 @@ engine_kernel(const __grid_constant__ DevIndex ix, const DevPlan* __restrict__ p
                 t0 = global_ns();
             }
         }
-        const int* src = reinterpret_cast<const int*>(plans + task.plan);
-        int* dst = reinterpret_cast<int*>(&sm.plan);
-        for (int i = threadIdx.x; i < (int)(sizeof(DevPlan) / 4); i += B) dst[i] = src[i];
-        __syncthreads();
+        if (task.plan != loaded) {   // (a plan's tasks often follow one another)
+            loaded = task.plan;
+            const int* src = reinterpret_cast<const int*>(plans + task.plan);
+            int* dst = reinterpret_cast<int*>(&sm.plan);
+            for (int i = threadIdx.x; i < (int)(sizeof(DevPlan) / 4); i += B) dst[i] = src[i];
+            __syncthreads();
+        }
         run_task<B, kC, kD, kS>(sm, ix, task, results, status, mt, sp, st);
         __syncthreads();
         if constexpr (kD) {
@@ -1679,6 +1721,40 @@ cudaError_t support_rows(const DevIndex& ix, const DevPlan* plans, const SupJob*
     const int grid = nJobs + (sp.ctl ? spillBlocks : 0);
     if (grid <= 0) return cudaSuccess;
     support_rows_kernel<<<grid, 256, 0, stream>>>(ix, plans, jobs, nJobs, results, sp);
+    return cudaGetLastError();
+}
+
+__global__ void widen_slots_kernel(const __grid_constant__ DevIndex ix, const HashSlot* hash16, long long n,
+                                   DevSlot* slots) {
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const HashSlot s = hash16[i];
+    DevSlot d{s.tag, s.key, s.beg, s.end, {0u, 0u}, -1, -1};
+    if (s.tag != kEmptyTag) {
+        const int dir = (int)(s.tag & 1u), pred = (int)(s.tag >> 1);
+        const uint64_t sig = ix.sufSig[dir][s.beg];
+        d.sig[0] = (uint32_t)sig;
+        d.sig[1] = (uint32_t)(sig >> 32);
+        d.rank = ix.srcRank[dir][s.beg];
+        d.hub = ix.hubOf[dir][ix.predRow[dir][pred] + d.rank];
+    }
+    slots[i] = d;
+}
+
+__global__ void row_records_kernel(const __grid_constant__ DevIndex ix, int dir, int n, DevRow* rows) {
+    const int r = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+    if (r >= n) return;
+    const int beg = ix.rowBeg[dir][r];
+    const uint64_t sig = ix.sufSig[dir][beg];
+    rows[r] = DevRow{ix.rowKey[dir][r], beg, ix.rowBeg[dir][r + 1], ix.hubOf[dir][r],
+                     {(uint32_t)sig, (uint32_t)(sig >> 32)}, {0, 0}};
+}
+
+cudaError_t build_lookup(const DevIndex& ix, const HashSlot* hash16, long long n, DevSlot* slots, DevRow* const* rows,
+                         const int* nRows) {
+    if (n > 0) widen_slots_kernel<<<(unsigned)((n + 255) / 256), 256>>>(ix, hash16, n, slots);
+    for (int d = 0; d < 2; ++d)
+        if (nRows[d] > 0) row_records_kernel<<<(nRows[d] + 255) / 256, 256>>>(ix, d, nRows[d], rows[d]);
     return cudaGetLastError();
 }
 
