@@ -56,9 +56,41 @@ struct Meter {
     }
 };
 
+// What a round needs to know of its level, worked out once per task (one
+// thread per level) instead of by every thread in every round: in rounds of
+// a few dozen candidates that was a third of the instructions.
+enum LevelFlag : int {
+    kLvLeaf = 1,         // the step is the plan's last
+    kLvHo = 2,           // kPairs: the step binds hO (its values' ranks are read)
+    kLvHasRank = 4,      // kPairs: the level's items carry hO's rank
+    kLvFilters = 8,      // checks or used-triple tests follow the step
+    kLvSig = 16,         // the next step expands the value this one binds: its signature is tested
+    kLvLook = 32,        // a new item is stored only if its row has a value that can take the step after
+    kLvLookHigh = 64,    // ... whose signature bit is in the high word
+    kLvScan = 128, kLvSameVar = 256, kLvRowScan = 512,
+    kLvTwo = 1024,       // the step binds two values
+    kLvWide = 2048,      // rounds may overflow the next level (see `wide`)
+    kLvClaims = 4096,    // hub or memo items are claimed (see kHubSeen)
+    kLvPath = 13,        // shift of the path kind (0 none, 1 hub, 2 memo, 3 existence, 4 three-step, 5 scan)
+};
+struct alignas(16) Level {
+    const int* vals;             // the step's values, by edge (or row)
+    const int* ranks;            // their ranks in hO's domain (kLvHo)
+    const uint32_t* sigs;        // their signature words (every second word; kLvSig)
+    int flags;
+    int len;                     // tuple length of the level's items
+    int at, nextAt;              // pool offsets of this level's and the next level's items
+    int nextLen;
+    int sigShift, lookShift;     // bits of the two signature tests
+    int rankBase;                // row scans: the predicate's first row
+    int maxTake;                 // candidates of a round
+    int pad[3];
+};
+
 template <int B>
 struct BlockState {
     static constexpr int kWarps = B / 32;
+    Level lv[kMaxBody];
     int task;
     int stop;                       // the block's deadline passed: abandon the task
     unsigned long long deadline;    // global-timer ns (0: none)
@@ -206,32 +238,37 @@ struct Smem;
 // every warp its total (warpSum), so item i's block-wide prefix is the
 // totals of the warps before i's warp plus wLoc[i] (WinCursor reads it
 // that way).  The barrier also ORs `flag` over the block.
+// Warps without any of the window's nw items only take the barrier.
 template <int B>
-__device__ __forceinline__ bool publish_window(int x, bool flag, Smem<B>& sm) {
+__device__ __forceinline__ bool publish_window(int x, bool flag, Smem<B>& sm, int nw) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (warp * 32 < nw) {
 #pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-        const int y = __shfl_up_sync(0xffffffffu, x, d);
-        if (lane >= d) x += y;
+        for (int d = 1; d < 32; d <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, x, d);
+            if (lane >= d) x += y;
+        }
+        sm.wLoc[threadIdx.x] = x;
+        if (lane == 31) sm.st.warpSum[warp] = x;
     }
-    sm.wLoc[threadIdx.x] = x;
-    if (lane == 31) sm.st.warpSum[warp] = x;
     return __syncthreads_or(flag) != 0;
 }
 
 // The window's candidate total: the warps' totals summed by shuffles.
 // (Up to 256 threads the eight totals are added directly; the two forms
-// differ only in the registers the kernel needs around them.)
+// differ only in the registers the kernel needs around them.)  Only warps
+// with items among the window's nw have published theirs.
 template <int B>
-__device__ __forceinline__ int window_total(const Smem<B>& sm) {
+__device__ __forceinline__ int window_total(const Smem<B>& sm, int nw) {
     if constexpr (B <= 256) {
         int v = 0;
 #pragma unroll
-        for (int w = 0; w < B / 32; ++w) v += sm.st.warpSum[w];
+        for (int w = 0; w < B / 32; ++w)
+            if (w * 32 < nw) v += sm.st.warpSum[w];
         return v;
     } else {
         const int lane = threadIdx.x & 31;
-        int v = lane < B / 32 ? sm.st.warpSum[lane] : 0;
+        int v = lane * 32 < nw ? sm.st.warpSum[lane] : 0;
 #pragma unroll
         for (int d = 16; d; d >>= 1) v += __shfl_xor_sync(0xffffffffu, v, d);
         return v;
@@ -846,6 +883,72 @@ __device__ __noinline__ bool spill_items(Smem<B>& sm, const DevTask& task, const
     return true;
 }
 
+// Fills the record of level l (one thread).
+template <int B>
+__device__ __noinline__ void level_info(Smem<B>& sm, const DevIndex& ix, int l, bool pairs, bool sortMode, bool sliced,
+                                        bool claims, int leafChunk, int wideChunk) {
+    const DevPlan& P = sm.plan;
+    Level& L = sm.st.lv[l];
+    const DevStep& st = P.steps[l];
+    const bool leaf = l + 1 == P.m;
+    const int len = P.tupleLen[l];
+    int at = 0;
+    for (int q = 0; q < l; ++q) at += P.cap * (P.tupleLen[q] + 2);
+    L.len = len;
+    L.at = at;
+    L.nextAt = at + P.cap * (len + 2);
+    L.nextLen = leaf ? 0 : P.tupleLen[l + 1];
+    const bool filters = (P.chkN[l + 1] | P.usedN[l + 1]) != 0;
+    int f = (leaf ? kLvLeaf : 0) | (pairs && st.hoWhich ? kLvHo : 0) |
+            (pairs && P.hoLevel >= 1 && l >= P.hoLevel ? kLvHasRank : 0) | (filters ? kLvFilters : 0) |
+            (st.kind == kScan ? kLvScan : 0) | (st.sameVar ? kLvSameVar : 0) | (st.kind == kRowScan ? kLvRowScan : 0) |
+            (st.nNew == 2 ? kLvTwo : 0) | (claims && l == P.claimLevel ? kLvClaims : 0);
+    L.vals = st.kind == kExpand ? ix.val[st.dir] : (st.kind == kRowScan ? ix.rowKey[st.dir] : ix.src[0]);
+    L.ranks = st.kind == kExpand ? ix.valRank[st.dir] : (st.hoWhich == 1 ? ix.srcRank[0] : ix.valRank[0]);
+    L.rankBase = st.kind == kRowScan ? ix.predRow[st.dir][st.pred] : 0;
+    // When the next step expands from the value this step binds, that value's
+    // row signature (stored beside it) drops most candidates whose next row
+    // is absent before any lookup.
+    L.sigs = nullptr;
+    L.sigShift = 0;
+    if (!leaf && st.kind == kExpand && P.steps[l + 1].kind == kExpand && P.steps[l + 1].keyRef == len) {
+        const int bit = sig_bit(P.steps[l + 1].pred, P.steps[l + 1].dir);
+        L.sigs = reinterpret_cast<const uint32_t*>(ix.valSig[st.dir]) + (bit >> 5);
+        L.sigShift = bit & 31;
+        f |= kLvSig | (sortMode ? 0 : kLvWide);
+    }
+    // A new item of the next level whose segment holds no value with a row
+    // under the step after it (keyed on that value) is not stored.
+    L.lookShift = 0;
+    if (l + 2 < P.m && P.steps[l + 1].kind == kExpand && P.steps[l + 2].kind == kExpand &&
+        P.steps[l + 2].keyRef == P.tupleLen[l + 1]) {
+        const int bit = sig_bit(P.steps[l + 2].pred, P.steps[l + 2].dir);
+        L.lookShift = bit & 31;
+        f |= kLvLook | (bit & 32 ? kLvLookHigh : 0);
+    }
+    L.maxTake = leaf ? leafChunk : ((f & kLvWide) ? wideChunk : P.cap);
+    // Hub path: when the leaf binds hO and tests nothing but injectivity, an
+    // item whose segment is a whole hub row is counted by OR-ing the row's
+    // rank bitmap into its pair row (32 candidates per word) instead of
+    // candidate by candidate.
+    // Memo path: the plan ends in two expand steps x -> y -> hO with nothing
+    // but injectivity to test; an item whose first segment is a hub row with
+    // a suffix memo is counted from the memo's maps (see memo_item).  A
+    // four-step plan may also have the three-step memo, at level 1.
+    // Scan path: the plan ends in a row scan binding hO and the free value
+    // behind it; the rows are counted from their scan memo.
+    int path = 0;
+    const bool whole = !(sliced && l == 0);   // (a slice is never a whole row)
+    if (pairs && !sortMode) {
+        if (leaf) {
+            if (st.hoWhich != 0 && st.kind == kExpand && st.nNew == 1 && !filters && ix.nHub > 0 && whole) path = 1;
+        } else if (P.memoTab != nullptr && l + 1 == P.memoLevel) path = 2;
+        else if (P.memo3Tab != nullptr && l == 1) path = 4;
+        else if (P.scanBits != nullptr && l + 1 == P.scanLevel && whole) path = 5;
+    } else if (!pairs && leaf && P.memoTab != nullptr && l + 1 == P.memoLevel && whole) path = 3;
+    L.flags = f | path << kLvPath;
+}
+
 // kS: the task may be spilled; st: the spill task to resume (`task` its
 // roots), or null.
 template <int B, bool kC, bool kD, bool kS>
@@ -862,9 +965,6 @@ __device__ __forceinline__ void run_task(Smem<B>& sm, const DevIndex& ix, const 
     // always has candidates left for the next window.
     constexpr int kMaxSeg = 1 << 21;
     static_assert(kLeafChunk < kMaxSeg && (long long)B * kMaxSeg <= 1 << 30, "window sums fit an int");
-    // candidates per thread per group (1, 2 and 4 measured on c3: 44.96,
-    // 45.22 and 46.92 ms per launch; 8 makes compilation impractical)
-    constexpr int kU = 1;
     const DevPlan& P = sm.plan;
     BlockState<B>& S = sm.st;
     const int tid = threadIdx.x;
@@ -930,6 +1030,7 @@ __device__ __forceinline__ void run_task(Smem<B>& sm, const DevIndex& ix, const 
             else if (P.m == 0 && l == 0) off += P.cap * P.tupleLen[0];
         }
     }
+    if (tid >= 32 && tid - 32 < P.m) level_info<B>(sm, ix, tid - 32, pairs, sortMode, sliced, claims, kLeafChunk, kWideChunk);
     __syncthreads();
 
     const int kBase = resumed ? st->level : 0;   // the search ends when this level is exhausted
@@ -1052,45 +1153,24 @@ __device__ __forceinline__ void run_task(Smem<B>& sm, const DevIndex& ix, const 
                 continue;
             }
             const int nw = min(B, cnt - w0);
-            const int lenK = P.tupleLen[k];
+            const Level lv = S.lv[k];   // uniform for the round: kept in registers
+            const int lenK = lv.len;
             const int strideK = lenK + 2;
-            const int* baseK = items + S.levelOff[k];
-            const DevStep stp = P.steps[k];   // uniform for the round: keep it in registers
-            const bool leaf = (k + 1 == P.m);
-            const bool hasFilters = (P.chkN[k + 1] | P.usedN[k + 1]) != 0;
-            const bool itemHasRank = pairs && P.hoLevel >= 1 && k >= P.hoLevel;
-            // Hub path: when the leaf binds hO and tests nothing but
-            // injectivity, an item whose segment is a whole hub row is
-            // counted by OR-ing the row's rank bitmap into its pair row (32
-            // candidates per word) instead of candidate by candidate.
-            const bool hubPath = leaf && pairs && !sortMode && stp.hoWhich != 0 && stp.kind == kExpand &&
-                                 stp.nNew == 1 && !hasFilters && ix.nHub > 0 && !(sliced && k == 0);
-            // Memo path: the plan ends in two expand steps x -> y -> hO with
-            // nothing but injectivity to test; an item whose first segment
-            // is a hub row with a suffix memo is counted from the memo's
-            // "one witness y" / "two witnesses y" bitmaps (see below).
-            // A four-step plan may also have the three-step memo, at level 1.
-            const bool memo3Path = !leaf && pairs && !sortMode && P.memo3Tab != nullptr && k == 1;
-            const bool memoPath = !leaf && pairs && !sortMode && P.memoTab != nullptr && k + 1 == P.memoLevel;
-            const bool existMemo = leaf && !pairs && P.memoTab != nullptr && k + 1 == P.memoLevel &&
-                                   !(sliced && k == 0);
-            // Scan path: the plan ends in a row scan binding hO and the free
-            // value behind it; the rows are counted from their scan memo.
-            const bool scanPath = !leaf && pairs && !sortMode && P.scanBits != nullptr && k + 1 == P.scanLevel &&
-                                  !(sliced && k == 0);
-            const int pathKind = hubPath ? 1 : (memoPath ? 2 : (existMemo ? 3 : (memo3Path ? 4 : (scanPath ? 5 : 0))));
+            int* const baseK = items + lv.at;
+            const bool leaf = (lv.flags & kLvLeaf) != 0;
+            const int pathKind = lv.flags >> kLvPath;
             bool isHub = false;   // item marked for the hub or memo pass
 
             // window: the stored neighbour segment of each item
             int myBeg = 0;
             int myLen = 0;
             if (tid < nw) {
-                int* it = items + S.levelOff[k] + (w0 + tid) * strideK;
+                int* it = baseK + (w0 + tid) * strideK;
                 bool pruned = false;
                 if (!pairs) {
                     pruned = (fb[it[0] >> 5] >> (it[0] & 31)) & 1u;
                     if (heavy) mt.add(4);
-                } else if (itemHasRank && !sortMode) {
+                } else if ((lv.flags & kLvHasRank) && !sortMode) {
                     pruned = (bm[(long long)it[0] * P.rowWords + (it[1] >> 5)] >> (it[1] & 31)) & 1u;
                     if (!shared) mt.add(4);
                 }
@@ -1112,7 +1192,7 @@ __device__ __forceinline__ void run_task(Smem<B>& sm, const DevIndex& ix, const 
                             } else if (pathKind == 1) {
                                 code = kItemHub + hub;   // the segment is a whole hub row
                             } else {
-                                const int c = classify_item(P, ix, stp, it, lenK, pathKind, myBeg, myLen, fb, heavy,
+                                const int c = classify_item(P, ix, P.steps[k], it, lenK, pathKind, myBeg, myLen, fb, heavy,
                                                             hub, mt);
                                 if (c == -4) myNew += 1;   // a new found bit of a split root
                                 code = c == -1 ? kItemEnum : (c >= 0 ? kItemHub + c : kItemDone);
@@ -1134,16 +1214,13 @@ __device__ __forceinline__ void run_task(Smem<B>& sm, const DevIndex& ix, const 
                     myLen = min(myLen, kMaxSeg);
                 }
             }
-            sm.wBeg[tid] = myBeg;
-            sm.wLen[tid] = myLen;
+            if (tid < ((nw + 31) & ~31)) {
+                sm.wBeg[tid] = myBeg;
+                sm.wLen[tid] = myLen;
+            }
             if (tid == 0 && !leaf) S.count[k + 1] = 0;
-            const bool anyHub = publish_window<B>(myLen, isHub, sm) && (hubPath || memoPath || memo3Path || scanPath);
-            const int total = window_total<B>(sm);
-            // When the next step expands from the value this step binds,
-            // that value's row signature (stored beside it) drops most
-            // candidates whose next row is absent before any lookup.
-            const bool sigTest = !leaf && stp.kind == kExpand && P.steps[k + 1].kind == kExpand &&
-                                 P.steps[k + 1].keyRef == lenK;
+            const bool anyHub = publish_window<B>(myLen, isHub, sm, nw);
+            const int total = window_total<B>(sm, nw);
             // Wide round: up to kWideChunk candidates although each survivor
             // takes a slot of the next level.  A survivor that finds it full
             // records its candidate index, and the level resumes from the
@@ -1154,38 +1231,29 @@ __device__ __forceinline__ void run_task(Smem<B>& sm, const DevIndex& ix, const 
             // exhausted, so the search always advances.  Sort mode keeps
             // capacity-sized rounds: its key count must not depend on how
             // the threads raced (a launch is staged again with that count).
-            const bool wide = sigTest && !sortMode && !((S.safeLevels >> k) & 1u);
-            const int take = min(total, leaf ? kLeafChunk : (wide ? kWideChunk : P.cap));
-            const int lenN = leaf ? 0 : P.tupleLen[k + 1];
-            const int strideN = lenN + 2;
-            int* baseN = leaf ? nullptr : items + S.levelOff[k + 1];
-
-            // A new item of level k + 1 whose segment holds no value with a
-            // row under step k + 2 (keyed on that value) is not stored.
-            const bool lookTest = k + 2 < P.m && P.steps[k + 1].kind == kExpand && P.steps[k + 2].kind == kExpand &&
-                                  P.steps[k + 2].keyRef == P.tupleLen[k + 1];
-            const int lookBit = lookTest ? sig_bit(P.steps[k + 2].pred, P.steps[k + 2].dir) : 0;
+            const bool wide = (lv.flags & kLvWide) && !((S.safeLevels >> k) & 1u);
+            const int take = min(total, (lv.flags & kLvWide) && !wide ? P.cap : lv.maxTake);
 
             // One candidate: its parent item `lo`, edge `e`, new value(s)
             // n0/n1 and (when this step binds hO) the loaded rank.
-            auto eval = [&](int lo, int e, int n0, int n1, int rankLoaded, int j) {
+            auto eval = [&](int lo, int n0, int n1, int rankLoaded, int j) {
                 const int* par = baseK + (w0 + lo) * strideK;
                 const int root = par[0];
                 if (!pairs && ((fb[root >> 5] >> (root & 31)) & 1u)) return;
-                if (stp.kind == kScan && (stp.sameVar ? (n0 != n1) : (n0 == n1))) return;
+                if ((lv.flags & kLvScan) && ((lv.flags & kLvSameVar) ? (n0 != n1) : (n0 == n1))) return;
                 if (n0 != kAnyValue)
                     for (int q = kTupleHead; q < lenK; ++q) {
                         const int x = par[q];
-                        if (x == n0 || (stp.nNew == 2 && x == n1)) return;
+                        if (x == n0 || ((lv.flags & kLvTwo) && x == n1)) return;
                     }
                 auto valN = [&](TermRef ref) -> int {
                     if (ref < 0) return P.consts[-1 - ref];
                     if (ref < lenK) return par[ref];
                     return ref == lenK ? n0 : n1;
                 };
-                if (hasFilters && !pass_filters(P, ix, k + 1, mt, valN)) return;
+                if ((lv.flags & kLvFilters) && !pass_filters(P, ix, k + 1, mt, valN)) return;
                 int rank = par[1];
-                if (pairs && stp.hoWhich) {
+                if (lv.flags & kLvHo) {
                     rank = rankLoaded;
                     if (!leaf && !sortMode) {
                         if (!shared) mt.add(4);
@@ -1209,68 +1277,47 @@ __device__ __forceinline__ void run_task(Smem<B>& sm, const DevIndex& ix, const 
                 } else {
                     const RowHit hit = step_row(P, ix, k + 1, mt, valN);
                     if (hit.seg.y <= hit.seg.x) return;
-                    if (lookTest && !(((lookBit & 32 ? hit.sig.y : hit.sig.x) >> (lookBit & 31)) & 1u)) return;
-                    if (!itemHasRank && !(pairs && stp.hoWhich)) rank = item_state(P.steps[k + 1], hit.hub);
+                    if ((lv.flags & kLvLook) &&
+                        !((((lv.flags & kLvLookHigh) ? hit.sig.y : hit.sig.x) >> lv.lookShift) & 1u))
+                        return;
+                    if (!(lv.flags & (kLvHasRank | kLvHo))) rank = item_state(P.steps[k + 1], hit.hub);
                     const int slot = atomicAdd(&S.count[k + 1], 1);
                     if (slot >= P.cap) {
                         if (wide) atomicMin(&S.firstFail, j);
                         else atomicOr(status, 8);   // a capacity-sized round cannot fill the level
                         return;
                     }
-                    int* dst = baseN + slot * strideN;
+                    const int lenN = lv.nextLen;
+                    int* dst = items + lv.nextAt + slot * (lenN + 2);
                     dst[0] = root;
                     dst[1] = rank;
                     for (int q = kTupleHead; q < lenK; ++q) dst[q] = par[q];
                     dst[lenK] = n0;
-                    if (stp.nNew == 2) dst[lenK + 1] = n1;
+                    if (lv.flags & kLvTwo) dst[lenK + 1] = n1;
                     dst[lenN] = hit.seg.x;
                     dst[lenN + 1] = hit.seg.y - hit.seg.x;
                 }
             };
 
-            // Candidates j = tid, tid + B, ... in groups of kU per thread: all
-            // group members are located first, then their loads are issued
-            // together, then they are evaluated.
-            const int* vbase = stp.kind == kExpand ? ix.val[stp.dir]
-                                                   : (stp.kind == kRowScan ? ix.rowKey[stp.dir] : ix.src[0]);
-            const int* rbase = stp.kind == kExpand ? ix.valRank[stp.dir]
-                                                   : (stp.hoWhich == 1 ? ix.srcRank[0] : ix.valRank[0]);
-            const bool wantRank = pairs && stp.hoWhich;
-            const int sigBit = sig_bit(P.steps[k + 1 < P.m ? k + 1 : k].pred, P.steps[k + 1 < P.m ? k + 1 : k].dir);
-            const uint32_t* sigWords = reinterpret_cast<const uint32_t*>(ix.valSig[stp.dir]) + (sigBit >> 5);
-            WinCursor<B> cur;
-            for (int jb = tid; jb < take; jb += B * kU) {
-                int lo_[kU], e_[kU], n0_[kU], n1_[kU], rk_[kU];
-                uint32_t sw_[kU];
-#pragma unroll
-                for (int u = 0; u < kU; ++u) {
-                    const int j = jb + u * B;
-                    lo_[u] = -1;
-                    e_[u] = 0;
-                    if (j < take) {
-                        cur.seek(sm, nw, j);
-                        lo_[u] = cur.item;
-                        e_[u] = sm.wBeg[cur.item] + (j - cur.first(sm));
-                    }
-                }
-#pragma unroll
-                for (int u = 0; u < kU; ++u) {
-                    n0_[u] = n1_[u] = rk_[u] = 0;
-                    sw_[u] = ~0u;
-                    if (lo_[u] < 0) continue;
-                    if (sigTest) { sw_[u] = __ldg(sigWords + 2 * (long long)e_[u]); mt.add(4); }
-                    n0_[u] = __ldg(vbase + e_[u]);
-                    if (stp.kind == kScan) { n1_[u] = __ldg(ix.val[0] + e_[u]); mt.add(8); } else mt.add(4);
-                    if (wantRank) {   // a row scan's rank is the row's place among the predicate's
-                        rk_[u] = stp.kind == kRowScan ? e_[u] - __ldg(ix.predRow[stp.dir] + stp.pred)
-                                                      : __ldg(rbase + e_[u]);
+            // Candidates j = tid, tid + B, ... one at a time (groups of 2 and 4
+            // with their loads issued together measured slower)
+            {
+                WinCursor<B> cur;
+                for (int j = tid; j < take; j += B) {
+                    cur.seek(sm, nw, j);
+                    const int lo = cur.item;
+                    const int e = sm.wBeg[lo] + (j - cur.first(sm));
+                    uint32_t sw = ~0u;
+                    int n1 = 0, rk = 0;
+                    if (lv.flags & kLvSig) { sw = __ldg(lv.sigs + 2 * (long long)e); mt.add(4); }
+                    const int n0 = __ldg(lv.vals + e);
+                    if (lv.flags & kLvScan) { n1 = __ldg(ix.val[0] + e); mt.add(8); } else mt.add(4);
+                    if (lv.flags & kLvHo) {   // a row scan's rank is the row's place among the predicate's
+                        rk = (lv.flags & kLvRowScan) ? e - lv.rankBase : __ldg(lv.ranks + e);
                         mt.add(4);
                     }
+                    if ((sw >> lv.sigShift) & 1u) eval(lo, n0, n1, rk, j);
                 }
-#pragma unroll
-                for (int u = 0; u < kU; ++u)
-                    if (lo_[u] >= 0 && ((sw_[u] >> (sigBit & 31)) & 1u))
-                        eval(lo_[u], e_[u], n0_[u], n1_[u], rk_[u], jb + u * B);
             }
             // where the next round at this level starts: the item holding
             // candidate `take` (items before it are consumed), and how much
@@ -1279,17 +1326,17 @@ __device__ __forceinline__ void run_task(Smem<B>& sm, const DevIndex& ix, const 
             int cut = nw;
             int cutOff = 0;
             {
-                if (take < window_total<B>(sm)) {
+                if (take < total) {
                     WinCursor<B> c;
                     c.seek(sm, nw, take);
                     cut = c.item;
                     cutOff = take - c.first(sm) + (c.item == 0 ? off : 0);
                 }
             }
-            if (anyHub && claims && k == P.claimLevel) {
+            if (anyHub && (lv.flags & kLvClaims)) {
                 // items of a (root, hub row) after enough middle values add nothing
                 hub_claims(P.hubSeen + (long long)blockIdx.x * kHubSeen, baseK + w0 * strideK, strideK, cut,
-                           stp.keyRef == kTupleHead + 1 ? kTupleHead + 2 : kTupleHead + 1, sm.wBeg, B,
+                           P.steps[k].keyRef == kTupleHead + 1 ? kTupleHead + 2 : kTupleHead + 1, sm.wBeg, B,
                            leaf ? 2u : 3u);
                 __syncthreads();
             }
@@ -1297,6 +1344,7 @@ __device__ __forceinline__ void run_task(Smem<B>& sm, const DevIndex& ix, const 
                 // hub items of the consumed part of the window: [0, cut)
                 const int lane = tid & 31, warp = tid >> 5;
                 constexpr int kWarps = B / 32;
+                const DevStep stp = P.steps[k];
                 const int words = P.rowWords;
                 // memo items and domains up to 1,024 words: one warp per item
                 // (a round's hub items in parallel); larger rows: the whole
@@ -1316,13 +1364,13 @@ __device__ __forceinline__ void run_task(Smem<B>& sm, const DevIndex& ix, const 
                         const int* par = baseK + (w0 + item) * strideK;
                         if (!leaf) {
                             const int slot = -2 - sm.wBeg[item];
-                            const int nEx3 = memo3Path
+                            const int nEx3 = pathKind == 4
                                 ? memo3_exceptions(P, ix, par, lenK, slot, words, S.exRank[warp], lane, mt) : 0;
                             DevStep stB = P.steps[k + 1];
-                            if (scanPath) stB.dir = (int8_t)(1 - stB.dir);
+                            if (pathKind == 5) stB.dir = (int8_t)(1 - stB.dir);
                             myNew += memo_item(P, ix, stp, stB, par, lenK, slot,
                                                bm + (long long)par[0] * words, words, S.exRank[warp],
-                                               lane, mt, shared, nEx3, scanPath);
+                                               lane, mt, shared, nEx3, pathKind == 5);
                             continue;
                         }
                         // hO must differ from every bound value: their ranks in hO's domain
