@@ -152,7 +152,7 @@ struct DevPlan {
     int32_t bitmapOff;       // where the dedup bitmap starts in the block's shared pool (ints)
     int32_t hoLevel;         // kPairs: level whose step binds hO (1..m)
     int32_t cap;             // frontier capacity per level (items)
-    int32_t groupMax;        // max roots per task
+    int32_t groupMax;        // roots a block takes at once (a task may hold several such groups)
     int32_t tupleLen[kMaxBody + 1];
     int32_t consts[kMaxConsts];
     DevStep steps[kMaxBody];
@@ -246,7 +246,8 @@ enum DedupMode : int32_t {
     kDedupSort = 3,       // 64-bit pair keys appended, radix-sorted and counted once each
 };
 
-// A unit of device work: the roots [beg, end) of one plan.  A heavy root is
+// A unit of device work: the roots [beg, end) of one plan, in groups of at
+// most the plan's groupMax.  A heavy root is
 // split over several tasks (gRow >= 0, end == beg + 1): each takes the slice
 // [sub0, sub1) of the root's first neighbour segment and deduplicates into
 // the plan's global row gRow, so the slices together count each pair (or
@@ -263,7 +264,7 @@ struct DevTask {
 // as records (tuple, segment) that a follow-up launch spreads over the GPU.
 // A spill task is a run of records of one task and level; its dedup rows (the
 // task's own, copied from shared memory, or its global ones) are shared by
-// all of them.
+// all of them.  Roots that the block had not begun go as tasks of level -1.
 struct SpillTask {
     int32_t plan, level;
     int32_t recBeg, recN;
@@ -271,8 +272,8 @@ struct SpillTask {
     uint32_t* rows;            // row of the first root (kExist: the found bits)
 };
 constexpr int kSpillRecInts = kMaxTuple + 2;   // tuple, first edge, edges
-constexpr int kSpillTasks = 8192;              // capacities of one list
-constexpr int kSpillRecs = 65536;
+constexpr int kSpillTasks = 1 << 14;           // capacities of one list
+constexpr int kSpillRecs = 1 << 17;
 constexpr int kSpillSups = 2048;
 constexpr long long kSpillRowWords = 1 << 21;  // rows copied out of shared memory (8 MiB a launch)
 
@@ -282,11 +283,13 @@ struct SpillSup {
     const uint32_t* rows;
 };
 
-// Counters of one launch's spilling (all zero before it).
+// Counters of one launch's spilling (all zero before it).  Follow-up k runs
+// list k, which lies in buffer k & 1, and may fill list k + 1.
+constexpr int kFollowUps = 4;
 struct SpillCtl {
-    unsigned long long used[2];   // per list: tasks << 32 | records
+    unsigned long long used[kFollowUps];   // per list: tasks << 32 | records
     unsigned long long rowWords;
-    int32_t next[2];              // task counters of the follow-up launches
+    int32_t next[kFollowUps];              // task counters of the follow-up launches
     int32_t sups;
     int32_t pad;
 };

@@ -243,7 +243,7 @@ void Staged::stage(Context& c, std::vector<DevPlan>& plans, const std::vector<co
     hostSect[1] += host_ms() - tSect;
     tSect = host_ms();
     std::vector<PhaseTasks> pts;
-    c.tasks->build(phases, c.grid, true, pts, walkBudget, costAware, &lim);
+    c.tasks->build(phases, c.grid, true, pts, walkBudget, costAware, &lim, true);
     hostSect[2] += host_ms() - tSect;
     tSect = host_ms();
     // split heavy roots of plans with fused support: counted after the launch
@@ -297,6 +297,7 @@ void Staged::stage(Context& c, std::vector<DevPlan>& plans, const std::vector<co
             }
         }
         plans[i].resultSlot = i;
+        plans[i].groupMax = pts[i].group;
         const int dm = dedup[i];
         uint32_t* gb = static_cast<uint32_t*>(dBitmap.p);
         plans[i].gBitmap = dm == kDedupRows ? gb + gOff[i] : (dm == kDedupBlockRows ? gb + regionOff : nullptr);
@@ -508,11 +509,19 @@ void Context::ensure_memos(const std::vector<std::array<int, 6>>& keys, cudaStre
     }
     if (take.empty()) return;
     const size_t tabTotal = tabBytes * take.size();
-    memoChunks.emplace_back(new DevBuf());
-    DevBuf& chunk = *memoChunks.back();
-    ck(cudaMalloc(&chunk.p, tabTotal + bitTotal), "cudaMalloc(memos)");   // exact: never resized
-    chunk.cap = tabTotal + bitTotal;
-    char* base = static_cast<char*>(chunk.p);
+    // from the last arena, or a new one: cudaMalloc waits for every stream,
+    // which a served request's first memo would pay for
+    const size_t need = (tabTotal + bitTotal + 255) & ~size_t(255);
+    if (memoChunks.empty() || memoUsed + need > memoChunks.back()->cap) {
+        auto chunk = std::make_unique<DevBuf>();
+        const size_t cap = std::max(need, kMemoArenaBytes);
+        ck(cudaMalloc(&chunk->p, cap), "cudaMalloc(memos)");   // never resized
+        chunk->cap = cap;
+        memoChunks.push_back(std::move(chunk));
+        memoUsed = 0;
+    }
+    char* base = static_cast<char*>(memoChunks.back()->p) + memoUsed;
+    memoUsed += need;
     std::vector<int32_t> tabs(tabTotal / 4, -1);
     std::vector<MemoJob> all;
     for (size_t t = 0; t < take.size(); ++t) {

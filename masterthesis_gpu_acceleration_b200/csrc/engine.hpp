@@ -158,12 +158,10 @@ struct Staged {
     DevBuf dSpill;                         // spill lists, rows and support jobs (see spill_args)
     // Where the control words of one launch lie in dCtl (kCtlBytes, cleared
     // before it): counters, status and per-plan words first, then spilling's.
-    static constexpr size_t kSpillCtlAt = 64, kCtlBytes = 128;
+    static constexpr size_t kSpillCtlAt = 64, kCtlBytes = 192;
     static_assert(kSpillCtlAt + sizeof(SpillCtl) <= kCtlBytes, "control words");
     bool spillable = false;                // launches of this staging may spill
     bool spillAlways = false;
-    // Follow-up launches after a launch that may spill (a list each).
-    static constexpr int kFollowUps = 2;
     SpillArgs spill_args() const;
     void enqueue_follow_ups(Context& c, cudaStream_t s, unsigned long long* results, int* status,
                             unsigned long long* span);
@@ -276,6 +274,7 @@ struct Staged {
 // of (p1, d1) worth it, the S1, S2 and S3 bitmaps over (p2, 1 - d2)'s rows (see
 // memo_item in kernels.cu).  Built once per context, never moved.
 constexpr size_t kMemoBudgetBytes = size_t(1) << 30;   // all suffix memos of a context
+constexpr size_t kMemoArenaBytes = size_t(32) << 20;
 
 struct SuffixMemo {   // its table and bits live in one of Context::memoChunks
     const int32_t* tab = nullptr;
@@ -312,7 +311,8 @@ struct Context {
     bool hubClaims = true;     // repeated leaf hub items of a root are skipped (see kHubSeen)
     bool hostProfile = false;  // one-shot batches print their host-side times
     std::unordered_map<uint64_t, std::unique_ptr<SuffixMemo>> memos;
-    std::vector<std::unique_ptr<DevBuf>> memoChunks;   // one allocation per ensure_memos call
+    std::vector<std::unique_ptr<DevBuf>> memoChunks;   // arenas the memos are taken from
+    size_t memoUsed = 0;                               // bytes taken of the last one
     size_t memoBytes = 0;
     // Builds the memos in `keys` that do not exist yet, {p1, d1, p2, d2, p3,
     // d3}: the transitions (p1, d1) -> (p2, d2), or with p3 >= 0 the

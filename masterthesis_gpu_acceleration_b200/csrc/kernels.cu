@@ -104,8 +104,8 @@ struct BlockState {
     unsigned long long red[kWarps];
     int exRank[kWarps][kMaxVars];   // per warp: hO-domain ranks of the bound values of a hub item
     int spill;                      // 1: the block gives its open items away
-    long long lookAt;               // thread 0: the clock at its last look at the queue,
-    int looks;                      // and the looks in a row that found idle blocks
+    long long lookAt;               // thread 0: the clock at its last look at the queue
+    int idle;                       // blocks that were past the queue's end when the group began
     int base;                       // the level the task's search starts at
     int nTasks;                     // of the launch, and its counter
     const int* queue;
@@ -532,6 +532,7 @@ __device__ __noinline__ unsigned long long memo_item(const DevPlan& P, const Dev
             mt.add(4);
             if (hit[0] & hit[1]) { m &= ~(hit[0] & hit[1] & ~__ldg(S2 + words + w)); mt.add(4); }
         }
+        if (m && !sharedDst) m &= ~__ldcg(dst + w);
         if (m) {
             const uint32_t old = atomicOr(dst + w, m);
             if (!sharedDst) mt.add(8);
@@ -728,6 +729,38 @@ __device__ __noinline__ unsigned long long fused_support(const DevPlan& P, const
     return n;
 }
 
+// Takes nTask task and nRec record slots of a list (one thread); false when
+// it is full.  `at` gets the first slots, tasks << 32 | records.
+__device__ __forceinline__ bool spill_take(unsigned long long* used, unsigned nTask, unsigned nRec,
+                                           unsigned long long& at) {
+    at = *reinterpret_cast<volatile unsigned long long*>(used);
+    for (;;) {
+        const unsigned t0 = (unsigned)(at >> 32), r0 = (unsigned)at;
+        if (t0 + nTask > (unsigned)kSpillTasks || r0 + nRec > (unsigned)kSpillRecs) return false;
+        const unsigned long long seen = atomicCAS(used, at, (unsigned long long)(t0 + nTask) << 32 | (r0 + nRec));
+        if (seen == at) return true;
+        at = seen;
+    }
+}
+
+// Gives the roots [beg, end) of a task away, a task per group; false when the
+// list is full.  The whole block calls this between two groups.
+template <int B>
+__device__ __noinline__ bool spill_groups(Smem<B>& sm, const SpillArgs& sp, int plan, int beg, int end) {
+    BlockState<B>& S = sm.st;
+    const int g = max(1, sm.plan.groupMax);
+    if (threadIdx.x == 0) {
+        unsigned long long at = 0;
+        S.spill = spill_take(&sp.ctl->used[sp.out], (unsigned)((end - beg + g - 1) / g), 0u, at) ? 1 : 0;
+        S.spillAt = (int)(at >> 32);
+    }
+    __syncthreads();
+    if (!S.spill) return false;
+    for (int b = beg + (int)threadIdx.x * g, j = S.spillAt + (int)threadIdx.x; b < end; b += B * g, j += B)
+        sp.tasks[sp.out & 1][j] = SpillTask{plan, -1, 0, 0, b, min(g, end - b), nullptr};
+    return true;
+}
+
 // What an item's rank slot holds before hO is bound: not looked at yet, with
 // hub index h (-1 - h) or with a scanned range (kItemNew); enumerated as
 // usual; nothing left to do; or kItemHub + the hub index (leaf items) or memo
@@ -737,11 +770,12 @@ __device__ __forceinline__ int item_state(const DevStep& next, int hub) {
     return next.kind != kExpand ? kItemNew : (hub >= 0 ? -1 - hub : kItemEnum);
 }
 
-// Clock cycles (about 8 us) between a block's looks at the task queue, and how
-// many looks in a row must find idle blocks before it spills (a follow-up
-// launch costs a few us; a round of memo items can take hundreds).
-constexpr long long kSpillEvery = 16000;
-constexpr int kSpillLooks = 2;
+// Clock cycles (about 32 us) between a block's looks at the task queue during
+// a group of roots: groups shorter than that are not worth the records (200
+// long rules 0.78 ms; 0.91 ms with 8 us).  A sixteenth of the launch idle is
+// enough (5,000 miner candidates 3.99 ms; a quarter on two looks 4.60 ms, an
+// eighth on two 4.59 ms).
+constexpr long long kSpillEvery = 64000;
 // Records of a spill task, and candidates of a record, at inner levels and at
 // the leaf: about a round's work each.
 constexpr int kSpillChunk = 8, kSpillChunkLeaf = 32;
@@ -756,7 +790,7 @@ constexpr int kSpillSeg = 256, kSpillSegLeaf = 8192;
 template <int B>
 __device__ __noinline__ bool spill_items(Smem<B>& sm, const DevTask& task, const SpillArgs& sp, uint32_t* rows,
                                          int nWords, bool shared, bool sup, int kBase, int k,
-                                         int w0, int off) {
+                                         int w0, int off, int rootsEnd) {
     const DevPlan& P = sm.plan;
     BlockState<B>& S = sm.st;
     const int tid = threadIdx.x;
@@ -800,6 +834,7 @@ __device__ __noinline__ bool spill_items(Smem<B>& sm, const DevTask& task, const
             nRec += S.spillN[l];
             nTask += (S.spillN[l] + c - 1) / c;
         }
+        nTask += (rootsEnd - task.end + P.groupMax - 1) / max(P.groupMax, 1);   // the groups behind it, a task each
         bool ok = nTask > 1 && nRec <= (unsigned)kSpillRecs;   // one task would gain nothing
         uint32_t* dst = rows;
         int supAt = -1;
@@ -814,19 +849,7 @@ __device__ __noinline__ bool spill_items(Smem<B>& sm, const DevTask& task, const
             }
         }
         unsigned long long old = 0;
-        if (ok) {
-            unsigned long long* used = &sp.ctl->used[sp.out];
-            old = *reinterpret_cast<volatile unsigned long long*>(used);
-            for (;;) {
-                const unsigned t0 = (unsigned)(old >> 32), r0 = (unsigned)old;
-                ok = t0 + nTask <= (unsigned)kSpillTasks && r0 + nRec <= (unsigned)kSpillRecs;
-                if (!ok) break;
-                const unsigned long long seen =
-                    atomicCAS(used, old, (unsigned long long)(t0 + nTask) << 32 | (r0 + nRec));
-                if (seen == old) break;
-                old = seen;
-            }
-        }
+        if (ok) ok = spill_take(&sp.ctl->used[sp.out], nTask, nRec, old);
         // (rows or a support slot taken before a list turned out full are lost to this launch)
         if (supAt >= 0 && supAt < kSpillSups)
             sp.sups[supAt] = SpillSup{ok ? task.plan : -1, task.beg, task.end - task.beg, 0, dst};
@@ -845,11 +868,13 @@ __device__ __noinline__ bool spill_items(Smem<B>& sm, const DevTask& task, const
     for (int l = kBase; l <= k; ++l) {
         const int n = S.spillN[l], c = l + 1 == P.m ? kSpillChunkLeaf : kSpillChunk;
         for (int j = tid; j * c < n; j += B)
-            sp.tasks[sp.out][t + j] = SpillTask{task.plan, l, r + j * c, min(c, n - j * c), task.beg,
+            sp.tasks[sp.out & 1][t + j] = SpillTask{task.plan, l, r + j * c, min(c, n - j * c), task.beg,
                                                 task.end - task.beg, dst};
         t += (n + c - 1) / c;
         r += n;
     }
+    for (int b = task.end + tid * P.groupMax, j = t + tid; b < rootsEnd; b += B * P.groupMax, j += B)
+        sp.tasks[sp.out & 1][j] = SpillTask{task.plan, -1, 0, 0, b, min(P.groupMax, rootsEnd - b), nullptr};
     __syncthreads();
     if (tid == 0) {
         int at = S.spillRec;
@@ -872,7 +897,7 @@ __device__ __noinline__ bool spill_items(Smem<B>& sm, const DevTask& task, const
             if (!n) continue;
             const int slot = atomicAdd(&S.spillN[l], n);
             for (int q = 0; q < n; ++q) {
-                int* rec = sp.recs[sp.out] + (long long)(slot + q) * kSpillRecInts;
+                int* rec = sp.recs[sp.out & 1] + (long long)(slot + q) * kSpillRecInts;
                 for (int j = 0; j < lenL; ++j) rec[j] = it[j];
                 const int b = skip + q * seg;
                 rec[lenL] = it[lenL] + b;
@@ -950,11 +975,12 @@ __device__ __noinline__ void level_info(Smem<B>& sm, const DevIndex& ix, int l, 
 }
 
 // kS: the task may be spilled; st: the spill task to resume (`task` its
-// roots), or null.
+// roots), or null.  rootsEnd: the roots [task.end, rootsEnd) are this block's
+// next groups, and are given away with it.
 template <int B, bool kC, bool kD, bool kS>
 __device__ __forceinline__ void run_task(Smem<B>& sm, const DevIndex& ix, const DevTask& task,
                                          unsigned long long* results, int* status, Meter<kC>& mt, const SpillArgs& sp,
-                                         const SpillTask* st) {
+                                         const SpillTask* st, int rootsEnd) {
     constexpr int kLeafChunk = 16 * B;
     // candidates of a non-leaf round whose next step has a signature test
     // (most candidates die on it): more than the next level's capacity, so
@@ -1017,7 +1043,7 @@ __device__ __forceinline__ void run_task(Smem<B>& sm, const DevIndex& ix, const 
     if (tid == 0) {
         S.firstFail = INT_MAX;
         S.safeLevels = 0;
-        S.spill = S.looks = 0;
+        S.spill = 0;
         S.lookAt = clock64();
         S.base = resumed ? st->level : 0;
         int off = 0;
@@ -1030,6 +1056,9 @@ __device__ __forceinline__ void run_task(Smem<B>& sm, const DevIndex& ix, const 
             else if (P.m == 0 && l == 0) off += P.cap * P.tupleLen[0];
         }
     }
+    if constexpr (kS) {   // (its latency hides behind the roots')
+        if (tid == B - 1 && sp.out >= 0) S.idle = *reinterpret_cast<const volatile int*>(S.queue) - S.nTasks;
+    }
     if (tid >= 32 && tid - 32 < P.m) level_info<B>(sm, ix, tid - 32, pairs, sortMode, sliced, claims, kLeafChunk, kWideChunk);
     __syncthreads();
 
@@ -1039,7 +1068,7 @@ __device__ __forceinline__ void run_task(Smem<B>& sm, const DevIndex& ix, const 
         const int n = min(st->recN, P.cap);
         for (int i = tid; i < n * ints; i += B) {
             const int r = i / ints, q = i - r * ints;
-            items[S.levelOff[kBase] + i] = sp.recs[sp.in][(long long)(st->recBeg + r) * kSpillRecInts + q];
+            items[S.levelOff[kBase] + i] = sp.recs[sp.in & 1][(long long)(st->recBeg + r) * kSpillRecInts + q];
         }
         if (tid == 0) S.count[kBase] = n;
     } else {
@@ -1138,7 +1167,7 @@ __device__ __forceinline__ void run_task(Smem<B>& sm, const DevIndex& ix, const 
                 if (S.spill) {   // set before the last round's barrier: all threads are here
                     if (spill_items<B>(sm, task, sp, pairs ? bm : fb,
                                        pairs ? G * P.rowWords : (G + 31) >> 5, !heavy && (shared || !pairs),
-                                       P.supN > 0 && !heavy, S.base, k, w0, off))
+                                       P.supN > 0 && !heavy, S.base, k, w0, off, rootsEnd))
                         break;
                 }
             }
@@ -1270,8 +1299,16 @@ __device__ __forceinline__ void run_task(Smem<B>& sm, const DevIndex& ix, const 
                         mt.add(8);
                     } else {
                         const uint32_t mask = 1u << (rank & 31);
-                        const uint32_t old = atomicOr(bm + (long long)root * P.rowWords + (rank >> 5), mask);
-                        if (!shared) mt.add(8);
+                        uint32_t* word = bm + (long long)root * P.rowWords + (rank >> 5);
+                        if (!shared) {
+                            // a global row may be shared by many blocks, and most
+                            // candidates find their bit set: a load costs a
+                            // contended word less than an atomic
+                            mt.add(4);
+                            if (__ldcg(word) & mask) return;
+                            mt.add(8);
+                        }
+                        const uint32_t old = atomicOr(word, mask);
                         myNew += (old & mask) ? 0ull : 1ull;
                     }
                 } else {
@@ -1389,6 +1426,7 @@ __device__ __forceinline__ void run_task(Smem<B>& sm, const DevIndex& ix, const 
                             for (int q = 0; q < nEx; ++q)
                                 if ((ex[q] >> 5) == w && ex[q] >= 0) m &= ~(1u << (ex[q] & 31));
                             mt.add(4);
+                            if (m && !shared) m &= ~__ldcg(dst + w);
                             if (m) {
                                 const uint32_t old = atomicOr(dst + w, m);
                                 if (!shared) mt.add(8);
@@ -1403,14 +1441,13 @@ __device__ __forceinline__ void run_task(Smem<B>& sm, const DevIndex& ix, const 
                 if (tid == 0 && global_ns() > S.deadline) S.stop = 1;
             }
             if constexpr (kS) {
-                // blocks past the end of the queue are idle; when a quarter
-                // of the launch has been for a while, the items left here are
-                // worth a follow-up launch
+                // blocks past the end of the queue are idle; once a sixteenth
+                // of the launch is, the items left here are worth a follow-up
+                // launch
                 if (tid == 0 && sp.out >= 0 && (clock64() - S.lookAt > kSpillEvery || sp.always)) {
                     S.lookAt = clock64();
                     const int idle = *reinterpret_cast<const volatile int*>(S.queue) - S.nTasks;
-                    S.looks = sp.always ? kSpillLooks : (idle * 4 >= (int)gridDim.x ? S.looks + 1 : 0);
-                    if (S.looks >= kSpillLooks && !sortMode && !blockRows) S.spill = 1;
+                    if ((idle * 16 >= (int)gridDim.x || sp.always) && !sortMode && !blockRows) S.spill = 1;
                 }
             }
             __syncthreads();
@@ -1514,8 +1551,9 @@ engine_kernel(const __grid_constant__ DevIndex ix, const DevPlan* __restrict__ p
         const SpillTask* st = nullptr;
         DevTask task;
         if (follow) {
-            st = sp.tasks[sp.in] + t;
+            st = sp.tasks[sp.in & 1] + t;
             task = DevTask{st->plan, st->beg, st->beg + st->G, 0, 0, -1};
+            if (st->level < 0) st = nullptr;   // roots that no block had begun
         } else {
             task = tasks[t];
         }
@@ -1540,8 +1578,23 @@ engine_kernel(const __grid_constant__ DevIndex ix, const DevPlan* __restrict__ p
             for (int i = threadIdx.x; i < (int)(sizeof(DevPlan) / 4); i += B) dst[i] = src[i];
             __syncthreads();
         }
-        run_task<B, kC, kD, kS>(sm, ix, task, results, status, mt, sp, st);
-        __syncthreads();
+        // a task of several groups of roots: one after the other
+        const int group = st ? INT_MAX : max(1, sm.plan.groupMax);
+        for (DevTask part = task; part.beg < task.end;) {
+            part.end = group < task.end - part.beg ? part.beg + group : task.end;
+            run_task<B, kC, kD, kS>(sm, ix, part, results, status, mt, sp, st, task.end);
+            __syncthreads();
+            if constexpr (kD) {
+                if (sm.st.stop) break;
+            }
+            if constexpr (kS) {
+                if (sm.st.spill) break;   // (the groups behind it went with it)
+                if (part.end < task.end && sp.out >= 0 && (sm.st.idle * 16 >= (int)gridDim.x || sp.always) &&
+                    spill_groups<B>(sm, sp, task.plan, part.end, task.end))
+                    break;
+            }
+            part.beg = part.end;
+        }
         if constexpr (kD) {
             if (threadIdx.x == 0 && sm.st.stop) atomicOr(prof.incomplete + task.plan, 1);
         }

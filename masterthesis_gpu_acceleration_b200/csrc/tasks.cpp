@@ -11,6 +11,11 @@ namespace gr {
 namespace {
 
 constexpr double kMinTarget = 4096.0;
+// Work units of a group of roots beside its candidates: clearing its rows,
+// its rounds' barriers and dependent loads (tasks of a few candidates measured
+// 5-10 us each).
+constexpr double kGroupUnits = 6000.0;
+constexpr int32_t kMaxGroups = 64;   // groups of a task
 constexpr size_t kCacheLimit = size_t(2) << 30;
 
 int64_t pd_key(int32_t pred, int dir) { return (int64_t)pred * 2 + dir; }
@@ -358,7 +363,7 @@ TaskBuilder::Walk TaskBuilder::compute_walk(const PhasePlan& ph) {
 
 void TaskBuilder::build(const std::vector<const PhasePlan*>& phases, int blocks, bool split,
                         std::vector<PhaseTasks>& out, double walkBudget, bool costAware,
-                        const std::vector<PhaseLimits>* limits) {
+                        const std::vector<PhaseLimits>* limits, bool groups) {
     size_t n = phases.size();
     out.assign(n, PhaseTasks{});
     if (cacheBytes_ > kCacheLimit) {  // only here: walks hand out references into the cache
@@ -438,7 +443,15 @@ void TaskBuilder::build(const std::vector<const PhasePlan*>& phases, int blocks,
     }
     // work in device-time units (learned ns per unit, where known)
     double total = 0;
-    for (size_t i = 0; i < n; ++i) total += out[i].work * scale[i];
+    for (size_t i = 0; i < n; ++i) {
+        const PhasePlan& ph = *phases[i];
+        int32_t g = std::max(ph.plan.groupMax, 1);
+        if (ph.needsGlobalBitmap) g = std::min(ph.plan.cap, 512);
+        if (limits && (*limits)[i].group > 0) g = std::min(g, (*limits)[i].group);
+        out[i].group = std::max(g, 1);
+        if (groups) out[i].work += kGroupUnits * ((ph.rootEnd - ph.rootBeg + g - 1) / out[i].group);
+        total += out[i].work * scale[i];
+    }
     const double target = forceTarget > 0 ? forceTarget
                                           : std::max(kMinTarget * defaultCalib_, total / (std::max(blocks, 1) * 8.0));
 
@@ -454,18 +467,21 @@ void TaskBuilder::build(const std::vector<const PhasePlan*>& phases, int blocks,
         PhaseTasks& pt = out[i];
         const double sc = forceTarget > 0 ? 1.0 : scale[i];
         pt.scale = scale[i];
-        int32_t g = std::max(P.groupMax, 1);
-        if (ph.needsGlobalBitmap) g = std::min(P.cap, 512);
         const PhaseLimits lim = limits ? (*limits)[i] : PhaseLimits{};
-        if (lim.group > 0) g = std::min(g, lim.group);
+        const int32_t one = pt.group;                                          // roots of a group
+        const double fixed = groups ? kGroupUnits : 0.0;                       // units a group costs by itself
+        const int32_t g = groups ? (int32_t)std::min<int64_t>((int64_t)one * kMaxGroups, INT32_MAX) : one;
         const int32_t R = ph.rootEnd - ph.rootBeg;
         const double uniform = R > 0 ? std::max(1.0, pt.work / R) : 1.0;
         const Walk* wk = walked[i];
         if (!wk) {
             // uniform cost per root: fixed-size chunks, no per-root pass
             const double per = uniform * sc;
+            // (uniform already holds the groups' own cost)
             int32_t chunk = g;
             if (per > 0 && per * chunk > target) chunk = std::max<int32_t>(1, (int32_t)(target / per));
+            if (groups && chunk > one) chunk -= chunk % one;
+            else chunk = std::min(chunk, one);
             for (int32_t b = ph.rootBeg; b < ph.rootEnd; b += chunk) {
                 const int32_t e = std::min(ph.rootEnd, b + chunk);
                 pt.tasks.push_back(DevTask{(int32_t)i, b, e, 0, 0, -1});
@@ -478,7 +494,7 @@ void TaskBuilder::build(const std::vector<const PhasePlan*>& phases, int blocks,
         auto flush = [&](int32_t end) {
             if (end > gb) {
                 pt.tasks.push_back(DevTask{(int32_t)i, gb, end, 0, 0, -1});
-                pt.cost.push_back(accUnits);
+                pt.cost.push_back(accUnits + fixed * ((end - gb + one - 1) / one));
             }
             gb = end;
             acc = 0;
@@ -501,8 +517,8 @@ void TaskBuilder::build(const std::vector<const PhasePlan*>& phases, int blocks,
                 // current task (roots below exceed neither bound one by one)
                 const size_t b = (size_t)(o / kWalkBlock);
                 const double bs = wk->bsum[b];
-                if ((!canSplit || (double)wk->bmax[b] * sc <= splitAt) && acc + bs * sc <= target &&
-                    r + kWalkBlock - 1 - gb < g) {
+                if ((!canSplit || (double)wk->bmax[b] * sc <= splitAt) &&
+                    acc + bs * sc + fixed * sc * ((r + kWalkBlock - gb) / one) <= target && r + kWalkBlock - 1 - gb < g) {
                     acc += bs * sc;
                     accUnits += bs;
                     r += kWalkBlock - 1;
@@ -541,7 +557,7 @@ void TaskBuilder::build(const std::vector<const PhasePlan*>& phases, int blocks,
                 gb = r + 1;
                 continue;
             }
-            if (r > gb && (r - gb >= g || acc + wr > target)) flush(r);
+            if (r > gb && (r - gb >= g || acc + wr + fixed * sc * ((r + 1 - gb) / one) > target)) flush(r);
             acc += wr;
             accUnits += wu;
         }

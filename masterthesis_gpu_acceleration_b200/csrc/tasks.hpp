@@ -27,6 +27,7 @@ struct PhaseLimits {
 struct PhaseTasks {
     std::vector<DevTask> tasks;
     std::vector<double> cost;   // estimated work per task
+    int32_t group = 0;          // most roots a block takes at once (tasks may hold several groups)
     int32_t heavyRows = 0;      // global dedup rows used by split roots
     double work = 0.0;          // estimated work of the whole phase
     double scale = 1.0;         // learned device ns per unit of work
@@ -42,6 +43,10 @@ struct PhaseTasks {
 // at most `target` (about 1/8 of a block's fair share of the batch); a root
 // heavier than that is split into slices of its first segment, each a task
 // of its own that deduplicates in a global row.
+// With groups, a task's size is that work alone, not the dedup rows a block
+// holds at once: a phase whose rows fill the shared pool with 20 roots made
+// hundreds of tasks of a few us, each fetched, listed, ordered and uploaded
+// (142,000 for 10,000 rules, 7,900 for the work they hold).
 // Host time of one step of a per-root walk (ns), for the cost-aware mode.
 constexpr double kWalkNsPerEdge = 8.0;
 
@@ -64,9 +69,11 @@ public:
     // the walk's own host time, and cut only roots above a block's fair
     // share of their phase (per-rule launches, where nothing overlaps).
     // limits (optional): one entry per phase.
+    // groups: tasks may hold several groups of roots, which a block takes one
+    // after the other (the kernel cuts them at the phase's `group`).
     void build(const std::vector<const PhasePlan*>& phases, int blocks, bool split,
                std::vector<PhaseTasks>& out, double walkBudget = 4.0e6, bool costAware = false,
-               const std::vector<PhaseLimits>* limits = nullptr);
+               const std::vector<PhaseLimits>* limits = nullptr, bool groups = false);
 
     // Estimated candidate bindings of a phase (average fan-outs; exact first
     // two levels for chain-shaped plans rooted at the first step's rows).
