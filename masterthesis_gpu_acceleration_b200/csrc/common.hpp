@@ -315,6 +315,22 @@ struct Geom {
     int poolInts() const { return pool_for(block); }
 };
 
+// A launch of one plan whose tasks are equal runs of its roots: the plan comes
+// with the launch instead of by a copy, the tasks follow from their number,
+// and the last block to end writes the control words to host memory and
+// clears them for the next launch (instead of a memset before and a copy
+// after).
+struct InlineLaunch {
+    int32_t on = 0;
+    int32_t beg = 0, end = 0, chunk = 0;   // task t: the roots [beg + t * chunk, ...)
+    int32_t publish = 0;                   // 1: the last launch on these control words
+    int32_t seq = 0;                       // written behind the published words, when they are there
+    void* ctl = nullptr;                   // the control words: kInlineWords, and the count of ended blocks behind them
+    void* host = nullptr;                  // where they go
+    DevPlan plan;
+};
+constexpr int kInlineWords = 16;
+
 constexpr int kMemoMaps = 3;   // S1, S2, S3 of a two-step memo: at least one, two, three witnesses
 
 // One suffix memo to build for hub row `row` of (p1, d1), or the part that

@@ -12,6 +12,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <climits>
 #include <cmath>
 #include <cstdio>
@@ -83,8 +84,45 @@ size_t spill_part(int part) {
 size_t spill_bytes() { return spill_part(6); }
 }  // namespace
 
+namespace {
+// Orders tasks [b, e) (and their costs) by falling cost x scale(i): a stable
+// counting sort by quarter-octaves of the estimate.
+template <class Scale>
+void longest_first(std::vector<DevTask>& tasks, std::vector<double>& cost, size_t b, size_t e, Scale scale) {
+    constexpr int kBuckets = 1024;
+    auto bucket = [](double v) {
+        if (!(v > 0.0)) return 0;
+        int ex;
+        const double m = std::frexp(v, &ex);   // v = m * 2^ex, m in [0.5, 1)
+        return std::max(1, std::min(kBuckets - 1, 512 + 4 * ex + (int)((m - 0.5) * 8.0)));
+    };
+    std::vector<uint16_t> bk(e - b);
+    std::vector<uint32_t> start(kBuckets + 1, 0);
+    for (size_t i = b; i < e; ++i) {
+        bk[i - b] = (uint16_t)bucket(cost[i] * scale(i));
+        ++start[kBuckets - 1 - bk[i - b]];
+    }
+    uint32_t acc = 0;
+    for (uint32_t& x : start) {
+        const uint32_t n = x;
+        x = acc;
+        acc += n;
+    }
+    std::vector<DevTask> t2(e - b);
+    std::vector<double> c2(e - b);
+    for (size_t i = b; i < e; ++i) {
+        const size_t at = start[kBuckets - 1 - bk[i - b]]++;
+        t2[at] = tasks[i];
+        c2[at] = cost[i];
+    }
+    std::copy(t2.begin(), t2.end(), tasks.begin() + (ptrdiff_t)b);
+    std::copy(c2.begin(), c2.end(), cost.begin() + (ptrdiff_t)b);
+}
+}  // namespace
+
 void Staged::stage(Context& c, std::vector<DevPlan>& plans, const std::vector<const PhasePlan*>& phases,
-                   bool sortTasks, cudaStream_t s, double walkBudget, bool costAware, bool allowSort) {
+                   bool sortTasks, cudaStream_t s, double walkBudget, bool costAware, bool allowSort, bool mayInline) {
+    inl.clear();
     nPlans = (int)plans.size();
     nResults = nPlans + extraResults;
     stagedBlock = c.geom.block;
@@ -326,35 +364,44 @@ void Staged::stage(Context& c, std::vector<DevPlan>& plans, const std::vector<co
         tasks.insert(tasks.end(), pts[i].tasks.begin(), pts[i].tasks.end());
         cost.insert(cost.end(), pts[i].cost.begin(), pts[i].cost.end());
     }
+    // Spilling pays where a task can outlast the others: not for launches
+    // whose estimated work is below about 60 us of the whole GPU (their
+    // follow-up launches, a few us, would cost more than a tail saves), and
+    // not for sort mode, whose key count must not depend on it.
+    double workNs = 0;
+    for (int i = 0; i < nPlans; ++i) workNs += pts[i].work * pts[i].scale;
+    spillAlways = c.spill == 2;
+    spillable = c.spill && nSort == 0 && (spillAlways || workNs > 60e3 * std::max(c.grid, 1));
+    if (dCtl.cap == 0) ctlClean = false;
+    dCtl.ensure(kCtlBytes, as);
+    if (hCtl.cap == 0) {
+        hCtl.ensure(kCtlBytes);
+        std::memset(hCtl.p, 0, kCtlBytes);
+    }
     hostSect[3] += host_ms() - tSect;
     tSect = host_ms();
+    if (mayInline && nPlans <= kMaxPerPlan && !spillable && !bitmapWords && !blockWords && !heavyWords && !nSort &&
+        std::all_of(pts.begin(), pts.end(), [](const PhaseTasks& t) { return t.chunk > 0; })) {
+        // no upload at all: every launch brings its plan
+        inl.resize(nPlans);
+        for (int i = 0; i < nPlans; ++i) {
+            InlineLaunch& L = inl[i];
+            L.on = 1;
+            L.beg = phases[i]->rootBeg;
+            L.end = phases[i]->rootEnd;
+            L.chunk = pts[i].chunk;
+            L.publish = i + 1 == nPlans ? 1 : 0;
+            L.ctl = dCtl.p;
+            L.host = hCtl.p;
+            L.plan = plans[i];
+        }
+        nTasks = (int)tasks.size();
+        d2hBytes = 64;
+        return;
+    }
     if (sortTasks && tasks.size() > 1) {
-        // longest (estimated device time) first, so the tail of the launch is
-        // short: a stable counting sort by quarter-octaves of the estimate
-        constexpr int kBuckets = 1024;
-        auto bucket = [](double v) {
-            if (!(v > 0.0)) return 0;
-            int e;
-            const double m = std::frexp(v, &e);   // v = m * 2^e, m in [0.5, 1)
-            return std::max(1, std::min(kBuckets - 1, 512 + 4 * e + (int)((m - 0.5) * 8.0)));
-        };
-        std::vector<uint16_t> bk(tasks.size());
-        std::vector<size_t> start(kBuckets + 1, 0);
-        for (size_t i = 0; i < tasks.size(); ++i) {
-            bk[i] = (uint16_t)bucket(cost[i] * pts[tasks[i].plan].scale);
-            ++start[kBuckets - 1 - bk[i]];
-        }
-        size_t acc = 0;
-        for (int b = 0; b <= kBuckets; ++b) { const size_t c = start[b]; start[b] = acc; acc += c; }
-        std::vector<DevTask> t2(tasks.size());
-        std::vector<double> c2(tasks.size());
-        for (size_t i = 0; i < tasks.size(); ++i) {
-            const size_t at = start[kBuckets - 1 - bk[i]]++;
-            t2[at] = tasks[i];
-            c2[at] = cost[i];
-        }
-        tasks.swap(t2);
-        cost.swap(c2);
+        // longest (estimated device time) first, so the tail of the launch is short
+        longest_first(tasks, cost, 0, tasks.size(), [&](size_t i) { return pts[tasks[i].plan].scale; });
     }
     nTasks = (int)tasks.size();
     planTaskEnd.clear();
@@ -362,18 +409,9 @@ void Staged::stage(Context& c, std::vector<DevPlan>& plans, const std::vector<co
         // one launch per plan: each plan's tasks stay contiguous, longest
         // first within the plan
         int32_t acc = 0;
-        std::vector<int32_t> ord;
         for (int i = 0; i < nPlans; ++i) {
             const int32_t b = acc, e = acc + (int32_t)pts[i].tasks.size();
-            ord.resize((size_t)(e - b));
-            std::iota(ord.begin(), ord.end(), b);
-            std::stable_sort(ord.begin(), ord.end(), [&](int32_t x, int32_t y) { return cost[x] > cost[y]; });
-            for (int32_t k = b; k < e; ++k) {
-                pts[i].tasks[k - b] = tasks[ord[k - b]];
-                pts[i].cost[k - b] = cost[ord[k - b]];
-            }
-            std::copy(pts[i].tasks.begin(), pts[i].tasks.end(), tasks.begin() + b);
-            std::copy(pts[i].cost.begin(), pts[i].cost.end(), cost.begin() + b);
+            if (pts[i].chunk <= 0) longest_first(tasks, cost, (size_t)b, (size_t)e, [](size_t) { return 1.0; });
             planTaskEnd.push_back(acc = e);
         }
     }
@@ -395,18 +433,8 @@ void Staged::stage(Context& c, std::vector<DevPlan>& plans, const std::vector<co
     dBlob.ensure(blob, as);
     nResults = nPlans + extraResults;
     dResults.ensure((size_t)nResults * sizeof(unsigned long long), as);
-    dCtl.ensure(kCtlBytes, as);
-    // Spilling pays where a task can outlast the others: not for launches
-    // whose estimated work is below about 60 us of the whole GPU (their
-    // follow-up launches, a few us, would cost more than a tail saves), and
-    // not for sort mode, whose key count must not depend on it.
-    double workNs = 0;
-    for (int i = 0; i < nPlans; ++i) workNs += pts[i].work * pts[i].scale;
-    spillAlways = c.spill == 2;
-    spillable = c.spill && nSort == 0 && (spillAlways || workNs > 60e3 * std::max(c.grid, 1));
     if (spillable) dSpill.ensure(spill_bytes(), as);
     hResults.ensure((size_t)nResults * sizeof(unsigned long long));
-    hCtl.ensure(64);
     ck(cudaMemcpyAsync(dBlob.p, hBlob.p, blob, cudaMemcpyHostToDevice, s), "H2D plans");
     dPlans = static_cast<const DevPlan*>(dBlob.p);
     dTasks = reinterpret_cast<const DevTask*>(static_cast<const char*>(dBlob.p) + planBytes);
@@ -637,6 +665,7 @@ void Staged::enqueue(Context& c, cudaStream_t s, int instr, int gridCap, unsigne
     budgeted = false;
     if (!nPlans) return;
     check_geometry(c);
+    ctlClean = false;
     ck(cudaMemsetAsync(dResults.p, 0, (size_t)nResults * sizeof(unsigned long long), s), "memset results");
     ck(cudaMemsetAsync(dCtl.p, 0, kCtlBytes, s), "memset ctl");
     if (bitmapWords) ck(cudaMemsetAsync(dBitmap.p, 0, bitmapWords * 4, s), "memset bitmap");
@@ -677,10 +706,30 @@ void Staged::enqueue(Context& c, cudaStream_t s, int instr, int gridCap, unsigne
 void Staged::enqueue_per_plan(Context& c, cudaStream_t s) {
     if (!nPlans) return;
     check_geometry(c);
+    if (!inl.empty()) {
+        static_assert(kInlineWords * 4 == 64 && kSpillCtlAt >= kInlineWords * 4 && kCtlBytes > kInlineWords * 4,
+                      "the ended blocks are counted behind the published words");
+        if (!ctlClean) ck(cudaMemsetAsync(dCtl.p, 0, kCtlBytes, s), "memset ctl");
+        ctlClean = false;   // until the launches are known to have ended (wait_published)
+        inlSeq = inlSeq % 0x3fffffff + 1;
+        for (InlineLaunch& L : inl) L.seq = inlSeq;
+        int* ctl = static_cast<int*>(dCtl.p);
+        for (int i = 0; i < nPlans; ++i) {
+            EngineProfile prof;
+            prof.span = reinterpret_cast<unsigned long long*>(static_cast<char*>(dCtl.p) + 16 + 16 * i);
+            const int n = (inl[i].end - inl[i].beg + inl[i].chunk - 1) / inl[i].chunk;
+            ck(engine_launch(c.dix, nullptr, nullptr, n, ctl + i,
+                             reinterpret_cast<unsigned long long*>(static_cast<char*>(dCtl.p) + kPerPlanResults),
+                             ctl + 2, std::max(1, std::min(n, c.grid)), c.geom.block, s, &prof, SpillArgs{}, &inl[i]),
+               "engine launch");
+        }
+        return;
+    }
     if (nPlans > kMaxPerPlan || (int)planTaskEnd.size() != nPlans) throw CudaError("bad per-plan staging");
     // control words: [0..1] task counters, [2] status (int), per plan two
     // u64 span words at byte 16 + 16 * i and its u64 result at
     // kPerPlanResults + 8 * i; all start at zero
+    ctlClean = false;
     ck(cudaMemsetAsync(dCtl.p, 0, kCtlBytes, s), "memset ctl");
     if (bitmapWords) ck(cudaMemsetAsync(dBitmap.p, 0, bitmapWords * 4, s), "memset bitmap");
     if (heavyWords) ck(cudaMemsetAsync(dHeavy.p, 0, heavyWords * 4, s), "memset heavy rows");
@@ -710,8 +759,24 @@ void Staged::enqueue_per_plan(Context& c, cudaStream_t s) {
     enqueue_sort(c, s, reinterpret_cast<unsigned long long*>(static_cast<char*>(dCtl.p) + kPerPlanResults), ctl + 2);
 }
 
+// Waits for the control words of an inline launch: the flag behind them in
+// host memory is a few us earlier than the stream's end.  Ends with the
+// stream in any case (an error is the following synchronisation's to report).
+void Staged::wait_published(cudaStream_t s) {
+    if (inl.empty()) return;
+    const volatile int* flag = static_cast<const volatile int*>(hCtl.p) + kInlineWords;
+    for (unsigned spins = 0;; ++spins) {
+        if (*flag == inlSeq) {
+            std::atomic_thread_fence(std::memory_order_acquire);
+            ctlClean = true;
+            return;
+        }
+        if (spins % 4096 == 4095 && cudaStreamQuery(s) != cudaErrorNotReady) return;
+    }
+}
+
 void Staged::download_spans(cudaStream_t s) {
-    if (!nPlans) return;
+    if (!nPlans || !inl.empty()) return;   // (an inline launch writes them itself)
     ck(cudaMemcpyAsync(hCtl.p, dCtl.p, 64, cudaMemcpyDeviceToHost, s), "D2H control words");
     download_cursor(s);
 }
@@ -800,11 +865,12 @@ int evaluate_parsed(Context& c, const Rule& rule, GpuRuleResult* out) {
     }
     if (!plans.empty()) {
         // one upload, one launch per phase (each timed on the device), one download
-        c.one.stage(c, plans, phases, false, c.stream, c.ruleWalkBudget, true);
+        c.one.stage(c, plans, phases, false, c.stream, c.ruleWalkBudget, true, true, true);
         for (int attempt = 0;; ++attempt) {
             with_rule_block(c, [&] { c.one.enqueue_per_plan(c, c.stream); });
             c.one.download_spans(c.stream);
-            ck(cudaStreamSynchronize(c.stream), "engine");
+            c.one.wait_published(c.stream);
+            ck(c.one.inl.empty() || !c.one.ctlClean ? cudaStreamSynchronize(c.stream) : cudaSuccess, "engine");
             if (attempt > 0 || !c.one.sort_overflow()) break;
             c.one.restage(c, c.stream);   // the exact key count is known now
         }

@@ -8,6 +8,7 @@
 #include <array>
 #include <climits>
 #include <cstdio>
+#include <cstring>
 #include <memory>
 #include <stdexcept>
 #include <string>
@@ -41,7 +42,8 @@ cudaError_t support_rows(const DevIndex& ix, const DevPlan* plans, const SupJob*
                          int spillBlocks = 0);
 cudaError_t engine_launch(const DevIndex& ix, const DevPlan* plans, const DevTask* tasks, int nTasks,
                           int* taskCounter, unsigned long long* results, int* status, int grid, int block,
-                          cudaStream_t stream, const EngineProfile* prof, const SpillArgs& sp = SpillArgs{});
+                          cudaStream_t stream, const EngineProfile* prof, const SpillArgs& sp = SpillArgs{},
+                          const InlineLaunch* in = nullptr);
 // Sort mode (sort.cu): radix sort of the appended pair keys and the count of
 // each plan's distinct keys into its result slot.
 size_t pairs_sort_hist_words(unsigned long long cap);
@@ -134,6 +136,12 @@ struct Staged {
     size_t bitmapWords = 0, heavyWords = 0;
     size_t h2dBytes = 0, d2hBytes = 0;
     bool streamOrdered = false;   // grow device buffers on the launch stream (serving slots)
+    // Plain per-rule staging whose plans all have equal tasks and need no
+    // memory of the launch's own: launched with the plan as an argument.
+    std::vector<InlineLaunch> inl;
+    int inlSeq = 0;                     // number of the last inline launch, its flag in host memory
+    void wait_published(cudaStream_t s);
+    bool ctlClean = false;              // the control words are zero (an inline launch left them so)
     std::vector<int32_t> planTaskEnd;   // tasks in plan order (unsorted staging): end of each plan's tasks
 
     // Deduplication of kPairs plans (DedupMode per plan).  Per-phase global
@@ -184,7 +192,7 @@ struct Staged {
     // when the key buffer overflows; the serving loop cannot).
     void stage(Context& c, std::vector<DevPlan>& plans, const std::vector<const PhasePlan*>& phases,
                bool sortTasks, cudaStream_t s, double walkBudget = 4.0e6, bool costAware = false,
-               bool allowSort = true);
+               bool allowSort = true, bool mayInline = false);
     // After download + synchronisation: whether sort-mode keys exceeded the
     // buffer (the counts are then incomplete).  restage() stages the same
     // plans again with a buffer of the exact size (one upload, no launch).
@@ -241,7 +249,10 @@ struct Staged {
         dResults.ensure(plans * sizeof(unsigned long long), s);
         hResults.ensure(plans * sizeof(unsigned long long));
         dCtl.ensure(kCtlBytes, s);
-        hCtl.ensure(64);
+        if (hCtl.cap == 0) {
+            hCtl.ensure(kCtlBytes);
+            std::memset(hCtl.p, 0, kCtlBytes);
+        }
         dHeavy.ensure(1 << 20, s);
         dBitmap.ensure(1 << 20, s);
         dBytes.ensure(8, s);

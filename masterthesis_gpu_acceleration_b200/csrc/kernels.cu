@@ -104,7 +104,11 @@ struct BlockState {
     unsigned long long red[kWarps];
     int exRank[kWarps][kMaxVars];   // per warp: hO-domain ranks of the bound values of a hub item
     int spill;                      // 1: the block gives its open items away
-    long long lookAt;               // thread 0: the clock at its last look at the queue
+    long long lookAt;               // thread 0: the clock at which it next looks at the queue
+    uint32_t* rows;                 // the group's dedup rows, of rowsWords words when in shared memory (else 0)
+    int rowsWords;
+    int rowsSup;                    // 1: their fused support is still to be counted
+    int rootsEnd;                   // end of the task's roots (the group's may lie before it)
     int idle;                       // blocks that were past the queue's end when the group began
     int base;                       // the level the task's search starts at
     int nTasks;                     // of the launch, and its counter
@@ -781,19 +785,20 @@ constexpr long long kSpillEvery = 64000;
 constexpr int kSpillChunk = 8, kSpillChunkLeaf = 32;
 constexpr int kSpillSeg = 256, kSpillSegLeaf = 8192;
 
-// Gives the open items of levels kBase..k away (see SpillTask); false when a
-// list is full (the block then carries on).  The task's dedup rows start at
-// `rows`; `shared`: they are nWords words in shared memory and move to global
-// ones.  The whole block calls this between two rounds;
-// level k continues at item w0, `off` candidates of it consumed.  Out of line:
-// it runs at most once per task.
+// Gives the open items of levels S.base..k away (see SpillTask), and the
+// groups of roots behind them; false when a list is full (the block then
+// carries on).  Rows in shared memory move to global ones.  The whole block
+// calls this between two rounds; level k continues at item w0, `off`
+// candidates of it consumed.  Out of line: it runs at most once per group.
 template <int B>
-__device__ __noinline__ bool spill_items(Smem<B>& sm, const DevTask& task, const SpillArgs& sp, uint32_t* rows,
-                                         int nWords, bool shared, bool sup, int kBase, int k,
-                                         int w0, int off, int rootsEnd) {
+__device__ __noinline__ bool spill_items(Smem<B>& sm, const DevTask& task, const SpillArgs& sp, int k, int w0,
+                                         int off) {
     const DevPlan& P = sm.plan;
     BlockState<B>& S = sm.st;
     const int tid = threadIdx.x;
+    uint32_t* const rows = S.rows;
+    const int nWords = S.rowsWords, kBase = S.base, rootsEnd = S.rootsEnd;
+    const bool shared = nWords > 0, sup = S.rowsSup != 0;
     // a level's first open item and the candidates of it already consumed
     auto level_pos = [&](int l, int& at, int& skip) {
         at = l == k ? w0 : S.curItem[l];
@@ -975,12 +980,11 @@ __device__ __noinline__ void level_info(Smem<B>& sm, const DevIndex& ix, int l, 
 }
 
 // kS: the task may be spilled; st: the spill task to resume (`task` its
-// roots), or null.  rootsEnd: the roots [task.end, rootsEnd) are this block's
-// next groups, and are given away with it.
+// roots), or null.
 template <int B, bool kC, bool kD, bool kS>
 __device__ __forceinline__ void run_task(Smem<B>& sm, const DevIndex& ix, const DevTask& task,
                                          unsigned long long* results, int* status, Meter<kC>& mt, const SpillArgs& sp,
-                                         const SpillTask* st, int rootsEnd) {
+                                         const SpillTask* st) {
     constexpr int kLeafChunk = 16 * B;
     // candidates of a non-leaf round whose next step has a signature test
     // (most candidates die on it): more than the next level's capacity, so
@@ -1044,7 +1048,10 @@ __device__ __forceinline__ void run_task(Smem<B>& sm, const DevIndex& ix, const 
         S.firstFail = INT_MAX;
         S.safeLevels = 0;
         S.spill = 0;
-        S.lookAt = clock64();
+        S.lookAt = !kS || sp.out < 0 || sortMode || blockRows ? LLONG_MAX : (sp.always ? 0 : clock64() + kSpillEvery);
+        S.rows = pairs ? bm : fb;
+        S.rowsWords = !heavy && (shared || !pairs) ? (pairs ? G * P.rowWords : (G + 31) >> 5) : 0;
+        S.rowsSup = P.supN > 0 && !heavy ? 1 : 0;
         S.base = resumed ? st->level : 0;
         int off = 0;
         for (int l = 0; l <= kMaxBody; ++l) {
@@ -1165,10 +1172,7 @@ __device__ __forceinline__ void run_task(Smem<B>& sm, const DevIndex& ix, const 
         for (;;) {
             if constexpr (kS) {
                 if (S.spill) {   // set before the last round's barrier: all threads are here
-                    if (spill_items<B>(sm, task, sp, pairs ? bm : fb,
-                                       pairs ? G * P.rowWords : (G + 31) >> 5, !heavy && (shared || !pairs),
-                                       P.supN > 0 && !heavy, S.base, k, w0, off, rootsEnd))
-                        break;
+                    if (spill_items<B>(sm, task, sp, k, w0, off)) break;
                 }
             }
             const int cnt = min(S.count[k], P.cap);
@@ -1182,12 +1186,13 @@ __device__ __forceinline__ void run_task(Smem<B>& sm, const DevIndex& ix, const 
                 continue;
             }
             const int nw = min(B, cnt - w0);
-            const Level lv = S.lv[k];   // uniform for the round: kept in registers
+            const Level& lv = S.lv[k];
+            const int lvf = lv.flags;   // uniform for the round; what only survivors need is read when they do
             const int lenK = lv.len;
             const int strideK = lenK + 2;
             int* const baseK = items + lv.at;
-            const bool leaf = (lv.flags & kLvLeaf) != 0;
-            const int pathKind = lv.flags >> kLvPath;
+            const bool leaf = (lvf & kLvLeaf) != 0;
+            const int pathKind = lvf >> kLvPath;
             bool isHub = false;   // item marked for the hub or memo pass
 
             // window: the stored neighbour segment of each item
@@ -1199,7 +1204,7 @@ __device__ __forceinline__ void run_task(Smem<B>& sm, const DevIndex& ix, const 
                 if (!pairs) {
                     pruned = (fb[it[0] >> 5] >> (it[0] & 31)) & 1u;
                     if (heavy) mt.add(4);
-                } else if ((lv.flags & kLvHasRank) && !sortMode) {
+                } else if ((lvf & kLvHasRank) && !sortMode) {
                     pruned = (bm[(long long)it[0] * P.rowWords + (it[1] >> 5)] >> (it[1] & 31)) & 1u;
                     if (!shared) mt.add(4);
                 }
@@ -1260,8 +1265,8 @@ __device__ __forceinline__ void run_task(Smem<B>& sm, const DevIndex& ix, const 
             // exhausted, so the search always advances.  Sort mode keeps
             // capacity-sized rounds: its key count must not depend on how
             // the threads raced (a launch is staged again with that count).
-            const bool wide = (lv.flags & kLvWide) && !((S.safeLevels >> k) & 1u);
-            const int take = min(total, (lv.flags & kLvWide) && !wide ? P.cap : lv.maxTake);
+            const bool wide = (lvf & kLvWide) && !((S.safeLevels >> k) & 1u);
+            const int take = min(total, (lvf & kLvWide) && !wide ? P.cap : lv.maxTake);
 
             // One candidate: its parent item `lo`, edge `e`, new value(s)
             // n0/n1 and (when this step binds hO) the loaded rank.
@@ -1269,20 +1274,20 @@ __device__ __forceinline__ void run_task(Smem<B>& sm, const DevIndex& ix, const 
                 const int* par = baseK + (w0 + lo) * strideK;
                 const int root = par[0];
                 if (!pairs && ((fb[root >> 5] >> (root & 31)) & 1u)) return;
-                if ((lv.flags & kLvScan) && ((lv.flags & kLvSameVar) ? (n0 != n1) : (n0 == n1))) return;
+                if ((lvf & kLvScan) && ((lvf & kLvSameVar) ? (n0 != n1) : (n0 == n1))) return;
                 if (n0 != kAnyValue)
                     for (int q = kTupleHead; q < lenK; ++q) {
                         const int x = par[q];
-                        if (x == n0 || ((lv.flags & kLvTwo) && x == n1)) return;
+                        if (x == n0 || ((lvf & kLvTwo) && x == n1)) return;
                     }
                 auto valN = [&](TermRef ref) -> int {
                     if (ref < 0) return P.consts[-1 - ref];
                     if (ref < lenK) return par[ref];
                     return ref == lenK ? n0 : n1;
                 };
-                if ((lv.flags & kLvFilters) && !pass_filters(P, ix, k + 1, mt, valN)) return;
+                if ((lvf & kLvFilters) && !pass_filters(P, ix, k + 1, mt, valN)) return;
                 int rank = par[1];
-                if (lv.flags & kLvHo) {
+                if (lvf & kLvHo) {
                     rank = rankLoaded;
                     if (!leaf && !sortMode) {
                         if (!shared) mt.add(4);
@@ -1314,10 +1319,10 @@ __device__ __forceinline__ void run_task(Smem<B>& sm, const DevIndex& ix, const 
                 } else {
                     const RowHit hit = step_row(P, ix, k + 1, mt, valN);
                     if (hit.seg.y <= hit.seg.x) return;
-                    if ((lv.flags & kLvLook) &&
-                        !((((lv.flags & kLvLookHigh) ? hit.sig.y : hit.sig.x) >> lv.lookShift) & 1u))
+                    if ((lvf & kLvLook) &&
+                        !((((lvf & kLvLookHigh) ? hit.sig.y : hit.sig.x) >> lv.lookShift) & 1u))
                         return;
-                    if (!(lv.flags & (kLvHasRank | kLvHo))) rank = item_state(P.steps[k + 1], hit.hub);
+                    if (!(lvf & (kLvHasRank | kLvHo))) rank = item_state(P.steps[k + 1], hit.hub);
                     const int slot = atomicAdd(&S.count[k + 1], 1);
                     if (slot >= P.cap) {
                         if (wide) atomicMin(&S.firstFail, j);
@@ -1330,7 +1335,7 @@ __device__ __forceinline__ void run_task(Smem<B>& sm, const DevIndex& ix, const 
                     dst[1] = rank;
                     for (int q = kTupleHead; q < lenK; ++q) dst[q] = par[q];
                     dst[lenK] = n0;
-                    if (lv.flags & kLvTwo) dst[lenK + 1] = n1;
+                    if (lvf & kLvTwo) dst[lenK + 1] = n1;
                     dst[lenN] = hit.seg.x;
                     dst[lenN + 1] = hit.seg.y - hit.seg.x;
                 }
@@ -1339,6 +1344,9 @@ __device__ __forceinline__ void run_task(Smem<B>& sm, const DevIndex& ix, const 
             // Candidates j = tid, tid + B, ... one at a time (groups of 2 and 4
             // with their loads issued together measured slower)
             {
+                const int* const vals = lv.vals;
+                const uint32_t* const sigs = lv.sigs;
+                const int sigShift = lv.sigShift;
                 WinCursor<B> cur;
                 for (int j = tid; j < take; j += B) {
                     cur.seek(sm, nw, j);
@@ -1346,14 +1354,14 @@ __device__ __forceinline__ void run_task(Smem<B>& sm, const DevIndex& ix, const 
                     const int e = sm.wBeg[lo] + (j - cur.first(sm));
                     uint32_t sw = ~0u;
                     int n1 = 0, rk = 0;
-                    if (lv.flags & kLvSig) { sw = __ldg(lv.sigs + 2 * (long long)e); mt.add(4); }
-                    const int n0 = __ldg(lv.vals + e);
-                    if (lv.flags & kLvScan) { n1 = __ldg(ix.val[0] + e); mt.add(8); } else mt.add(4);
-                    if (lv.flags & kLvHo) {   // a row scan's rank is the row's place among the predicate's
-                        rk = (lv.flags & kLvRowScan) ? e - lv.rankBase : __ldg(lv.ranks + e);
+                    if (lvf & kLvSig) { sw = __ldg(sigs + 2 * (long long)e); mt.add(4); }
+                    const int n0 = __ldg(vals + e);
+                    if (lvf & kLvScan) { n1 = __ldg(ix.val[0] + e); mt.add(8); } else mt.add(4);
+                    if (lvf & kLvHo) {   // a row scan's rank is the row's place among the predicate's
+                        rk = (lvf & kLvRowScan) ? e - lv.rankBase : __ldg(lv.ranks + e);
                         mt.add(4);
                     }
-                    if ((sw >> lv.sigShift) & 1u) eval(lo, n0, n1, rk, j);
+                    if ((sw >> sigShift) & 1u) eval(lo, n0, n1, rk, j);
                 }
             }
             // where the next round at this level starts: the item holding
@@ -1370,7 +1378,7 @@ __device__ __forceinline__ void run_task(Smem<B>& sm, const DevIndex& ix, const 
                     cutOff = take - c.first(sm) + (c.item == 0 ? off : 0);
                 }
             }
-            if (anyHub && (lv.flags & kLvClaims)) {
+            if (anyHub && (lvf & kLvClaims)) {
                 // items of a (root, hub row) after enough middle values add nothing
                 hub_claims(P.hubSeen + (long long)blockIdx.x * kHubSeen, baseK + w0 * strideK, strideK, cut,
                            P.steps[k].keyRef == kTupleHead + 1 ? kTupleHead + 2 : kTupleHead + 1, sm.wBeg, B,
@@ -1444,10 +1452,10 @@ __device__ __forceinline__ void run_task(Smem<B>& sm, const DevIndex& ix, const 
                 // blocks past the end of the queue are idle; once a sixteenth
                 // of the launch is, the items left here are worth a follow-up
                 // launch
-                if (tid == 0 && sp.out >= 0 && (clock64() - S.lookAt > kSpillEvery || sp.always)) {
-                    S.lookAt = clock64();
+                if (tid == 0 && clock64() > S.lookAt) {
                     const int idle = *reinterpret_cast<const volatile int*>(S.queue) - S.nTasks;
-                    if ((idle * 16 >= (int)gridDim.x || sp.always) && !sortMode && !blockRows) S.spill = 1;
+                    S.lookAt = sp.always ? 0 : clock64() + kSpillEvery;
+                    if (idle * 16 >= (int)gridDim.x || sp.always) S.spill = 1;
                 }
             }
             __syncthreads();
@@ -1513,15 +1521,17 @@ __device__ __forceinline__ void run_task(Smem<B>& sm, const DevIndex& ix, const 
 // the algorithmic bytes; 3 records task times under a deadline (served
 // launches: past prof.budgetNs from the block's start the block abandons
 // its task at the end of a frontier round, skips the rest, and marks the
-// plans that lost a task in prof.incomplete).
+// plans that lost a task in prof.incomplete); 4 one plan that comes with the
+// launch (InlineLaunch).
 template <int B, int kI>
 __global__ void __launch_bounds__(B, 1024 / B)
 engine_kernel(const __grid_constant__ DevIndex ix, const DevPlan* __restrict__ plans, const DevTask* __restrict__ tasks,
               int nTasks, int* taskCounter, unsigned long long* results, int* status, EngineProfile prof,
-              const __grid_constant__ SpillArgs sp) {
+              const __grid_constant__ SpillArgs sp, const __grid_constant__ InlineLaunch in) {
     constexpr bool kC = kI == 2;
     constexpr bool kD = kI == 3;
     constexpr bool kS = kI == 0;   // only the plain variant spills: the others time whole tasks
+    constexpr bool kIn = kI == 4;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     Smem<B>& sm = *reinterpret_cast<Smem<B>*>(smem_raw);
     Meter<kC> mt;
@@ -1537,12 +1547,13 @@ engine_kernel(const __grid_constant__ DevIndex ix, const DevPlan* __restrict__ p
         if (nTasks == 0) return;
     }
     if (threadIdx.x == 0) {
-        sm.st.nTasks = nTasks;
+        sm.st.nTasks = nTasks - (int)gridDim.x;   // those the counter deals out
         sm.st.queue = taskCounter;
     }
-    for (;;) {
+    // a block's first task is its own number, the others come from the counter
+    for (bool first = true;; first = false) {
         if (threadIdx.x == 0) {
-            sm.st.task = atomicAdd(taskCounter, 1);
+            sm.st.task = first ? (int)blockIdx.x : (int)gridDim.x + atomicAdd(taskCounter, 1);
             if constexpr (kD) sm.st.stop = global_ns() > sm.st.deadline ? 1 : 0;
         }
         __syncthreads();
@@ -1554,6 +1565,9 @@ engine_kernel(const __grid_constant__ DevIndex ix, const DevPlan* __restrict__ p
             st = sp.tasks[sp.in & 1] + t;
             task = DevTask{st->plan, st->beg, st->beg + st->G, 0, 0, -1};
             if (st->level < 0) st = nullptr;   // roots that no block had begun
+        } else if constexpr (kIn) {
+            const int b = in.beg + t * in.chunk;
+            task = DevTask{0, b, min(in.end, b + in.chunk), 0, 0, -1};
         } else {
             task = tasks[t];
         }
@@ -1565,7 +1579,7 @@ engine_kernel(const __grid_constant__ DevIndex ix, const DevPlan* __restrict__ p
             }
         }
         unsigned long long t0 = 0;
-        if constexpr (kI >= 1) {
+        if constexpr (kI >= 1 && kI <= 3) {
             if (threadIdx.x == 0) {
                 mt.add(sizeof(DevTask) + sizeof(DevPlan) + 8);
                 t0 = global_ns();
@@ -1573,16 +1587,17 @@ engine_kernel(const __grid_constant__ DevIndex ix, const DevPlan* __restrict__ p
         }
         if (task.plan != loaded) {   // (a plan's tasks often follow one another)
             loaded = task.plan;
-            const int* src = reinterpret_cast<const int*>(plans + task.plan);
+            const int* src = reinterpret_cast<const int*>(kIn ? &in.plan : plans + task.plan);
             int* dst = reinterpret_cast<int*>(&sm.plan);
             for (int i = threadIdx.x; i < (int)(sizeof(DevPlan) / 4); i += B) dst[i] = src[i];
             __syncthreads();
         }
         // a task of several groups of roots: one after the other
         const int group = st ? INT_MAX : max(1, sm.plan.groupMax);
+        if (kS && threadIdx.x == 0) sm.st.rootsEnd = task.end;   // (read after run_task's first barrier)
         for (DevTask part = task; part.beg < task.end;) {
             part.end = group < task.end - part.beg ? part.beg + group : task.end;
-            run_task<B, kC, kD, kS>(sm, ix, part, results, status, mt, sp, st, task.end);
+            run_task<B, kC, kD, kS>(sm, ix, part, results, status, mt, sp, st);
             __syncthreads();
             if constexpr (kD) {
                 if (sm.st.stop) break;
@@ -1595,10 +1610,11 @@ engine_kernel(const __grid_constant__ DevIndex ix, const DevPlan* __restrict__ p
             }
             part.beg = part.end;
         }
+        if (kIn && nTasks <= (int)gridDim.x) break;   // every block has had its one task
         if constexpr (kD) {
             if (threadIdx.x == 0 && sm.st.stop) atomicOr(prof.incomplete + task.plan, 1);
         }
-        if constexpr (kI >= 1) {
+        if constexpr (kI >= 1 && kI <= 3) {
             if (threadIdx.x == 0 && prof.taskNs) {
                 prof.taskNs[2 * t] = t0;
                 prof.taskNs[2 * t + 1] = global_ns();
@@ -1611,6 +1627,25 @@ engine_kernel(const __grid_constant__ DevIndex ix, const DevPlan* __restrict__ p
         if ((threadIdx.x & 31) == 0 && b && prof.bytes) atomicAdd(prof.bytes, b);
     }
     if (prof.span && threadIdx.x == 0) atomicMax(prof.span + 1, global_ns());
+    if (kIn && in.publish) {
+        __syncthreads();   // the block's results are out
+        if (threadIdx.x == 0) {
+            int* words = static_cast<int*>(in.ctl);
+            __threadfence();
+            if (atomicAdd(words + kInlineWords, 1) == (int)gridDim.x - 1) {   // the last block
+                __threadfence();
+                int4* src = static_cast<int4*>(in.ctl);
+                int4* dst = static_cast<int4*>(in.host);
+                for (int i = 0; i < kInlineWords / 4; ++i) {
+                    dst[i] = __ldcg(src + i);
+                    src[i] = make_int4(0, 0, 0, 0);
+                }
+                words[kInlineWords] = 0;
+                __threadfence_system();   // the words before their flag; the cleared ones before the next launch's
+                *(static_cast<volatile int*>(in.host) + kInlineWords) = in.seq;
+            }
+        }
+    }
 }
 
 template <int B>
@@ -1623,6 +1658,8 @@ static cudaError_t configure_b() {
         e = cudaFuncSetAttribute(engine_kernel<B, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(engine_kernel<B, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(engine_kernel<B, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     return e;
 }
 
@@ -1644,17 +1681,19 @@ cudaError_t engine_configure() {
 template <int B>
 static void launch_b(const DevIndex& ix, const DevPlan* plans, const DevTask* tasks, int nTasks, int* taskCounter,
                      unsigned long long* results, int* status, int grid, cudaStream_t stream,
-                     const EngineProfile* prof, const SpillArgs& sp) {
+                     const EngineProfile* prof, const SpillArgs& sp, const InlineLaunch& in) {
     const size_t smem = sizeof(Smem<B>);
     const EngineProfile p = prof ? *prof : EngineProfile{};
-    if (p.bytes)
-        engine_kernel<B, 2><<<grid, B, smem, stream>>>(ix, plans, tasks, nTasks, taskCounter, results, status, p, sp);
+    if (in.on)
+        engine_kernel<B, 4><<<grid, B, smem, stream>>>(ix, plans, tasks, nTasks, taskCounter, results, status, p, sp, in);
+    else if (p.bytes)
+        engine_kernel<B, 2><<<grid, B, smem, stream>>>(ix, plans, tasks, nTasks, taskCounter, results, status, p, sp, in);
     else if (p.budgetNs && p.incomplete && p.taskNs)
-        engine_kernel<B, 3><<<grid, B, smem, stream>>>(ix, plans, tasks, nTasks, taskCounter, results, status, p, sp);
+        engine_kernel<B, 3><<<grid, B, smem, stream>>>(ix, plans, tasks, nTasks, taskCounter, results, status, p, sp, in);
     else if (p.taskNs)
-        engine_kernel<B, 1><<<grid, B, smem, stream>>>(ix, plans, tasks, nTasks, taskCounter, results, status, p, sp);
+        engine_kernel<B, 1><<<grid, B, smem, stream>>>(ix, plans, tasks, nTasks, taskCounter, results, status, p, sp, in);
     else
-        engine_kernel<B, 0><<<grid, B, smem, stream>>>(ix, plans, tasks, nTasks, taskCounter, results, status, p, sp);
+        engine_kernel<B, 0><<<grid, B, smem, stream>>>(ix, plans, tasks, nTasks, taskCounter, results, status, p, sp, in);
 }
 
 // Suffix memos (see memo_item): one block per job (a hub row x of one
@@ -1876,12 +1915,14 @@ cudaError_t memo_build(const DevIndex& ix, const MemoJob* jobs, int nJobs, int m
 // prof->span is set (any variant).
 cudaError_t engine_launch(const DevIndex& ix, const DevPlan* plans, const DevTask* tasks, int nTasks,
                           int* taskCounter, unsigned long long* results, int* status, int grid, int block,
-                          cudaStream_t stream, const EngineProfile* prof, const SpillArgs& sp) {
+                          cudaStream_t stream, const EngineProfile* prof, const SpillArgs& sp, const InlineLaunch* in) {
     if (nTasks <= 0 && sp.in < 0) return cudaSuccess;
+    static const InlineLaunch none{};
+    const InlineLaunch& il = in ? *in : none;
     switch (block) {
-        case 128: launch_b<128>(ix, plans, tasks, nTasks, taskCounter, results, status, grid, stream, prof, sp); break;
-        case 256: launch_b<256>(ix, plans, tasks, nTasks, taskCounter, results, status, grid, stream, prof, sp); break;
-        case 512: launch_b<512>(ix, plans, tasks, nTasks, taskCounter, results, status, grid, stream, prof, sp); break;
+        case 128: launch_b<128>(ix, plans, tasks, nTasks, taskCounter, results, status, grid, stream, prof, sp, il); break;
+        case 256: launch_b<256>(ix, plans, tasks, nTasks, taskCounter, results, status, grid, stream, prof, sp, il); break;
+        case 512: launch_b<512>(ix, plans, tasks, nTasks, taskCounter, results, status, grid, stream, prof, sp, il); break;
         default: return cudaErrorInvalidValue;
     }
     return cudaGetLastError();

@@ -110,13 +110,19 @@ private:
     const pid_t pid_;
 };
 
+// The host's logical processors (asking the system costs microseconds, more
+// than a small loop's work).
+inline unsigned host_threads() {
+    static const unsigned n = std::max(1u, std::thread::hardware_concurrency());
+    return n;
+}
+
 // Calls fn(i) for i in [0, n) on up to maxThreads threads (the calling
 // thread included), in chunks of `grain`; serial below 2 * grain items.
 // The first exception thrown by fn stops the loop and is rethrown here.
 template <class Fn>
 void parallel_for(size_t n, Fn fn, size_t grain = 64, unsigned maxThreads = 16) {
-    const unsigned hw = std::max(1u, std::thread::hardware_concurrency());
-    const unsigned t = (unsigned)std::min<size_t>(std::min(hw, maxThreads), n / std::max<size_t>(grain, 1));
+    const unsigned t = (unsigned)std::min<size_t>(std::min(host_threads(), maxThreads), n / std::max<size_t>(grain, 1));
     if (t <= 1) {
         for (size_t i = 0; i < n; ++i) fn(i);
         return;
@@ -159,8 +165,7 @@ void parallel_for(size_t n, Fn fn, size_t grain = 64, unsigned maxThreads = 16) 
 // merged pairwise, level by level, in parallel.
 template <class T, class Cmp>
 void parallel_sort(std::vector<T>& v, Cmp cmp, size_t minChunk = size_t(1) << 16) {
-    const unsigned hw = std::max(1u, std::thread::hardware_concurrency());
-    size_t parts = std::min<size_t>(std::min(hw, 16u), v.size() / std::max<size_t>(minChunk, 1));
+    size_t parts = std::min<size_t>(std::min(host_threads(), 16u), v.size() / std::max<size_t>(minChunk, 1));
     if (parts < 2) {
         std::sort(v.begin(), v.end(), cmp);
         return;

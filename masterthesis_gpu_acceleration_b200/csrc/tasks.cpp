@@ -482,6 +482,10 @@ void TaskBuilder::build(const std::vector<const PhasePlan*>& phases, int blocks,
             if (per > 0 && per * chunk > target) chunk = std::max<int32_t>(1, (int32_t)(target / per));
             if (groups && chunk > one) chunk -= chunk % one;
             else chunk = std::min(chunk, one);
+            pt.chunk = chunk;
+            const size_t nt = (size_t)((R + chunk - 1) / std::max(chunk, 1));
+            pt.tasks.reserve(nt);
+            pt.cost.reserve(nt);
             for (int32_t b = ph.rootBeg; b < ph.rootEnd; b += chunk) {
                 const int32_t e = std::min(ph.rootEnd, b + chunk);
                 pt.tasks.push_back(DevTask{(int32_t)i, b, e, 0, 0, -1});

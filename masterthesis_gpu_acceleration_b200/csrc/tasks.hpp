@@ -31,6 +31,7 @@ struct PhaseTasks {
     int32_t heavyRows = 0;      // global dedup rows used by split roots
     double work = 0.0;          // estimated work of the whole phase
     double scale = 1.0;         // learned device ns per unit of work
+    int32_t chunk = 0;          // > 0: the tasks are equal runs of this many roots (the last may be shorter)
 };
 
 // Builds tasks for a batch of phases.  Work is measured in candidate
