@@ -243,8 +243,9 @@ enum DedupMode : int32_t {
     kDedupShared = 0,     // bitmap rows in the block's shared pool (the task's roots)
     kDedupRows = 1,       // one global bitmap row per root of the phase, cleared before the launch
     kDedupBlockRows = 2,  // global rows per resident block for its current task, cleared by the block
-    kDedupSort = 3,       // 64-bit pair keys appended, radix-sorted and counted once each
+    kDedupSort = 3,       // 64-bit pair keys appended, parted by a hash and counted once each
 };
+constexpr int kSortSetKeys = 6144;   // most keys of a part's hash set (sort.cu)
 
 // A unit of device work: the roots [beg, end) of one plan, in groups of at
 // most the plan's groupMax.  A heavy root is

@@ -639,7 +639,7 @@ void Staged::enqueue_sort(Context& c, cudaStream_t s, unsigned long long* result
     auto* tmp = keys + keyCap;
     auto* hist = reinterpret_cast<uint32_t*>(tmp + keyCap);
     ck(pairs_sort_count(keys, tmp, cursor, keyCap, sortBits, sortSlotShift, dSortSlots, nSort, results, status,
-                        hist, std::max(c.sms, 1) * 8, s),
+                        hist, std::max(c.sms, 1) * 8, c.sortSet, s),
        "pair sort");
 }
 
@@ -1120,6 +1120,10 @@ void finish_load(Context* c) {
     // task spills after its first round
     if (const char* h = std::getenv("GPU_RULES_SPILL")) c->spill = std::max(0, std::min(2, std::atoi(h)));
     // GPU_RULES_HOST_PROFILE=1: one stderr line of host-side times per one-shot batch
+    // GPU_RULES_SORT_SET: keys a hash set of sort mode takes before its part of
+    // the keys is split (fewer: more splits)
+    if (const char* h = std::getenv("GPU_RULES_SORT_SET"))
+        c->sortSet = std::max(16, std::min(kSortSetKeys, std::atoi(h)));
     if (const char* h = std::getenv("GPU_RULES_HOST_PROFILE")) c->hostProfile = std::atoi(h) != 0;
     c->tasks.reset(new TaskBuilder(c->hix));
     // GPU_RULES_PLAN_BOTH_ENDS=0: body sizes always from the head subject's end

@@ -44,9 +44,10 @@ cudaError_t engine_launch(const DevIndex& ix, const DevPlan* plans, const DevTas
                           int* taskCounter, unsigned long long* results, int* status, int grid, int block,
                           cudaStream_t stream, const EngineProfile* prof, const SpillArgs& sp = SpillArgs{},
                           const InlineLaunch* in = nullptr);
-// Sort mode (sort.cu): radix sort of the appended pair keys and the count of
-// each plan's distinct keys into its result slot.
+// Sort mode (sort.cu): parts the appended pair keys by a hash and counts each
+// plan's distinct keys into its result slot.
 size_t pairs_sort_hist_words(unsigned long long cap);
+int pairs_sort_passes(unsigned long long cap);   // radix passes that part `cap` keys into buckets
 // Sorts min(*count, cap) keys by their low `bits` bits (8 bits a pass,
 // stable), ping-ponging with tmp; returns the buffer that holds the result.
 unsigned long long* radix_sort_keys(unsigned long long* keys, unsigned long long* tmp, const unsigned long long* count,
@@ -54,7 +55,7 @@ unsigned long long* radix_sort_keys(unsigned long long* keys, unsigned long long
                                     cudaError_t* err);
 cudaError_t pairs_sort_count(unsigned long long* keys, unsigned long long* tmp, const unsigned long long* count,
                              unsigned long long cap, int bits, int slotShift, const int32_t* slotOf, int nSlots,
-                             unsigned long long* results, int* status, uint32_t* hist, int grid,
+                             unsigned long long* results, int* status, uint32_t* hist, int grid, int setKeys,
                              cudaStream_t stream);
 
 // Records the calling thread's last error (gpu_last_error) and logs it.
@@ -206,7 +207,7 @@ struct Staged {
     int kernels_per_enqueue() const {
         if (!nPlans) return 0;
         return (nTasks > 0 ? 1 : 0) + (nTasks > 0 && spillable ? kFollowUps : 0) +
-               (nSupJobs > 0 || (spillable && extraResults > 0) ? 1 : 0) + (nSort ? 3 * ((sortBits + 7) / 8) + 1 : 0);
+               (nSupJobs > 0 || (spillable && extraResults > 0) ? 1 : 0) + (nSort ? 3 * pairs_sort_passes(keyCap) + 1 : 0);
     }
     // instr: 0 plain, 1 task times into dTaskNs, 2 also algorithmic bytes
     // into dBytes.  gridCap > 0 limits the launch to that many blocks (a
@@ -321,6 +322,7 @@ struct Context {
     int spill = 1;             // 1: long tasks spill into follow-up launches (see SpillTask); 2: every task (tests)
     bool hubClaims = true;     // repeated leaf hub items of a root are skipped (see kHubSeen)
     bool hostProfile = false;  // one-shot batches print their host-side times
+    int sortSet = kSortSetKeys;   // keys of a hash set of sort mode
     std::unordered_map<uint64_t, std::unique_ptr<SuffixMemo>> memos;
     std::vector<std::unique_ptr<DevBuf>> memoChunks;   // arenas the memos are taken from
     size_t memoUsed = 0;                               // bytes taken of the last one
