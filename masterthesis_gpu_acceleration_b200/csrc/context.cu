@@ -365,13 +365,15 @@ void Staged::stage(Context& c, std::vector<DevPlan>& plans, const std::vector<co
         cost.insert(cost.end(), pts[i].cost.begin(), pts[i].cost.end());
     }
     // Spilling pays where a task can outlast the others: not for launches
-    // whose estimated work is below about 60 us of the whole GPU (their
-    // follow-up launches, a few us, would cost more than a tail saves), and
-    // not for sort mode, whose key count must not depend on it.
+    // whose estimated work is below about 150 us of the whole GPU, and not for
+    // sort mode, whose key count must not depend on it.  (Measured with and
+    // without: at 66 us, 25 rules of a dense graph, 219 and 151 us; at 169 us,
+    // 200 long rules, 805 and 778 us; at 188 us, 1,329 mined rules, 836 and
+    // 924 us; at 4,500 us, 10,000 rules, 5.5 and 6.9 ms.)
     double workNs = 0;
     for (int i = 0; i < nPlans; ++i) workNs += pts[i].work * pts[i].scale;
     spillAlways = c.spill == 2;
-    spillable = c.spill && nSort == 0 && (spillAlways || workNs > 60e3 * std::max(c.grid, 1));
+    spillable = c.spill && nSort == 0 && (spillAlways || workNs > 150e3 * std::max(c.grid, 1));
     if (dCtl.cap == 0) ctlClean = false;
     dCtl.ensure(kCtlBytes, as);
     if (hCtl.cap == 0) {
