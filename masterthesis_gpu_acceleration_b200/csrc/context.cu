@@ -373,7 +373,7 @@ void Staged::stage(Context& c, std::vector<DevPlan>& plans, const std::vector<co
     double workNs = 0;
     for (int i = 0; i < nPlans; ++i) workNs += pts[i].work * pts[i].scale;
     spillAlways = c.spill == 2;
-    spillable = c.spill && nSort == 0 && (spillAlways || workNs > 150e3 * std::max(c.grid, 1));
+    spillable = maySpill && c.spill && nSort == 0 && (spillAlways || workNs > 150e3 * std::max(c.grid, 1));
     if (dCtl.cap == 0) ctlClean = false;
     dCtl.ensure(kCtlBytes, as);
     if (hCtl.cap == 0) {
@@ -539,19 +539,33 @@ void Context::ensure_memos(const std::vector<std::array<int, 6>>& keys, cudaStre
     }
     if (take.empty()) return;
     const size_t tabTotal = tabBytes * take.size();
-    // from the last arena, or a new one: cudaMalloc waits for every stream,
-    // which a served request's first memo would pay for
+    // one block per slice of a row's values, so that the paths of a long row
+    // spread over the SMs
+    constexpr int32_t kSlice = 64, kScanRows = 2048;
+    size_t nJobs = 0;
+    for (size_t i : take)
+        for (int32_t r : rowsOf[i])
+            nJobs += r < 0 ? (size_t)((domain(fresh[i]) + kScanRows - 1) / kScanRows)
+                           : (size_t)((h.rowBeg[fresh[i][1]][r + 1] - h.rowBeg[fresh[i][1]][r] + kSlice - 1) / kSlice);
+    // From the last arena, or a new one; the job list uses the room behind the
+    // memos until they are built.  Stream-ordered: cudaMalloc and cudaFree wait
+    // for every stream, and a server's launch that met new memos stalled for
+    // 10-900 ms in them (p99 latency of 10,000 requests/s 100-730 ms where a
+    // stall fell, 2 ms otherwise).
     const size_t need = (tabTotal + bitTotal + 255) & ~size_t(255);
-    if (memoChunks.empty() || memoUsed + need > memoChunks.back()->cap) {
+    const size_t jobBytes = nJobs * sizeof(MemoJob);
+    if (memoChunks.empty() || memoUsed + need + jobBytes > memoChunks.back()->cap) {
         auto chunk = std::make_unique<DevBuf>();
-        const size_t cap = std::max(need, kMemoArenaBytes);
-        ck(cudaMalloc(&chunk->p, cap), "cudaMalloc(memos)");   // never resized
+        const size_t cap = std::max(need + jobBytes, kMemoArenaBytes);
+        ck(cudaMallocAsync(&chunk->p, cap, s), "cudaMallocAsync(memos)");   // never resized
         chunk->cap = cap;
+        chunk->pooled = true;
         memoChunks.push_back(std::move(chunk));
         memoUsed = 0;
     }
     char* base = static_cast<char*>(memoChunks.back()->p) + memoUsed;
     memoUsed += need;
+    MemoJob* const dJobs = reinterpret_cast<MemoJob*>(base + need);
     std::vector<int32_t> tabs(tabTotal / 4, -1);
     std::vector<MemoJob> all;
     for (size_t t = 0; t < take.size(); ++t) {
@@ -568,16 +582,12 @@ void Context::ensure_memos(const std::vector<std::array<int, 6>>& keys, cudaStre
         const std::vector<int32_t>& rows = rowsOf[i];
         for (size_t j = 0; j < rows.size(); ++j) {
             if (p1 < 0) {
-                constexpr int32_t kRows = 2048;   // rows a block
-                for (int32_t b0 = 0; b0 < wo; b0 += kRows)
-                    all.push_back(MemoJob{p2, d2, p2, d2, -1, words, -1, 0, wo, b0, std::min(wo, b0 + kRows), 0, bits});
+                for (int32_t b0 = 0; b0 < wo; b0 += kScanRows)
+                    all.push_back(MemoJob{p2, d2, p2, d2, -1, words, -1, 0, wo, b0, std::min(wo, b0 + kScanRows), 0, bits});
                 continue;
             }
             tab[h.hubOf[d1][rows[j]]] = (int32_t)j;
             m->rowHasMemo[(size_t)(rows[j] - h.predRow[d1][p1])] = 1;
-            // one block per slice of the row's values, so that the paths of a
-            // long row spread over the SMs
-            constexpr int32_t kSlice = 64;
             const int32_t len = h.rowBeg[d1][rows[j] + 1] - h.rowBeg[d1][rows[j]];
             for (int32_t b0 = 0; b0 < len; b0 += kSlice)
                 all.push_back(MemoJob{p1, d1, p2, d2, rows[j], words, p3, d3, wo, b0, std::min(len, b0 + kSlice), 0,
@@ -592,13 +602,11 @@ void Context::ensure_memos(const std::vector<std::array<int, 6>>& keys, cudaStre
     }
     ck(cudaMemcpyAsync(base, tabs.data(), tabTotal, cudaMemcpyHostToDevice, s), "H2D memo tables");
     ck(cudaMemsetAsync(base + tabTotal, 0, bitTotal, s), "clear memo bits");
-    memoJobs.ensure(all.size() * sizeof(MemoJob));
-    ck(cudaMemcpyAsync(memoJobs.p, all.data(), all.size() * sizeof(MemoJob), cudaMemcpyHostToDevice, s),
-       "H2D memo jobs");
+    ck(cudaMemcpyAsync(dJobs, all.data(), all.size() * sizeof(MemoJob), cudaMemcpyHostToDevice, s), "H2D memo jobs");
     int maxWo = 0;
     for (const MemoJob& j : all)
         if (j.p3 >= 0) maxWo = std::max(maxWo, j.wo);
-    ck(memo_build(dix, static_cast<const MemoJob*>(memoJobs.p), (int)all.size(), maxWo, s), "memo build");
+    ck(memo_build(dix, dJobs, (int)all.size(), maxWo, s), "memo build");
     ck(cudaStreamSynchronize(s), "memo build");   // memos are shared by every stream afterwards
 }
 

@@ -169,6 +169,7 @@ struct Staged {
     // before it): counters, status and per-plan words first, then spilling's.
     static constexpr size_t kSpillCtlAt = 64, kCtlBytes = 192;
     static_assert(kSpillCtlAt + sizeof(SpillCtl) <= kCtlBytes, "control words");
+    bool maySpill = true;                  // false: only timed launches (served ones), which never spill
     bool spillable = false;                // launches of this staging may spill
     bool spillAlways = false;
     SpillArgs spill_args() const;
@@ -336,7 +337,6 @@ struct Context {
     // The memo of a key if built, null when none exists or no hub row of
     // (p1, d1) is worth one.
     const SuffixMemo* memo_for(int p1, int d1, int p2, int d2, int p3 = -1, int d3 = 0) const;
-    DevBuf memoJobs;
     int serveLanes = 1;        // servers started on this context keep a heavy lane
     int serveHeavyShare = 2;   // the heavy lane launches on grid / serveHeavyShare blocks
     double serveHeavyNs = 5.0e6;

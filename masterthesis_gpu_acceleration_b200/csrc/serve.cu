@@ -356,6 +356,7 @@ void* gpu_serve_start(void* ctx, int slots, int maxBatch, long long memBudgetByt
             ck(cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking), "cudaStreamCreate");
             for (cudaEvent_t* ev : {&s->start, &s->kend, &s->done}) ck(cudaEventCreate(ev), "cudaEventCreate");
             s->st.streamOrdered = true;
+            s->st.maySpill = false;
             s->st.reserve(std::min<size_t>(kReservePlans, 2 * (size_t)maxBatch), kReserveTasks, s->stream);
             s->hTaskNs.ensure(kReserveTasks * 16);
             sv->slots.push_back(std::move(s));
