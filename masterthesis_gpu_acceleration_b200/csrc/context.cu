@@ -120,10 +120,10 @@ void longest_first(std::vector<DevTask>& tasks, std::vector<double>& cost, size_
 }
 }  // namespace
 
-void Staged::stage(Context& c, std::vector<DevPlan>& plans, const std::vector<const PhasePlan*>& phases,
+void Staged::stage(Context& c, const std::vector<const PhasePlan*>& phases, const std::vector<PlanSup>& sups,
                    bool sortTasks, cudaStream_t s, double walkBudget, bool costAware, bool allowSort, bool mayInline) {
     inl.clear();
-    nPlans = (int)plans.size();
+    nPlans = (int)phases.size();
     nResults = nPlans + extraResults;
     stagedBlock = c.geom.block;
     nTasks = 0;
@@ -153,9 +153,16 @@ void Staged::stage(Context& c, std::vector<DevPlan>& plans, const std::vector<co
         return est[i];
     };
     size_t fullTotal = 0;
+    // the phases lie in their rules' plans, a few cache lines each: passes over
+    // all of them run on host threads
+    auto plan = [&](int i) -> const DevPlan& { return phases[i]->plan; };
+    std::vector<uint8_t> global(nPlans, 0);
+    parallel_for((size_t)nPlans, [&](size_t i) {
+        global[i] = plan((int)i).mode == kPairs && (phases[i]->needsGlobalBitmap || c.dedupForce != 0) ? 1 : 0;
+    }, 256);
     for (int i = 0; i < nPlans; ++i) {
-        if (plans[i].mode != kPairs || (!phases[i]->needsGlobalBitmap && c.dedupForce == 0)) continue;
-        fullWords[i] = (size_t)(phases[i]->rootEnd - phases[i]->rootBeg) * (size_t)std::max(plans[i].rowWords, 1);
+        if (!global[i]) continue;
+        fullWords[i] = (size_t)(phases[i]->rootEnd - phases[i]->rootBeg) * (size_t)std::max(plan(i).rowWords, 1);
         fullTotal += fullWords[i];
         dedup[i] = kDedupRows;
     }
@@ -177,7 +184,7 @@ void Staged::stage(Context& c, std::vector<DevPlan>& plans, const std::vector<co
     for (int i = 0; i < nPlans; ++i)
         if (dedup[i] == kDedupSort) {
             sortPlans.push_back(i);
-            rankBits = std::max(rankBits, bits_for((uint64_t)std::max(plans[i].wo, 1)));
+            rankBits = std::max(rankBits, bits_for((uint64_t)std::max(plan(i).wo, 1)));
             rowBits = std::max(rowBits, bits_for((uint64_t)std::max(phases[i]->rootEnd - phases[i]->rootBeg, 1)));
         }
     if (!sortPlans.empty()) {
@@ -193,14 +200,14 @@ void Staged::stage(Context& c, std::vector<DevPlan>& plans, const std::vector<co
     }
     if (nSort) {
         // kept so that a run whose keys overflow can be staged again
-        inPlans = plans;
+        inSups = sups;
         inPhases = phases;
         inSortTasks = sortTasks;
         inWalk = walkBudget;
         inCostAware = costAware;
         inAllowSort = allowSort;
     } else {
-        inPlans.clear();
+        inSups.clear();
         inPhases.clear();
     }
     // block rows: every resident block owns a region that holds its current
@@ -209,16 +216,16 @@ void Staged::stage(Context& c, std::vector<DevPlan>& plans, const std::vector<co
     {
         size_t maxRow = 0;
         for (int i = 0; i < nPlans; ++i)
-            if (dedup[i] == kDedupBlockRows) maxRow = std::max(maxRow, (size_t)std::max(plans[i].rowWords, 1));
+            if (dedup[i] == kDedupBlockRows) maxRow = std::max(maxRow, (size_t)std::max(plan(i).rowWords, 1));
         if (maxRow) {
             blockRegions = (size_t)std::max(c.grid, 1);
             const size_t regionCap = std::max(maxRow, budgetWords / blockRegions);
             size_t need = 0;
             for (int i = 0; i < nPlans; ++i) {
                 if (dedup[i] != kDedupBlockRows) continue;
-                const size_t rw = (size_t)std::max(plans[i].rowWords, 1);
+                const size_t rw = (size_t)std::max(plan(i).rowWords, 1);
                 const int32_t g = (int32_t)std::max<size_t>(
-                    1, std::min<size_t>(regionCap / rw, (size_t)std::max(1, std::min(plans[i].cap, 512))));
+                    1, std::min<size_t>(regionCap / rw, (size_t)std::max(1, std::min(plan(i).cap, 512))));
                 lim[i].group = g;
                 lim[i].maxHeavy = (int32_t)std::min<size_t>(INT_MAX, budgetWords / 4 / rw);
                 need = std::max(need, (size_t)g * rw);
@@ -260,22 +267,33 @@ void Staged::stage(Context& c, std::vector<DevPlan>& plans, const std::vector<co
     auto memo3_key_of = [](const DevPlan& P) -> std::array<int, 6> {
         return {P.steps[1].pred, P.steps[1].dir, P.steps[2].pred, P.steps[2].dir, P.steps[3].pred, P.steps[3].dir};
     };
-    for (int i = 0; i < nPlans; ++i) {
-        if (!c.memo3) plans[i].memoSteps = 0;   // three-step memos switched off
-        if (plans[i].memoLevel > 0) {
+    // which of a plan's memos apply in this staging: bit 0 two-step, 1
+    // three-step, 2 scan; and those that are not built yet
+    std::vector<uint8_t> memoUse(nPlans, 0), memoNew(nPlans, 0);
+    parallel_for((size_t)nPlans, [&](size_t i) {
+        if (dedup[i] == kDedupSort) return;   // memos set bitmap words; keys carry every pair
+        const DevPlan& P = plan((int)i);
+        int use = (P.memoLevel > 0 ? 1 : 0) | (P.memoSteps == 3 && c.memo3 ? 2 : 0) | (P.scanLevel > 0 ? 4 : 0);
+        if (use & 1) {
             // the memo leaves x out of x's own neighbours, as injectivity
             // does for a variable; a constant that is its own neighbour stays
             // one, so such a plan enumerates
-            const DevStep& a = plans[i].steps[plans[i].memoLevel - 1];
+            const DevStep& a = P.steps[P.memoLevel - 1];
             if (a.keyRef < 0) {
-                const int32_t e = plans[i].consts[-1 - a.keyRef];
-                if (e >= 0 && c.hix.has_triple(a.pred, e, e)) plans[i].memoLevel = 0;
+                const int32_t e = P.consts[-1 - a.keyRef];
+                if (e >= 0 && c.hix.has_triple(a.pred, e, e)) use &= ~1;
             }
         }
-        if (dedup[i] == kDedupSort) continue;
-        if (plans[i].scanLevel > 0) memoKeys.push_back(scan_key_of(plans[i]));
-        if (plans[i].memoLevel > 0) memoKeys.push_back(memo_key_of(plans[i]));
-        if (plans[i].memoSteps == 3) memoKeys.push_back(memo3_key_of(plans[i]));
+        memoUse[i] = (uint8_t)use;
+        if ((use & 1) && !c.memo_known(memo_key_of(P))) memoNew[i] |= 1;
+        if ((use & 2) && !c.memo_known(memo3_key_of(P))) memoNew[i] |= 2;
+        if ((use & 4) && !c.memo_known(scan_key_of(P))) memoNew[i] |= 4;
+    }, 128);
+    for (int i = 0; i < nPlans; ++i) {
+        if (!memoNew[i]) continue;
+        if (memoNew[i] & 4) memoKeys.push_back(scan_key_of(plan(i)));
+        if (memoNew[i] & 1) memoKeys.push_back(memo_key_of(plan(i)));
+        if (memoNew[i] & 2) memoKeys.push_back(memo3_key_of(plan(i)));
     }
     if (!memoKeys.empty()) c.ensure_memos(memoKeys, s);
     hostSect[1] += host_ms() - tSect;
@@ -287,7 +305,7 @@ void Staged::stage(Context& c, std::vector<DevPlan>& plans, const std::vector<co
     // split heavy roots of plans with fused support: counted after the launch
     std::vector<SupJob> supJobs;
     for (int i = 0; i < nPlans; ++i) {
-        if (plans[i].supN == 0 || pts[i].heavyRows == 0) continue;
+        if (pts[i].heavyRows == 0 || sups.empty() || sups[i].n == 0) continue;
         std::vector<char> seenRow((size_t)pts[i].heavyRows, 0);
         for (const DevTask& t : pts[i].tasks)
             if (t.gRow >= 0 && !seenRow[(size_t)t.gRow]) {
@@ -298,72 +316,91 @@ void Staged::stage(Context& c, std::vector<DevPlan>& plans, const std::vector<co
     nSupJobs = (int)supJobs.size();
     std::vector<size_t> hOff(nPlans, 0);
     heavyWords = 0;
+    auto row_words = [&](int i) -> int32_t { return plan(i).mode == kPairs ? (plan(i).wo + 31) / 32 : 1; };
     for (int i = 0; i < nPlans; ++i) {
-        plans[i].rowWords = plans[i].mode == kPairs ? (plans[i].wo + 31) / 32 : 1;
         hOff[i] = heavyWords;
-        if (dedup[i] != kDedupSort) heavyWords += (size_t)pts[i].heavyRows * plans[i].rowWords;   // keys need no rows
+        if (pts[i].heavyRows && dedup[i] != kDedupSort)
+            heavyWords += (size_t)pts[i].heavyRows * row_words(i);   // keys need no rows
     }
     if (heavyWords) dHeavy.ensure(heavyWords * 4, as);
+    std::vector<int32_t> claimAt(nPlans, -1);
+    if (c.hubClaims)
+        parallel_for((size_t)nPlans, [&](size_t i) {
+            if (dedup[i] != kDedupSort) claimAt[i] = claim_level(plan((int)i));
+        }, 256);
+    bool anyClaims = false;
+    for (int i = 0; i < nPlans; ++i) anyClaims |= claimAt[i] >= 0;
+    if (anyClaims) dHubSeen.ensure((size_t)std::max(c.grid, 1) * kHubSeen * 8, as);
     std::vector<DevTask> tasks;
     std::vector<double> cost;
-    bool anyClaims = false;
-    for (int i = 0; i < nPlans; ++i) anyClaims |= c.hubClaims && dedup[i] != kDedupSort && claim_level(plans[i]) >= 0;
-    if (anyClaims) dHubSeen.ensure((size_t)std::max(c.grid, 1) * kHubSeen * 8, as);
-    for (int i = 0; i < nPlans; ++i) {
-        plans[i].memoTab = plans[i].memo3Tab = nullptr;
-        plans[i].memoBits = plans[i].memo3Bits = plans[i].scanBits = nullptr;
-        if (plans[i].scanLevel > 0) {
-            const std::array<int, 6> k = scan_key_of(plans[i]);
-            const SuffixMemo* m = c.memo_for(k[0], k[1], k[2], k[3], k[4], k[5]);
-            if (m && m->words == plans[i].rowWords) plans[i].scanBits = m->bits;
+    {
+        size_t nt = 0;
+        for (int i = 0; i < nPlans; ++i) nt += pts[i].tasks.size();
+        tasks.reserve(nt);
+        cost.reserve(nt);
+        for (int i = 0; i < nPlans; ++i) {
+            tasks.insert(tasks.end(), pts[i].tasks.begin(), pts[i].tasks.end());
+            cost.insert(cost.end(), pts[i].cost.begin(), pts[i].cost.end());
         }
-        if (plans[i].memoLevel > 0) {
-            const std::array<int, 6> k = memo_key_of(plans[i]);
-            const SuffixMemo* m = c.memo_for(k[0], k[1], k[2], k[3], k[4], k[5]);
-            if (m && (plans[i].mode != kPairs || m->words == plans[i].rowWords)) {
-                plans[i].memoTab = m->tab;
-                plans[i].memoBits = m->bits;
-                plans[i].memoWords = m->words;
+    }
+    // The device's copy of plan i, written straight into the upload buffer
+    // (8,000 plans of 1 KB: copied twice before).
+    auto fill = [&](int i, DevPlan& P) {
+        P = plan(i);
+        P.rowWords = row_words(i);
+        if (!(memoUse[i] & 1)) P.memoLevel = 0;
+        if (!(memoUse[i] & 2)) P.memoSteps = 0;
+        if (memoUse[i] & 4) {
+            const SuffixMemo* m = c.memo_for(scan_key_of(P));
+            if (m && m->words == P.rowWords) P.scanBits = m->bits;
+        }
+        if (memoUse[i] & 1) {
+            const SuffixMemo* m = c.memo_for(memo_key_of(P));
+            if (m && (P.mode != kPairs || m->words == P.rowWords)) {
+                P.memoTab = m->tab;
+                P.memoBits = m->bits;
+                P.memoWords = m->words;
             }
         }
-        if (plans[i].memoSteps == 3) {
-            const std::array<int, 6> k = memo3_key_of(plans[i]);
-            const SuffixMemo* m = c.memo_for(k[0], k[1], k[2], k[3], k[4], k[5]);
-            if (m && m->words == plans[i].rowWords && m->wo == plans[i].wo) {
-                plans[i].memo3Tab = m->tab;
-                plans[i].memo3Bits = m->bits;
+        if (memoUse[i] & 2) {
+            const SuffixMemo* m = c.memo_for(memo3_key_of(P));
+            if (m && m->words == P.rowWords && m->wo == P.wo) {
+                P.memo3Tab = m->tab;
+                P.memo3Bits = m->bits;
             }
         }
-        plans[i].resultSlot = i;
-        plans[i].groupMax = pts[i].group;
+        if (!sups.empty() && sups[i].n > 0) {
+            const auto dom = ho_domain(P);
+            P.supN = sups[i].n;
+            P.supDomPred = dom.first;
+            P.supDomDir = dom.second;
+            for (int j = 0; j < P.supN; ++j) {
+                P.supPred[j] = sups[i].pred[j];
+                P.supSlot[j] = nPlans + sups[i].slot[j];
+            }
+        }
+        P.resultSlot = i;
+        P.groupMax = pts[i].group;
         const int dm = dedup[i];
         uint32_t* gb = static_cast<uint32_t*>(dBitmap.p);
-        plans[i].gBitmap = dm == kDedupRows ? gb + gOff[i] : (dm == kDedupBlockRows ? gb + regionOff : nullptr);
-        plans[i].gRowBase = (dm == kDedupRows || dm == kDedupSort) ? phases[i]->rootBeg : 0;
-        plans[i].gBlockWords = dm == kDedupBlockRows ? (int64_t)blockWords : 0;
-        plans[i].gHeavy = (pts[i].heavyRows && dm != kDedupSort) ? static_cast<uint32_t*>(dHeavy.p) + hOff[i] : nullptr;
-        plans[i].claimLevel = claim_level(plans[i]);
-        plans[i].hubSeen = (anyClaims && dm != kDedupSort && plans[i].claimLevel >= 0)
-                               ? static_cast<unsigned long long*>(dHubSeen.p) : nullptr;
-        plans[i].pairKeys = nullptr;
-        plans[i].keyCursor = nullptr;
-        plans[i].keyCap = 0;
-        plans[i].keyBase = 0;
-        plans[i].rankBits = 0;
+        P.gBitmap = dm == kDedupRows ? gb + gOff[i] : (dm == kDedupBlockRows ? gb + regionOff : nullptr);
+        P.gRowBase = (dm == kDedupRows || dm == kDedupSort) ? phases[i]->rootBeg : 0;
+        P.gBlockWords = dm == kDedupBlockRows ? (int64_t)blockWords : 0;
+        P.gHeavy = (pts[i].heavyRows && dm != kDedupSort) ? static_cast<uint32_t*>(dHeavy.p) + hOff[i] : nullptr;
+        P.claimLevel = claimAt[i];
+        P.hubSeen = claimAt[i] >= 0 ? static_cast<unsigned long long*>(dHubSeen.p) : nullptr;
         if (dm == kDedupSort) {
             const int k = (int)(std::find(sortPlans.begin(), sortPlans.end(), i) - sortPlans.begin());
             char* sb = static_cast<char*>(dSort.p);
-            plans[i].keyCursor = reinterpret_cast<unsigned long long*>(sb);
-            plans[i].pairKeys = reinterpret_cast<unsigned long long*>(sb + 256);
-            plans[i].keyCap = keyCap;
-            plans[i].keyBase = (unsigned long long)k << sortSlotShift;
-            plans[i].rankBits = rankBits;
-            plans[i].memoTab = plans[i].memo3Tab = nullptr;   // memos set bitmap words; keys carry every pair
-            plans[i].memoBits = plans[i].memo3Bits = plans[i].scanBits = nullptr;
+            P.keyCursor = reinterpret_cast<unsigned long long*>(sb);
+            P.pairKeys = reinterpret_cast<unsigned long long*>(sb + 256);
+            P.keyCap = keyCap;
+            P.keyBase = (unsigned long long)k << sortSlotShift;
+            P.rankBits = rankBits;
         }
-        tasks.insert(tasks.end(), pts[i].tasks.begin(), pts[i].tasks.end());
-        cost.insert(cost.end(), pts[i].cost.begin(), pts[i].cost.end());
-    }
+    };
+    anyFused = !supJobs.empty();
+    for (const PlanSup& u : sups) anyFused |= u.n > 0;
     // Spilling pays where a task can outlast the others: not for launches
     // whose estimated work is below about 150 us of the whole GPU, and not for
     // sort mode, whose key count must not depend on it.  (Measured with and
@@ -395,7 +432,7 @@ void Staged::stage(Context& c, std::vector<DevPlan>& plans, const std::vector<co
             L.publish = i + 1 == nPlans ? 1 : 0;
             L.ctl = dCtl.p;
             L.host = hCtl.p;
-            L.plan = plans[i];
+            fill(i, L.plan);
         }
         nTasks = (int)tasks.size();
         d2hBytes = 64;
@@ -424,7 +461,7 @@ void Staged::stage(Context& c, std::vector<DevPlan>& plans, const std::vector<co
     const size_t sortBytes = ((size_t)nSort * sizeof(int32_t) + 15) & ~size_t(15);
     size_t blob = planBytes + taskBytes + sortBytes + (size_t)nSupJobs * sizeof(SupJob);
     hBlob.ensure(blob);
-    std::memcpy(hBlob.p, plans.data(), planBytes);
+    parallel_for((size_t)nPlans, [&](size_t i) { fill((int)i, static_cast<DevPlan*>(hBlob.p)[i]); }, 64);
     std::memcpy(static_cast<char*>(hBlob.p) + planBytes, tasks.data(), taskBytes);
     if (nSort) std::memcpy(static_cast<char*>(hBlob.p) + planBytes + taskBytes, sortPlans.data(), nSort * sizeof(int32_t));
     if (nSupJobs)
@@ -460,9 +497,13 @@ uint64_t memo_key(int p1, int d1, int p2, int d2, int p3 = -1, int d3 = 0) {
 }
 }  // namespace
 
-const SuffixMemo* Context::memo_for(int p1, int d1, int p2, int d2, int p3, int d3) const {
-    auto it = memos.find(memo_key(p1, d1, p2, d2, p3, d3));
+const SuffixMemo* Context::memo_for(const std::array<int, 6>& k) const {
+    auto it = memos.find(memo_key(k[0], k[1], k[2], k[3], k[4], k[5]));
     return it == memos.end() ? nullptr : it->second.get();
+}
+
+bool Context::memo_known(const std::array<int, 6>& k) const {
+    return memos.count(memo_key(k[0], k[1], k[2], k[3], k[4], k[5])) != 0;
 }
 
 void Context::ensure_memos(const std::vector<std::array<int, 6>>& keys, cudaStream_t s) {
@@ -656,9 +697,9 @@ void Staged::enqueue_sort(Context& c, cudaStream_t s, unsigned long long* result
 void Staged::restage(Context& c, cudaStream_t s) {
     if (!nSort) return;
     keyHint = *static_cast<const unsigned long long*>(hSort.p);
-    std::vector<DevPlan> p = inPlans;
-    std::vector<const PhasePlan*> ph = inPhases;
-    stage(c, p, ph, inSortTasks, s, inWalk, inCostAware, inAllowSort);
+    const std::vector<const PhasePlan*> ph = inPhases;
+    const std::vector<PlanSup> su = inSups;
+    stage(c, ph, su, inSortTasks, s, inWalk, inCostAware, inAllowSort);
 }
 
 void Staged::check_geometry(const Context& c) const {
@@ -708,7 +749,7 @@ void Staged::enqueue(Context& c, cudaStream_t s, int instr, int gridCap, unsigne
     if (!instr)
         enqueue_follow_ups(c, s, static_cast<unsigned long long*>(dResults.p), static_cast<int*>(dCtl.p) + 1, nullptr);
     ck(support_rows(c.dix, dPlans, dSupJobs, nSupJobs, static_cast<unsigned long long*>(dResults.p), s,
-                    !instr && extraResults > 0 ? spill_args() : SpillArgs{}, c.sms),
+                    !instr && anyFused ? spill_args() : SpillArgs{}, c.sms),
        "fused support of split roots and spilled tasks");
     enqueue_sort(c, s, static_cast<unsigned long long*>(dResults.p), static_cast<int*>(dCtl.p) + 1);
 }
@@ -759,12 +800,9 @@ void Staged::enqueue_per_plan(Context& c, cudaStream_t s) {
     // (timed with the last plan's phase, the body size where there is one)
     enqueue_follow_ups(c, s, reinterpret_cast<unsigned long long*>(static_cast<char*>(dCtl.p) + kPerPlanResults), ctl + 2,
                        reinterpret_cast<unsigned long long*>(static_cast<char*>(dCtl.p) + 16 + 16 * (nPlans - 1)));
-    bool fusedHere = false;
-    for (const DevPlan* P = static_cast<const DevPlan*>(hBlob.p); P != static_cast<const DevPlan*>(hBlob.p) + nPlans; ++P)
-        fusedHere |= P->supN > 0;
     ck(support_rows(c.dix, dPlans, dSupJobs, nSupJobs,
                     reinterpret_cast<unsigned long long*>(static_cast<char*>(dCtl.p) + kPerPlanResults), s,
-                    fusedHere ? spill_args() : SpillArgs{}, c.sms),
+                    anyFused ? spill_args() : SpillArgs{}, c.sms),
        "fused support of split roots and spilled tasks");
     enqueue_sort(c, s, reinterpret_cast<unsigned long long*>(static_cast<char*>(dCtl.p) + kPerPlanResults), ctl + 2);
 }
@@ -810,8 +848,8 @@ namespace {
 
 // One phase in its own launch (the plain per-rule form), timed by events.
 int64_t run_one_phase(Context& c, const PhasePlan& ph, float* ms) {
-    std::vector<DevPlan> plans{ph.plan};
-    c.one.stage(c, plans, {&ph}, false, c.stream, c.ruleWalkBudget, true);
+    c.one.extraResults = 0;
+    c.one.stage(c, {&ph}, {}, false, c.stream, c.ruleWalkBudget, true);
     for (int attempt = 0;; ++attempt) {
         ck(cudaEventRecord(c.ev[0], c.stream), "event");
         c.one.enqueue(c, c.stream, 0);
@@ -842,11 +880,6 @@ void with_rule_block(Context& c, Fn fn) {
     fn();
 }
 
-// Whether supports may be counted by their body-size plans (fused
-// support, see RulePlan::supFuse): both phases run and no dedup mode is
-// forced.
-bool fusing(const Context& c) { return c.fuseSupport && (c.batchPhases & 3) == 3 && c.dedupForce == 0; }
-
 // Both phases of one rule, each in its own launch timed by its own events,
 // issued back to back with one host synchronisation; a fused support takes
 // no launch of its own.
@@ -856,26 +889,21 @@ int evaluate_parsed(Context& c, const Rule& rule, GpuRuleResult* out) {
     float supMs = 0.f, confMs = 0.f;
     const bool runS = rp.status == kRuleOk && rp.support.how == kDevice;
     const bool runB = rp.status == kRuleOk && rp.body.how == kDevice;
-    std::vector<DevPlan> plans;
+    std::vector<PlanSup> sups;
     std::vector<const PhasePlan*> phases;
     // fused support (see prepare): the body-size launch also counts the
     // support, into per-plan result slot 1; the support takes no launch
-    const bool fused = runS && runB && fusing(c) && rp.supFuse >= 0 && rp.body.plan.mode == kPairs &&
-                       !rp.body.needsGlobalBitmap;
-    if (runS && !fused) { plans.push_back(rp.support.plan); phases.push_back(&rp.support); }
-    if (runB) { plans.push_back(rp.body.plan); phases.push_back(&rp.body); }
+    const bool fused = runS && runB && fusing(c) && fuses(rp);
+    if (runS && !fused) phases.push_back(&rp.support);
+    if (runB) phases.push_back(&rp.body);
     if (fused) {
-        DevPlan& B = plans.back();
-        const auto dom = ho_domain(B);
-        B.supN = 1;
-        B.supDomPred = dom.first;
-        B.supDomDir = dom.second;
-        B.supPred[0] = rp.supFuse;
-        B.supSlot[0] = 1;
+        sups.resize(1);
+        sups[0].n = 1;
+        sups[0].pred[0] = rp.supFuse;   // (its slot, 0, comes after the one plan's own)
     }
-    if (!plans.empty()) {
+    if (!phases.empty()) {
         // one upload, one launch per phase (each timed on the device), one download
-        c.one.stage(c, plans, phases, false, c.stream, c.ruleWalkBudget, true, true, true);
+        c.one.stage(c, phases, sups, false, c.stream, c.ruleWalkBudget, true, true, true);
         for (int attempt = 0;; ++attempt) {
             with_rule_block(c, [&] { c.one.enqueue_per_plan(c, c.stream); });
             c.one.download_spans(c.stream);
@@ -922,34 +950,32 @@ void evaluate_shard(Context& c, const Rule& rule, int shard, int nShards, long l
 }
 
 // Parses and plans n rules and stages their device phases.
-// keepPlans: keep a copy of the plans for restaging (prepared batches that
-// may be autotuned); one-shot chunks skip it.
-void prepare(Batch& b, Context& c, const char* const* rules, int n, int isJson, bool keepPlans = true) {
+// oneShot: for one run (the task builder then walks only what pays).
+void prepare(Batch& b, Context& c, const char* const* rules, int n, int isJson, bool oneShot = false) {
     const double tStart = host_ms();
     b.c = &c;
     b.n = n;
     b.owner.clear();
     b.shared.clear();
-    std::unordered_multimap<uint64_t, int> seen;
-    seen.reserve(2 * (size_t)n);
     if (b.exec) { cudaGraphExecDestroy(b.exec); b.exec = nullptr; }
     if (b.graph) { cudaGraphDestroy(b.graph); b.graph = nullptr; }
-    b.rps.assign(n, RulePlan{});
+    if ((int)b.rps.size() < n) b.rps.resize(n);   // every entry is written below
     b.parseStatus.assign(n, 0);
-    std::vector<DevPlan> plans;
-    std::vector<const PhasePlan*> phases;
-    plans.reserve(2 * (size_t)n);
-    std::vector<uint64_t> hash(2 * (size_t)n, 0);   // per rule: support and body phase hashes
+    b.hash.resize(2 * (size_t)n);   // per rule: support and body phase hashes
+    uint64_t* const hash = b.hash.data();
+    const bool fuse = fusing(c);
     // parsing, planning and hashing only read the graph and the
     // dictionaries: in parallel
     parallel_for((size_t)n, [&](size_t i) {
+        RulePlan& rp = b.rps[i];
         if (!rules[i]) { b.parseStatus[i] = -1; return; }
         try {
             Rule r = isJson ? c.parser->parse_json(rules[i]) : c.parser->parse_text(rules[i]);
-            b.rps[i] = plan_rule(r, c.hix, c.geom, c.fans.get());
-            if (b.rps[i].status == kRuleOk) {
-                if (b.rps[i].support.how == kDevice) hash[2 * i] = phase_hash(b.rps[i].support);
-                if (b.rps[i].body.how == kDevice) hash[2 * i + 1] = phase_hash(b.rps[i].body);
+            rp = plan_rule(r, c.hix, c.geom, c.fans.get());
+            if (rp.status == kRuleOk) {
+                // (a fused support is only hashed if its plan turns out to be full)
+                if (rp.support.how == kDevice && !(fuse && fuses(rp))) hash[2 * i] = phase_hash(rp.support);
+                if (rp.body.how == kDevice) hash[2 * i + 1] = phase_hash(rp.body);
             }
         } catch (const RuleError&) {
             b.parseStatus[i] = -1;
@@ -959,10 +985,19 @@ void prepare(Batch& b, Context& c, const char* const* rules, int n, int isJson, 
     // RulePlan::supFuse) gets no support plan when that plan keeps its pair
     // rows in shared memory (no global dedup bitmap, no forced mode); the
     // count lands in a result slot after the plans' own
-    const bool fuse = fusing(c);
     b.supOf.assign(n, -1);
-    std::vector<std::array<int, 3>> fused;   // {body plan, head predicate, first rule}
-    std::unordered_map<uint64_t, int> fusedAt;
+    std::vector<const PhasePlan*>& phases = b.phases;
+    std::vector<PlanSup>& sups = b.sups;
+    phases.clear();
+    sups.clear();
+    phases.reserve(2 * (size_t)n);
+    sups.reserve(2 * (size_t)n);
+    int nFused = 0;
+    // plans by hash, open addressing: {hash, plan}
+    size_t slots = 64;
+    while (slots < 4 * (size_t)n) slots *= 2;
+    b.seen.assign(slots, -1);
+    b.seenHash.resize(slots);
     for (int i = 0; i < n; ++i) {
         if (b.parseStatus[i] != 0) continue;
         RulePlan& rp = b.rps[i];
@@ -971,69 +1006,59 @@ void prepare(Batch& b, Context& c, const char* const* rules, int n, int isJson, 
         for (int k : {1, 0}) {
             const PhasePlan& ph = k == 0 ? rp.support : rp.body;
             if (ph.how != kDevice || !(c.batchPhases & (1 << k))) continue;
-            if (k == 0 && fuse && rp.supFuse >= 0 && bodyPlan >= 0 && phases[bodyPlan]->plan.mode == kPairs &&
-                !phases[bodyPlan]->needsGlobalBitmap) {
-                const uint64_t key = ((uint64_t)(uint32_t)bodyPlan << 32) | (uint32_t)rp.supFuse;
-                auto it = fusedAt.find(key);
-                if (it != fusedAt.end()) {
-                    b.supOf[i] = it->second;
+            if (k == 0 && fuse && bodyPlan >= 0 && fuses(rp)) {
+                PlanSup& u = sups[(size_t)bodyPlan];
+                int j = 0;
+                while (j < u.n && u.pred[j] != rp.supFuse) ++j;
+                if (j < u.n) {   // one body under one head predicate again
+                    b.supOf[i] = u.slot[j];
                     continue;
                 }
-                DevPlan& B = plans[(size_t)bodyPlan];
-                if (B.supN < kMaxSupFused) {
-                    if (B.supN == 0) {
-                        const auto dom = ho_domain(B);
-                        B.supDomPred = dom.first;
-                        B.supDomDir = dom.second;
-                    }
-                    B.supPred[B.supN] = rp.supFuse;
-                    B.supSlot[B.supN] = (int32_t)fused.size();   // made absolute below
-                    ++B.supN;
-                    fusedAt.emplace(key, (int)fused.size());
-                    b.supOf[i] = (int)fused.size();
-                    fused.push_back({bodyPlan, rp.supFuse, i});
+                if (u.n < kMaxSupFused) {
+                    u.pred[u.n] = rp.supFuse;
+                    u.slot[u.n] = b.supOf[i] = nFused++;
+                    ++u.n;
                     continue;
                 }
+                hash[2 * (size_t)i] = phase_hash(ph);
             }
             // identical computations (same plan and roots, e.g. one body under
             // several heads) run once; the others share the count
             // keyed by hash, confirmed by the full signature (plans are
             // zero-initialised, so equal signatures mean equal computations)
             const uint64_t h = hash[2 * (size_t)i + k];
-            auto range = seen.equal_range(h);
+            size_t at = (size_t)h & (slots - 1);
             int same = -1;
-            for (auto it = range.first; it != range.second && same < 0; ++it)
-                if (phase_equal(*phases[it->second], ph)) same = it->second;
+            for (; b.seen[at] >= 0; at = (at + 1) & (slots - 1))
+                if (b.seenHash[at] == h && phase_equal(*phases[(size_t)b.seen[at]], ph)) {
+                    same = b.seen[at];
+                    break;
+                }
             if (same >= 0) {
                 b.shared.emplace_back(2 * i + k, same);
                 if (k == 1) bodyPlan = same;
                 continue;
             }
-            seen.emplace(h, (int)plans.size());
-            if (k == 1) bodyPlan = (int)plans.size();
-            plans.push_back(ph.plan);
+            b.seen[at] = (int)phases.size();
+            b.seenHash[at] = h;
+            if (k == 1) bodyPlan = (int)phases.size();
             phases.push_back(&ph);
+            sups.emplace_back();
             b.owner.push_back(2 * i + k);
         }
     }
     // fused counts follow the plans' own result slots
-    const int nPlansOwn = (int)plans.size();
-    for (DevPlan& P : plans)
-        for (int j = 0; j < P.supN; ++j) P.supSlot[j] += nPlansOwn;
     for (int i = 0; i < n; ++i)
-        if (b.supOf[i] >= 0) b.supOf[i] += nPlansOwn;
-    b.st.extraResults = (int)fused.size();
+        if (b.supOf[i] >= 0) b.supOf[i] += (int)phases.size();
+    b.st.extraResults = nFused;
     if (!b.stream) ck(cudaStreamCreateWithFlags(&b.stream, cudaStreamNonBlocking), "cudaStreamCreate");
     if (!b.ev0) ck(cudaEventCreate(&b.ev0), "cudaEventCreate");
     if (!b.ev1) ck(cudaEventCreate(&b.ev1), "cudaEventCreate");
-    if (keepPlans) b.plans0 = plans;
-    else b.plans0.clear();
-    b.phases = phases;
     // a one-shot batch walks a phase only when the walk costs less host time
     // than the phase is expected to take on the device; a prepared batch,
     // replayed many times, walks every phase the budget allows
     const double tPlanned = host_ms();
-    b.st.stage(c, plans, phases, true, b.stream, b.walkBudget, !keepPlans);
+    b.st.stage(c, phases, sups, true, b.stream, b.walkBudget, oneShot);
     b.hostPlanMs = tPlanned - tStart;
     b.hostStageMs = host_ms() - tPlanned;
 }
@@ -1299,7 +1324,7 @@ int gpu_evaluate_rules_batch(void* ctx, const char* const* rules, int n, int isJ
         for (int k = 0; k < K; ++k) {
             const int lo = (int)((long long)n * k / K), hi = (int)((long long)n * (k + 1) / K);
             Batch& b = *c.pipe[k];
-            prepare(b, c, rules + lo, hi - lo, isJson, false);
+            prepare(b, c, rules + lo, hi - lo, isJson, true);
             planMs += b.hostPlanMs;
             stageMs += b.hostStageMs;
             ck(cudaEventRecord(b.ev0, b.stream), "event");
@@ -1507,8 +1532,7 @@ int gpu_batch_autotune(void* batch, int rounds) {
             ck(cudaStreamSynchronize(b.stream), "autotune");
             c.tasks->learn(b.phases, b.st.hTasks, b.st.hCost, ns.data(), c.grid);
             drop_graph(b);
-            std::vector<DevPlan> pl = b.plans0;
-            b.st.stage(c, pl, b.phases, true, b.stream, b.walkBudget);
+            b.st.stage(c, b.phases, b.sups, true, b.stream, b.walkBudget);
             ck(cudaStreamSynchronize(b.stream), "restage");
         }
         return 0;

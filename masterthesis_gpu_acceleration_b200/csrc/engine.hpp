@@ -124,6 +124,13 @@ inline int64_t clamp_int(int64_t v) { return std::min<int64_t>(v, INT_MAX); }
 
 struct Context;
 
+// The supports that one body-size plan of a staging counts as well (fused
+// support): head predicates, and result slots counted from the plans' own.
+struct PlanSup {
+    int32_t n = 0;
+    int32_t pred[kMaxSupFused] = {}, slot[kMaxSupFused] = {};
+};
+
 // A set of plans and their tasks resident on the device, with the buffers
 // one launch over them needs.
 struct Staged {
@@ -169,6 +176,7 @@ struct Staged {
     // before it): counters, status and per-plan words first, then spilling's.
     static constexpr size_t kSpillCtlAt = 64, kCtlBytes = 192;
     static_assert(kSpillCtlAt + sizeof(SpillCtl) <= kCtlBytes, "control words");
+    bool anyFused = false;                 // some plan counts supports
     bool maySpill = true;                  // false: only timed launches (served ones), which never spill
     bool spillable = false;                // launches of this staging may spill
     bool spillAlways = false;
@@ -183,7 +191,7 @@ struct Staged {
     bool budgeted = false;              // the last enqueue ran under a deadline
     // inputs of the last staging, kept while it has sort-mode plans so that
     // an overflowing run can be staged again with the exact key count
-    std::vector<DevPlan> inPlans;
+    std::vector<PlanSup> inSups;
     std::vector<const PhasePlan*> inPhases;
     bool inSortTasks = true, inCostAware = false, inAllowSort = true;
     double inWalk = 4.0e6;
@@ -192,7 +200,8 @@ struct Staged {
     // (prepared batches afford more than one-shot or served launches).
     // allowSort: sort mode may be chosen (launches that can be run again
     // when the key buffer overflows; the serving loop cannot).
-    void stage(Context& c, std::vector<DevPlan>& plans, const std::vector<const PhasePlan*>& phases,
+    // sups: per phase, the supports it counts (empty: none).
+    void stage(Context& c, const std::vector<const PhasePlan*>& phases, const std::vector<PlanSup>& sups,
                bool sortTasks, cudaStream_t s, double walkBudget = 4.0e6, bool costAware = false,
                bool allowSort = true, bool mayInline = false);
     // After download + synchronisation: whether sort-mode keys exceeded the
@@ -208,7 +217,7 @@ struct Staged {
     int kernels_per_enqueue() const {
         if (!nPlans) return 0;
         return (nTasks > 0 ? 1 : 0) + (nTasks > 0 && spillable ? kFollowUps : 0) +
-               (nSupJobs > 0 || (spillable && extraResults > 0) ? 1 : 0) + (nSort ? 3 * pairs_sort_passes(keyCap) + 1 : 0);
+               (nSupJobs > 0 || (spillable && anyFused) ? 1 : 0) + (nSort ? 3 * pairs_sort_passes(keyCap) + 1 : 0);
     }
     // instr: 0 plain, 1 task times into dTaskNs, 2 also algorithmic bytes
     // into dBytes.  gridCap > 0 limits the launch to that many blocks (a
@@ -335,8 +344,10 @@ struct Context {
     // by every stream afterwards).
     void ensure_memos(const std::vector<std::array<int, 6>>& keys, cudaStream_t s);
     // The memo of a key if built, null when none exists or no hub row of
-    // (p1, d1) is worth one.
-    const SuffixMemo* memo_for(int p1, int d1, int p2, int d2, int p3 = -1, int d3 = 0) const;
+    // (p1, d1) is worth one; whether the key has been looked at.  (Both only
+    // read: safe on several threads between ensure_memos calls.)
+    const SuffixMemo* memo_for(const std::array<int, 6>& key) const;
+    bool memo_known(const std::array<int, 6>& key) const;
     int serveLanes = 1;        // servers started on this context keep a heavy lane
     int serveHeavyShare = 2;   // the heavy lane launches on grid / serveHeavyShare blocks
     double serveHeavyNs = 5.0e6;
@@ -485,10 +496,12 @@ struct Batch {
     std::vector<int> parseStatus;
     std::vector<int> owner;  // plan -> rule * 2 + phase
     std::vector<int> supOf;  // rule -> result slot of its fused support count, or -1
+    std::vector<uint64_t> hash, seenHash;   // scratch of prepare, kept between its calls
+    std::vector<int> seen;
     // phases identical to an earlier one of the batch (same plan and roots):
     // (rule * 2 + phase, plan whose count they share); computed once per run
     std::vector<std::pair<int, int>> shared;
-    std::vector<DevPlan> plans0;
+    std::vector<PlanSup> sups;               // per staged phase
     std::vector<const PhasePlan*> phases;
     Staged st;
     cudaStream_t stream = nullptr;
@@ -511,6 +524,16 @@ struct Batch {
     }
 };
 
+
+// Whether supports may be counted by their body-size plans (fused support,
+// see RulePlan::supFuse): both phases run and no dedup mode is forced.
+inline bool fusing(const Context& c) { return c.fuseSupport && (c.batchPhases & 3) == 3 && c.dedupForce == 0; }
+// Whether a rule's support can be: its body-size plan keeps its pair rows in
+// shared memory.
+inline bool fuses(const RulePlan& rp) {
+    return rp.support.how == kDevice && rp.body.how == kDevice && rp.supFuse >= 0 && rp.body.plan.mode == kPairs &&
+           !rp.body.needsGlobalBitmap;
+}
 
 inline void Context::free_pipe() {
     for (Batch* b : pipe) delete b;

@@ -25,9 +25,10 @@ enum PhaseHow : int32_t {
 };
 
 struct PhasePlan {
+    PhasePlan() {}                      // (the plan of a static phase stays unset)
     int32_t how = kStatic;
     int64_t value = 0;
-    DevPlan plan{};
+    DevPlan plan;
     int32_t rootBeg = 0, rootEnd = 0;   // root range (edges or rows)
     bool needsGlobalBitmap = false;     // kPairs whose hO domain exceeds the shared bitmap
     double estCost = 0.0;               // autotuner estimate (relative units)

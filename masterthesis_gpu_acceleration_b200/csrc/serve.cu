@@ -239,14 +239,13 @@ struct Server {
             q.pop_front();
         }
         if (s.reqs.empty()) return false;
-        std::vector<DevPlan> plans;
         std::vector<const PhasePlan*> phases;
         s.owner.clear();
         for (size_t i = 0; i < s.reqs.size(); ++i) {
             RulePlan& rp = s.reqs[i].rp;
             if (s.reqs[i].status != 0 || rp.status != kRuleOk) continue;
-            if (rp.support.how == kDevice) { plans.push_back(rp.support.plan); phases.push_back(&rp.support); s.owner.push_back(2 * (int)i); }
-            if (rp.body.how == kDevice) { plans.push_back(rp.body.plan); phases.push_back(&rp.body); s.owner.push_back(2 * (int)i + 1); }
+            if (rp.support.how == kDevice) { phases.push_back(&rp.support); s.owner.push_back(2 * (int)i); }
+            if (rp.body.how == kDevice) { phases.push_back(&rp.body); s.owner.push_back(2 * (int)i + 1); }
         }
         s.mem = mem;
         {
@@ -256,7 +255,7 @@ struct Server {
         s.busy = true;
         const bool heavyWork = s.heavyLane || overflow;
         // no sort mode: a served launch is never run a second time
-        s.st.stage(*c, plans, phases, true, s.stream, heavyWork ? 4.0e6 : 2.0e5, false, false);
+        s.st.stage(*c, phases, {}, true, s.stream, heavyWork ? 4.0e6 : 2.0e5, false, false);
         // Launches record task times, from which the task builder learns
         // each plan shape's cost (the launches that follow split slow plans
         // finer and classify requests by it).

@@ -25,44 +25,13 @@ uint64_t signature(const PhasePlan& ph) { return phase_hash(ph); }
 
 }  // namespace
 
-namespace {
-// The plan without its per-launch fields.
-DevPlan plan_identity(const PhasePlan& ph) {
-    DevPlan p = ph.plan;
-    p.resultSlot = 0;
-    p.gBitmap = nullptr;
-    p.gRowBase = 0;
-    p.gHeavy = nullptr;
-    p.rowWords = 0;
-    p.memoTab = nullptr;
-    p.memoBits = nullptr;
-    p.memo3Tab = nullptr;
-    p.memo3Bits = nullptr;
-    p.scanBits = nullptr;
-    p.memoWords = 0;
-    p.gBlockWords = 0;
-    p.pairKeys = nullptr;
-    p.keyCursor = nullptr;
-    p.keyCap = 0;
-    p.keyBase = 0;
-    p.rankBits = 0;
-    p.pad0 = 0;
-    p.pad2 = 0;
-    p.pad3 = 0;
-    return p;
-}
-}  // namespace
-
 bool phase_equal(const PhasePlan& a, const PhasePlan& b) {
-    if (a.rootBeg != b.rootBeg || a.rootEnd != b.rootEnd) return false;
-    const DevPlan pa = plan_identity(a), pb = plan_identity(b);
-    return std::memcmp(&pa, &pb, sizeof(DevPlan)) == 0;
+    return a.rootBeg == b.rootBeg && a.rootEnd == b.rootEnd && std::memcmp(&a.plan, &b.plan, sizeof(DevPlan)) == 0;
 }
 
 uint64_t phase_hash(const PhasePlan& ph) {
     static_assert(sizeof(DevPlan) % 8 == 0, "plan hashed in 8-byte words");
-    const DevPlan p = plan_identity(ph);
-    const unsigned char* b = reinterpret_cast<const unsigned char*>(&p);
+    const unsigned char* b = reinterpret_cast<const unsigned char*>(&ph.plan);
     // four independent lanes (a quarter of the dependent multiplies each),
     // combined at the end
     uint64_t h[4] = {0x243F6A8885A308D3ull ^ ((uint64_t)(uint32_t)ph.rootBeg << 32 | (uint32_t)ph.rootEnd),

@@ -51,8 +51,9 @@ struct PhaseTasks {
 // Host time of one step of a per-root walk (ns), for the cost-aware mode.
 constexpr double kWalkNsPerEdge = 8.0;
 
-// The signature of a phase is the identity of its device computation: the
-// plan without its per-launch fields, and its root range.  Phases with equal
+// The signature of a phase is the identity of its device computation: its
+// plan as the planner made it (per-launch fields are set in copies of it, so
+// they are zero here), and its root range.  Phases with equal
 // signatures produce equal counts.  phase_equal compares two signatures;
 // phase_hash is a 64-bit hash of one (the key of the task builder's caches).
 bool phase_equal(const PhasePlan& a, const PhasePlan& b);
