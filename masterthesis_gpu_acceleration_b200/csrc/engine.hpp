@@ -230,6 +230,8 @@ struct Staged {
     bool plan_incomplete(int i) const {
         return budgeted && static_cast<const int*>(hIncomplete.p)[i] != 0;
     }
+    // Tasks of the largest launch of enqueue_per_plan.
+    int max_launch_tasks() const;
     // One launch per plan of an unsorted staging (at most kMaxPerPlan plans),
     // each with its own task counter, launch span and result in the 64
     // control bytes (counters and status at 0, spans at 16, results at
@@ -470,8 +472,8 @@ struct Context {
         grid = sms * (1024 / b);
         return true;
     }
-    // Plain per-rule calls launch on 512-thread blocks: one rule has few
-    // tasks, which finish sooner on larger blocks.  Their plans keep the
+    // Plain per-rule calls with few tasks launch on 512-thread blocks, on
+    // which each task ends sooner (see with_rule_block).  Their plans keep the
     // layout of geom.block.  0 (or a size not above geom.block): geom.block.
     int ruleBlock = 512;
 
