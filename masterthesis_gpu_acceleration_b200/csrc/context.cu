@@ -712,6 +712,15 @@ void Staged::check_geometry(const Context& c) const {
                         "); prepare the batch again after changing the block size");
 }
 
+// The block size of a launch of `tasks` tasks: larger blocks than the plans'
+// while all tasks are resident at once.  They shorten each task, but half as
+// many are resident: rules through hub rows with 2,000-4,800 tasks take 182 us
+// on 256 threads and 333 us on 512; a rule with 95 tasks 28 and 26 us, a
+// dense batch with 293 tasks 191 and 175 us.
+static int few_task_block(const Context& c, int tasks) {
+    return c.ruleBlock > c.geom.block && tasks <= c.sms * (1024 / c.ruleBlock) ? c.ruleBlock : c.geom.block;
+}
+
 void Staged::enqueue(Context& c, cudaStream_t s, int instr, int gridCap, unsigned long long budgetNs) {
     budgeted = false;
     if (!nPlans) return;
@@ -740,11 +749,14 @@ void Staged::enqueue(Context& c, cudaStream_t s, int instr, int gridCap, unsigne
         prof.incomplete = static_cast<int*>(dIncomplete.p);
         budgeted = true;
     }
+    // few tasks: larger blocks (see few_task_block); launches that spill keep
+    // the blocks of their follow-ups, timed ones those that costs are learnt for
+    const int block = instr || gridCap > 0 || spillable ? c.geom.block : few_task_block(c, nTasks);
     int grid = std::max(1, std::min(nTasks, gridCap > 0 ? std::min(gridCap, c.grid) : c.grid));
     if (blockWords && (size_t)grid > blockRegions) throw CudaError("launch grid exceeds the block-row regions");
     ck(engine_launch(c.dix, dPlans, dTasks, nTasks, static_cast<int*>(dCtl.p),
                      static_cast<unsigned long long*>(dResults.p), static_cast<int*>(dCtl.p) + 1, grid,
-                     c.geom.block, s, instr ? &prof : nullptr, instr ? SpillArgs{} : spill_args()),
+                     block, s, instr ? &prof : nullptr, instr ? SpillArgs{} : spill_args()),
        "engine launch");
     if (!instr)
         enqueue_follow_ups(c, s, static_cast<unsigned long long*>(dResults.p), static_cast<int*>(dCtl.p) + 1, nullptr);
@@ -873,16 +885,11 @@ int64_t run_one_phase(Context& c, const PhasePlan& ph, float* ms) {
     return (int64_t)c.one.counts()[0];
 }
 
-// Runs fn with the context's launch block size and grid switched to the
-// per-rule block size, restoring them afterwards (also when fn throws).
+// Runs fn with the context's launch block size and grid switched to those of
+// a launch of `tasks` tasks, restoring them afterwards (also when fn throws).
 // Only launches run under it: plans keep the batch geometry, whose shared
 // pool is a prefix of the larger block's, so per-rule calls share the
 // batch's cached walks and learnt costs (both keyed by plan signature).
-//
-// Larger blocks only while all of a launch's tasks are resident at once: they
-// shorten each task, but hold half as many tasks a GPU (rules through hub
-// rows with 2,000-4,800 tasks: 182 us instead of 333 us on 256 threads; 36-95
-// tasks: 28 us instead of 26 us).
 template <class Fn>
 void with_rule_block(Context& c, int tasks, Fn fn) {
     struct Restore {
@@ -890,7 +897,7 @@ void with_rule_block(Context& c, int tasks, Fn fn) {
         int block, grid;
         ~Restore() { c.geom.block = block; c.grid = grid; }
     } restore{c, c.geom.block, c.grid};
-    if (c.ruleBlock > c.geom.block && tasks <= c.sms * (1024 / c.ruleBlock)) c.set_block(c.ruleBlock);
+    c.set_block(few_task_block(c, tasks));
     fn();
 }
 

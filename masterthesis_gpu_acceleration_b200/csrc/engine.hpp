@@ -472,9 +472,8 @@ struct Context {
         grid = sms * (1024 / b);
         return true;
     }
-    // Plain per-rule calls with few tasks launch on 512-thread blocks, on
-    // which each task ends sooner (see with_rule_block).  Their plans keep the
-    // layout of geom.block.  0 (or a size not above geom.block): geom.block.
+    // Launches with few tasks take 512-thread blocks, on which each task ends
+    // sooner (see few_task_block).  Their plans keep the layout of geom.block.  0 (or a size not above geom.block): geom.block.
     int ruleBlock = 512;
 
     void init_device() {
