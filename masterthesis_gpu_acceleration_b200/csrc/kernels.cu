@@ -30,6 +30,13 @@
 // the block (16 ints of frontier and 32 bitmap words per thread), so 8, 4 or
 // 2 blocks stay resident per SM.
 //
+// What bounds it: 1,024 threads an SM (64 registers, 55 KB of shared memory
+// for 256 threads), which fill 48 % of the issue slots; a warp waits for block
+// barriers (4.6 cycles per issue), dependent loads (3.6) and fixed latencies
+// (3.2), and DRAM is idle (the index lies in L2; 5,000 miner candidates,
+// 1.9e9 warp instructions in 3.9 ms).  So a step pays that saves instructions
+// or rounds.
+//
 // The reference's kernels (GPU_03/gpu_kernels.cuh:34-443) run one thread
 // per head triple or per first-atom triple with template-unrolled
 // recursion; this engine replaces them as a whole.
@@ -1517,12 +1524,14 @@ __device__ __forceinline__ void run_task(Smem<B>& sm, const DevIndex& ix, const 
     if (tid == 0) mt.add(8);
 }
 
-// kI: 0 plain; 1 records each task's start and end time; 2 also counts
-// the algorithmic bytes; 3 records task times under a deadline (served
-// launches: past prof.budgetNs from the block's start the block abandons
-// its task at the end of a frontier round, skips the rest, and marks the
-// plans that lost a task in prof.incomplete); 4 one plan that comes with the
-// launch (InlineLaunch).
+// kI: 0 plain, may spill; 5 plain, may not: most small launches, without the
+// registers that spilling takes (10 biomedical rules 143 -> 125 us, a dense
+// batch 80 -> 74 us, short rules one by one 5.6 -> 5.4 ms); 1 records each
+// task's start and end time; 2 also counts the algorithmic bytes; 3 records
+// task times under a deadline (served launches: past prof.budgetNs from the
+// block's start the block abandons its task at the end of a frontier round,
+// skips the rest, and marks the plans that lost a task in prof.incomplete);
+// 4 one plan that comes with the launch (InlineLaunch).
 template <int B, int kI>
 __global__ void __launch_bounds__(B, 1024 / B)
 engine_kernel(const __grid_constant__ DevIndex ix, const DevPlan* __restrict__ plans, const DevTask* __restrict__ tasks,
@@ -1660,6 +1669,8 @@ static cudaError_t configure_b() {
         e = cudaFuncSetAttribute(engine_kernel<B, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(engine_kernel<B, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(engine_kernel<B, 5>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     return e;
 }
 
@@ -1692,6 +1703,8 @@ static void launch_b(const DevIndex& ix, const DevPlan* plans, const DevTask* ta
         engine_kernel<B, 3><<<grid, B, smem, stream>>>(ix, plans, tasks, nTasks, taskCounter, results, status, p, sp, in);
     else if (p.taskNs)
         engine_kernel<B, 1><<<grid, B, smem, stream>>>(ix, plans, tasks, nTasks, taskCounter, results, status, p, sp, in);
+    else if (!sp.ctl)
+        engine_kernel<B, 5><<<grid, B, smem, stream>>>(ix, plans, tasks, nTasks, taskCounter, results, status, p, sp, in);
     else
         engine_kernel<B, 0><<<grid, B, smem, stream>>>(ix, plans, tasks, nTasks, taskCounter, results, status, p, sp, in);
 }
