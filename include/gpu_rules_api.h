@@ -149,7 +149,7 @@ void gpu_batch_free(void* batch);
  * GPU_03/gpu_rules_lib.cu:296-316): modes[i] (n entries) = 0 bitmap rows in
  * shared memory, 1 one global bitmap row per head subject, 2 global rows per
  * resident block (memory bounded by the launch, not the rows), 3 pair keys
- * radix-sorted and counted once each; -1 when rule i's body size needs no
+ * parted by a hash and counted once each; -1 when rule i's body size needs no
  * pair deduplication on the device.  sortKeys (optional): pair keys the last
  * run appended.  Returns 0, or -1 on null arguments. */
 int gpu_batch_dedup(void* batch, int* modes, long long* sortKeys);
@@ -172,9 +172,9 @@ int gpu_evaluate_rule_noalloc(void* ctx, const char* ruleText, GpuRuleResult* ou
  * variable GPU_RULES_BLOCK sets it at load).  "task_target": fixed work per
  * task in candidate bindings (0 = automatic balancing).  "walk_threshold":
  * estimated work above which a phase's roots are measured one by one before
- * splitting (default 200000).  "rule_block": block size the plain per-rule
- * calls launch on (default 512; 0, or a size not above "block", = "block");
- * their plans keep the layout of "block", so they reuse what batches learnt.
+ * splitting (default 200000).  "rule_block": block size of launches
+ * whose tasks are all resident on it at once (default 512; 0, or a size not
+ * above "block", = "block"); their plans keep the layout of "block".
  * "rule_walk_budget": per-root measurement allowed per per-rule call.
  * "batch_chunks": pipelined chunks of gpu_evaluate_rules_batch (0 =
  * automatic).  "batch_phases": which phases batches prepared afterwards run
@@ -191,7 +191,7 @@ int gpu_evaluate_rule_noalloc(void* ctx, const char* ruleText, GpuRuleResult* ou
  * refused at admission with status -4; 0, the default: none).  "dedup_budget": device bytes that one
  * launch's global pair bitmaps may take (default 8 GiB); beyond it each
  * body-size phase whose pairs do not fit shared memory uses either bitmap
- * rows per resident block or pair keys sorted on the device, whichever
+ * rows per resident block or pair keys parted by a hash, whichever
  * moves fewer bytes (see gpu_batch_dedup).  "dedup_mode": 0 automatic, or
  * force 1, 2 or 3 of gpu_batch_dedup's modes on every pair-counting phase
  * (for tests).  Returns 0, or -1 for an unknown name or value. */

@@ -585,7 +585,7 @@ __device__ __noinline__ int memo_exists(const DevPlan& P, const DevIndex& ix, co
 // the paths through a must reach at most kMemo3List values (the warp's
 // list) and a's reverse row under the second step must be short.
 template <bool kC>
-__device__ __forceinline__ bool memo3_fits(const DevPlan& P, const DevIndex& ix, int a, Meter<kC>& mt) {
+__device__ __forceinline__ bool memo3_fits(const DevPlan& P, const DevIndex& ix, int a, int x, Meter<kC>& mt) {
     const DevStep s2 = P.steps[2], s3 = P.steps[3];
     const int2 rInv = row_lookup(ix, s2.pred, 1 - s2.dir, a, mt);
     if (rInv.y - rInv.x > 64) return false;
@@ -594,7 +594,9 @@ __device__ __forceinline__ bool memo3_fits(const DevPlan& P, const DevIndex& ix,
     const int2 r3a = row_lookup(ix, s3.pred, s3.dir, a, mt);
     int reach = r3a.y - r3a.x;
     for (int e2 = r2.x; e2 < r2.y && reach <= kMemo3List; ++e2) {
-        const int2 r3 = row_lookup(ix, s3.pred, s3.dir, __ldg(ix.val[s2.dir] + e2), mt);
+        const int v3 = __ldg(ix.val[s2.dir] + e2);
+        if (v3 == x) continue;   // (its row is a hub's, and no path through a takes it)
+        const int2 r3 = row_lookup(ix, s3.pred, s3.dir, v3, mt);
         reach += r3.y - r3.x;
     }
     return reach <= kMemo3List;
@@ -623,7 +625,7 @@ __device__ __noinline__ int classify_item(const DevPlan& P, const DevIndex& ix, 
     const int slot = __ldg((kind == 4 ? P.memo3Tab : P.memoTab) + hub);
     mt.add(4);
     if (slot < 0) return -1;
-    if (kind == 4) return memo3_fits(P, ix, it[kTupleHead], mt) ? slot : -1;
+    if (kind == 4) return memo3_fits(P, ix, it[kTupleHead], it[kTupleHead + 1], mt) ? slot : -1;
     if (kind == 2) {
         // bound values that are also first-step neighbours are witnesses the
         // memo must not count (x itself never is one); up to two are
