@@ -94,6 +94,9 @@ struct alignas(16) Level {
     int pad[3];
 };
 
+// What a block does after a group of a task's roots.
+enum GroupNext : int { kGroupGoOn, kGroupGive, kGroupLeave };
+
 template <int B>
 struct BlockState {
     static constexpr int kWarps = B / 32;
@@ -117,6 +120,7 @@ struct BlockState {
     int rowsSup;                    // 1: their fused support is still to be counted
     int rootsEnd;                   // end of the task's roots (the group's may lie before it)
     int idle;                       // blocks that were past the queue's end when the group began
+    int next;                       // what follows the group (GroupNext): thread 0's one decision for the block
     int base;                       // the level the task's search starts at
     int nTasks;                     // of the launch, and its counter
     const int* queue;
@@ -1039,7 +1043,11 @@ __device__ __forceinline__ void run_task(Smem<B>& sm, const DevIndex& ix, const 
                                            : (pairs ? 0 : ((G + 31) >> 5)));
     for (int i = tid; i < nWords; i += B) sbits[i] = 0u;
     if (blockRows && (long long)G * P.rowWords > P.gBlockWords) {   // the task builder keeps tasks this small
-        if (tid == 0) atomicOr(status, 32);
+        if (tid == 0) {
+            S.spill = 0;
+            atomicOr(status, 32);
+        }
+        __syncthreads();   // as on the way out below: the caller's last reads of `next` are done
         return;
     }
     if (blockRows) {
@@ -1609,15 +1617,26 @@ engine_kernel(const __grid_constant__ DevIndex ix, const DevPlan* __restrict__ p
         for (DevTask part = task; part.beg < task.end;) {
             part.end = group < task.end - part.beg ? part.beg + group : task.end;
             run_task<B, kC, kD, kS>(sm, ix, part, results, status, mt, sp, st);
+            if constexpr (kS) {
+                // One thread decides for the block: `spill` and `idle` are
+                // written again as soon as a block goes on, so a warp that
+                // looked at them itself after the barrier could decide
+                // otherwise.  (`spill` is this thread's own; `idle` was
+                // written before barriers of run_task.)
+                if (threadIdx.x == 0)
+                    sm.st.next = sm.st.spill ? kGroupLeave   // (the groups behind it went with it)
+                                 : part.end < task.end && sp.out >= 0 &&
+                                           (sm.st.idle * 16 >= (int)gridDim.x || sp.always)
+                                       ? kGroupGive : kGroupGoOn;
+            }
             __syncthreads();
             if constexpr (kD) {
                 if (sm.st.stop) break;
             }
             if constexpr (kS) {
-                if (sm.st.spill) break;   // (the groups behind it went with it)
-                if (part.end < task.end && sp.out >= 0 && (sm.st.idle * 16 >= (int)gridDim.x || sp.always) &&
-                    spill_groups<B>(sm, sp, task.plan, part.end, task.end))
-                    break;
+                const int next = sm.st.next;   // written again behind the next run_task's barriers
+                if (next == kGroupLeave) break;
+                if (next == kGroupGive && spill_groups<B>(sm, sp, task.plan, part.end, task.end)) break;
             }
             part.beg = part.end;
         }
