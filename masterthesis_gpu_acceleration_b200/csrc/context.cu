@@ -156,9 +156,14 @@ void Staged::stage(Context& c, const std::vector<const PhasePlan*>& phases, cons
     // the phases lie in their rules' plans, a few cache lines each: passes over
     // all of them run on host threads
     auto plan = [&](int i) -> const DevPlan& { return phases[i]->plan; };
+    // (supports are fused when a batch is prepared, the mode is chosen by each
+    // staging: a plan that counts supports needs rows to count them from, so
+    // one that is forced to keys keeps its rows in shared memory)
     std::vector<uint8_t> global(nPlans, 0);
     parallel_for((size_t)nPlans, [&](size_t i) {
-        global[i] = plan((int)i).mode == kPairs && (phases[i]->needsGlobalBitmap || c.dedupForce != 0) ? 1 : 0;
+        const bool fused = !sups.empty() && sups[i].n > 0;
+        const bool forced = c.dedupForce != 0 && !(fused && c.dedupForce == kDedupSort);
+        global[i] = plan((int)i).mode == kPairs && (phases[i]->needsGlobalBitmap || forced) ? 1 : 0;
     }, 256);
     for (int i = 0; i < nPlans; ++i) {
         if (!global[i]) continue;

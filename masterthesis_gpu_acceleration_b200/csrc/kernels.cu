@@ -861,10 +861,10 @@ __device__ __noinline__ bool spill_items(Smem<B>& sm, const DevTask& task, const
             const unsigned long long at = atomicAdd(&sp.ctl->rowWords, need);
             ok = at + need <= (unsigned long long)kSpillRowWords;
             dst = sp.rows + at;
-            if (ok && sup) {
-                supAt = atomicAdd(&sp.ctl->sups, 1);
-                ok = supAt < kSpillSups;
-            }
+        }
+        if (ok && sup) {   // (also of rows that are global already: this task's fused count is put off either way)
+            supAt = atomicAdd(&sp.ctl->sups, 1);
+            ok = supAt < kSpillSups;
         }
         unsigned long long old = 0;
         if (ok) ok = spill_take(&sp.ctl->used[sp.out], nTask, nRec, old);
