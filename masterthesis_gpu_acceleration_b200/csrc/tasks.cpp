@@ -23,6 +23,19 @@ int64_t pd_key(int32_t pred, int dir) { return (int64_t)pred * 2 + dir; }
 
 uint64_t signature(const PhasePlan& ph) { return phase_hash(ph); }
 
+// Roots a block takes at once (limit > 0: at most that many).
+int32_t group_of(const PhasePlan& ph, int32_t limit) {
+    int32_t g = ph.needsGlobalBitmap ? std::min(ph.plan.cap, 512) : ph.plan.groupMax;
+    if (limit > 0) g = std::min(g, limit);
+    return std::max(g, 1);
+}
+
+// The work of a phase of `cand` candidates in groups of g roots: the one unit
+// that tasks are cut by, learnt rates are per, and times are expected from.
+double units_of(const PhasePlan& ph, double cand, int32_t g) {
+    return cand + kGroupUnits * (double)((ph.rootEnd - ph.rootBeg + g - 1) / g);
+}
+
 }  // namespace
 
 bool phase_equal(const PhasePlan& a, const PhasePlan& b) {
@@ -360,11 +373,14 @@ void TaskBuilder::build(const std::vector<const PhasePlan*>& phases, int blocks,
         if (learned || split) sig[i] = signature(*phases[i]);
         if (learned) {
             auto c = calib_.find(sig[i]);
-            if (c != calib_.end()) scale[i] = c->second;
+            if (c != calib_.end()) scale[i] = c->second.rate;
             forced[i] = mustWalk_.count(sig[i]) ? 1 : 0;
         }
         if (split) cached[i] = walks_.count(sig[i]) ? 1 : 0;
     }, 16);
+    for (size_t i = 0; i < n; ++i) out[i].group = group_of(*phases[i], limits ? (*limits)[i].group : 0);
+    // a phase's work for `cand` candidates (without groups every task is one)
+    auto units = [&](size_t i, double cand) { return groups ? units_of(*phases[i], cand, out[i].group) : cand; };
     if (split) {
         std::vector<size_t> ord(n);
         std::iota(ord.begin(), ord.end(), 0);
@@ -387,7 +403,9 @@ void TaskBuilder::build(const std::vector<const PhasePlan*>& phases, int blocks,
             if (!forced[i] && !cached[i] && used + edges > walkBudget) continue;
             // a walk whose own cost exceeds the phase's expected device time
             // cannot pay for itself (a single rule on the whole GPU)
-            if (costAware && !cached[i] && std::max(estAvg[i], estHub[i]) * scale[i] < kWalkNsPerEdge * edges) continue;
+            if (costAware && !cached[i] &&
+                units(i, std::max(estAvg[i], estHub[i])) * scale[i] < kWalkNsPerEdge * edges)
+                continue;
             if (!cached[i]) used += edges;   // cached walks cost nothing
             sel.push_back(i);
         }
@@ -413,12 +431,7 @@ void TaskBuilder::build(const std::vector<const PhasePlan*>& phases, int blocks,
     // work in device-time units (learned ns per unit, where known)
     double total = 0;
     for (size_t i = 0; i < n; ++i) {
-        const PhasePlan& ph = *phases[i];
-        int32_t g = std::max(ph.plan.groupMax, 1);
-        if (ph.needsGlobalBitmap) g = std::min(ph.plan.cap, 512);
-        if (limits && (*limits)[i].group > 0) g = std::min(g, (*limits)[i].group);
-        out[i].group = std::max(g, 1);
-        if (groups) out[i].work += kGroupUnits * ((ph.rootEnd - ph.rootBeg + g - 1) / out[i].group);
+        out[i].work = units(i, out[i].work);
         total += out[i].work * scale[i];
     }
     const double target = forceTarget > 0 ? forceTarget
@@ -560,11 +573,9 @@ double TaskBuilder::expected_ns(const PhasePlan& ph) {
     if (ph.how != kDevice) return 0.0;
     if (!calib_.empty()) {
         auto it = calib_.find(signature(ph));
-        if (it != calib_.end()) return estimate2(ph) * it->second;
+        if (it != calib_.end()) return it->second.ns;
     }
-    // the average-fan-out estimate, raised at most tenfold toward the
-    // hub-aware one (which assumes every step lands on a hub)
-    return estimate2(ph) * defaultCalib_;
+    return units_of(ph, estimate2(ph), group_of(ph, 0)) * defaultCalib_;
 }
 
 void TaskBuilder::learn(const std::vector<const PhasePlan*>& phases, const std::vector<DevTask>& tasks,
@@ -590,8 +601,9 @@ void TaskBuilder::learn(const std::vector<const PhasePlan*>& phases, const std::
         if (units[p] <= 0) continue;
         const uint64_t sig = signature(*phases[p]);
         auto it = calib_.find(sig);
-        const double now = ns[p] / units[p];
-        calib_[sig] = it == calib_.end() ? now : blend(it->second, now);
+        const Learnt now{ns[p] / units[p], ns[p]};
+        if (it == calib_.end()) calib_.emplace(sig, now);
+        else it->second = Learnt{blend(it->second.rate, now.rate), blend(it->second.ns, now.ns)};
         if (worst[p] > limit) mustWalk_[sig] = true;
     }
 }

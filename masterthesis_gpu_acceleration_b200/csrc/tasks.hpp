@@ -91,9 +91,10 @@ public:
     // (cached; safe to call from several threads).
     const int32_t* degrees(int32_t pred, int dir);
 
-    // Estimated device time of a phase: learned ns per unit for plans seen
-    // by learn(), otherwise the work estimate times the learned default
-    // (1 ns per unit before any learning).
+    // Expected device time of a phase, summed over blocks: what learn() saw
+    // of its plan, otherwise its estimated work (candidates and groups, the
+    // units of tasks built with `groups`) times the learned default rate (1 ns
+    // per unit before any learning).
     double expected_ns(const PhasePlan& ph);
 
     // Feedback from an instrumented run of tasks built by build(): taskNs
@@ -160,7 +161,11 @@ private:
         std::unordered_map<uint64_t, double> map;
     };
     std::unique_ptr<TransShard[]> trans_;
-    std::unordered_map<uint64_t, double> calib_;                // phase hash -> ns per work unit
+    struct Learnt {
+        double rate = 0.0;   // ns per work unit
+        double ns = 0.0;     // ns of the whole phase
+    };
+    std::unordered_map<uint64_t, Learnt> calib_;                // phase hash -> what learn() saw
     std::unordered_map<uint64_t, bool> mustWalk_;               // phase hash -> walk next time
     double defaultCalib_ = 1.0;
     std::atomic<size_t> cacheBytes_{0};

@@ -1,0 +1,51 @@
+"""The task builder's costs on CPU (tests/native/costs_check.cpp, compiled
+here with g++), for rules planned from either end and tasks of several groups
+of roots: they cover every root once, times that were learnt come back as the
+expected times, and phases never run are expected in the units that tasks are
+built in (the serving loop admits requests by these times)."""
+import re
+import subprocess
+
+import pytest
+
+from conftest import ROOT, fuzz_names, load_fixture
+from masterthesis_gpu_acceleration_b200 import synth
+
+CSRC = ROOT / "masterthesis_gpu_acceleration_b200" / "csrc"
+
+
+@pytest.fixture(scope="module")
+def checker(tmp_path_factory):
+    out = tmp_path_factory.mktemp("native") / "costs_check"
+    subprocess.run(["g++", "-O2", "-std=c++17", "-pthread", "-o", str(out),
+                    str(ROOT / "tests" / "native" / "costs_check.cpp")] +
+                   [str(CSRC / f) for f in ("turtle.cpp", "index.cpp", "rules.cpp", "planner.cpp", "tasks.cpp")],
+                   check=True)
+    return out
+
+
+def _run(checker, ttl, rules):
+    r = subprocess.run([str(checker), str(ttl), str(rules)], capture_output=True, text=True, timeout=600)
+    assert r.returncode == 0, r.stdout + r.stderr
+    return [int(x) for x in re.findall(r"\d+", r.stdout)]
+
+
+def test_costs_fixtures(checker, tmp_path):
+    for name in fuzz_names() + ["edge_cases.json"]:
+        fx = load_fixture(name)
+        ttl, rules = tmp_path / f"{name}.ttl", tmp_path / f"{name}.txt"
+        ttl.write_text(fx["ttl"])
+        texts = fx["rules"] if "rules" in fx else [c["rule"] for c in fx["cases"]]
+        rules.write_text("\n".join(texts) + "\n")
+        _run(checker, ttl, rules)
+
+
+@pytest.mark.parametrize("cfg,n", [("c2s", None), ("c4s", None), ("c3", 1500)])
+def test_costs_synthetic(checker, data_dir, cfg, n):
+    d = synth.generate(cfg, data_dir / f"{cfg}_costs", seed=0)
+    rules = data_dir / f"{cfg}_costs" / "some.txt"
+    rules.write_text("\n".join(synth.read_rules(d)[:n]) + "\n")
+    phases, multi, split, unseen = _run(checker, d / "graph.ttl", rules)[:4]
+    assert phases > 0 and unseen > 0
+    if cfg == "c3":
+        assert multi > 0 and split > 0
