@@ -121,7 +121,7 @@ void longest_first(std::vector<DevTask>& tasks, std::vector<double>& cost, size_
 }  // namespace
 
 void Staged::stage(Context& c, const std::vector<const PhasePlan*>& phases, const std::vector<PlanSup>& sups,
-                   bool sortTasks, cudaStream_t s, double walkBudget, bool costAware, bool allowSort, bool mayInline) {
+                   bool sortTasks, cudaStream_t s, double walkBudget, int walkRule, bool allowSort, bool mayInline) {
     inl.clear();
     nPlans = (int)phases.size();
     nResults = nPlans + extraResults;
@@ -209,7 +209,7 @@ void Staged::stage(Context& c, const std::vector<const PhasePlan*>& phases, cons
         inPhases = phases;
         inSortTasks = sortTasks;
         inWalk = walkBudget;
-        inCostAware = costAware;
+        inWalkRule = walkRule;
         inAllowSort = allowSort;
     } else {
         inSups.clear();
@@ -304,7 +304,7 @@ void Staged::stage(Context& c, const std::vector<const PhasePlan*>& phases, cons
     hostSect[1] += host_ms() - tSect;
     tSect = host_ms();
     std::vector<PhaseTasks> pts;
-    c.tasks->build(phases, c.grid, true, pts, walkBudget, costAware, &lim, true);
+    c.tasks->build(phases, c.grid, true, pts, walkBudget, walkRule, &lim, true);
     hostSect[2] += host_ms() - tSect;
     tSect = host_ms();
     // split heavy roots of plans with fused support: counted after the launch
@@ -704,7 +704,7 @@ void Staged::restage(Context& c, cudaStream_t s) {
     keyHint = *static_cast<const unsigned long long*>(hSort.p);
     const std::vector<const PhasePlan*> ph = inPhases;
     const std::vector<PlanSup> su = inSups;
-    stage(c, ph, su, inSortTasks, s, inWalk, inCostAware, inAllowSort);
+    stage(c, ph, su, inSortTasks, s, inWalk, inWalkRule, inAllowSort);
 }
 
 void Staged::check_geometry(const Context& c) const {
@@ -875,7 +875,7 @@ namespace {
 // One phase in its own launch (the plain per-rule form), timed by events.
 int64_t run_one_phase(Context& c, const PhasePlan& ph, float* ms) {
     c.one.extraResults = 0;
-    c.one.stage(c, {&ph}, {}, false, c.stream, c.ruleWalkBudget, true);
+    c.one.stage(c, {&ph}, {}, false, c.stream, c.ruleWalkBudget, kWalkPays);
     for (int attempt = 0;; ++attempt) {
         ck(cudaEventRecord(c.ev[0], c.stream), "event");
         c.one.enqueue(c, c.stream, 0);
@@ -929,7 +929,7 @@ int evaluate_parsed(Context& c, const Rule& rule, GpuRuleResult* out) {
     }
     if (!phases.empty()) {
         // one upload, one launch per phase (each timed on the device), one download
-        c.one.stage(c, phases, sups, false, c.stream, c.ruleWalkBudget, true, true, true);
+        c.one.stage(c, phases, sups, false, c.stream, c.ruleWalkBudget, kWalkPays, true, true);
         for (int attempt = 0;; ++attempt) {
             with_rule_block(c, c.one.max_launch_tasks(), [&] { c.one.enqueue_per_plan(c, c.stream); });
             c.one.download_spans(c.stream);
@@ -1084,7 +1084,7 @@ void prepare(Batch& b, Context& c, const char* const* rules, int n, int isJson, 
     // than the phase is expected to take on the device; a prepared batch,
     // replayed many times, walks every phase the budget allows
     const double tPlanned = host_ms();
-    b.st.stage(c, phases, sups, true, b.stream, b.walkBudget, oneShot);
+    b.st.stage(c, phases, sups, true, b.stream, b.walkBudget, oneShot ? kWalkPays : kWalkBudget);
     b.hostPlanMs = tPlanned - tStart;
     b.hostStageMs = host_ms() - tPlanned;
 }

@@ -193,7 +193,8 @@ struct Staged {
     // an overflowing run can be staged again with the exact key count
     std::vector<PlanSup> inSups;
     std::vector<const PhasePlan*> inPhases;
-    bool inSortTasks = true, inCostAware = false, inAllowSort = true;
+    bool inSortTasks = true, inAllowSort = true;
+    int inWalkRule = kWalkBudget;
     double inWalk = 4.0e6;
 
     // walkBudget: how much per-root measurement the task builder may do
@@ -202,7 +203,7 @@ struct Staged {
     // when the key buffer overflows; the serving loop cannot).
     // sups: per phase, the supports it counts (empty: none).
     void stage(Context& c, const std::vector<const PhasePlan*>& phases, const std::vector<PlanSup>& sups,
-               bool sortTasks, cudaStream_t s, double walkBudget = 4.0e6, bool costAware = false,
+               bool sortTasks, cudaStream_t s, double walkBudget = 4.0e6, int walkRule = kWalkBudget,
                bool allowSort = true, bool mayInline = false);
     // After download + synchronisation: whether sort-mode keys exceeded the
     // buffer (the counts are then incomplete).  restage() stages the same

@@ -255,7 +255,7 @@ struct Server {
         s.busy = true;
         const bool heavyWork = s.heavyLane || overflow;
         // no sort mode: a served launch is never run a second time
-        s.st.stage(*c, phases, {}, true, s.stream, heavyWork ? 4.0e6 : 2.0e5, false, false);
+        s.st.stage(*c, phases, {}, true, s.stream, heavyWork ? 4.0e6 : 2.0e5, kWalkServed, false);
         // Launches record task times, from which the task builder learns
         // each plan shape's cost (the launches that follow split slow plans
         // finer and classify requests by it).

@@ -344,7 +344,7 @@ TaskBuilder::Walk TaskBuilder::compute_walk(const PhasePlan& ph) {
 }
 
 void TaskBuilder::build(const std::vector<const PhasePlan*>& phases, int blocks, bool split,
-                        std::vector<PhaseTasks>& out, double walkBudget, bool costAware,
+                        std::vector<PhaseTasks>& out, double walkBudget, int walkRule,
                         const std::vector<PhaseLimits>* limits, bool groups) {
     size_t n = phases.size();
     out.assign(n, PhaseTasks{});
@@ -403,8 +403,11 @@ void TaskBuilder::build(const std::vector<const PhasePlan*>& phases, int blocks,
             if (!forced[i] && !cached[i] && used + edges > walkBudget) continue;
             // a walk whose own cost exceeds the phase's expected device time
             // cannot pay for itself (a single rule on the whole GPU)
-            if (costAware && !cached[i] &&
+            if (walkRule == kWalkPays && !cached[i] &&
                 units(i, std::max(estAvg[i], estHub[i])) * scale[i] < kWalkNsPerEdge * edges)
+                continue;
+            if (walkRule == kWalkServed && !forced[i] && !cached[i] &&
+                units(i, estAvg[i]) * scale[i] < kWalkNsPerEdge * edges * std::max(blocks, 1))
                 continue;
             if (!cached[i]) used += edges;   // cached walks cost nothing
             sel.push_back(i);
@@ -489,10 +492,10 @@ void TaskBuilder::build(const std::vector<const PhasePlan*>& phases, int blocks,
         const std::vector<float>& w = wk->w;
         const bool canSplit = split && P.m >= 1;
         // Roots heavier than splitAt are cut into slices of `target`.  A
-        // launch of one rule (costAware) cuts only roots above a block's fair
+        // launch made once (kWalkPays) cuts only roots above a block's fair
         // share of the phase: lighter ones cannot hold up its end, and each
         // cut costs host time per first-segment edge.
-        const double splitAt = costAware ? std::max(target, pt.work * sc / std::max(blocks, 1)) : target;
+        const double splitAt = walkRule == kWalkPays ? std::max(target, pt.work * sc / std::max(blocks, 1)) : target;
         const double tail = chain_tail(P);
         const int32_t* deg2 =
             (canSplit && P.m >= 2 && P.steps[1].kind == kExpand) ? degrees(P.steps[1].pred, P.steps[1].dir) : nullptr;

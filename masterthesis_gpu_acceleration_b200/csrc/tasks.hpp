@@ -34,6 +34,34 @@ struct PhaseTasks {
     int32_t chunk = 0;          // > 0: the tasks are equal runs of this many roots (the last may be shorter)
 };
 
+// Host time of one step of a per-root walk (ns), for the rules below.
+constexpr double kWalkNsPerEdge = 8.0;
+
+// Which phases build() walks, within its budget and beside those learn()
+// marked:
+enum WalkRule : int {
+    kWalkBudget = 0,   // all it can (prepared batches, replayed many times)
+    // those whose device time, at the larger of the two estimates, exceeds the
+    // walk's host time; and only roots above a block's fair share of their
+    // phase are cut (launches made once, where nothing overlaps)
+    kWalkPays = 1,
+    // those expected to hold the whole GPU for longer than the walk takes: the
+    // one thread that stages launches has requests of all sizes behind it, and
+    // a phase whose slowest task turns out long is walked the next time.
+    // (Two graphs served at 50k requests/s, second pass over the stream: walks
+    // for hub-graph requests of 5-20 ms of block time took 2.5-10 ms a launch;
+    // p99 121-164 ms, 3-14 ms without them.)
+    kWalkServed = 2,
+};
+
+// The signature of a phase is the identity of its device computation: its
+// plan as the planner made it (per-launch fields are set in copies of it, so
+// they are zero here), and its root range.  Phases with equal
+// signatures produce equal counts.  phase_equal compares two signatures;
+// phase_hash is a 64-bit hash of one (the key of the task builder's caches).
+bool phase_equal(const PhasePlan& a, const PhasePlan& b);
+uint64_t phase_hash(const PhasePlan& ph);
+
 // Builds tasks for a batch of phases.  Work is measured in candidate
 // bindings.  Every phase gets a cheap estimate from average fan-outs and a
 // hub-aware one from size-biased fan-outs (the degree of a row reached by
@@ -48,17 +76,6 @@ struct PhaseTasks {
 // holds at once: a phase whose rows fill the shared pool with 20 roots made
 // hundreds of tasks of a few us, each fetched, listed, ordered and uploaded
 // (142,000 for 10,000 rules, 7,900 for the work they hold).
-// Host time of one step of a per-root walk (ns), for the cost-aware mode.
-constexpr double kWalkNsPerEdge = 8.0;
-
-// The signature of a phase is the identity of its device computation: its
-// plan as the planner made it (per-launch fields are set in copies of it, so
-// they are zero here), and its root range.  Phases with equal
-// signatures produce equal counts.  phase_equal compares two signatures;
-// phase_hash is a 64-bit hash of one (the key of the task builder's caches).
-bool phase_equal(const PhasePlan& a, const PhasePlan& b);
-uint64_t phase_hash(const PhasePlan& ph);
-
 class TaskBuilder {
 public:
     explicit TaskBuilder(const HostIndex& ix);
@@ -67,14 +84,12 @@ public:
     // launch.  split=false keeps every root in shared-memory tasks.
     // walkBudget: first-segment edges that may be newly walked (cached
     // walks and phases marked by learn() are not counted).
-    // costAware: walk a phase only when its expected device time exceeds
-    // the walk's own host time, and cut only roots above a block's fair
-    // share of their phase (per-rule launches, where nothing overlaps).
+    // walkRule: which phases are worth a walk (WalkRule).
     // limits (optional): one entry per phase.
     // groups: tasks may hold several groups of roots, which a block takes one
     // after the other (the kernel cuts them at the phase's `group`).
     void build(const std::vector<const PhasePlan*>& phases, int blocks, bool split,
-               std::vector<PhaseTasks>& out, double walkBudget = 4.0e6, bool costAware = false,
+               std::vector<PhaseTasks>& out, double walkBudget = 4.0e6, int walkRule = kWalkBudget,
                const std::vector<PhaseLimits>* limits = nullptr, bool groups = false);
 
     // Estimated candidate bindings of a phase (average fan-outs; exact first

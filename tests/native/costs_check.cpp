@@ -8,6 +8,8 @@
 //   * Phases never run are expected at the rate of those that were: with
 //     every task at the same rate, expected_ns() is that rate times the work
 //     build() gives the phase.
+//   * A served launch walks only phases expected to hold the whole GPU for
+//     longer than the walk takes, and those whose tasks turned out long.
 // Usage: costs_check GRAPH.ttl RULES.txt
 #include <algorithm>
 #include <cmath>
@@ -144,7 +146,37 @@ int main(int argc, char** argv) {
             if (std::fabs(got - want) > 1e-4 * want) ++badRate;
         }
     }
-    std::printf("phases %zu multi-group tasks %zu split roots %zu unseen %zu; cover %ld times %ld rates %ld\n",
-                phases.size(), multi, split, unseen, bad, badNs, badRate);
-    return bad + badNs + badRate == 0 ? 0 : 1;
+    long badServed = 0;
+    {
+        TaskBuilder tb(ix), all(ix);
+        tb.walkThreshold = 0.0;
+        all.walkThreshold = std::numeric_limits<double>::infinity();
+        std::vector<PhaseTasks> out, whole;
+        all.build(phases, blocks, true, whole, 0.0, false, nullptr, true);
+        tb.build(phases, blocks, true, out, 1e12, kWalkServed, nullptr, true);
+        for (size_t i = 0; i < phases.size(); ++i) {
+            // (a walk takes a step per root at least; chunk 0: walked)
+            const double least = kWalkNsPerEdge * (phases[i]->rootEnd - phases[i]->rootBeg);
+            badServed += out[i].chunk == 0 && whole[i].work < least * blocks;
+        }
+        const Launch run(out, 1e3);   // every task takes more than the ms below
+        tb.learn(phases, run.tasks, run.cost, run.ns.data(), blocks, 1.0, 1.0e6);
+        tb.build(phases, blocks, true, out, 0.0, kWalkServed, nullptr, true);
+        size_t at = 0;
+        for (size_t i = 0; i < phases.size(); ++i) {
+            double worst = 0, sum = 0;
+            for (; at < run.tasks.size() && run.tasks[at].plan == (int)i; ++at) {
+                const double d = (double)(run.ns[2 * at + 1] - run.ns[2 * at]);
+                worst = std::max(worst, d);
+                sum += d;
+            }
+            double every = 0;
+            for (double t : run.total) every += t;
+            badServed += worst > std::max(1.0e6, every / (blocks * 8.0)) && out[i].chunk != 0;
+        }
+    }
+    std::printf("phases %zu multi-group tasks %zu split roots %zu unseen %zu; cover %ld times %ld rates %ld served %ld\n",
+                phases.size(), multi, split, unseen, bad, badNs, badRate,
+                badServed);
+    return bad + badNs + badRate + badServed == 0 ? 0 : 1;
 }
