@@ -401,13 +401,14 @@ void TaskBuilder::build(const std::vector<const PhasePlan*>& phases, int blocks,
                          : (double)(ph.rootEnd - ph.rootBeg) *
                            (s0.kind == kExpand ? std::max(1.0, ix_.avg_degree(s0.pred, s0.dir)) : avg_fan(s0));
             if (!forced[i] && !cached[i] && used + edges > walkBudget) continue;
-            // a walk whose own cost exceeds the phase's expected device time
+            // a walk whose own cost exceeds the device time of what it weighs,
+            // the candidates (a group's own cost is the same for every group),
             // cannot pay for itself (a single rule on the whole GPU)
             if (walkRule == kWalkPays && !cached[i] &&
-                units(i, std::max(estAvg[i], estHub[i])) * scale[i] < kWalkNsPerEdge * edges)
+                std::max(estAvg[i], estHub[i]) * scale[i] < kWalkNsPerEdge * edges)
                 continue;
             if (walkRule == kWalkServed && !forced[i] && !cached[i] &&
-                units(i, estAvg[i]) * scale[i] < kWalkNsPerEdge * edges * std::max(blocks, 1))
+                estAvg[i] * scale[i] < kWalkNsPerEdge * edges * std::max(blocks, 1))
                 continue;
             if (!cached[i]) used += edges;   // cached walks cost nothing
             sel.push_back(i);

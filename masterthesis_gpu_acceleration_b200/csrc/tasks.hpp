@@ -41,13 +41,15 @@ constexpr double kWalkNsPerEdge = 8.0;
 // marked:
 enum WalkRule : int {
     kWalkBudget = 0,   // all it can (prepared batches, replayed many times)
-    // those whose device time, at the larger of the two estimates, exceeds the
-    // walk's host time; and only roots above a block's fair share of their
-    // phase are cut (launches made once, where nothing overlaps)
+    // those whose candidates, at the larger of the two estimates, take the
+    // device longer than the walk takes the host; and only roots above a
+    // block's fair share of their phase are cut (launches made once, where
+    // nothing overlaps)
     kWalkPays = 1,
-    // those expected to hold the whole GPU for longer than the walk takes: the
-    // one thread that stages launches has requests of all sizes behind it, and
-    // a phase whose slowest task turns out long is walked the next time.
+    // those whose candidates hold the whole GPU for longer than the walk
+    // takes: the one thread that stages launches has requests of all sizes
+    // behind it, and a phase whose slowest task turns out long is walked the
+    // next time.
     // (Two graphs served at 50k requests/s, second pass over the stream: walks
     // for hub-graph requests of 5-20 ms of block time took 2.5-10 ms a launch;
     // p99 121-164 ms, 3-14 ms without them.)
