@@ -280,6 +280,32 @@ const TaskBuilder::Walk& TaskBuilder::keep_walk(uint64_t sig, Walk&& wk) {
     return walks_.emplace(sig, std::move(wk)).first->second;
 }
 
+const std::vector<uint8_t>* TaskBuilder::walk_memo(const DevPlan& P, double* cost) const {
+    const DevStep& s1 = P.steps[1];
+    if (!memoRows || !chain_shaped(P) || P.mode != kPairs || P.memoLevel != 2) return nullptr;
+    if (P.m == 3) return memoRows(s1.pred, s1.dir, P.steps[2].pred, P.steps[2].dir, -1, 0, cost);
+    if (P.m == 4 && P.memoSteps == 3)
+        return memoRows(s1.pred, s1.dir, P.steps[2].pred, P.steps[2].dir, P.steps[3].pred, P.steps[3].dir, cost);
+    return nullptr;
+}
+
+// Whether the second step costs the same after every value of the first: it
+// scans, expands from a root value or a constant, or is free.
+static bool uniform_child(const DevPlan& P) {
+    const DevStep& s1 = P.steps[1];
+    return P.m >= 2 && (s1.kind != kExpand || s1.free || s1.keyRef < P.tupleLen[0]);
+}
+
+double TaskBuilder::walk_cost(const PhasePlan& ph) const {
+    const DevPlan& P = ph.plan;
+    const DevStep& s0 = P.steps[0];
+    double edges = ph.rootEnd - ph.rootBeg, memoCost = 0.0;
+    if (P.m < 2 || uniform_child(P)) return edges;
+    // (the rows of different roots hold different edges)
+    if (chain_shaped(P)) return edges + (walk_memo(P, &memoCost) ? (double)ix_.pred_size(s0.pred) : 0.0);
+    return edges + (double)(s0.kind == kRowScan ? ix_.pred_rows(s0.pred, s0.dir) : ix_.pred_size(s0.pred));
+}
+
 TaskBuilder::Walk TaskBuilder::compute_walk(const PhasePlan& ph) {
     const DevPlan& P = ph.plan;
     const double tail = chain_tail(P);
@@ -288,19 +314,12 @@ TaskBuilder::Walk TaskBuilder::compute_walk(const PhasePlan& ph) {
     const int32_t* deg2 = (!chain && P.m >= 2 && P.steps[1].kind == kExpand) ? degrees(P.steps[1].pred, P.steps[1].dir) : nullptr;
     // plans whose last two (three) steps are memoised: an item of level 1
     // costs the memo's price when its row has a memo, else its enumeration
-    const std::vector<uint8_t>* memo = nullptr;
     double memoCost = 0.0;
+    const std::vector<uint8_t>* memo = walk_memo(P, &memoCost);
     const DevStep& s1 = P.steps[1];
-    if (chain && P.mode == kPairs && P.memoLevel == 2 && memoRows) {
-        if (P.m == 3)
-            memo = memoRows(s1.pred, s1.dir, P.steps[2].pred, P.steps[2].dir, -1, 0, &memoCost);
-        else if (P.m == 4 && P.memoSteps == 3)
-            memo = memoRows(s1.pred, s1.dir, P.steps[2].pred, P.steps[2].dir, P.steps[3].pred, P.steps[3].dir,
-                            &memoCost);
-    }
-    // a second step that scans, or expands from a root value or a constant,
-    // costs the same after every edge of the first step
-    const bool uniformChild = P.m >= 2 && (s1.kind != kExpand || s1.keyRef < P.tupleLen[0]);
+    const bool uniformChild = uniform_child(P);
+    double scanned = -1.0;   // a scan's rows, the same for every root
+    size_t steps = (size_t)(ph.rootEnd - ph.rootBeg);
     std::vector<float> w((size_t)(ph.rootEnd - ph.rootBeg));
     int32_t vals[2];
     for (int32_t r = ph.rootBeg; r < ph.rootEnd; ++r) {
@@ -310,6 +329,7 @@ TaskBuilder::Walk TaskBuilder::compute_walk(const PhasePlan& ph) {
         if (P.m < 2) acc += seg.second - seg.first;
         else if (chain && memo) {
             acc += seg.second - seg.first;
+            steps += (size_t)(seg.second - seg.first);
             const int d0 = P.steps[0].dir;
             for (int32_t e = seg.first; e < seg.second; ++e) {
                 const auto rr = ix_.row_range(s1.pred, s1.dir, ix_.val[d0][e]);
@@ -325,10 +345,19 @@ TaskBuilder::Walk TaskBuilder::compute_walk(const PhasePlan& ph) {
             // every edge of the segment costs the same
             if (seg.second > seg.first)
                 acc += (double)(seg.second - seg.first) * child_work(P, vals, seg.first, deg2, tail);
-        } else
-            for (int32_t e = seg.first; e < seg.second; ++e) acc += child_work(P, vals, e, deg2, tail);
+        } else {
+            // the first step scans and the second expands from what it binds:
+            // the same edges and work for every root
+            if (scanned < 0) {
+                scanned = 1.0;
+                for (int32_t e = seg.first; e < seg.second; ++e) scanned += child_work(P, vals, e, deg2, tail);
+                steps += (size_t)(seg.second - seg.first);
+            }
+            acc = scanned;
+        }
         w[r - ph.rootBeg] = (float)acc;
     }
+    walkSteps_ += steps;
     Walk entry;
     for (float x : w) entry.sum += x;
     const size_t nb = w.size() / kWalkBlock;
@@ -394,12 +423,7 @@ void TaskBuilder::build(const std::vector<const PhasePlan*>& phases, int blocks,
         for (size_t i : ord) {
             if (!forced[i] && estHub[i] < walkThreshold) break;
             const PhasePlan& ph = *phases[i];
-            const DevStep& s0 = ph.plan.steps[0];
-            // cost of a walk: one lookup per root for chain-shaped plans,
-            // otherwise every first-segment edge
-            double edges = chain_shaped(ph.plan) ? (double)(ph.rootEnd - ph.rootBeg)
-                         : (double)(ph.rootEnd - ph.rootBeg) *
-                           (s0.kind == kExpand ? std::max(1.0, ix_.avg_degree(s0.pred, s0.dir)) : avg_fan(s0));
+            const double edges = walk_cost(ph);
             if (!forced[i] && !cached[i] && used + edges > walkBudget) continue;
             // a walk whose own cost exceeds the device time of what it weighs,
             // the candidates (a group's own cost is the same for every group),

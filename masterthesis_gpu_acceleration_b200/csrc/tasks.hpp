@@ -84,8 +84,8 @@ public:
 
     // phases[i] is planned as plan number i.  blocks: resident blocks of the
     // launch.  split=false keeps every root in shared-memory tasks.
-    // walkBudget: first-segment edges that may be newly walked (cached
-    // walks and phases marked by learn() are not counted).
+    // walkBudget: steps (roots and first-segment edges) that new walks may
+    // take (cached walks and phases marked by learn() are not counted).
     // walkRule: which phases are worth a walk (WalkRule).
     // limits (optional): one entry per phase.
     // groups: tasks may hold several groups of roots, which a block takes one
@@ -103,6 +103,8 @@ public:
     double hub_estimate(const PhasePlan& ph) { return estimate(ph, true); }
 
     size_t cache_bytes() const { return cacheBytes_; }
+    // Roots and edges that walks have visited so far.
+    size_t walk_steps() const { return walkSteps_; }
 
     // Row length of every entity under (pred, dir), indexed by entity
     // (cached; safe to call from several threads).
@@ -185,7 +187,7 @@ private:
     std::unordered_map<uint64_t, Learnt> calib_;                // phase hash -> what learn() saw
     std::unordered_map<uint64_t, bool> mustWalk_;               // phase hash -> walk next time
     double defaultCalib_ = 1.0;
-    std::atomic<size_t> cacheBytes_{0};
+    std::atomic<size_t> cacheBytes_{0}, walkSteps_{0};
     // guards deg_ while the estimates of a build run on several threads
     // (entries are never erased during a build, so references handed out
     // stay valid)
@@ -207,6 +209,11 @@ private:
     // the average-fan-out estimate.
     double estimate2(const PhasePlan& ph);
     const Walk& walk(const PhasePlan& ph, uint64_t sig);
+    // Roots and edges a walk of the phase visits (at most): a step per root,
+    // and the edges it has to look at one by one.
+    double walk_cost(const PhasePlan& ph) const;
+    // The memo flags by which a walk weighs the phase's items of level 1.
+    const std::vector<uint8_t>* walk_memo(const DevPlan& P, double* cost) const;
     // The per-root walk of a phase (thread-safe: reads the index and the
     // lock-guarded estimate caches), and its insertion into the cache.
     Walk compute_walk(const PhasePlan& ph);

@@ -8,6 +8,7 @@
 //   * Phases never run are expected at the rate of those that were: with
 //     every task at the same rate, expected_ns() is that rate times the work
 //     build() gives the phase.
+//   * New walks visit no more roots and edges than the budget allows.
 //   * A served launch walks only phases expected to hold the whole GPU for
 //     longer than the walk takes, and those whose tasks turned out long.
 // Usage: costs_check GRAPH.ttl RULES.txt
@@ -146,6 +147,20 @@ int main(int argc, char** argv) {
             if (std::fabs(got - want) > 1e-4 * want) ++badRate;
         }
     }
+    long badSteps = 0;
+    size_t steps = 0;
+    for (double budget : {2.0e4, 2.0e5, 4.0e6})
+        for (bool memos : {false, true}) {
+            TaskBuilder tb(ix);
+            tb.walkThreshold = 0.0;
+            std::vector<uint8_t> flags((size_t)ix.nEnt, 1);   // (longer than any predicate's rows)
+            if (memos)
+                tb.memoRows = [&](int, int, int, int, int, int, double* cost) { *cost = 256.0; return &flags; };
+            std::vector<PhaseTasks> out;
+            tb.build(phases, blocks, true, out, budget, kWalkBudget, nullptr, true);
+            badSteps += (double)tb.walk_steps() > budget;
+            steps += tb.walk_steps();
+        }
     long badServed = 0;
     {
         TaskBuilder tb(ix), all(ix);
@@ -175,8 +190,8 @@ int main(int argc, char** argv) {
             badServed += worst > std::max(1.0e6, every / (blocks * 8.0)) && out[i].chunk != 0;
         }
     }
-    std::printf("phases %zu multi-group tasks %zu split roots %zu unseen %zu; cover %ld times %ld rates %ld served %ld\n",
+    std::printf("phases %zu multi-group tasks %zu split roots %zu unseen %zu; cover %ld times %ld rates %ld served %ld steps %ld (%zu)\n",
                 phases.size(), multi, split, unseen, bad, badNs, badRate,
-                badServed);
-    return bad + badNs + badRate + badServed == 0 ? 0 : 1;
+                badServed, badSteps, steps);
+    return bad + badNs + badRate + badServed + badSteps == 0 ? 0 : 1;
 }

@@ -2,7 +2,9 @@
 here with g++), for rules planned from either end and tasks of several groups
 of roots: they cover every root once, times that were learnt come back as the
 expected times, and phases never run are expected in the units that tasks are
-built in (the serving loop admits requests by these times)."""
+built in (the serving loop admits requests by these times).  Walks keep to
+their budget, also where the second step is a free variable's and the
+subjects are skewed."""
 import re
 import subprocess
 
@@ -49,3 +51,18 @@ def test_costs_synthetic(checker, data_dir, cfg, n):
     assert phases > 0 and unseen > 0
     if cfg == "c3":
         assert multi > 0 and split > 0
+
+
+def test_costs_free_second_step(checker, data_dir):
+    """Dangling refinements of a skewed graph: ?f occurs once, behind ?x or ?b."""
+    d = synth.generate("c3", data_dir / "c3_costs", seed=0)
+    preds = sorted(set(re.findall(r"<[^>]*>", "\n".join(synth.read_rules(d)))))[::7]
+    rules = data_dir / "c3_costs" / "free.txt"
+    with open(rules, "w") as f:
+        for i, p in enumerate(preds):
+            q, h = preds[(i + 1) % len(preds)], preds[(i + 2) % len(preds)]
+            f.write(f"(?a {p} ?x) ^ (?x {q} ?f) => (?a {h} ?b)\n")
+            f.write(f"(?x {p} ?a) ^ (?f {q} ?x) => (?a {h} ?b)\n")
+            f.write(f"(?a {p} ?b) ^ (?b {q} ?f) => (?a {h} ?b)\n")
+            f.write(f"(?b {p} ?f) ^ (?a {q} ?x) => (?a {h} ?b)\n")
+    assert _run(checker, d / "graph.ttl", rules)[0] > 0
