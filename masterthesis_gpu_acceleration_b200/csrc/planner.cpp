@@ -26,6 +26,7 @@
 // whichever order finds it (the reference's greedy choice in
 // SupportCounting.cpp:38-79 is likewise a speed heuristic).
 #include "planner.hpp"
+#include "parallel.hpp"
 
 #include <algorithm>
 #include <cstring>
@@ -436,9 +437,42 @@ double plan_cost(const PhasePlan& ph, FanSamples& fans) {
     return cost;
 }
 
+// Candidates the plan may visit at most, as its steps are likely to go: every
+// step at the mean row length that a random edge sees.
+double plan_bound(const DevPlan& P, int32_t roots, const FanSamples& fans) {
+    double w = std::max(1, roots);
+    for (int s = 0; s < P.m; ++s) {
+        const DevStep& st = P.steps[s];
+        double f;
+        if (st.kind == kExpand) f = st.free ? 2.0 : fans.biased(st.pred, st.dir);
+        else f = (double)(st.kind == kScan ? fans.index().pred_size(st.pred) : fans.index().pred_rows(st.pred, st.dir));
+        w *= std::max(1.0, f);
+    }
+    return w;
+}
+
+// Body sizes below this bound stay at hS's end (see plan_rule).
+constexpr double kWorthTwoEnds = 2.0e5;
+
 }  // namespace
 
-FanSamples::FanSamples(const HostIndex& ix) : ix_(ix), shards_(new Shard[kShards]) {}
+std::vector<double> size_biased_fans(const HostIndex& ix) {
+    std::vector<double> fan((size_t)std::max(ix.nPred, 0) * 2, 0.0);
+    parallel_for(fan.size(), [&](size_t k) {
+        const int32_t p = (int32_t)(k / 2);
+        const int dir = (int)(k & 1);
+        double s1 = 0, s2 = 0;
+        for (int32_t r = ix.predRow[dir][p]; r < ix.predRow[dir][p + 1]; ++r) {
+            const double d = ix.rowBeg[dir][r + 1] - ix.rowBeg[dir][r];
+            s1 += d;
+            s2 += d * d;
+        }
+        fan[k] = s1 > 0 ? s2 / s1 : 0.0;
+    }, 4);
+    return fan;
+}
+
+FanSamples::FanSamples(const HostIndex& ix) : ix_(ix), biased_(size_biased_fans(ix)), shards_(new Shard[kShards]) {}
 
 FanSamples::Fan FanSamples::get(int32_t p0, int d0, int32_t p1, int d1, bool perEdge) {
     const uint64_t key = ((uint64_t)(uint32_t)p0 << 35) | ((uint64_t)(uint32_t)p1 << 3) | (uint64_t)(d0 << 2) |
@@ -449,6 +483,7 @@ FanSamples::Fan FanSamples::get(int32_t p0, int d0, int32_t p1, int d1, bool per
         auto it = sh.map.find(key);
         if (it != sh.map.end()) return it->second;
     }
+    sampled_.fetch_add(1, std::memory_order_relaxed);
     const int32_t beg = perEdge ? ix_.predEdge[d0][p0] : ix_.predRow[d0][p0];
     const int32_t n = (perEdge ? ix_.predEdge[d0][p0 + 1] : ix_.predRow[d0][p0 + 1]) - beg;
     const int32_t k = std::min(n, kSamples);
@@ -574,8 +609,12 @@ RulePlan plan_rule(const Rule& rule, const HostIndex& ix, const Geom& geom, FanS
         // memoised, so the end with the lower estimate is taken (half or
         // less, as the estimates are sampled).
         // Plans whose rows do not fit the shared pool keep hS's end: their
-        // memory (and what a scratch limit refuses) depends on it.
-        if (fans && pairs && rp.status == kRuleOk && B.how == kDevice && B.plan.m >= 2 && !B.needsGlobalBitmap) {
+        // memory (and what a scratch limit refuses) depends on it.  So do small
+        // ones: they take a few us from either end, and sampling their
+        // transitions costs a first call more than that (200 rules of 4 to 8 atoms
+        // on a uniform graph: planned in 1.6 ms on 8 threads, 0.5 ms without).
+        if (fans && pairs && rp.status == kRuleOk && B.how == kDevice && B.plan.m >= 2 && !B.needsGlobalBitmap &&
+            plan_bound(B.plan, B.rootEnd - B.rootBeg, *fans) >= kWorthTwoEnds) {
             PhasePlan R;
             if (build_body(rule, ix, geom, hO, hS, true, R) && R.how == kDevice &&
                 !R.needsGlobalBitmap && plan_cost(R, *fans) < 0.5 * plan_cost(B, *fans)) {

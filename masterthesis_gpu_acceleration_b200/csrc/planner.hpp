@@ -1,5 +1,6 @@
 // planner.hpp — rule -> device plans (support phase and body-size phase).
 #pragma once
+#include <atomic>
 #include <cstdint>
 #include <memory>
 #include <shared_mutex>
@@ -50,6 +51,10 @@ struct RulePlan {
 // pair (the step binding hO looks its value up there).
 std::pair<int32_t, int32_t> ho_domain(const DevPlan& P);
 
+// Per predicate and direction (pred * 2 + dir): the mean row length that a
+// random edge sees, sum(d^2) / sum(d).
+std::vector<double> size_biased_fans(const HostIndex& ix);
+
 // Mean row lengths of predicate transitions, estimated from a few evenly
 // spaced edges (or rows) of the first predicate and cached: what the planner
 // compares grounding orders by.  Safe to call from several threads.
@@ -60,6 +65,10 @@ public:
     };
     explicit FanSamples(const HostIndex& ix);
     const HostIndex& index() const { return ix_; }
+    // size-biased row length of (pred, dir)
+    double biased(int32_t pred, int dir) const { return biased_[(size_t)pred * 2 + (size_t)dir]; }
+    // transitions sampled so far
+    size_t sampled() const { return sampled_; }
     // row length under (p1, d1) of the value an edge of (p0, d0) leads to
     Fan edges(int32_t p0, int d0, int32_t p1, int d1) { return get(p0, d0, p1, d1, true); }
     // row length under (p1, d1) of a row key of (p0, d0)
@@ -73,7 +82,9 @@ private:
         std::unordered_map<uint64_t, Fan> map;
     };
     const HostIndex& ix_;
+    const std::vector<double> biased_;
     std::unique_ptr<Shard[]> shards_;
+    std::atomic<size_t> sampled_{0};
     Fan get(int32_t p0, int d0, int32_t p1, int d1, bool perEdge);
 };
 

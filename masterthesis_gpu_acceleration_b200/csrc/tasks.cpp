@@ -72,19 +72,9 @@ uint64_t phase_hash(const PhasePlan& ph) {
 }
 
 TaskBuilder::TaskBuilder(const HostIndex& ix)
-    : ix_(ix), degAt_((size_t)std::max(ix.nPred, 0) * 2), sbFan_((size_t)std::max(ix.nPred, 0) * 2, 0.0),
+    : ix_(ix), degAt_((size_t)std::max(ix.nPred, 0) * 2), sbFan_(size_biased_fans(ix)),
       hop2_(new Hop2Shard[kHop2Shards]), trans_(new TransShard[kHop2Shards]) {
     for (auto& a : degAt_) a.store(nullptr, std::memory_order_relaxed);
-    for (int32_t p = 0; p < ix.nPred; ++p)
-        for (int dir = 0; dir < 2; ++dir) {
-            double s1 = 0, s2 = 0;
-            for (int32_t r = ix.predRow[dir][p]; r < ix.predRow[dir][p + 1]; ++r) {
-                const double d = ix.rowBeg[dir][r + 1] - ix.rowBeg[dir][r];
-                s1 += d;
-                s2 += d * d;
-            }
-            sbFan_[(size_t)p * 2 + dir] = s1 > 0 ? s2 / s1 : 0.0;
-        }
 }
 
 const int32_t* TaskBuilder::degrees(int32_t pred, int dir) {

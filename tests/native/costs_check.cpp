@@ -190,8 +190,8 @@ int main(int argc, char** argv) {
             badServed += worst > std::max(1.0e6, every / (blocks * 8.0)) && out[i].chunk != 0;
         }
     }
-    std::printf("phases %zu multi-group tasks %zu split roots %zu unseen %zu; cover %ld times %ld rates %ld served %ld steps %ld (%zu)\n",
+    std::printf("phases %zu multi-group tasks %zu split roots %zu unseen %zu; cover %ld times %ld rates %ld served %ld steps %ld (%zu) sampled %zu\n",
                 phases.size(), multi, split, unseen, bad, badNs, badRate,
-                badServed, badSteps, steps);
+                badServed, badSteps, steps, fans.sampled());
     return bad + badNs + badRate + badServed + badSteps == 0 ? 0 : 1;
 }

@@ -4,10 +4,12 @@ of roots: they cover every root once, times that were learnt come back as the
 expected times, and phases never run are expected in the units that tasks are
 built in (the serving loop admits requests by these times).  Walks keep to
 their budget, also where the second step is a free variable's and the
-subjects are skewed."""
+subjects are skewed, and rules that are small from either end are planned
+without sampling the graph's transitions."""
 import re
 import subprocess
 
+import numpy as np
 import pytest
 
 from conftest import ROOT, fuzz_names, load_fixture
@@ -47,8 +49,9 @@ def test_costs_synthetic(checker, data_dir, cfg, n):
     d = synth.generate(cfg, data_dir / f"{cfg}_costs", seed=0)
     rules = data_dir / f"{cfg}_costs" / "some.txt"
     rules.write_text("\n".join(synth.read_rules(d)[:n]) + "\n")
-    phases, multi, split, unseen = _run(checker, d / "graph.ttl", rules)[:4]
+    phases, multi, split, unseen, *_, sampled = _run(checker, d / "graph.ttl", rules)
     assert phases > 0 and unseen > 0
+    assert sampled > 0   # skewed or with hubs
     if cfg == "c3":
         assert multi > 0 and split > 0
 
@@ -66,3 +69,23 @@ def test_costs_free_second_step(checker, data_dir):
             f.write(f"(?a {p} ?b) ^ (?b {q} ?f) => (?a {h} ?b)\n")
             f.write(f"(?b {p} ?f) ^ (?a {q} ?x) => (?a {h} ?b)\n")
     assert _run(checker, d / "graph.ttl", rules)[0] > 0
+
+
+def test_costs_uniform_graph(checker, tmp_path):
+    """Chains of 4 to 8 atoms on a graph without skew."""
+    rng = np.random.default_rng(5)
+    ttl, rules = tmp_path / "uniform.ttl", tmp_path / "rules.txt"
+    t = np.unique(np.stack([rng.integers(0, 10000, 100000), rng.integers(0, 20, 100000),
+                            rng.integers(0, 10000, 100000)], axis=1), axis=0)
+    ttl.write_text("".join(f"<http://u/e{s}> <http://u/p{p}> <http://u/e{o}> .\n" for s, p, o in t.tolist()))
+    with open(rules, "w") as f:
+        for i in range(60):
+            names = ["a"] + [f"v{k}" for k in range(3 + i % 5)] + ["b"]
+            atoms = []
+            for x, y in zip(names, names[1:]):
+                if rng.integers(0, 2):
+                    x, y = y, x
+                atoms.append(f"(?{x} <http://u/p{rng.integers(0, 20)}> ?{y})")
+            f.write(" ^ ".join(atoms) + f" => (?a <http://u/p{rng.integers(0, 20)}> ?b)\n")
+    phases, *_, sampled = _run(checker, ttl, rules)
+    assert phases > 0 and sampled == 0
