@@ -1677,20 +1677,29 @@ void* noalloc_scratch(int dev) {
 
 size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
 
-int64_t run_phase_noalloc(Context& c, const PhasePlan& ph, char* scratch, float* ms) {
+// A phase's tasks and its place in the scratch array.
+struct NoallocPhase {
+    std::vector<DevTask> tasks;
+    size_t taskOff = 0, bitmapOff = 0, bitmapWords = 0, need = 0;
+    NoallocPhase(Context& c, const PhasePlan& ph) {
+        if (ph.how != kDevice) return;
+        std::vector<PhaseTasks> pts;
+        c.tasks->build({&ph}, c.grid, false, pts);
+        tasks = std::move(pts[0].tasks);
+        taskOff = align256(kNoAllocHeader + sizeof(DevPlan));
+        bitmapOff = align256(taskOff + tasks.size() * sizeof(DevTask));
+        if (ph.needsGlobalBitmap)
+            bitmapWords = (size_t)(ph.rootEnd - ph.rootBeg) * (size_t)std::max(ph.plan.rowWords, 1);
+        need = bitmapOff + bitmapWords * 4;
+    }
+};
+
+int64_t run_phase_noalloc(Context& c, const PhasePlan& ph, const NoallocPhase& np, char* scratch, float* ms) {
     DevPlan plan = ph.plan;
-    std::vector<PhaseTasks> pts;
-    c.tasks->build({&ph}, c.grid, false, pts);
-    std::vector<DevTask>& tasks = pts[0].tasks;
-    const size_t planOff = kNoAllocHeader;
-    const size_t taskOff = align256(planOff + sizeof(DevPlan));
-    const size_t bitmapOff = align256(taskOff + tasks.size() * sizeof(DevTask));
-    size_t bitmapWords = 0;
-    if (ph.needsGlobalBitmap)
-        bitmapWords = (size_t)(ph.rootEnd - ph.rootBeg) * (size_t)std::max(plan.rowWords, 1);
-    const size_t need = bitmapOff + bitmapWords * 4;
-    if (need > kNoAllocScratchBytes)
-        throw CudaError("rule needs " + std::to_string(need) + " bytes of scratch; the no-allocation limit is " +
+    const std::vector<DevTask>& tasks = np.tasks;
+    const size_t planOff = kNoAllocHeader, taskOff = np.taskOff, bitmapOff = np.bitmapOff, bitmapWords = np.bitmapWords;
+    if (np.need > kNoAllocScratchBytes)
+        throw CudaError("rule needs " + std::to_string(np.need) + " bytes of scratch; the no-allocation limit is " +
                         std::to_string(kNoAllocScratchBytes) + " bytes");
     plan.resultSlot = 0;
     plan.gBitmap = bitmapWords ? reinterpret_cast<uint32_t*>(scratch + bitmapOff) : nullptr;
@@ -1731,10 +1740,18 @@ extern "C" int gpu_evaluate_rule_noalloc(void* ctx, const char* ruleText, GpuRul
         char* scratch = static_cast<char*>(noalloc_scratch(c.device));
         Rule r = c.parser->parse_text(ruleText);
         RulePlan rp = plan_rule(r, c.hix, c.geom, c.fans.get());
+        NoallocPhase ns(c, rp.support), nb(c, rp.body);
+        if (ns.need > kNoAllocScratchBytes || nb.need > kNoAllocScratchBytes) {
+            // a plan made for speed may need more memory (a larger hO domain,
+            // more tasks): what the array holds depends on the plain one
+            rp = plan_rule(r, c.hix, c.geom, nullptr, false);
+            ns = NoallocPhase(c, rp.support);
+            nb = NoallocPhase(c, rp.body);
+        }
         int64_t sup = rp.support.value, body = rp.body.value;
         float supMs = 0.f, confMs = 0.f;
-        if (rp.status == kRuleOk && rp.support.how == kDevice) sup = run_phase_noalloc(c, rp.support, scratch, &supMs);
-        if (rp.status == kRuleOk && rp.body.how == kDevice) body = run_phase_noalloc(c, rp.body, scratch, &confMs);
+        if (rp.status == kRuleOk && rp.support.how == kDevice) sup = run_phase_noalloc(c, rp.support, ns, scratch, &supMs);
+        if (rp.status == kRuleOk && rp.body.how == kDevice) body = run_phase_noalloc(c, rp.body, nb, scratch, &confMs);
         compose(rp, sup, body, supMs, confMs, out);
         return 0;
     } catch (const std::exception& e) {

@@ -87,7 +87,7 @@ int check_dir(const HostIndex& ix, int32_t p) {
 // body that nothing bound reaches would be scanned edge by edge, the rows of
 // such an atom are scanned instead, and its free variable is looked for
 // behind each.
-bool build_steps(Builder& b, const Rule& rule, const Atom* head, int32_t hO, bool pairs) {
+bool build_steps(Builder& b, const Rule& rule, const Atom* head, int32_t hO, bool pairs, bool freeVars) {
     const std::vector<Atom>& body = rule.body;
     DevPlan& P = b.P;
     const HostIndex& ix = b.ix;
@@ -116,6 +116,7 @@ bool build_steps(Builder& b, const Rule& rule, const Atom* head, int32_t hO, boo
     int freeSide[kMaxBody];
     for (int i = 0; i < nb; ++i) {
         freeSide[i] = 0;
+        if (!freeVars) continue;
         auto occurs = [&](const Term& t) {
             int n = 0;
             for (const Atom& a : body) n += (a.s.isVar && a.s.id == t.id) + (a.o.isVar && a.o.id == t.id);
@@ -318,7 +319,7 @@ bool finish_capacity(DevPlan& P, const Geom& geom) {
 // for plans beyond the engine's limits; `B` stays static (count 0) when hS is
 // in no body atom or two atoms always collide.
 bool build_body(const Rule& rule, const HostIndex& ix, const Geom& geom, int32_t hS, int32_t hO, bool pairs,
-                PhasePlan& B) {
+                bool freeVars, PhasePlan& B) {
     int seedPred = -1, seedDir = 0;
     int64_t bestSize = std::numeric_limits<int32_t>::max();
     for (const auto& a : rule.body) {
@@ -335,7 +336,7 @@ bool build_body(const Rule& rule, const HostIndex& ix, const Geom& geom, int32_t
     P.rootDir = seedDir;
     P.rootPred = seedPred;
     b.bind(hS);
-    if (!build_steps(b, rule, nullptr, hO, pairs)) return true;
+    if (!build_steps(b, rule, nullptr, hO, pairs, freeVars)) return true;
     if (!b.ok) return false;
     if (pairs) {
         for (int l = 0; l < P.m; ++l) {
@@ -505,7 +506,7 @@ FanSamples::Fan FanSamples::get(int32_t p0, int d0, int32_t p1, int d1, bool per
     return f;
 }
 
-RulePlan plan_rule(const Rule& rule, const HostIndex& ix, const Geom& geom, FanSamples* fans) {
+RulePlan plan_rule(const Rule& rule, const HostIndex& ix, const Geom& geom, FanSamples* fans, bool freeVars) {
     RulePlan rp;
     const Atom& h = rule.head;
     int nb = (int)rule.body.size();
@@ -578,7 +579,7 @@ RulePlan plan_rule(const Rule& rule, const HostIndex& ix, const Geom& geom, FanS
                 range = ix.row_range(h.pred, 0, h.s.id);
                 P.rootValConst = b.ref(h.o);
             }
-            if (build_steps(b, rule, &h, -1, false) && b.ok) {
+            if (build_steps(b, rule, &h, -1, false, freeVars) && b.ok) {
                 finish_capacity(P, geom);
                 exist_memo_eligibility(P);
                 S.how = kDevice;
@@ -601,7 +602,7 @@ RulePlan plan_rule(const Rule& rule, const HostIndex& ix, const Geom& geom, FanS
         for (const auto& a : rule.body)
             hoInBody |= (a.s.isVar && a.s.id == hO) || (a.o.isVar && a.o.id == hO);
         const bool pairs = hS != hO && hoInBody;
-        if (!build_body(rule, ix, geom, hS, hO, pairs, B)) rp.status = kRuleUnsupported;
+        if (!build_body(rule, ix, geom, hS, hO, pairs, freeVars, B)) rp.status = kRuleUnsupported;
         // Distinct (hS, hO) pairs can be counted from either end: rows of hS
         // values with bits for hO, or the reverse.  What a grounding order
         // costs is the bindings of its inner levels, and a hub costs least
@@ -616,7 +617,7 @@ RulePlan plan_rule(const Rule& rule, const HostIndex& ix, const Geom& geom, FanS
         if (fans && pairs && rp.status == kRuleOk && B.how == kDevice && B.plan.m >= 2 && !B.needsGlobalBitmap &&
             plan_bound(B.plan, B.rootEnd - B.rootBeg, *fans) >= kWorthTwoEnds) {
             PhasePlan R;
-            if (build_body(rule, ix, geom, hO, hS, true, R) && R.how == kDevice &&
+            if (build_body(rule, ix, geom, hO, hS, true, freeVars, R) && R.how == kDevice &&
                 !R.needsGlobalBitmap && plan_cost(R, *fans) < 0.5 * plan_cost(B, *fans)) {
                 R.plan.supDir = 1;
                 B = R;

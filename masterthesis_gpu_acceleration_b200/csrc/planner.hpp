@@ -91,7 +91,10 @@ private:
 // Plans both phases.  Semantics follow CPU_01_nonparallel/SupportCounting.cpp:
 // support (474-552) with the head triple counted as used, body size
 // (563-631) with the seed atom's keys as headS candidates, or from hO's end
-// where `fans` (optional) says that costs less.
-RulePlan plan_rule(const Rule& rule, const HostIndex& ix, const Geom& geom, FanSamples* fans = nullptr);
+// where `fans` (optional) says that costs less.  freeVars false: free
+// variables are grounded as any other (no free steps, no row scans).  Without
+// both a plan's memory depends on the rule and the predicates' rows alone.
+RulePlan plan_rule(const Rule& rule, const HostIndex& ix, const Geom& geom, FanSamples* fans = nullptr,
+                   bool freeVars = true);
 
 }  // namespace gr
