@@ -185,13 +185,21 @@ struct Server {
             Planned& q = qs[i];
             q.req = std::move(got[i]);
             try {
-                q.rp = plan_rule(c->parser->parse_text(q.req.text), c->hix, c->geom, c->fans.get());
+                const Rule rule = c->parser->parse_text(q.req.text);
+                q.rp = plan_rule(rule, c->hix, c->geom, c->fans.get());
+                q.mem = estimate_mem(q.rp);
+                if (q.mem > memBudget) {
+                    // a plan made for speed may need more memory: what the
+                    // budget refuses depends on the plain one
+                    q.rp = plan_rule(rule, c->hix, c->geom, nullptr, false);
+                    q.mem = estimate_mem(q.rp);
+                }
             } catch (const std::exception&) {
                 q.status = -1;
+                q.mem = 0;
             }
             double ns = 0;
             if (q.status == 0) {
-                q.mem = estimate_mem(q.rp);
                 if (q.mem > memBudget) { q.status = -2; q.mem = 0; }
                 if (q.rp.status == kRuleOk)
                     ns = c->tasks->expected_ns(q.rp.support) + c->tasks->expected_ns(q.rp.body);

@@ -7,7 +7,9 @@ p2 (390,000, each with a free object) are fewer than p3's or p5's edges
 (391,000 each, from 20 subjects), so the row scan of p2 is cheaper than the
 scan of p3, but binds ?b in a domain whose bitmap rows lie in global memory:
 220 head subjects need 10.7 MB of the 8 MiB that gpu_evaluate_rule_noalloc
-has.  From p3 the domain has 20 values."""
+has, or of a server's budget.  From p3 the domain has 20 values."""
+import time
+
 import numpy as np
 import pytest
 
@@ -55,3 +57,17 @@ def test_noalloc_keeps_accepting(parts):
         for _ in range(2):
             r = lib.evaluate_rule_noalloc(RULE)
             assert [getattr(r, f) for f in FIELDS] == exp
+
+
+def test_serving_keeps_accepting(parts):
+    ttl, exp = parts
+    with eng.GpuRulesLib(ttl) as lib:
+        with lib.serve(slots=2, max_batch=4, mem_budget=4 << 20) as sv:
+            sv.submit(7, RULE)
+            got = []
+            t0 = time.time()
+            while not got and time.time() - t0 < 60:
+                got = sv.poll(wait_ms=50)
+    rid, status, r, _ = got[0]
+    assert (rid, status) == (7, 0)
+    assert [getattr(r, f) for f in FIELDS] == exp
