@@ -412,10 +412,13 @@ void Staged::stage(Context& c, const std::vector<const PhasePlan*>& phases, cons
     // without: at 66 us, 25 rules of a dense graph, 219 and 151 us; at 169 us,
     // 200 long rules, 805 and 778 us; at 188 us, 1,329 mined rules, 836 and
     // 924 us; at 4,500 us, 10,000 rules, 5.5 and 6.9 ms.)
+    // What is given away costs several times its work, so sets with much work
+    // but no long task lose: a prepared batch spills where that measured faster.
     double workNs = 0;
     for (int i = 0; i < nPlans; ++i) workNs += pts[i].work * pts[i].scale;
     spillAlways = c.spill == 2;
-    spillable = maySpill && c.spill && nSort == 0 && (spillAlways || workNs > 150e3 * std::max(c.grid, 1));
+    spillable = maySpill && c.spill && nSort == 0 &&
+                (spillAlways || (spillMeasured ? spillPays : workNs > 150e3 * std::max(c.grid, 1)));
     if (dCtl.cap == 0) ctlClean = false;
     dCtl.ensure(kCtlBytes, as);
     if (hCtl.cap == 0) {
@@ -654,6 +657,12 @@ void Context::ensure_memos(const std::vector<std::array<int, 6>>& keys, cudaStre
         if (j.p3 >= 0) maxWo = std::max(maxWo, j.wo);
     ck(memo_build(dix, dJobs, (int)all.size(), maxWo, s), "memo build");
     ck(cudaStreamSynchronize(s), "memo build");   // memos are shared by every stream afterwards
+}
+
+void Staged::set_spill(bool on, cudaStream_t s) {
+    spillable = on;
+    if (on) dSpill.ensure(spill_bytes(), streamOrdered ? s : nullptr);
+    else dSpill.release();
 }
 
 SpillArgs Staged::spill_args() const {
@@ -1159,6 +1168,34 @@ void run_batch(Batch& b, bool useGraph, size_t flushBytes, bool retried = false)
     b.lastMs = ms;
 }
 
+// Times a prepared batch's launch with and without spilling (the best of two
+// runs after one) and keeps the faster way; spilling has to gain 3 %.  50
+// rules on a graph with hubs: four sets 0.85-1.56 ms without and 1.10-1.81 ms
+// with, two others 2.19 and 1.26 ms without, 1.59 and 1.15 ms with.  10,000
+// rules: 3.35 and 3.56 ms without, 3.73 and 3.89 ms with; four other sets
+// 6.2-7.2 ms without, 4.4-6.0 ms with.
+void tune_spill(Batch& b) {
+    Context& c = *b.c;
+    if (c.spill != 1 || !b.st.nPlans || b.st.nSort) return;
+    float best[2] = {0.f, 0.f};
+    for (int on = 0; on < 2; ++on) {
+        b.st.set_spill(on != 0, b.stream);
+        for (int run = 0; run < 3; ++run) {
+            ck(cudaEventRecord(b.ev0, b.stream), "event");
+            b.st.enqueue(c, b.stream, 0);
+            ck(cudaEventRecord(b.ev1, b.stream), "event");
+            b.st.download(b.stream);
+            ck(cudaStreamSynchronize(b.stream), "tune");
+            b.st.check_status();
+            float ms = 0.f;
+            ck(cudaEventElapsedTime(&ms, b.ev0, b.ev1), "elapsed");
+            if (run == 1 || (run > 1 && ms < best[on])) best[on] = ms;
+        }
+    }
+    b.st.spillPays = best[1] < 0.97f * best[0];
+    if (!b.st.spillPays) b.st.set_spill(false, b.stream);
+}
+
 Context* as_ctx(void* p) { return static_cast<Context*>(p); }
 
 }  // namespace
@@ -1424,6 +1461,7 @@ void* gpu_batch_prepare(void* ctx, const char* const* rules, int n, int isJson) 
         cudaSetDevice(c.device);
         b = new Batch();
         b->walkBudget = 4.0e7;   // prepared once, replayed many times
+        b->st.spillMeasured = true;
         prepare(*b, c, rules, n, isJson);
         ck(cudaStreamSynchronize(b->stream), "stage");
         return b;
@@ -1561,6 +1599,7 @@ int gpu_batch_autotune(void* batch, int rounds) {
             b.st.stage(c, b.phases, b.sups, true, b.stream, b.walkBudget);
             ck(cudaStreamSynchronize(b.stream), "restage");
         }
+        if (rounds > 0) tune_spill(b);
         return 0;
     } catch (const std::exception& e) {
         set_error(std::string("gpu_batch_autotune error: ") + e.what());

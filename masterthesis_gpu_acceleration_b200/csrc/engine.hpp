@@ -179,6 +179,10 @@ struct Staged {
     bool anyFused = false;                 // some plan counts supports
     bool maySpill = true;                  // false: only timed launches (served ones), which never spill
     bool spillable = false;                // launches of this staging may spill
+    // Prepared batches: whether launches spill is measured when the batch is
+    // tuned (tune_spill) instead of estimated by each staging.
+    bool spillMeasured = false, spillPays = false;
+    void set_spill(bool on, cudaStream_t s);
     bool spillAlways = false;
     SpillArgs spill_args() const;
     void enqueue_follow_ups(Context& c, cudaStream_t s, unsigned long long* results, int* status,
