@@ -480,7 +480,9 @@ void Staged::stage(Context& c, const std::vector<const PhasePlan*>& phases, cons
     dBlob.ensure(blob, as);
     nResults = nPlans + extraResults;
     dResults.ensure((size_t)nResults * sizeof(unsigned long long), as);
-    if (spillable) dSpill.ensure(spill_bytes(), as);
+    // 31 MB, stream-ordered also for staging that is not: cudaMalloc waits for
+    // every stream, and a call of several chunks takes one buffer each
+    if (spillable) dSpill.ensure(spill_bytes(), s, true);
     hResults.ensure((size_t)nResults * sizeof(unsigned long long));
     ck(cudaMemcpyAsync(dBlob.p, hBlob.p, blob, cudaMemcpyHostToDevice, s), "H2D plans");
     dPlans = static_cast<const DevPlan*>(dBlob.p);
@@ -661,7 +663,7 @@ void Context::ensure_memos(const std::vector<std::array<int, 6>>& keys, cudaStre
 
 void Staged::set_spill(bool on, cudaStream_t s) {
     spillable = on;
-    if (on) dSpill.ensure(spill_bytes(), streamOrdered ? s : nullptr);
+    if (on) dSpill.ensure(spill_bytes(), s, true);
     else dSpill.release();
 }
 

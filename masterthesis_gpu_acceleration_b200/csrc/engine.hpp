@@ -77,9 +77,10 @@ struct DevBuf {
     // must be rare when request sizes vary.  With a stream, the old buffer
     // is freed and the new one allocated in that stream's order (no device
     // synchronisation); the buffer must then only be used on that stream.
-    void ensure(size_t bytes, cudaStream_t s = nullptr) {
+    // exact: sizes that never change take no more than they need.
+    void ensure(size_t bytes, cudaStream_t s = nullptr, bool exact = false) {
         if (bytes <= cap) return;
-        size_t want = std::max<size_t>(bytes + bytes / 2, 4096);
+        size_t want = exact ? bytes : std::max<size_t>(bytes + bytes / 2, 4096);
         if (s) {
             if (p && pooled) ck(cudaFreeAsync(p, s), "cudaFreeAsync");
             else release();
