@@ -82,6 +82,7 @@ size_t spill_part(int part) {
     return at;
 }
 size_t spill_bytes() { return spill_part(6); }
+constexpr double kSpillSkew = 4.0;   // least PhaseTasks::skew among the phases of a launch that may spill
 }  // namespace
 
 namespace {
@@ -412,13 +413,20 @@ void Staged::stage(Context& c, const std::vector<const PhasePlan*>& phases, cons
     // without: at 66 us, 25 rules of a dense graph, 219 and 151 us; at 169 us,
     // 200 long rules, 805 and 778 us; at 188 us, 1,329 mined rules, 836 and
     // 924 us; at 4,500 us, 10,000 rules, 5.5 and 6.9 ms.)
+    // Nor where no step's rows differ much in length, so that no task can
+    // outlast the others by far (200 to 1,600 long rules on a uniform graph:
+    // 0.83-5.9 ms with, 0.68-5.3 ms without).
     // What is given away costs several times its work, so sets with much work
     // but no long task lose: a prepared batch spills where that measured faster.
-    double workNs = 0;
-    for (int i = 0; i < nPlans; ++i) workNs += pts[i].work * pts[i].scale;
+    double workNs = 0, skew = 0;
+    for (int i = 0; i < nPlans; ++i) {
+        workNs += pts[i].work * pts[i].scale;
+        skew = std::max(skew, pts[i].skew);
+    }
     spillAlways = c.spill == 2;
     spillable = maySpill && c.spill && nSort == 0 &&
-                (spillAlways || (spillMeasured ? spillPays : workNs > 150e3 * std::max(c.grid, 1)));
+                (spillAlways || (spillMeasured ? spillPays
+                                     : skew >= kSpillSkew && workNs > 150e3 * std::max(c.grid, 1)));
     if (dCtl.cap == 0) ctlClean = false;
     dCtl.ensure(kCtlBytes, as);
     if (hCtl.cap == 0) {

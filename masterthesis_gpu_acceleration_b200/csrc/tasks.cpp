@@ -90,7 +90,18 @@ const int32_t* TaskBuilder::degrees(int32_t pred, int dir) {
     return ins.first->second.data();
 }
 
-double TaskBuilder::sb_fan(int32_t pred, int dir) { return sbFan_[(size_t)pred * 2 + (size_t)dir]; }
+double TaskBuilder::skew(const DevPlan& P) const {
+    double most = 0.0;
+    for (int s = 0; s < P.m; ++s) {
+        const DevStep& st = P.steps[s];
+        if (st.kind != kExpand || st.free) continue;
+        const double avg = ix_.avg_degree(st.pred, st.dir);
+        if (avg > 0) most = std::max(most, sb_fan(st.pred, st.dir) / avg);
+    }
+    return most;
+}
+
+double TaskBuilder::sb_fan(int32_t pred, int dir) const { return sbFan_[(size_t)pred * 2 + (size_t)dir]; }
 
 double TaskBuilder::avg_fan(const DevStep& st) const {
     if (st.kind == kScan) return (double)ix_.pred_size(st.pred);
@@ -389,6 +400,7 @@ void TaskBuilder::build(const std::vector<const PhasePlan*>& phases, int blocks,
         estAvg[i] = estimate2(*phases[i]);
         estHub[i] = split ? estimate(*phases[i], true) : estAvg[i];
         out[i].work = estAvg[i];
+        out[i].skew = skew(phases[i]->plan);
         if (learned || split) sig[i] = signature(*phases[i]);
         if (learned) {
             auto c = calib_.find(sig[i]);

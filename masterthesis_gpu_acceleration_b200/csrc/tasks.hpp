@@ -31,6 +31,7 @@ struct PhaseTasks {
     int32_t heavyRows = 0;      // global dedup rows used by split roots
     double work = 0.0;          // estimated work of the whole phase
     double scale = 1.0;         // learned device ns per unit of work
+    double skew = 0.0;          // of its steps: the row length a random edge sees over the mean one, at most
     int32_t chunk = 0;          // > 0: the tasks are equal runs of this many roots (the last may be shorter)
 };
 
@@ -193,7 +194,8 @@ private:
     // stay valid)
     mutable std::shared_mutex cacheMu_;
 
-    double sb_fan(int32_t pred, int dir);
+    double sb_fan(int32_t pred, int dir) const;
+    double skew(const DevPlan& P) const;
     double avg_fan(const DevStep& st) const;
     double estimate(const PhasePlan& ph, bool hubAware);
     // Two-hop sums of the transition from (p0, d0) to (p1, d1), shared by

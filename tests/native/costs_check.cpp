@@ -147,6 +147,13 @@ int main(int argc, char** argv) {
             if (std::fabs(got - want) > 1e-4 * want) ++badRate;
         }
     }
+    double skew = 0;
+    {
+        TaskBuilder tb(ix);
+        std::vector<PhaseTasks> out;
+        tb.build(phases, blocks, true, out, 4.0e6, kWalkPays, nullptr, true);
+        for (const PhaseTasks& pt : out) skew = std::max(skew, pt.skew);
+    }
     long badSteps = 0;
     size_t steps = 0;
     for (double budget : {2.0e4, 2.0e5, 4.0e6})
@@ -190,8 +197,8 @@ int main(int argc, char** argv) {
             badServed += worst > std::max(1.0e6, every / (blocks * 8.0)) && out[i].chunk != 0;
         }
     }
-    std::printf("phases %zu multi-group tasks %zu split roots %zu unseen %zu; cover %ld times %ld rates %ld served %ld steps %ld (%zu) sampled %zu\n",
+    std::printf("phases %zu multi-group tasks %zu split roots %zu unseen %zu; cover %ld times %ld rates %ld served %ld steps %ld (%zu) sampled %zu skew x1000 %.0f\n",
                 phases.size(), multi, split, unseen, bad, badNs, badRate,
-                badServed, badSteps, steps, fans.sampled());
+                badServed, badSteps, steps, fans.sampled(), 1000 * skew);
     return bad + badNs + badRate + badServed + badSteps == 0 ? 0 : 1;
 }
