@@ -675,11 +675,11 @@ void Staged::set_spill(bool on, cudaStream_t s) {
     else dSpill.release();
 }
 
-SpillArgs Staged::spill_args() const {
+SpillArgs Staged::spill_args(int launch) const {
     SpillArgs a;
     if (!spillable) return a;
     char* p = static_cast<char*>(dSpill.p);
-    a.ctl = reinterpret_cast<SpillCtl*>(static_cast<char*>(dCtl.p) + kSpillCtlAt);
+    a.ctl = reinterpret_cast<SpillCtl*>(static_cast<char*>(dCtl.p) + kSpillCtlAt) + launch;
     for (int k = 0; k < 2; ++k) {
         a.tasks[k] = reinterpret_cast<SpillTask*>(p + spill_part(k));
         a.recs[k] = reinterpret_cast<int32_t*>(p + spill_part(2 + k));
@@ -693,12 +693,12 @@ SpillArgs Staged::spill_args() const {
 
 // The launches that run what the one before spilled; the last may not spill.
 void Staged::enqueue_follow_ups(Context& c, cudaStream_t s, unsigned long long* results, int* status,
-                                unsigned long long* span) {
+                                unsigned long long* span, int launch) {
     if (!spillable) return;
     EngineProfile prof;
     prof.span = span;
     for (int k = 0; k < kFollowUps; ++k) {
-        SpillArgs a = spill_args();
+        SpillArgs a = spill_args(launch);
         a.in = k;
         a.out = k + 1 < kFollowUps ? k + 1 : -1;
         ck(engine_launch(c.dix, dPlans, dTasks, 0, nullptr, results, status, c.grid, c.geom.block, s, &prof, a),
@@ -822,25 +822,26 @@ void Staged::enqueue_per_plan(Context& c, cudaStream_t s) {
     if (heavyWords) ck(cudaMemsetAsync(dHeavy.p, 0, heavyWords * 4, s), "memset heavy rows");
     if (nSort) ck(cudaMemsetAsync(dSort.p, 0, 8, s), "memset key cursor");
     int* ctl = static_cast<int*>(dCtl.p);
+    auto* results = reinterpret_cast<unsigned long long*>(static_cast<char*>(dCtl.p) + kPerPlanResults);
     for (int i = 0; i < nPlans; ++i) {
         const int32_t b = i ? planTaskEnd[i - 1] : 0, e = planTaskEnd[i];
         EngineProfile prof;
         prof.span = reinterpret_cast<unsigned long long*>(static_cast<char*>(dCtl.p) + 16 + 16 * i);
         const int grid = std::max(1, std::min(e - b, c.grid));
         if (blockWords && (size_t)grid > blockRegions) throw CudaError("launch grid exceeds the block-row regions");
-        ck(engine_launch(c.dix, dPlans, dTasks + b, e - b, ctl + i,
-                         reinterpret_cast<unsigned long long*>(static_cast<char*>(dCtl.p) + kPerPlanResults), ctl + 2,
-                         grid, c.geom.block, s, &prof, spill_args()),
+        ck(engine_launch(c.dix, dPlans, dTasks + b, e - b, ctl + i, results, ctl + 2,
+                         grid, c.geom.block, s, &prof, spill_args(i)),
            "engine launch");
+        // each plan's spilled tasks before the next plan's launch: timed with
+        // their own phase, and the lists and rows are free again (the rows of
+        // fused supports once those are counted)
+        enqueue_follow_ups(c, s, results, ctl + 2, prof.span, i);
+        const bool last = i + 1 == nPlans;
+        ck(support_rows(c.dix, dPlans, dSupJobs, last ? nSupJobs : 0, results, s,
+                        anyFused ? spill_args(i) : SpillArgs{}, c.sms),
+           "fused support of split roots and spilled tasks");
     }
-    // (timed with the last plan's phase, the body size where there is one)
-    enqueue_follow_ups(c, s, reinterpret_cast<unsigned long long*>(static_cast<char*>(dCtl.p) + kPerPlanResults), ctl + 2,
-                       reinterpret_cast<unsigned long long*>(static_cast<char*>(dCtl.p) + 16 + 16 * (nPlans - 1)));
-    ck(support_rows(c.dix, dPlans, dSupJobs, nSupJobs,
-                    reinterpret_cast<unsigned long long*>(static_cast<char*>(dCtl.p) + kPerPlanResults), s,
-                    anyFused ? spill_args() : SpillArgs{}, c.sms),
-       "fused support of split roots and spilled tasks");
-    enqueue_sort(c, s, reinterpret_cast<unsigned long long*>(static_cast<char*>(dCtl.p) + kPerPlanResults), ctl + 2);
+    enqueue_sort(c, s, results, ctl + 2);
 }
 
 int Staged::max_launch_tasks() const {

@@ -174,9 +174,9 @@ struct Staged {
     DevBuf dHubSeen;                       // hub and memo claims: kHubSeen words per resident block
     DevBuf dSpill;                         // spill lists, rows and support jobs (see spill_args)
     // Where the control words of one launch lie in dCtl (kCtlBytes, cleared
-    // before it): counters, status and per-plan words first, then spilling's.
+    // before it): counters, status and per-plan words first, then spilling's,
+    // for each plan with a launch of its own.
     static constexpr size_t kSpillCtlAt = 64, kCtlBytes = 192;
-    static_assert(kSpillCtlAt + sizeof(SpillCtl) <= kCtlBytes, "control words");
     bool anyFused = false;                 // some plan counts supports
     bool maySpill = true;                  // false: only timed launches (served ones), which never spill
     bool spillable = false;                // launches of this staging may spill
@@ -185,9 +185,9 @@ struct Staged {
     bool spillMeasured = false, spillPays = false;
     void set_spill(bool on, cudaStream_t s);
     bool spillAlways = false;
-    SpillArgs spill_args() const;
+    SpillArgs spill_args(int launch = 0) const;
     void enqueue_follow_ups(Context& c, cudaStream_t s, unsigned long long* results, int* status,
-                            unsigned long long* span);
+                            unsigned long long* span, int launch = 0);
     // host ms of the staging sections (dedup and fusion, memos, task build,
     // plan fields, task order, upload), summed until read
     double hostSect[6] = {0, 0, 0, 0, 0, 0};
@@ -245,6 +245,7 @@ struct Staged {
     // back in one copy.  The plain per-rule form: support and body size of
     // one rule.
     static constexpr int kMaxPerPlan = 2;
+    static_assert(kSpillCtlAt + kMaxPerPlan * sizeof(SpillCtl) <= kCtlBytes, "control words");
     static constexpr int kPerPlanResults = 16 + 16 * kMaxPerPlan;
     static_assert(kPerPlanResults + 8 * kMaxPerPlan <= 64, "per-plan control words fit the 64 control bytes");
     void enqueue_per_plan(Context& c, cudaStream_t s);
