@@ -930,7 +930,7 @@ void with_rule_block(Context& c, int tasks, Fn fn) {
 // issued back to back with one host synchronisation; a fused support takes
 // no launch of its own.
 int evaluate_parsed(Context& c, const Rule& rule, GpuRuleResult* out) {
-    RulePlan rp = plan_rule(rule, c.hix, c.geom, c.fans.get());
+    RulePlan rp = plan_rule(rule, c.hix, c.geom, c.fans());
     int64_t sup = rp.support.value, body = rp.body.value;
     float supMs = 0.f, confMs = 0.f;
     const bool runS = rp.status == kRuleOk && rp.support.how == kDevice;
@@ -971,12 +971,14 @@ int evaluate_parsed(Context& c, const Rule& rule, GpuRuleResult* out) {
 
 // Counts of one rule restricted to slice `shard` of `nShards` of each device
 // phase's roots (slices of about equal estimated work).  Support roots are
-// head triples and body-size roots are rows of the seed atom keyed by the
-// head subject, so the slices' counts add up to the whole rule's: distinct
-// (hS, hO) pairs of different hS never collide.  Static parts count in
-// slice 0 only.
+// head triples and body-size roots are rows of the seed atom keyed by one of
+// the head's variables, so the slices' counts add up to the whole rule's:
+// distinct (hS, hO) pairs of different roots never collide.  Which variable,
+// and where the roots are cut, follows from the rule and the graph alone:
+// each slice may be evaluated by another process.  Static parts count in slice
+// 0 only.
 void evaluate_shard(Context& c, const Rule& rule, int shard, int nShards, long long* counts) {
-    RulePlan rp = plan_rule(rule, c.hix, c.geom, c.fans.get());
+    RulePlan rp = plan_rule(rule, c.hix, c.geom, c.samples.get());   // (whatever this process's bothEnds)
     int64_t part[2] = {shard == 0 ? rp.support.value : 0, shard == 0 ? rp.body.value : 0};
     PhasePlan* phs[2] = {&rp.support, &rp.body};
     for (int k = 0; k < 2 && rp.status == kRuleOk; ++k) {
@@ -1017,7 +1019,7 @@ void prepare(Batch& b, Context& c, const char* const* rules, int n, int isJson, 
         if (!rules[i]) { b.parseStatus[i] = -1; return; }
         try {
             Rule r = isJson ? c.parser->parse_json(rules[i]) : c.parser->parse_text(rules[i]);
-            rp = plan_rule(r, c.hix, c.geom, c.fans.get());
+            rp = plan_rule(r, c.hix, c.geom, c.fans());
             if (rp.status == kRuleOk) {
                 // (a fused support is only hashed if its plan turns out to be full)
                 if (rp.support.how == kDevice && !(fuse && fuses(rp))) hash[2 * i] = phase_hash(rp.support);
@@ -1237,7 +1239,8 @@ void finish_load(Context* c) {
     c->tasks.reset(new TaskBuilder(c->hix));
     // GPU_RULES_PLAN_BOTH_ENDS=0: body sizes always from the head subject's end
     const char* ends = std::getenv("GPU_RULES_PLAN_BOTH_ENDS");
-    if (!ends || std::atoi(ends) != 0) c->fans.reset(new FanSamples(c->hix));
+    c->bothEnds = !ends || std::atoi(ends) != 0;
+    c->samples.reset(new FanSamples(c->hix));
     c->tasks->memoRows = [c](int p1, int d1, int p2, int d2, int p3, int d3,
                              double* cost) -> const std::vector<uint8_t>* {
         auto it = c->memos.find(memo_key(p1, d1, p2, d2, p3, d3));
@@ -1789,7 +1792,7 @@ extern "C" int gpu_evaluate_rule_noalloc(void* ctx, const char* ruleText, GpuRul
         ck(cudaSetDevice(c.device), "cudaSetDevice");
         char* scratch = static_cast<char*>(noalloc_scratch(c.device));
         Rule r = c.parser->parse_text(ruleText);
-        RulePlan rp = plan_rule(r, c.hix, c.geom, c.fans.get());
+        RulePlan rp = plan_rule(r, c.hix, c.geom, c.fans());
         NoallocPhase ns(c, rp.support), nb(c, rp.body);
         if (ns.need > kNoAllocScratchBytes || nb.need > kNoAllocScratchBytes) {
             // a plan made for speed may need more memory (a larger hO domain,

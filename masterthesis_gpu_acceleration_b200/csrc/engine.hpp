@@ -328,7 +328,9 @@ struct Context {
     Staged one;          // per-rule launches
     std::vector<struct Batch*> pipe;  // reusable chunks of one-shot batches
     std::unique_ptr<TaskBuilder> tasks;
-    std::unique_ptr<FanSamples> fans;   // sampled fan-outs (null: plans start at the head subject)
+    std::unique_ptr<FanSamples> samples;   // sampled fan-outs
+    bool bothEnds = true;                  // body sizes are planned from the cheaper end
+    FanSamples* fans() const { return bothEnds ? samples.get() : nullptr; }
     Geom geom;
     double ruleWalkBudget = 4.0e6;   // per-root measurement allowed per plain per-rule launch
     int batchChunks = 0;             // pipelined chunks of one-shot batches (0: automatic)

@@ -186,7 +186,7 @@ struct Server {
             q.req = std::move(got[i]);
             try {
                 const Rule rule = c->parser->parse_text(q.req.text);
-                q.rp = plan_rule(rule, c->hix, c->geom, c->fans.get());
+                q.rp = plan_rule(rule, c->hix, c->geom, c->fans());
                 q.mem = estimate_mem(q.rp);
                 if (q.mem > memBudget) {
                     // a plan made for speed may need more memory: what the
