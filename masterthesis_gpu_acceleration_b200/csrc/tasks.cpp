@@ -270,15 +270,9 @@ double TaskBuilder::child_work(const DevPlan& P, const int32_t* vals, int32_t e,
     return 1.0 + d2 * tail;
 }
 
-const TaskBuilder::Walk& TaskBuilder::walk(const PhasePlan& ph, uint64_t sig) {
-    auto it = walks_.find(sig);
-    if (it != walks_.end()) return it->second;
-    return keep_walk(sig, compute_walk(ph));
-}
-
-const TaskBuilder::Walk& TaskBuilder::keep_walk(uint64_t sig, Walk&& wk) {
+const TaskBuilder::Walk& TaskBuilder::keep_walk(std::unordered_map<uint64_t, Walk>& walks, uint64_t sig, Walk&& wk) {
     cacheBytes_ += wk.w.size() * sizeof(float) + wk.bsum.size() * (sizeof(double) + sizeof(float)) + sizeof(Walk);
-    return walks_.emplace(sig, std::move(wk)).first->second;
+    return walks.emplace(sig, std::move(wk)).first->second;
 }
 
 const std::vector<uint8_t>* TaskBuilder::walk_memo(const DevPlan& P, double* cost) const {
@@ -307,7 +301,7 @@ double TaskBuilder::walk_cost(const PhasePlan& ph) const {
     return edges + (double)(s0.kind == kRowScan ? ix_.pred_rows(s0.pred, s0.dir) : ix_.pred_size(s0.pred));
 }
 
-TaskBuilder::Walk TaskBuilder::compute_walk(const PhasePlan& ph) {
+TaskBuilder::Walk TaskBuilder::compute_walk(const PhasePlan& ph, bool memos) {
     const DevPlan& P = ph.plan;
     const double tail = chain_tail(P);
     const bool chain = chain_shaped(P);
@@ -316,7 +310,7 @@ TaskBuilder::Walk TaskBuilder::compute_walk(const PhasePlan& ph) {
     // plans whose last two (three) steps are memoised: an item of level 1
     // costs the memo's price when its row has a memo, else its enumeration
     double memoCost = 0.0;
-    const std::vector<uint8_t>* memo = walk_memo(P, &memoCost);
+    const std::vector<uint8_t>* memo = memos ? walk_memo(P, &memoCost) : nullptr;
     const DevStep& s1 = P.steps[1];
     const bool uniformChild = uniform_child(P);
     double scanned = -1.0;   // a scan's rows, the same for every root
@@ -380,6 +374,7 @@ void TaskBuilder::build(const std::vector<const PhasePlan*>& phases, int blocks,
     out.assign(n, PhaseTasks{});
     if (cacheBytes_ > kCacheLimit) {  // only here: walks hand out references into the cache
         walks_.clear();
+        plainWalks_.clear();
         deg_.clear();
         for (auto& a : degAt_) a.store(nullptr, std::memory_order_relaxed);
         for (int k = 0; k < kHop2Shards; ++k) {
@@ -449,9 +444,9 @@ void TaskBuilder::build(const std::vector<const PhasePlan*>& phases, int blocks,
         }
         std::vector<Walk> made(fresh.size());
         // threads only pay for themselves on large walks (~0.1 ms and up)
-        parallel_for(fresh.size(), [&](size_t k) { made[k] = compute_walk(*phases[fresh[k]]); },
+        parallel_for(fresh.size(), [&](size_t k) { made[k] = compute_walk(*phases[fresh[k]], true); },
                      used > 1.0e5 ? 1 : fresh.size() + 1);
-        for (size_t k = 0; k < fresh.size(); ++k) keep_walk(sig[fresh[k]], std::move(made[k]));
+        for (size_t k = 0; k < fresh.size(); ++k) keep_walk(walks_, sig[fresh[k]], std::move(made[k]));
         for (size_t i : sel) {
             const Walk& wk = walks_.find(sig[i])->second;
             walked[i] = &wk;
@@ -587,7 +582,10 @@ std::vector<int32_t> TaskBuilder::split_roots(const PhasePlan& ph, int n) {
     cut[0] = ph.rootBeg;
     const int32_t R = ph.rootEnd - ph.rootBeg;
     if (R <= 0) return cut;
-    const std::vector<float>& w = walk(ph).w;
+    const uint64_t sig = signature(ph);
+    auto it = plainWalks_.find(sig);
+    const std::vector<float>& w =
+        it != plainWalks_.end() ? it->second.w : keep_walk(plainWalks_, sig, compute_walk(ph, false)).w;
     double total = 0;
     for (float x : w) total += x;
     double acc = 0;

@@ -130,7 +130,9 @@ public:
 
     // Boundaries of n contiguous slices of a device phase's roots with about
     // equal estimated work (per-root walk): slice k is [cut[k], cut[k+1]),
-    // cut[0] = rootBeg, cut[n] = rootEnd.
+    // cut[0] = rootBeg, cut[n] = rootEnd.  They follow from the phase and the
+    // graph alone (not from memos or times that this builder happens to know):
+    // every process that evaluates a slice has to cut alike.
     std::vector<int32_t> split_roots(const PhasePlan& ph, int n);
 
     // Suffix memos known to the context: per-row flags of (p1, d1) for the
@@ -163,6 +165,7 @@ private:
         double sum = 0.0;
     };
     std::unordered_map<uint64_t, Walk> walks_;                   // phase hash -> per-root work
+    std::unordered_map<uint64_t, Walk> plainWalks_;              // the same without memos (split_roots)
     struct Hop2 {
         std::vector<float> perRow;   // per row of (p0, d0): sum over its edges of the next degree
         double total = 0.0;
@@ -210,7 +213,6 @@ private:
     // chain-shaped plans whose roots are the first step's rows; otherwise
     // the average-fan-out estimate.
     double estimate2(const PhasePlan& ph);
-    const Walk& walk(const PhasePlan& ph, uint64_t sig);
     // Roots and edges a walk of the phase visits (at most): a step per root,
     // and the edges it has to look at one by one.
     double walk_cost(const PhasePlan& ph) const;
@@ -218,9 +220,9 @@ private:
     const std::vector<uint8_t>* walk_memo(const DevPlan& P, double* cost) const;
     // The per-root walk of a phase (thread-safe: reads the index and the
     // lock-guarded estimate caches), and its insertion into the cache.
-    Walk compute_walk(const PhasePlan& ph);
-    const Walk& keep_walk(uint64_t sig, Walk&& wk);
-    const Walk& walk(const PhasePlan& ph) { return walk(ph, phase_hash(ph)); }
+    // memos: weigh items by the memos known now.
+    Walk compute_walk(const PhasePlan& ph, bool memos);
+    const Walk& keep_walk(std::unordered_map<uint64_t, Walk>& walks, uint64_t sig, Walk&& wk);
     double child_work(const DevPlan& P, const int32_t* rootVals, int32_t e, const int32_t* deg2, double tail) const;
 
 public:

@@ -8,6 +8,8 @@
 //   * Phases never run are expected at the rate of those that were: with
 //     every task at the same rate, expected_ns() is that rate times the work
 //     build() gives the phase.
+//   * Where a phase's roots are cut into slices does not depend on the memos
+//     or times that the builder knows.
 //   * New walks visit no more roots and edges than the budget allows.
 //   * A served launch walks only phases expected to hold the whole GPU for
 //     longer than the walk takes, and those whose tasks turned out long.
@@ -154,6 +156,18 @@ int main(int argc, char** argv) {
         tb.build(phases, blocks, true, out, 4.0e6, kWalkPays, nullptr, true);
         for (const PhaseTasks& pt : out) skew = std::max(skew, pt.skew);
     }
+    long badCuts = 0;
+    {
+        TaskBuilder plain(ix), used(ix);
+        std::vector<uint8_t> flags((size_t)ix.nEnt, 1);
+        used.memoRows = [&](int, int, int, int, int, int, double* cost) { *cost = 256.0; return &flags; };
+        used.walkThreshold = 0.0;
+        std::vector<PhaseTasks> out;
+        used.build(phases, blocks, true, out, 4.0e6, kWalkBudget, nullptr, true);
+        const Launch run(out, 0.0);
+        used.learn(phases, run.tasks, run.cost, run.ns.data(), blocks);
+        for (const PhasePlan* ph : phases) badCuts += plain.split_roots(*ph, 3) != used.split_roots(*ph, 3);
+    }
     long badSteps = 0;
     size_t steps = 0;
     for (double budget : {2.0e4, 2.0e5, 4.0e6})
@@ -197,8 +211,8 @@ int main(int argc, char** argv) {
             badServed += worst > std::max(1.0e6, every / (blocks * 8.0)) && out[i].chunk != 0;
         }
     }
-    std::printf("phases %zu multi-group tasks %zu split roots %zu unseen %zu; cover %ld times %ld rates %ld served %ld steps %ld (%zu) sampled %zu skew x1000 %.0f\n",
+    std::printf("phases %zu multi-group tasks %zu split roots %zu unseen %zu; cover %ld times %ld rates %ld served %ld cuts %ld steps %ld (%zu) sampled %zu skew x1000 %.0f\n",
                 phases.size(), multi, split, unseen, bad, badNs, badRate,
-                badServed, badSteps, steps, fans.sampled(), 1000 * skew);
-    return bad + badNs + badRate + badServed + badSteps == 0 ? 0 : 1;
+                badServed, badCuts, badSteps, steps, fans.sampled(), 1000 * skew);
+    return bad + badNs + badRate + badServed + badCuts + badSteps == 0 ? 0 : 1;
 }

@@ -18,6 +18,7 @@ def test_slices_of_different_contexts(hub_chains, monkeypatch):   # noqa: F811
         monkeypatch.setenv("GPU_RULES_PLAN_BOTH_ENDS", ends)
         libs.append(eng.GpuRulesLib(ttl))
     try:
+        libs[1].evaluate_rules_batch(rules)   # its memos exist before it cuts anything
         for n in (2, 3):
             for i, r in enumerate(rules):
                 parts = [libs[k % 2].evaluate_rule_shard(r, k, n) for k in range(n)]
