@@ -488,9 +488,7 @@ void Staged::stage(Context& c, const std::vector<const PhasePlan*>& phases, cons
     dBlob.ensure(blob, as);
     nResults = nPlans + extraResults;
     dResults.ensure((size_t)nResults * sizeof(unsigned long long), as);
-    // 31 MB, stream-ordered also for staging that is not: cudaMalloc waits for
-    // every stream, and a call of several chunks takes one buffer each
-    if (spillable) dSpill.ensure(spill_bytes(), s, true);
+    if (spillable) set_spill(true, s);
     hResults.ensure((size_t)nResults * sizeof(unsigned long long));
     ck(cudaMemcpyAsync(dBlob.p, hBlob.p, blob, cudaMemcpyHostToDevice, s), "H2D plans");
     dPlans = static_cast<const DevPlan*>(dBlob.p);
@@ -615,10 +613,14 @@ void Context::ensure_memos(const std::vector<std::array<int, 6>>& keys, cudaStre
     const size_t jobBytes = nJobs * sizeof(MemoJob);
     if (memoChunks.empty() || memoUsed + need + jobBytes > memoChunks.back()->cap) {
         auto chunk = std::make_unique<DevBuf>();
-        const size_t cap = std::max(need + jobBytes, kMemoArenaBytes);
-        ck(cudaMallocAsync(&chunk->p, cap, s), "cudaMallocAsync(memos)");   // never resized
+        size_t cap = std::max(need + jobBytes, kMemoArenaBytes);
+        chunk->pooled = cudaMallocAsync(&chunk->p, cap, s) == cudaSuccess;   // never resized
+        if (!chunk->pooled) {   // no room for an arena: what these memos need, as long as that fits
+            cudaGetLastError();
+            cap = need + jobBytes;
+            ck(cudaMalloc(&chunk->p, cap), "cudaMalloc(memos)");
+        }
         chunk->cap = cap;
-        chunk->pooled = true;
         memoChunks.push_back(std::move(chunk));
         memoUsed = 0;
     }
@@ -627,6 +629,7 @@ void Context::ensure_memos(const std::vector<std::array<int, 6>>& keys, cudaStre
     MemoJob* const dJobs = reinterpret_cast<MemoJob*>(base + need);
     std::vector<int32_t> tabs(tabTotal / 4, -1);
     std::vector<MemoJob> all;
+    std::vector<std::pair<uint64_t, std::unique_ptr<SuffixMemo>>> built;   // known once the device has them
     for (size_t t = 0; t < take.size(); ++t) {
         const size_t i = take[t];
         const int p1 = fresh[i][0], d1 = fresh[i][1], p2 = fresh[i][2], d2 = fresh[i][3];
@@ -657,7 +660,7 @@ void Context::ensure_memos(const std::vector<std::array<int, 6>>& keys, cudaStre
         m->words = words;
         m->wo = p3 >= 0 ? wo : 0;
         m->slots = (int)rows.size();
-        memos[memo_key(p1, d1, p2, d2, p3, d3)] = std::move(m);
+        built.emplace_back(memo_key(p1, d1, p2, d2, p3, d3), std::move(m));
     }
     ck(cudaMemcpyAsync(base, tabs.data(), tabTotal, cudaMemcpyHostToDevice, s), "H2D memo tables");
     ck(cudaMemsetAsync(base + tabTotal, 0, bitTotal, s), "clear memo bits");
@@ -667,12 +670,24 @@ void Context::ensure_memos(const std::vector<std::array<int, 6>>& keys, cudaStre
         if (j.p3 >= 0) maxWo = std::max(maxWo, j.wo);
     ck(memo_build(dix, dJobs, (int)all.size(), maxWo, s), "memo build");
     ck(cudaStreamSynchronize(s), "memo build");   // memos are shared by every stream afterwards
+    for (auto& m : built) memos[m.first] = std::move(m.second);
 }
 
+// Its buffer is stream-ordered also for staging that is not: cudaMalloc waits
+// for every stream, and a call of several chunks takes one buffer (31 MB) each.
+// Without room for it launches do not spill.
 void Staged::set_spill(bool on, cudaStream_t s) {
     spillable = on;
-    if (on) dSpill.ensure(spill_bytes(), s, true);
-    else dSpill.release();
+    if (!on) {
+        dSpill.release();
+        return;
+    }
+    try {
+        dSpill.ensure(spill_bytes(), s, true);
+    } catch (const CudaError&) {
+        cudaGetLastError();
+        spillable = false;
+    }
 }
 
 SpillArgs Staged::spill_args(int launch) const {
@@ -1191,8 +1206,10 @@ void tune_spill(Batch& b) {
     Context& c = *b.c;
     if (c.spill != 1 || !b.st.nPlans || b.st.nSort) return;
     float best[2] = {0.f, 0.f};
+    b.st.spillPays = false;
     for (int on = 0; on < 2; ++on) {
         b.st.set_spill(on != 0, b.stream);
+        if (b.st.spillable != (on != 0)) return;   // no room for the buffer
         for (int run = 0; run < 3; ++run) {
             ck(cudaEventRecord(b.ev0, b.stream), "event");
             b.st.enqueue(c, b.stream, 0);
