@@ -130,7 +130,7 @@ void Staged::stage(Context& c, const std::vector<const PhasePlan*>& phases, cons
     nTasks = 0;
     bitmapWords = 0;
     blockWords = blockRegions = 0;
-    nSort = sortBits = sortSlotShift = 0;
+    nSort = sortSlotShift = 0;
     keyCap = 0;
     h2dBytes = d2hBytes = 0;
     dedup.assign(nPlans, kDedupShared);
@@ -143,9 +143,12 @@ void Staged::stage(Context& c, const std::vector<const PhasePlan*>& phases, cons
     // ---- how each kPairs plan deduplicates ----
     // Per-phase global rows (one bitmap row per root, cleared before the
     // launch) while all of them fit the budget.  Beyond it, per plan: sort
-    // mode when the estimated keys (sorted in ~7 passes of 8 bits) cost fewer
-    // bytes than clearing and setting the rows, else block rows, whose
-    // memory grows with the launch's blocks instead of the phase's roots.
+    // mode when the estimated keys cost fewer bytes than clearing and setting
+    // the rows, else block rows, whose memory grows with the launch's blocks
+    // instead of the phase's roots.  (A key is priced at 22 times its size, as
+    // a full sort in seven passes moves it.  Parting the keys by a hash moves
+    // them one to three times, so close to the line keys would be the cheaper
+    // choice; where the line should lie now has not been measured.)
     const size_t budgetWords = std::max<size_t>(c.dedupBudget / 4, 1);
     std::vector<size_t> fullWords(nPlans, 0);
     std::vector<double> est(nPlans, -1.0);
@@ -201,7 +204,6 @@ void Staged::stage(Context& c, const std::vector<const PhasePlan*>& phases, cons
         } else {
             nSort = (int)sortPlans.size();
             sortSlotShift = rankBits + rowBits;
-            sortBits = sortSlotShift + slotBits;
         }
     }
     if (nSort) {
@@ -728,7 +730,7 @@ void Staged::enqueue_sort(Context& c, cudaStream_t s, unsigned long long* result
     auto* keys = reinterpret_cast<unsigned long long*>(base + 256);
     auto* tmp = keys + keyCap;
     auto* hist = reinterpret_cast<uint32_t*>(tmp + keyCap);
-    ck(pairs_sort_count(keys, tmp, cursor, keyCap, sortBits, sortSlotShift, dSortSlots, nSort, results, status,
+    ck(pairs_sort_count(keys, tmp, cursor, keyCap, sortSlotShift, dSortSlots, nSort, results, status,
                         hist, std::max(c.sms, 1) * 8, c.sortSet, s),
        "pair sort");
 }

@@ -54,7 +54,7 @@ unsigned long long* radix_sort_keys(unsigned long long* keys, unsigned long long
                                     unsigned long long cap, int bits, uint32_t* hist, int grid, cudaStream_t stream,
                                     cudaError_t* err);
 cudaError_t pairs_sort_count(unsigned long long* keys, unsigned long long* tmp, const unsigned long long* count,
-                             unsigned long long cap, int bits, int slotShift, const int32_t* slotOf, int nSlots,
+                             unsigned long long cap, int slotShift, const int32_t* slotOf, int nSlots,
                              unsigned long long* results, int* status, uint32_t* hist, int grid, int setKeys,
                              cudaStream_t stream);
 
@@ -161,7 +161,7 @@ struct Staged {
     // estimate favours.
     std::vector<int32_t> dedup;
     size_t blockWords = 0, blockRegions = 0;
-    int nSort = 0, sortBits = 0, sortSlotShift = 0;
+    int nSort = 0, sortSlotShift = 0;
     unsigned long long keyCap = 0;
     unsigned long long keyHint = 0;     // exact keys of a run that overflowed keyCap
     const int32_t* dSortSlots = nullptr;   // result slot of each sort index (in dBlob)

@@ -366,11 +366,11 @@ int pairs_sort_passes(unsigned long long cap) {
 // pairs_sort_hist_words(cap) words.  grid: blocks of the per-tile kernels
 // (they loop over tiles).  setKeys: most keys a hash set takes in one round.
 cudaError_t pairs_sort_count(unsigned long long* keys, unsigned long long* tmp, const unsigned long long* count,
-                             unsigned long long cap, int bits, int slotShift, const int32_t* slotOf, int nSlots,
+                             unsigned long long cap, int slotShift, const int32_t* slotOf, int nSlots,
                              unsigned long long* results, int* status, uint32_t* hist, int grid, int setKeys,
                              cudaStream_t stream) {
     if (cap == 0) return cudaSuccess;
-    if (bits < 1 || bits > 64 || slotShift < 0 || slotShift > 63 || cap > 0xffffffffull) return cudaErrorInvalidValue;
+    if (slotShift < 0 || slotShift > 63 || cap > 0xffffffffull) return cudaErrorInvalidValue;
     cudaError_t e = cudaSuccess;
     const int passes = pairs_sort_passes(cap);
     unsigned long long* a = radix_passes<true>(keys, tmp, count, cap, 8 * passes, hist, grid, stream, &e);
