@@ -788,10 +788,11 @@ __device__ __forceinline__ int item_state(const DevStep& next, int hub) {
 }
 
 // Clock cycles (about 32 us) between a block's looks at the task queue during
-// a group of roots: groups shorter than that are not worth the records (200
-// long rules 0.78 ms; 0.91 ms with 8 us).  A sixteenth of the launch idle is
-// enough (5,000 miner candidates 3.99 ms; a quarter on two looks 4.60 ms, an
-// eighth on two 4.59 ms).
+// a group of roots: shorter groups are not worth the records (first look after
+// 100, 200 and 500 us: 10,000 rules 5.54 -> 5.66, 5.83 and 6.39 ms, of the
+// biomedical sets one 1.25 -> 1.01-1.34 ms, others 1.59 -> 1.54-2.19 ms).  A
+// sixteenth of the launch idle is enough (5,000 miner candidates 3.99 ms; a
+// quarter on two looks 4.60 ms, an eighth on two 4.59 ms).
 constexpr long long kSpillEvery = 64000;
 // Records of a spill task, and candidates of a record, at inner levels and at
 // the leaf: about a round's work each.
@@ -1703,8 +1704,14 @@ size_t engine_smem_bytes(int block) {
     }
 }
 
+__global__ void memo_build_kernel(DevIndex ix, const MemoJob* jobs, int nJobs);
+
 cudaError_t engine_configure() {
     cudaError_t e = configure_b<128>();
+    // (its limit, once: a launch that set what it needs itself could be
+    // overtaken by another thread's smaller one)
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(memo_build_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMemoSmemRanks * 4);
     if (e == cudaSuccess) e = configure_b<256>();
     if (e == cudaSuccess) e = configure_b<512>();
     return e;
@@ -1935,11 +1942,6 @@ cudaError_t build_lookup(const DevIndex& ix, const HashSlot* hash16, long long n
 cudaError_t memo_build(const DevIndex& ix, const MemoJob* jobs, int nJobs, int maxWo, cudaStream_t stream) {
     if (nJobs <= 0) return cudaSuccess;
     const size_t smem = (size_t)std::min(maxWo, kMemoSmemRanks) * 4;
-    if (smem > 48 * 1024) {
-        const cudaError_t e =
-            cudaFuncSetAttribute(memo_build_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-    }
     memo_build_kernel<<<nJobs, 256, smem, stream>>>(ix, jobs, nJobs);
     return cudaGetLastError();
 }
