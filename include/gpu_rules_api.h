@@ -98,9 +98,10 @@ int gpu_batch_counts(void* batch, long long* counts, int* status);
 
 /* One rule split over nShards workers (one per GPU): evaluates only slice
  * `shard` of each device phase's roots — head triples for support, rows of
- * the seed atom keyed by the head subject for body size — cut so that the
- * slices carry about equal estimated work.  Body pairs of different head
- * subjects are distinct, so summing counts[0] (support) and counts[3]
+ * a body atom keyed by one of the head's variables for body size — cut so that
+ * the slices carry about equal estimated work.  Variable and cuts follow from
+ * the rule and the graph alone, so that every worker agrees on them.  Body pairs
+ * of different roots are distinct, so summing counts[0] (support) and counts[3]
  * (bodySize) over all shards gives the whole rule's counts (one int64 sum
  * all-reduce across GPUs); counts[1..2] (headSize, headSupport) are the
  * whole rule's in every shard.  No counterpart in the reference.  Returns
@@ -135,7 +136,9 @@ int gpu_batch_profile(void* batch, unsigned long long* bytes, unsigned long long
  * times; after each run the context's task builder learns, per plan
  * signature, the device time per unit of estimated work, marks the phases
  * whose slowest task held up the launch for an exact per-root measurement,
- * and the batch's tasks are rebuilt and re-uploaded.  What is learnt stays
+ * and the batch's tasks are rebuilt and re-uploaded.  At the end the batch is
+ * timed with and without giving long tasks' open work to follow-up launches,
+ * and keeps the faster way (not tuned: without).  What is learnt stays
  * with the context and also balances later batches and per-rule calls with
  * the same plans.  Returns 0, or -1 on a CUDA error. */
 int gpu_batch_autotune(void* batch, int rounds);
@@ -161,8 +164,8 @@ int gpu_batch_dedup(void* batch, int* modes, long long* sortKeys);
  * synchronise the whole device.  The per-call device buffers (plan, tasks,
  * counters, status and, for very large hO domains, the pair bitmap) come from
  * one 8 MiB array built into the library (held on every GPU that loads it
- * until the process exits); a rule that needs more returns -1 with the size
- * in gpu_last_error().  The first call on a device looks up the array's
+ * until the process exits); a rule that needs more, also planned plainly,
+ * returns -1 with the size in gpu_last_error().  The first call on a device looks up the array's
  * device address (make it before any stream capture).  Calls share the array:
  * calls that overlap on the same GPU race and must be serialised. */
 int gpu_evaluate_rule_noalloc(void* ctx, const char* ruleText, GpuRuleResult* out);

@@ -10,11 +10,11 @@ every rank loads the same graph and evaluates its own rules.  Two layouts:
   in the original order on the host (``gather_results``).
 
 * one giant rule: every rank evaluates its slice of the rule's roots
-  (``gpu_evaluate_rule_shard``: head triples for support, head-subject rows
-  for body size, cut for equal estimated work) and one int64 sum all-reduce
-  adds the partial support and body-size counts (``evaluate_rule_split``).
-  Distinct (hS, hO) pairs of different head subjects never collide, so the
-  sum is exact.
+  (``gpu_evaluate_rule_shard``: head triples for support, rows of one of the
+  head's variables for body size, cut for equal estimated work) and one int64
+  sum all-reduce adds the partial support and body-size counts
+  (``evaluate_rule_split``).  Distinct (hS, hO) pairs of different roots never
+  collide, and every rank plans and cuts alike, so the sum is exact.
 
 Apart from that all-reduce the cross-rank communication is host-side
 plumbing through torch.distributed: a barrier, the maximum of the ranks'
